@@ -1744,6 +1744,9 @@ static gs_status fused_setup(gs_group g, StepDev& d, const Grid& grid, unsigned 
             g->auto_cap_valid = true;
         }
         d.enum_cap = g->auto_cap;
+        // a capacity fixed by the caller asks for that scan; otherwise small
+        // groups step with a group of lanes per agent
+        d.lanes = lanes_preferred(g->n, (d.need & NEED_WALLS) != 0) ? 1u : 0u;
     }
 
     fill_launch(g, d, w, L);

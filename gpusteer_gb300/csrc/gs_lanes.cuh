@@ -1,0 +1,226 @@
+// An agent's neighbour search and neighbour pass spread over a group of G
+// lanes (8, 16 or 32; k <= G): lane r of the group ends up with the agent's
+// r-th neighbour.
+//
+// With one thread per agent a small group leaves most SMs empty and its step
+// takes as long as one thread's serial chain: the box's candidates one after
+// another into a k-list, then k dependent neighbour gathers.  A lane group
+// takes G candidates at a time and gathers all k neighbours at once, so the
+// chain is a few rounds long and a few thousand agents fill the chip.  It
+// costs more issue slots per agent (the list lives across lanes and every
+// merge is shuffles), so large groups keep one thread per agent.
+//
+// Every key is exact, (distance bits, agent index), so no candidate order is
+// left open and nothing is redone.  All lanes of a warp run the same number
+// of rounds (the busiest group's), so every shuffle is warp-converged.
+#pragma once
+
+#include "gs_behaviours.cuh"
+#include "gs_knn.cuh"
+
+namespace gs {
+
+constexpr unsigned kAllLanes = 0xffffffffu;
+
+template <int G>
+struct LaneEntry {
+    unsigned long long key;  // (distance bits, agent index), KEY_EMPTY for none
+    unsigned slot;           // the neighbour's slot, UINT_MAX for none
+
+    // Keeps the smaller (keep_min) or larger of this entry and the one
+    // `stride` lanes away.  Keys are unique but for KEY_EMPTY, whose slot is
+    // the same everywhere.
+    __device__ __forceinline__ void exchange(int stride, bool keep_min) {
+        const unsigned long long ok = __shfl_xor_sync(kAllLanes, key, stride);
+        const unsigned os = __shfl_xor_sync(kAllLanes, slot, stride);
+        if ((ok < key) == keep_min) {
+            key = ok;
+            slot = os;
+        }
+    }
+    // Ascending bitonic sort over the group's lanes.
+    __device__ __forceinline__ void sort(unsigned lane) {
+#pragma unroll
+        for (int size = 2; size <= G; size <<= 1) {
+#pragma unroll
+            for (int stride = size >> 1; stride > 0; stride >>= 1)
+                exchange(stride, ((lane & unsigned(stride)) == 0) == ((lane & unsigned(size)) == 0));
+        }
+    }
+    // Merges the group's sorted chunk c into this sorted list, keeping the G
+    // smallest: laid reversed against the list, the elementwise minima are
+    // bitonic and hold them; log2(G) half-cleaners sort them again.
+    __device__ __forceinline__ void merge(const LaneEntry& c, unsigned lane) {
+        const unsigned long long rk = __shfl_xor_sync(kAllLanes, c.key, G - 1);
+        const unsigned rs = __shfl_xor_sync(kAllLanes, c.slot, G - 1);
+        if (rk < key) {
+            key = rk;
+            slot = rs;
+        }
+#pragma unroll
+        for (int stride = G >> 1; stride > 0; stride >>= 1)
+            exchange(stride, (lane & unsigned(stride)) == 0);
+    }
+};
+
+// Takes one candidate per lane (c; KEY_EMPTY for none) into the list.
+// `first`: the list is still empty.  Warp-converged; a chunk with nothing
+// below any group's k-th key is dropped after one vote.
+template <int G>
+__device__ __forceinline__ void lanes_take(LaneEntry<G>& list, LaneEntry<G> c, bool first,
+                                           unsigned k, unsigned lane) {
+    if (first) {
+        c.sort(lane);
+        list = c;
+        return;
+    }
+    const unsigned long long kth = __shfl_sync(kAllLanes, list.key, int(k) - 1, G);
+    if (!__any_sync(kAllLanes, c.key < kth)) return;
+    c.sort(lane);
+    list.merge(c, lane);
+}
+
+template <int G>
+__device__ __forceinline__ LaneEntry<G> lanes_candidate(V3 p, unsigned self_id, float4 q,
+                                                        unsigned slot, bool ok) {
+    LaneEntry<G> c{KEY_EMPTY, UINT_MAX};
+    const unsigned id = __float_as_uint(q.w);
+    const unsigned long long kk = knn_key(distance(p, v3(q)), id);
+    if (ok && id != self_id && kk < KEY_EMPTY) {
+        c.key = kk;
+        c.slot = slot;
+    }
+    return c;
+}
+
+// The k nearest of the box around cell (ix, iy, iz), in (distance, index)
+// order over the group's lanes: lane r holds rank r (ranks past the last
+// neighbour hold the empty entry; lanes r >= k hold leftovers).
+// R: rows of cells in the box at search radius 1 (9, or 3 on a grid one cell
+// high in y); 0 for any radius.  Rows 1..R are laid end to end, so a group
+// takes ceil(candidates / G) chunks whatever the rows' lengths.
+template <int G, int R>
+__device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 p,
+                                                  unsigned self_id, const Grid& g, const Box& b,
+                                                  unsigned cell_offset,
+                                                  const unsigned* __restrict__ start,
+                                                  const float4* __restrict__ pos_id) {
+    LaneEntry<G> list{KEY_EMPTY, UINT_MAX};
+    const unsigned span = b.x1 - b.x0 + 1;
+    if constexpr (R > 0) {
+        constexpr int Q = (R + G - 1) / G;
+        unsigned s0[Q], len[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const unsigned i = lane + unsigned(q * G);
+            const unsigned cy = b.y0 + (R == 3 ? 0u : i / 3u), cz = b.z0 + (R == 3 ? i : i % 3u);
+            s0[q] = len[q] = 0;
+            if (i < unsigned(R) && cy <= b.y1 && cz <= b.z1) {
+                const unsigned c0 = cell_offset + cell_label(g, b.x0, cy, cz);
+                s0[q] = __ldg(start + c0);
+                len[q] = __ldg(start + c0 + span) - s0[q];
+            }
+        }
+        unsigned rs[R], pre[R + 1];
+        pre[0] = 0;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            rs[i] = __shfl_sync(kAllLanes, s0[i / G], i % G, G);
+            pre[i + 1] = pre[i] + __shfl_sync(kAllLanes, len[i / G], i % G, G);
+        }
+        const unsigned total = pre[R], rounds = __reduce_max_sync(kAllLanes, total);
+        auto at = [&](unsigned j) {
+            unsigned s = rs[0] + j;
+#pragma unroll
+            for (int i = 1; i < R; ++i)
+                if (j >= pre[i]) s = rs[i] + (j - pre[i]);
+            return s;
+        };
+        // the next chunk's position is on its way while this one is sorted in
+        unsigned sl = at(lane);
+        float4 q = lane < total ? __ldg(pos_id + sl) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (unsigned j0 = 0; j0 < rounds; j0 += G) {
+            const unsigned j = j0 + lane, jn = j + G;
+            const unsigned sn = at(jn);
+            const float4 qn = jn < total ? __ldg(pos_id + sn) : make_float4(0.f, 0.f, 0.f, 0.f);
+            lanes_take(list, lanes_candidate<G>(p, self_id, q, sl, j < total), j0 == 0, k, lane);
+            sl = sn;
+            q = qn;
+        }
+    } else {
+        bool first = true;
+        // (an empty box has y1 < y0)
+        const unsigned ny = __reduce_max_sync(kAllLanes, b.y1 >= b.y0 ? b.y1 - b.y0 : 0u),
+                       nz = __reduce_max_sync(kAllLanes, b.z1 >= b.z0 ? b.z1 - b.z0 : 0u);
+        for (unsigned y = 0; y <= ny; ++y)
+            for (unsigned z = 0; z <= nz; ++z) {
+                unsigned s0 = 0, len = 0;
+                if (b.y0 + y <= b.y1 && b.z0 + z <= b.z1) {
+                    const unsigned c0 = cell_offset + cell_label(g, b.x0, b.y0 + y, b.z0 + z);
+                    s0 = __ldg(start + c0);
+                    len = __ldg(start + c0 + span) - s0;
+                }
+                const unsigned rounds = __reduce_max_sync(kAllLanes, len);
+                for (unsigned j = lane; j < rounds + lane; j += G) {
+                    const float4 q = j < len ? __ldg(pos_id + s0 + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    lanes_take(list, lanes_candidate<G>(p, self_id, q, s0 + j, j < len), first, k,
+                               lane);
+                    first = false;
+                }
+            }
+    }
+    return list;
+}
+
+// This group's bits of a warp vote, lane 0 of the group in bit 0.
+template <int G>
+__device__ __forceinline__ unsigned lanes_ballot(bool pred) {
+    const unsigned all = __ballot_sync(kAllLanes, pred);
+    if (G == 32) return all;
+    return (all >> (threadIdx.x & 31u & ~unsigned(G - 1))) & ((1u << (G & 31)) - 1u);
+}
+template <int G>
+__device__ __forceinline__ V3 lanes_get(V3 v, unsigned from) {
+    return v3(__shfl_sync(kAllLanes, v.x, int(from), G), __shfl_sync(kAllLanes, v.y, int(from), G),
+              __shfl_sync(kAllLanes, v.z, int(from), G));
+}
+
+// One value per lane of a group summed in lane order, for up to 9 value
+// columns at once: each column is a row of shared memory and one lane adds
+// up one row from 0, as the reference's loop over the list does (a lane that
+// is not in the sum holds +0, which changes no partial sum: those start at
+// +0 and never become -0).  Rows are padded to G + 4 words, so eight lanes'
+// 16-byte reads of eight rows meet no bank twice.
+template <int G>
+struct LaneSums {
+    static constexpr unsigned kRow = G + 4;
+    static constexpr unsigned kWords = 9 * kRow + 12;
+    float* w;  // this group's kWords words, 16-byte aligned
+    __device__ __forceinline__ void put(unsigned first, unsigned lane, V3 v) {
+        w[first * kRow + lane] = v.x;
+        w[(first + 1) * kRow + lane] = v.y;
+        w[(first + 2) * kRow + lane] = v.z;
+    }
+    __device__ __forceinline__ void add_rows(unsigned lane) {
+        __syncwarp();
+        for (unsigned c = lane; c < 9; c += G) {
+            const float4* row = reinterpret_cast<const float4*>(w + c * kRow);
+            float s = 0.f;
+#pragma unroll
+            for (int i = 0; i < G / 4; ++i) {
+                const float4 v = row[i];
+                s = s + v.x;
+                s = s + v.y;
+                s = s + v.z;
+                s = s + v.w;
+            }
+            w[9 * kRow + c] = s;
+        }
+        __syncwarp();
+    }
+    __device__ __forceinline__ V3 sum(unsigned first) const {
+        return v3(w[9 * kRow + first], w[9 * kRow + first + 1], w[9 * kRow + first + 2]);
+    }
+};
+
+}  // namespace gs

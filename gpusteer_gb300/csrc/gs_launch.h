@@ -174,6 +174,7 @@ struct StepDev {
     unsigned persistent;  // run a supported step as one persistent launch
     unsigned bar_limit;   // its barrier poll limit
     unsigned fresh;       // A is in agent order (first step after an upload)
+    unsigned lanes;       // step with a group of lanes per agent (lanes_preferred)
     PathDev path;       // path following (GS_B_FOLLOW_PATH)
     float path_time, w_path;
     unsigned mask_path;
@@ -259,6 +260,11 @@ gs_status fused_step_persistent(const FusedLaunch& L, const StepDev& p, const Pe
                                 cudaStream_t st);
 gs_status fused_step(const FusedLaunch& L, const StepDev& p, cudaStream_t st,
                      PhaseHook* hook = nullptr);
+// The same step with a group of lanes per agent (gs_lanes.cu); fused_step takes
+// it when p.lanes is set.  lanes_preferred: the sizes where it is the faster.
+gs_status fused_step_lanes(const FusedLaunch& L, const StepDev& p, cudaStream_t st,
+                           PhaseHook* hook);
+bool lanes_preferred(unsigned n, bool walls);
 // slot_of: capacity words of scratch (each agent's slot, then the gather).
 gs_status fused_to_reference(Fused A, unsigned n, const Scene* scenes, unsigned* slot_of,
                              GroupView g, cudaStream_t st);

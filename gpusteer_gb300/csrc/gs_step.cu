@@ -31,31 +31,9 @@
 #include <mutex>
 
 #include "gs_launch.h"
+#include "gs_step.cuh"
 
 namespace gs {
-
-__device__ __forceinline__ unsigned u(float x) { return __float_as_uint(x); }
-__device__ __forceinline__ float fb(unsigned x) { return __uint_as_float(x); }
-
-// Adds 1 to the scan tile total of `cell`, once per group of active lanes in
-// the same tile (a warp's agents are mostly in one).
-__device__ __forceinline__ void add_to_tile(unsigned* tile, unsigned cell) {
-    const unsigned t = cell / kScanTile;
-    const unsigned peers = __match_any_sync(__activemask(), t);
-    if ((threadIdx.x & 31u) == unsigned(__ffs(int(peers)) - 1))
-        atomicAdd(tile + t, unsigned(__popc(int(peers))));
-}
-
-// The agent's cell for the next step's counting sort: counted (the old count
-// is its rank in the cell) and, given tile totals (tile not null), added to
-// its tile's total.
-__device__ __forceinline__ unsigned count_next(const Scene& sc, V3 pos, int wrap_mode,
-                                               unsigned* count, unsigned* tile, unsigned& cell) {
-    const V3 wp = wrap_world(pos, sc.grid.ws, wrap_mode);
-    cell = sc.cell_offset + cell_of(sc.grid, wp);
-    if (tile) add_to_tile(tile, cell);
-    return atomicAdd(count + cell, 1u);
-}
 
 // Reference layout -> A (identity order), counting the first step's cells.
 __global__ void k_from_reference(GroupView g, const unsigned* __restrict__ agent_scene,
@@ -399,44 +377,6 @@ __device__ __forceinline__ void init_accs(Accs& a, const StepDev& p) {
     close_init(a.close);
 }
 
-__device__ __forceinline__ void store_next(const FusedLaunch& L, unsigned s, const Self& me,
-                                           unsigned id, unsigned scene, const Scene& sc,
-                                           int wrap_mode) {
-    // the cell count's atomic first: its round trip overlaps the state stores
-    unsigned cell;
-    const unsigned rank = count_next(sc, me.pos, wrap_mode, L.count, L.tile, cell);
-    L.A.f[0][s] = make_float4(me.pos.x, me.pos.y, me.pos.z, fb(id));
-    L.A.f[1][s] = make_float4(me.dir.x, me.dir.y, me.dir.z, me.speed);
-    L.A.f[2][s] = make_float4(me.side.x, me.side.y, me.side.z, me.radius);
-    L.A.f[3][s] = make_float4(me.up.x, me.up.y, me.up.z, me.mass);
-    L.A.f[4][s] = make_float4(me.max_speed, me.max_force, fb(0u), fb(scene));
-    L.cellrank[s] = make_uint2(cell, rank);
-}
-
-// The scene number alone (f4.w): the KNN needs position, index and scene;
-// the rest of the state is loaded after it, so it is not held in registers
-// through the scan.
-__device__ __forceinline__ unsigned load_scene(const Fused& B, unsigned s) {
-    return __float_as_uint(reinterpret_cast<const float*>(B.f[4] + s)[3]);
-}
-
-// Everything but position and index, after the KNN.
-__device__ __forceinline__ Self load_rest(const Fused& B, unsigned s, V3 pos, float4& f4v) {
-    const float4 f1 = B.f[1][s], f2 = B.f[2][s], f3 = B.f[3][s];
-    f4v = B.f[4][s];
-    Self me;
-    me.pos = pos;
-    me.dir = v3(f1);
-    me.speed = f1.w;
-    me.side = v3(f2);
-    me.radius = f2.w;
-    me.up = v3(f3);
-    me.mass = f3.w;
-    me.max_speed = f4v.x;
-    me.max_force = f4v.y;
-    return me;
-}
-
 // ---- KNN of one agent (fast path, or exact redo) ----------------------------------
 // The exact (distance, index) list of one agent out of line: the collecting
 // scan's kernels call it for the rare agents whose fast scan could not vouch
@@ -647,10 +587,6 @@ __global__ void __launch_bounds__(kBlock) k_knn_retry(FusedLaunch L, StepDev p) 
 constexpr unsigned kNbrChunk = 1;  // measured best for the flock (2: +2.5 %, 4: +9 %)
 constexpr unsigned kRestChunk = 2;  // the rest phase's (1: +7 %, 3: +6 %, 4: +12 %; spills)
 
-// NEEDC: the behaviours that read the neighbour list, fixed at compile time
-// (kNeedRuntime: taken from p.need).
-constexpr unsigned kNeedRuntime = ~0u;
-constexpr unsigned kNeedList = NEED_SEP | NEED_ALI | NEED_COH | NEED_AVOID | NEED_CLOSE;
 template <int KMAX, unsigned ENUM, bool EXACT, unsigned NEEDC = kNeedRuntime, bool FLAT = false>
 __global__ void __launch_bounds__(kBlock, 3) k_fused(FusedLaunch L, StepDev p) {
     const unsigned need = NEEDC == kNeedRuntime ? p.need : NEEDC;
@@ -1167,6 +1103,7 @@ gs_status fused_step(const FusedLaunch& L, const StepDev& p, cudaStream_t st, Ph
     if (L.n == 0) return GS_OK;
     if ((p.need & NEED_WALLS) && p.knw > 8)
         return fail(GS_ERR_UNSUPPORTED, "knw > 8 in the fused step");
+    if (p.lanes) return fused_step_lanes(L, p, st, hook);
     if (p.k <= 8) return launch_fused<8>(L, p, st, hook);
     if (p.k <= 16) return launch_fused<16>(L, p, st, hook);
     return launch_fused<32>(L, p, st, hook);
