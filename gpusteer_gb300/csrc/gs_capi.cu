@@ -985,7 +985,6 @@ static gs_status knn_pairs(const gs_group* groups, unsigned n_groups, gs_bins bi
             gs_group a = groups[i], b = groups[j];
             if (o->n != a->n) return fail(GS_ERR_INVALID_ARG, "KNNData size differs from its group");
             KnnPair& q = P.pair[P.n_pairs++];
-            q.a_sorted = a->db.sorted;
             q.a_pos_id = a->db.pos_id;
             q.b_start = b->db.start;
             q.b_pos_id = b->db.pos_id;

@@ -233,115 +233,6 @@ gs_status db_build(Database& db, const float4* pos, unsigned n, const Grid& grid
     return GS_OK;
 }
 
-// ---- binned KNN, reference output layout (KNNBinningV2Kernel.cu:417-528) ----------
-// One thread per agent of A in bucketed order (neighbouring threads scan the
-// same cells); results go to idx/dist[a + i * nA].
-template <int KMAX>
-__global__ void __launch_bounds__(kBlock) k_knn_binned(
-    const unsigned* __restrict__ a_sorted, const float4* __restrict__ a_pos_id, unsigned nA,
-    const unsigned* __restrict__ b_start, const float4* __restrict__ b_pos_id, Grid g,
-    unsigned r, unsigned k, bool self, unsigned* __restrict__ idx, float* __restrict__ dist) {
-    const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nA) return;
-    const unsigned a = a_sorted[s];
-    const V3 p = v3(a_pos_id[s]);
-    unsigned ix, iy, iz;
-    cell_coords(g, p, ix, iy, iz);
-    const Box box = cell_box(g, ix, iy, iz, r);
-    extern __shared__ unsigned sh_col[];
-    unsigned* col = sh_col + threadIdx.x;
-    const unsigned bd = blockDim.x;
-    knn_neighbours<KMAX, 64>(int(k), p, self ? a : UINT_MAX, g, box, 0u, b_start, b_pos_id, col,
-                             bd);
-    for (unsigned r = 0; r < k; ++r) {
-        const unsigned bs = col[r * bd];
-        const float4 q = bs == UINT_MAX ? make_float4(0.f, 0.f, 0.f, 0.f) : b_pos_id[bs];
-        idx[a + size_t(r) * nA] = bs == UINT_MAX ? UINT_MAX : __float_as_uint(q.w);
-        dist[a + size_t(r) * nA] = bs == UINT_MAX ? FLT_MAX : distance(p, v3(q));
-    }
-}
-
-template <int KMAX>
-static gs_status knn_binned_k(const Database& A, unsigned nA, const Database& B, bool self,
-                              unsigned r, unsigned k, unsigned* idx, float* dist,
-                              cudaStream_t st) {
-    const size_t smem = size_t(2 * 64) * kBlock * sizeof(unsigned);
-    if (smem > 48 * 1024)
-        GS_CUDA(cudaFuncSetAttribute(k_knn_binned<KMAX>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    k_knn_binned<KMAX><<<blocks_for(nA), kBlock, smem, st>>>(A.sorted, A.pos_id, nA, B.start,
-                                                             B.pos_id, B.grid, r, k, self, idx,
-                                                             dist);
-    GS_LAUNCHED("knn_binned");
-    return GS_OK;
-}
-
-// ---- batched binned KNN over group pairs --------------------------------------
-// The k_knn_binned search for several (A, B) database pairs in one launch: the
-// pair table rides in the kernel parameters, each pair owns a contiguous run
-// of blocks, and a block finds its pair by a scan of the (few) block offsets.
-template <int KMAX>
-__global__ void __launch_bounds__(kBlock) k_knn_binned_pairs(KnnPairs P) {
-    unsigned q = 0;
-    while (q + 1 < P.n_pairs && blockIdx.x >= P.pair[q + 1].block_begin) ++q;
-    const KnnPair& pr = P.pair[q];
-    const unsigned s = (blockIdx.x - pr.block_begin) * blockDim.x + threadIdx.x;
-    if (s >= pr.nA) return;
-    const unsigned a = pr.a_sorted[s];
-    const V3 p = v3(pr.a_pos_id[s]);
-    unsigned ix, iy, iz;
-    cell_coords(P.grid, p, ix, iy, iz);
-    const Box box = cell_box(P.grid, ix, iy, iz, P.r);
-    extern __shared__ unsigned sh_col[];
-    unsigned* col = sh_col + threadIdx.x;
-    const unsigned bd = blockDim.x;
-    knn_neighbours<KMAX, 64>(int(pr.k), p, pr.self ? a : UINT_MAX, P.grid, box, 0u, pr.b_start,
-                             pr.b_pos_id, col, bd);
-    for (unsigned r = 0; r < pr.k; ++r) {
-        const unsigned bs = col[r * bd];
-        const float4 v = bs == UINT_MAX ? make_float4(0.f, 0.f, 0.f, 0.f) : pr.b_pos_id[bs];
-        pr.idx[a + size_t(r) * pr.nA] = bs == UINT_MAX ? UINT_MAX : __float_as_uint(v.w);
-        pr.dist[a + size_t(r) * pr.nA] = bs == UINT_MAX ? FLT_MAX : distance(p, v3(v));
-    }
-}
-
-template <int KMAX>
-static gs_status knn_pairs_k(const KnnPairs& P, unsigned blocks, cudaStream_t st) {
-    const size_t smem = size_t(2 * 64) * kBlock * sizeof(unsigned);
-    if (smem > 48 * 1024)
-        GS_CUDA(cudaFuncSetAttribute(k_knn_binned_pairs<KMAX>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    k_knn_binned_pairs<KMAX><<<blocks, kBlock, smem, st>>>(P);
-    GS_LAUNCHED("knn_binned_pairs");
-    return GS_OK;
-}
-static_assert(sizeof(KnnPairs) <= 4096, "batched KNN parameters exceed 4 KiB");
-
-gs_status launch_knn_binned_pairs(KnnPairs& P, cudaStream_t st) {
-    if (P.n_pairs == 0 || P.n_pairs > kMaxKnnPairs)
-        return fail(GS_ERR_INVALID_ARG, "between 1 and 49 group pairs per batched KNN");
-    unsigned blocks = 0, kmax = 0;
-    for (unsigned q = 0; q < P.n_pairs; ++q) {
-        P.pair[q].block_begin = blocks;
-        blocks += blocks_for(P.pair[q].nA);
-        kmax = std::max(kmax, P.pair[q].k);
-    }
-    if (blocks == 0) return GS_OK;
-    if (kmax <= 8) return knn_pairs_k<8>(P, blocks, st);
-    if (kmax <= 16) return knn_pairs_k<16>(P, blocks, st);
-    if (kmax <= 32) return knn_pairs_k<32>(P, blocks, st);
-    return knn_pairs_k<64>(P, blocks, st);
-}
-
-gs_status launch_knn_binned(const Database& A, unsigned nA, const Database& B, bool self,
-                            unsigned r, unsigned k, unsigned* idx, float* dist, cudaStream_t st) {
-    if (nA == 0) return GS_OK;
-    if (k <= 8) return knn_binned_k<8>(A, nA, B, self, r, k, idx, dist, st);
-    if (k <= 16) return knn_binned_k<16>(A, nA, B, self, r, k, idx, dist, st);
-    if (k <= 32) return knn_binned_k<32>(A, nA, B, self, r, k, idx, dist, st);
-    return knn_binned_k<64>(A, nA, B, self, r, k, idx, dist, st);
-}
-
 // ---- brute-force KNN (KNNBruteForceCudaKernel.cu:207-283) ---------------------------
 // A candidate needs its square root only when its squared distance is within
 // a rounded-up bound of the current k-th distance squared: a larger squared

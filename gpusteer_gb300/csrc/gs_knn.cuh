@@ -527,23 +527,4 @@ __device__ __forceinline__ void knn_neighbours_exact(int k, V3 p, unsigned self_
     });
 }
 
-// The k nearest of `box` as slots in (distance, index) order at
-// col[r * stride] (UINT_MAX after the last neighbour): the fast scan, or the
-// exact list when the fast scan cannot vouch for its order.  col needs
-// ENUM + KMAX entries.
-template <int KMAX, unsigned ENUM>
-__device__ __forceinline__ void knn_neighbours(int k, V3 p, unsigned self_id, const Grid& g,
-                                               const Box& b, unsigned cell_offset,
-                                               const unsigned* __restrict__ cell_start,
-                                               const float4* __restrict__ pos_id,
-                                               unsigned* col, unsigned stride) {
-    // col holds the slot table (ENUM entries) then the key table / result
-    if (knn_neighbours_fast<KMAX, ENUM>(k, p, self_id, g, b, cell_offset, cell_start, pos_id, col,
-                                        col + ENUM * stride, stride)) {
-        for (int r = 0; r < k; ++r) col[r * stride] = col[(ENUM + r) * stride];
-        return;
-    }
-    knn_neighbours_exact<KMAX>(k, p, self_id, g, b, cell_offset, cell_start, pos_id, col, stride);
-}
-
 }  // namespace gs

@@ -12,121 +12,31 @@ namespace gs {
 
 constexpr unsigned kLaneBlock = 128;
 
-// The neighbour pass and the behaviours order[first..] of one agent: lane r
-// holds neighbour r (ok: there is one) in b0 (position), b1 (heading | speed),
-// br (radius) and its KNN distance kd.  Each lane evaluates its neighbour's
-// terms with the reference's expressions; the sums run in list order.
+// The behaviours order[first..] of one agent over its lanes' neighbours.
 template <int G>
 __device__ __forceinline__ void lanes_behaviours(const StepDev& p, unsigned need, unsigned first,
-                                                 const Self& me, unsigned lane, bool ok, V3 bpos,
-                                                 V3 bdir, float bspeed, float br, float kd,
-                                                 float* shared, unsigned& applied, V3& steer) {
-    const V3 zero = v3(0.f, 0.f, 0.f);
-    V3 r_sep = zero, r_ali = zero, r_coh = zero;
-    if (need & (NEED_SEP | NEED_ALI | NEED_COH)) {
-        LaneSums<G> sums{shared + (threadIdx.x / G) * LaneSums<G>::kWords};
-        const V3 offset = sub(bpos, me.pos);
-        const float dsq = dot(offset, offset), d = sqrtf(dsq);
-        const float ahead = dot(me.dir, dvd(offset, d));
-        auto member = [&](const float v[5]) {
-            return ok && (d < v[0] || (!(d > v[1]) && ahead > v[2]));
-        };
-        unsigned n_sep = 0, n_ali = 0, n_coh = 0;
-        if (need & NEED_SEP) {
-            const bool in = member(p.sep);
-            n_sep = __popc(lanes_ballot<G>(in));
-            sums.put(0, lane, in ? dvd(offset, -dsq) : zero);
-        }
-        if (need & NEED_ALI) {
-            const bool in = member(p.ali);
-            n_ali = __popc(lanes_ballot<G>(in));
-            sums.put(3, lane, in ? bdir : zero);
-        }
-        if (need & NEED_COH) {
-            const bool in = member(p.coh);
-            n_coh = __popc(lanes_ballot<G>(in));
-            sums.put(6, lane, in ? bpos : zero);
-        }
-        sums.add_rows(lane);
-        // lanes 0, 1, 2: the three behaviours' finish (flock_finish) side by side
-        const unsigned kind = lane < 2 ? lane : 2u;
-        const unsigned n = kind == 0 ? n_sep : kind == 1 ? n_ali : n_coh;
-        const float w = kind == 0 ? p.sep[3] : kind == 1 ? p.ali[3] : p.coh[3];
-        V3 r = n ? sums.sum(3 * kind) : zero;
-        if (n) {
-            const V3 mean = dvd(r, float(n));
-            r = normalize(kind == 0 ? mean : sub(mean, kind == 1 ? me.dir : me.pos));
-        }
-        r = mul(r, w);
-        if (need & NEED_SEP) r_sep = lanes_get<G>(r, 0);
-        if (need & NEED_ALI) r_ali = lanes_get<G>(r, 1);
-        if (need & NEED_COH) r_coh = lanes_get<G>(r, 2);
-    }
+                                                 const Self& me, unsigned lane,
+                                                 const LaneNeighbour& nb, LaneSums<G> sums,
+                                                 unsigned& applied, V3& steer) {
+    const FlockParams fs = flock_params(p.sep, p.sep_dsq), fa = flock_params(p.ali, p.ali_dsq),
+                      fc = flock_params(p.coh, p.coh_dsq);
+    V3 r_sep, r_ali, r_coh;
+    lanes_flock(need, fs, fa, fc, me, lane, nb, sums, r_sep, r_ali, r_coh);
     CloseAcc close;
-    close_init(close);
     AvoidAcc avoid;
-    avoid_init(avoid, p.min_time_col);
-    if (need & NEED_CLOSE) {
-        CloseAcc c;
-        close_init(c);
-        if (ok) close_add(c, me, p.min_sep, kd, bpos, br);
-        const unsigned m = lanes_ballot<G>(c.found);
-        const V3 s = lanes_get<G>(c.steer, m ? unsigned(__ffs(int(m)) - 1) : 0u);
-        if (m) close.steer = s;
-    }
-    if (need & NEED_AVOID) {
-        // every lane its neighbour's approach time and distance; then the
-        // reference's pass over them in list order (avoid_add), whose window
-        // [0, min_t) only narrows
-        V3 at = zero;
-        float t = __int_as_float(0x7f800000);
-        bool danger = false;
-        if (ok) {
-            const float time =
-                nearest_approach_time(me.pos, me.dir, me.speed, bpos, bdir, bspeed);
-            if (time >= 0.f) t = time;
-            danger = nearest_approach_positions(me.pos, me.dir, me.speed, bpos, bdir, bspeed, time,
-                                                at) < me.radius + br;
-        }
-        const unsigned hits = lanes_ballot<G>(danger);
-        unsigned last = UINT_MAX, threat = UINT_MAX;
-        for (unsigned r = 0; r < p.k; ++r) {
-            const float tr = __shfl_sync(kAllLanes, t, int(r), G);
-            if (tr < avoid.min_t) {
-                last = r;
-                if ((hits >> r) & 1u) {
-                    avoid.min_t = tr;
-                    threat = r;
-                }
-            }
-        }
-        const unsigned lf = last == UINT_MAX ? 0u : last, tf = threat == UINT_MAX ? 0u : threat;
-        const V3 la = lanes_get<G>(at, lf), tp = lanes_get<G>(bpos, tf), td = lanes_get<G>(bdir, tf);
-        const float ts = __shfl_sync(kAllLanes, bspeed, int(tf), G);
-        if (last != UINT_MAX) avoid.threat_at = la;
-        if (threat != UINT_MAX) {
-            avoid.threat = threat;
-            avoid.threat_pos = tp;
-            avoid.threat_dir = td;
-            avoid.threat_speed = ts;
-        }
-    }
-    auto flock = [&](V3 r, const float v[5], unsigned bit) {
-        if (applied & __float_as_uint(v[4])) return;
-        if (!is_zero(r)) applied |= bit;
-        steer = add(r, steer);
-    };
+    if (need & NEED_CLOSE) close = lanes_close<G>(me, p.min_sep, nb);
+    if (need & NEED_AVOID) avoid = lanes_avoid<G>(me, p.min_time_col, p.k, nb);
 #pragma unroll 1
     for (unsigned o = first; o < p.n_order; ++o) {
         switch ((p.order_packed >> (3u * o)) & 7u) {
             case GS_B_SEPARATION:
-                if (need & NEED_SEP) flock(r_sep, p.sep, SEPARATION_BIT);
+                if (need & NEED_SEP) flock_apply(r_sep, fs, SEPARATION_BIT, applied, steer);
                 break;
             case GS_B_ALIGNMENT:
-                if (need & NEED_ALI) flock(r_ali, p.ali, ALIGNMENT_BIT);
+                if (need & NEED_ALI) flock_apply(r_ali, fa, ALIGNMENT_BIT, applied, steer);
                 break;
             case GS_B_COHESION:
-                if (need & NEED_COH) flock(r_coh, p.coh, COHESION_BIT);
+                if (need & NEED_COH) flock_apply(r_coh, fc, COHESION_BIT, applied, steer);
                 break;
             case GS_B_SEEK:
                 seek_finish(v3(p.seek_target[0], p.seek_target[1], p.seek_target[2]), p.w_seek,
@@ -134,7 +44,8 @@ __device__ __forceinline__ void lanes_behaviours(const StepDev& p, unsigned need
                 break;
             case GS_B_AVOID_NEIGHBORS:
                 if (need & NEED_AVOID) {
-                    if (p.avoid_close) close_finish(close, p.w_avoid, p.mask_avoid, applied, steer);
+                    if (need & NEED_CLOSE)
+                        close_finish(close, p.w_avoid, p.mask_avoid, applied, steer);
                     avoid_finish(avoid, p.w_avoid, p.mask_avoid, me, applied, steer);
                 }
                 break;
@@ -149,6 +60,8 @@ __device__ __forceinline__ void lanes_behaviours(const StepDev& p, unsigned need
 // ---- whole step without walls -----------------------------------------------------------
 template <int G, int R, unsigned NEEDC>
 __global__ void __launch_bounds__(kLaneBlock) k_lanes_step(FusedLaunch L, StepDev p) {
+    __shared__ unsigned row_sh[R ? 1 : kLaneBlock / G * kLaneRowWords];
+    unsigned* rows = row_sh + (R ? 0u : threadIdx.x / G * kLaneRowWords);
     __shared__ __align__(16) float sh[kLaneBlock / G * LaneSums<G>::kWords];
     const unsigned need = NEEDC == kNeedRuntime ? p.need : NEEDC;
     const unsigned lane = threadIdx.x & unsigned(G - 1);
@@ -165,7 +78,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_step(FusedLaunch L, StepDe
     cell_coords(sc.grid, me.pos, ix, iy, iz);
     const Box box = cell_box(sc.grid, ix, iy, iz, p.r);
     const LaneEntry<G> nb = lanes_knn<G, R>(p.k, lane, me.pos, id, sc.grid, box, sc.cell_offset,
-                                            L.start, L.B.f[0]);
+                                            L.start, L.B.f[0], rows);
     const bool ok = lane < p.k && nb.slot != UINT_MAX;
     const unsigned bs = ok ? nb.slot : s;
     const float4 b0 = L.B.f[0][bs], b1 = L.B.f[1][bs];
@@ -180,8 +93,8 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_step(FusedLaunch L, StepDe
     }
     unsigned applied = p.clear_applied ? 0u : __float_as_uint(f4v.z);
     V3 steer = p.dirty ? v3(L.B.f[5][s]) : v3(0.f, 0.f, 0.f);
-    lanes_behaviours<G>(p, need, 0, me, lane, ok, v3(b0), v3(b1), b1.w, br, key_dist(nb.key), sh,
-                        applied, steer);
+    const LaneNeighbour n{ok, v3(b0), v3(b1), b1.w, br, key_dist(nb.key)};
+    lanes_behaviours<G>(p, need, 0, me, lane, n, LaneSums<G>::of(sh), applied, steer);
     integrate(me, steer, p.dt);
     if (act && lane == 0) store_next(L, s, me, id, scene, sc, p.wrap_mode);
 }
@@ -222,6 +135,8 @@ __device__ __forceinline__ void lanes_wall_line(WallAcc& wa, const Self& me, uns
 
 template <int G, int R>
 __global__ void __launch_bounds__(kLaneBlock) k_lanes_walls(FusedLaunch L, StepDev p) {
+    __shared__ unsigned row_sh[R ? 1 : kLaneBlock / G * kLaneRowWords];
+    unsigned* rows = row_sh + (R ? 0u : threadIdx.x / G * kLaneRowWords);
     const unsigned lane = threadIdx.x & unsigned(G - 1);
     const unsigned a = (blockIdx.x * kLaneBlock + threadIdx.x) / G;
     const bool act = a < L.n;
@@ -235,7 +150,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_walls(FusedLaunch L, StepD
     cell_coords(sc.grid, me.pos, ix, iy, iz);
     const Box box = cell_box(sc.grid, ix, iy, iz, p.r);
     const LaneEntry<G> nb = lanes_knn<G, R>(p.k, lane, me.pos, id, sc.grid, box, sc.cell_offset,
-                                            L.start, L.B.f[0]);
+                                            L.start, L.B.f[0], rows);
     if (act && lane < p.k) {
         L.knn_slot[size_t(s) * p.k + lane] = nb.slot;
         // the KNN distance (before any wall correction moves agents), read by
@@ -253,7 +168,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_walls(FusedLaunch L, StepD
         }
         const LaneEntry<G> wl =
             lanes_knn<G, R>(p.knw, lane, me.pos, UINT_MAX, sc.grid, wb, sc.wall_cell_offset,
-                            L.w_cell_start, L.w_pos_id);
+                            L.w_cell_start, L.w_pos_id, rows);
         const unsigned found = lanes_ballot<G>(walls && lane < p.knw && wl.slot != UINT_MAX &&
                                                key_id(wl.key) < sc.n_walls);
         WallAcc wa;
@@ -303,8 +218,8 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_rest(FusedLaunch L, StepDe
     const unsigned scene = __float_as_uint(f4v.w);
     unsigned applied = __float_as_uint(w2.w);
     V3 steer = v3(w2);
-    lanes_behaviours<G>(p, need, 1, me, lane, ok, v3(b0), v3(b1), b1.w, b0.w, kd, sh, applied,
-                        steer);
+    const LaneNeighbour n{ok, v3(b0), v3(b1), b1.w, b0.w, kd};
+    lanes_behaviours<G>(p, need, 1, me, lane, n, LaneSums<G>::of(sh), applied, steer);
     integrate(me, steer, p.dt);
     const Scene sc = L.scenes[scene];
     if (act && lane == 0) store_next(L, s, me, id, scene, sc, p.wrap_mode);

@@ -17,6 +17,7 @@
 
 #include "gs_behaviours.cuh"
 #include "gs_knn.cuh"
+#include "gs_launch.h"
 
 namespace gs {
 
@@ -97,14 +98,18 @@ __device__ __forceinline__ LaneEntry<G> lanes_candidate(V3 p, unsigned self_id, 
 // order over the group's lanes: lane r holds rank r (ranks past the last
 // neighbour hold the empty entry; lanes r >= k hold leftovers).
 // R: rows of cells in the box at search radius 1 (9, or 3 on a grid one cell
-// high in y); 0 for any radius.  Rows 1..R are laid end to end, so a group
-// takes ceil(candidates / G) chunks whatever the rows' lengths.
+// high in y); 0 for any radius.  The rows are laid end to end, so a group
+// takes ceil(candidates / G) chunks whatever the rows' lengths; with R = 0
+// their table is the group's kLaneRowWords words `rows` of shared memory, and
+// a box of more than kLaneRows rows is taken row by row.
+constexpr unsigned kLaneRows = 64, kLaneRowWords = 2 * kLaneRows + 1;
 template <int G, int R>
 __device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 p,
                                                   unsigned self_id, const Grid& g, const Box& b,
                                                   unsigned cell_offset,
                                                   const unsigned* __restrict__ start,
-                                                  const float4* __restrict__ pos_id) {
+                                                  const float4* __restrict__ pos_id,
+                                                  unsigned* rows = nullptr) {
     LaneEntry<G> list{KEY_EMPTY, UINT_MAX};
     const unsigned span = b.x1 - b.x0 + 1;
     if constexpr (R > 0) {
@@ -148,26 +153,63 @@ __device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 
             q = qn;
         }
     } else {
-        bool first = true;
         // (an empty box has y1 < y0)
-        const unsigned ny = __reduce_max_sync(kAllLanes, b.y1 >= b.y0 ? b.y1 - b.y0 : 0u),
-                       nz = __reduce_max_sync(kAllLanes, b.z1 >= b.z0 ? b.z1 - b.z0 : 0u);
-        for (unsigned y = 0; y <= ny; ++y)
-            for (unsigned z = 0; z <= nz; ++z) {
-                unsigned s0 = 0, len = 0;
-                if (b.y0 + y <= b.y1 && b.z0 + z <= b.z1) {
-                    const unsigned c0 = cell_offset + cell_label(g, b.x0, b.y0 + y, b.z0 + z);
-                    s0 = __ldg(start + c0);
-                    len = __ldg(start + c0 + span) - s0;
+        const unsigned nz = b.z1 - b.z0 + 1;
+        const unsigned nr = b.y1 >= b.y0 ? (b.y1 - b.y0 + 1) * nz : 0u;
+        const unsigned most = __reduce_max_sync(kAllLanes, nr);
+        auto row = [&](unsigned i, unsigned& s0) {
+            const unsigned c0 = cell_offset + cell_label(g, b.x0, b.y0 + i / nz, b.z0 + i % nz);
+            s0 = __ldg(start + c0);
+            return __ldg(start + c0 + span) - s0;
+        };
+        if (most <= kLaneRows) {
+            unsigned* rs = rows;
+            unsigned* pre = rows + kLaneRows;
+            unsigned total = 0;
+            for (unsigned i = lane; i < most + lane; i += G) {
+                unsigned s0 = 0, len = i < nr ? row(i, s0) : 0u;
+                unsigned sum = len;
+#pragma unroll
+                for (int o = 1; o < G; o <<= 1) {
+                    const unsigned y = __shfl_up_sync(kAllLanes, sum, o, G);
+                    if (lane >= unsigned(o)) sum += y;
                 }
+                if (i < nr) {
+                    rs[i] = s0;
+                    pre[i] = total + sum - len;
+                }
+                total += __shfl_sync(kAllLanes, sum, G - 1, G);
+            }
+            if (lane == 0) pre[nr] = total;
+            __syncwarp();
+            const unsigned rounds = __reduce_max_sync(kAllLanes, total);
+            unsigned at = 0;
+            for (unsigned j = lane; j < rounds + lane; j += G) {
+                const bool ok = j < total;
+                unsigned sl = 0;
+                if (ok) {
+                    while (j >= pre[at + 1]) ++at;
+                    sl = rs[at] + (j - pre[at]);
+                }
+                const float4 q = ok ? __ldg(pos_id + sl) : make_float4(0.f, 0.f, 0.f, 0.f);
+                lanes_take(list, lanes_candidate<G>(p, self_id, q, sl, ok), j < G, k, lane);
+            }
+            __syncwarp();  // the rows may be written again
+        } else {
+            bool first = true;
+            for (unsigned i = 0; i < most; ++i) {
+                unsigned s0 = 0;
+                const unsigned len = i < nr ? row(i, s0) : 0u;
                 const unsigned rounds = __reduce_max_sync(kAllLanes, len);
                 for (unsigned j = lane; j < rounds + lane; j += G) {
-                    const float4 q = j < len ? __ldg(pos_id + s0 + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 q =
+                        j < len ? __ldg(pos_id + s0 + j) : make_float4(0.f, 0.f, 0.f, 0.f);
                     lanes_take(list, lanes_candidate<G>(p, self_id, q, s0 + j, j < len), first, k,
                                lane);
                     first = false;
                 }
             }
+        }
     }
     return list;
 }
@@ -196,6 +238,9 @@ struct LaneSums {
     static constexpr unsigned kRow = G + 4;
     static constexpr unsigned kWords = 9 * kRow + 12;
     float* w;  // this group's kWords words, 16-byte aligned
+    __device__ __forceinline__ static LaneSums of(float* shared) {
+        return LaneSums{shared + threadIdx.x / G * kWords};
+    }
     __device__ __forceinline__ void put(unsigned first, unsigned lane, V3 v) {
         w[first * kRow + lane] = v.x;
         w[(first + 1) * kRow + lane] = v.y;
@@ -222,5 +267,129 @@ struct LaneSums {
         return v3(w[9 * kRow + first], w[9 * kRow + first + 1], w[9 * kRow + first + 2]);
     }
 };
+
+// ---- the neighbour pass over lanes -----------------------------------------------------
+// Lane r's neighbour (rank r of the list): ok when there is one; `dist` is its
+// KNN distance.  Each lane evaluates its neighbour's terms with the
+// reference's expressions; what the reference does in list order happens in
+// lane order.
+struct LaneNeighbour {
+    bool ok;
+    V3 pos, dir;
+    float speed, radius, dist;
+};
+
+// The weighted separation, alignment and cohesion vectors (flock_finish up to
+// its mask test) of the behaviours in `need`; the others' are left unset.
+template <int G>
+__device__ __forceinline__ void lanes_flock(unsigned need, const FlockParams& fs,
+                                            const FlockParams& fa, const FlockParams& fc,
+                                            const Self& me, unsigned lane,
+                                            const LaneNeighbour& nb, LaneSums<G> sums, V3& r_sep,
+                                            V3& r_ali, V3& r_coh) {
+    if (!(need & (NEED_SEP | NEED_ALI | NEED_COH))) return;
+    const V3 zero = v3(0.f, 0.f, 0.f);
+    const V3 offset = sub(nb.pos, me.pos);
+    const float dsq = dot(offset, offset), d = sqrtf(dsq);
+    const float ahead = dot(me.dir, dvd(offset, d));
+    auto member = [&](const FlockParams& f) {  // inBoidNeighborhood, FlockingCommon.cuh:4-30
+        return nb.ok && (d < f.min_d || (!(d > f.max_d) && ahead > f.cos_max));
+    };
+    unsigned n_sep = 0, n_ali = 0, n_coh = 0;
+    if (need & NEED_SEP) {
+        const bool in = member(fs);
+        n_sep = __popc(lanes_ballot<G>(in));
+        sums.put(0, lane, in ? dvd(offset, -dsq) : zero);
+    }
+    if (need & NEED_ALI) {
+        const bool in = member(fa);
+        n_ali = __popc(lanes_ballot<G>(in));
+        sums.put(3, lane, in ? nb.dir : zero);
+    }
+    if (need & NEED_COH) {
+        const bool in = member(fc);
+        n_coh = __popc(lanes_ballot<G>(in));
+        sums.put(6, lane, in ? nb.pos : zero);
+    }
+    sums.add_rows(lane);
+    // lanes 0, 1, 2: the three behaviours' finish side by side
+    const unsigned kind = lane < 2 ? lane : 2u;
+    const unsigned n = kind == 0 ? n_sep : kind == 1 ? n_ali : n_coh;
+    const float w = kind == 0 ? fs.w : kind == 1 ? fa.w : fc.w;
+    V3 r = zero;
+    if (n) {
+        const V3 mean = dvd(sums.sum(3 * kind), float(n));
+        r = normalize(kind == 0 ? mean : sub(mean, kind == 1 ? me.dir : me.pos));
+    }
+    r = mul(r, w);
+    if (need & NEED_SEP) r_sep = lanes_get<G>(r, 0);
+    if (need & NEED_ALI) r_ali = lanes_get<G>(r, 1);
+    if (need & NEED_COH) r_coh = lanes_get<G>(r, 2);
+    __syncwarp();  // the sums may be written again
+}
+// The rest of flock_finish.
+__device__ __forceinline__ void flock_apply(V3 r, const FlockParams& f, unsigned bit,
+                                            unsigned& applied, V3& steer) {
+    if (applied & f.mask) return;
+    if (!is_zero(r)) applied |= bit;
+    steer = add(r, steer);
+}
+
+// close_add over the list: its first hit.
+template <int G>
+__device__ __forceinline__ CloseAcc lanes_close(const Self& me, float min_sep,
+                                                const LaneNeighbour& nb) {
+    CloseAcc c;
+    close_init(c);
+    if (nb.ok) close_add(c, me, min_sep, nb.dist, nb.pos, nb.radius);
+    const unsigned m = lanes_ballot<G>(c.found);
+    const V3 s = lanes_get<G>(c.steer, m ? unsigned(__ffs(int(m)) - 1) : 0u);
+    c.found = m != 0;
+    c.steer = m ? s : v3(0.f, 0.f, 0.f);
+    return c;
+}
+
+// avoid_add over the list: every lane its neighbour's approach time and
+// distance, then the reference's pass over them, whose window [0, min_t) only
+// narrows (`at` keeps the last neighbour in it, threat or not).
+template <int G>
+__device__ __forceinline__ AvoidAcc lanes_avoid(const Self& me, float min_time, unsigned k,
+                                                const LaneNeighbour& nb) {
+    AvoidAcc a;
+    avoid_init(a, min_time);
+    V3 at = v3(0.f, 0.f, 0.f);
+    float t = __int_as_float(0x7f800000);
+    bool danger = false;
+    if (nb.ok) {
+        const float time =
+            nearest_approach_time(me.pos, me.dir, me.speed, nb.pos, nb.dir, nb.speed);
+        if (time >= 0.f) t = time;
+        danger = nearest_approach_positions(me.pos, me.dir, me.speed, nb.pos, nb.dir, nb.speed,
+                                            time, at) < me.radius + nb.radius;
+    }
+    const unsigned hits = lanes_ballot<G>(danger);
+    unsigned last = UINT_MAX;
+    for (unsigned r = 0; r < k; ++r) {
+        const float tr = __shfl_sync(kAllLanes, t, int(r), G);
+        if (tr < a.min_t) {
+            last = r;
+            if ((hits >> r) & 1u) {
+                a.min_t = tr;
+                a.threat = r;
+            }
+        }
+    }
+    const unsigned lf = last == UINT_MAX ? 0u : last, tf = a.threat == UINT_MAX ? 0u : a.threat;
+    const V3 la = lanes_get<G>(at, lf), tp = lanes_get<G>(nb.pos, tf),
+             td = lanes_get<G>(nb.dir, tf);
+    const float ts = __shfl_sync(kAllLanes, nb.speed, int(tf), G);
+    if (last != UINT_MAX) a.threat_at = la;
+    if (a.threat != UINT_MAX) {
+        a.threat_pos = tp;
+        a.threat_dir = td;
+        a.threat_speed = ts;
+    }
+    return a;
+}
 
 }  // namespace gs

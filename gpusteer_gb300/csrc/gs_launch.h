@@ -38,7 +38,6 @@ gs_status launch_knn_binned(const Database& A, unsigned nA, const Database& B, b
 // 49 pairs (seven groups, every pair) keep the parameter block under 4 KiB.
 constexpr unsigned kMaxKnnPairs = 49;
 struct KnnPair {
-    const unsigned* a_sorted;
     const float4* a_pos_id;
     const unsigned* b_start;
     const float4* b_pos_id;
