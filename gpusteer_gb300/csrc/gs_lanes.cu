@@ -225,6 +225,188 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_rest(FusedLaunch L, StepDe
     if (act && lane == 0) store_next(L, s, me, id, scene, sc, p.wrap_mode);
 }
 
+// ---- one behaviour per launch ------------------------------------------------------------------
+// The per-function behaviours of small groups: lane r of an agent's group takes
+// list entry r.  An index past the other group ends the list, as in the
+// reference's kernels.
+template <int G>
+__device__ __forceinline__ bool lanes_entry(const unsigned* __restrict__ knn, unsigned i,
+                                            unsigned n, unsigned k, unsigned n_other,
+                                            unsigned lane, unsigned& b) {
+    b = lane < k ? knn[i + size_t(lane) * n] : UINT_MAX;
+    const unsigned bad = lanes_ballot<G>(b >= n_other);
+    const bool ok = bad == 0 || lane < unsigned(__ffs(int(bad)) - 1);
+    if (!ok) b = 0;
+    return ok;
+}
+
+// Agent, lane and validity of the thread; spare groups run along as the last
+// agent and store nothing.
+template <int G>
+__device__ __forceinline__ bool lanes_agent(unsigned n, unsigned& i, unsigned& lane) {
+    const unsigned a = (blockIdx.x * kLaneBlock + threadIdx.x) / G;
+    lane = threadIdx.x & unsigned(G - 1);
+    i = a < n ? a : n - 1;
+    return a < n;
+}
+
+// KIND: 0 separation, 1 alignment, 2 cohesion
+template <int G, int KIND>
+__global__ void __launch_bounds__(kLaneBlock) k_flock_lanes(GroupView g,
+                                                            const unsigned* __restrict__ knn,
+                                                            unsigned k, OtherView o,
+                                                            FlockParams fp) {
+    __shared__ __align__(16) float sh[kLaneBlock / G * LaneSums<G>::kWords];
+    constexpr unsigned need = KIND == 0 ? NEED_SEP : KIND == 1 ? NEED_ALI : NEED_COH;
+    unsigned i, lane, b;
+    const bool act = lanes_agent<G>(g.n, i, lane);
+    LaneNeighbour nb;
+    nb.ok = lanes_entry<G>(knn, i, g.n, k, o.n, lane, b);
+    unsigned applied = g.applied[i];
+    Self me;
+    me.pos = v3(g.position[i]);
+    me.dir = v3(g.direction[i]);
+    V3 steer = v3(g.steering[i]);
+    nb.pos = nb.ok ? v3(o.position[b]) : me.pos;
+    nb.dir = nb.ok && KIND == 1 ? v3(o.direction[b]) : me.dir;
+    V3 r_sep, r_ali, r_coh;
+    lanes_flock(need, fp, fp, fp, me, lane, nb, LaneSums<G>::of(sh), r_sep, r_ali, r_coh);
+    if (!act || lane != 0 || (applied & fp.mask)) return;
+    flock_apply(KIND == 0 ? r_sep : KIND == 1 ? r_ali : r_coh, fp,
+                KIND == 0 ? SEPARATION_BIT : KIND == 1 ? ALIGNMENT_BIT : COHESION_BIT, applied,
+                steer);
+    g.steering[i] = f4(steer, 0.f);
+    g.applied[i] = applied;
+}
+
+// steerToAvoidNeighbors: the close pass (CLOSE) or the main pass.
+template <int G, bool CLOSE>
+__global__ void __launch_bounds__(kLaneBlock) k_avoid_lanes(GroupView g,
+                                                            const unsigned* __restrict__ knn,
+                                                            const float* __restrict__ knn_dist,
+                                                            unsigned k, OtherView o, float limit,
+                                                            float w, unsigned mask) {
+    unsigned i, lane, b;
+    const bool act = lanes_agent<G>(g.n, i, lane);
+    LaneNeighbour nb;
+    nb.ok = lanes_entry<G>(knn, i, g.n, k, o.n, lane, b);
+    nb.dist = CLOSE && nb.ok ? knn_dist[i + size_t(lane) * g.n] : 0.f;
+    unsigned applied = g.applied[i];
+    Self me;
+    me.pos = v3(g.position[i]);
+    me.dir = v3(g.direction[i]);
+    me.speed = g.speed[i];
+    me.radius = g.radius[i];
+    const float3 sd = g.side[i];
+    me.side = v3(sd.x, sd.y, sd.z);
+    V3 steer = v3(g.steering[i]);
+    if (nb.ok) {
+        nb.pos = v3(o.position[b]);
+        nb.radius = o.radius[b];
+        if (!CLOSE) {
+            nb.dir = v3(o.direction[b]);
+            nb.speed = o.speed[b];
+        }
+    } else {
+        nb.pos = nb.dir = v3(0.f, 0.f, 0.f);
+        nb.speed = nb.radius = 0.f;
+    }
+    if constexpr (CLOSE) {
+        const CloseAcc c = lanes_close<G>(me, limit, nb);
+        if (!act || lane != 0 || (applied & mask)) return;
+        close_finish(c, w, mask, applied, steer);
+    } else {
+        const AvoidAcc a = lanes_avoid<G>(me, limit, k, nb);
+        if (!act || lane != 0 || a.threat == UINT_MAX) return;
+        avoid_finish(a, w, mask, me, applied, steer);
+    }
+    g.steering[i] = f4(steer, 0.f);
+    g.applied[i] = applied;
+}
+
+template <int G>
+__global__ void __launch_bounds__(kLaneBlock) k_avoid_walls_lanes(
+    GroupView g, const unsigned* __restrict__ knw, unsigned kw, const float4* __restrict__ ls,
+    const float4* __restrict__ le, const float4* __restrict__ ln, unsigned n_lines, float min_time,
+    float w, unsigned mask) {
+    unsigned i, lane, line;
+    const bool act = lanes_agent<G>(g.n, i, lane);
+    const bool ok = lanes_entry<G>(knw, i, g.n, kw, n_lines, lane, line);
+    unsigned applied = g.applied[i];
+    Self me;
+    me.pos = v3(g.position[i]);
+    me.dir = v3(g.direction[i]);
+    me.speed = g.speed[i];
+    me.radius = g.radius[i];
+    const float3 sd = g.side[i];
+    me.side = v3(sd.x, sd.y, sd.z);
+    V3 steer = v3(g.steering[i]);
+    const unsigned lines = __popc(lanes_ballot<G>(ok));
+    const unsigned most = __reduce_max_sync(kAllLanes, lines);
+    WallAcc wa;
+    walls_init(wa, me, min_time);
+    for (unsigned r = 0; r < most; ++r) {
+        const unsigned at = __shfl_sync(kAllLanes, line, int(r), G);
+        const bool on = r < lines;
+        const unsigned s = on ? at : 0u;
+        lanes_wall_line<G>(wa, me, lane, at, on, v3(ls[s]), v3(le[s]), v3(ln[s]));
+    }
+    if (!act || lane != 0 || (applied & mask)) return;
+    walls_finish(wa, w, mask, me, applied, steer);
+    g.steering[i] = f4(steer, 0.f);
+    g.position[i] = f4(me.pos, 0.f);
+    g.direction[i] = f4(me.dir, 0.f);
+    g.applied[i] = applied;
+}
+
+template <int G>
+static void flock_lanes_go(int kind, GroupView g, const unsigned* knn, unsigned k, OtherView o,
+                           FlockParams fp, cudaStream_t st) {
+    const unsigned nb = blocks_for(g.n, kLaneBlock / G);
+    if (kind == 0) k_flock_lanes<G, 0><<<nb, kLaneBlock, 0, st>>>(g, knn, k, o, fp);
+    else if (kind == 1) k_flock_lanes<G, 1><<<nb, kLaneBlock, 0, st>>>(g, knn, k, o, fp);
+    else k_flock_lanes<G, 2><<<nb, kLaneBlock, 0, st>>>(g, knn, k, o, fp);
+}
+void launch_flock_lanes(int kind, GroupView g, const unsigned* knn, unsigned k, OtherView o,
+                        FlockParams fp, cudaStream_t st) {
+    if (k <= 8) flock_lanes_go<8>(kind, g, knn, k, o, fp, st);
+    else if (k <= 16) flock_lanes_go<16>(kind, g, knn, k, o, fp, st);
+    else flock_lanes_go<32>(kind, g, knn, k, o, fp, st);
+}
+
+template <int G>
+static void avoid_lanes_go(GroupView g, const unsigned* knn, const float* knn_dist, unsigned k,
+                           OtherView o, float min_time, float min_sep, bool close, float w,
+                           unsigned mask, cudaStream_t st) {
+    const unsigned nb = blocks_for(g.n, kLaneBlock / G);
+    if (close)
+        k_avoid_lanes<G, true><<<nb, kLaneBlock, 0, st>>>(g, knn, knn_dist, k, o, min_sep, w, mask);
+    k_avoid_lanes<G, false><<<nb, kLaneBlock, 0, st>>>(g, knn, nullptr, k, o, min_time, w, mask);
+}
+void launch_avoid_lanes(GroupView g, const unsigned* knn, const float* knn_dist, unsigned k,
+                        OtherView o, float min_time, float min_sep, bool close, float w,
+                        unsigned mask, cudaStream_t st) {
+    if (k <= 8) avoid_lanes_go<8>(g, knn, knn_dist, k, o, min_time, min_sep, close, w, mask, st);
+    else if (k <= 16)
+        avoid_lanes_go<16>(g, knn, knn_dist, k, o, min_time, min_sep, close, w, mask, st);
+    else avoid_lanes_go<32>(g, knn, knn_dist, k, o, min_time, min_sep, close, w, mask, st);
+}
+
+void launch_avoid_walls_lanes(GroupView g, const unsigned* knw, unsigned kw, const float4* start,
+                              const float4* end, const float4* normal, unsigned n_lines,
+                              float min_time, float w, unsigned mask, cudaStream_t st) {
+    k_avoid_walls_lanes<8><<<blocks_for(g.n, kLaneBlock / 8), kLaneBlock, 0, st>>>(
+        g, knw, kw, start, end, normal, n_lines, min_time, w, mask);
+}
+
+// Under ncu, lanes / threads (us; a launch's floor is about 3): one flocking
+// behaviour, k = 7, 30,000 agents 7.5 / 6.5; k = 16, 10,000 6.5 / 11.3, 32,768
+// 10.2 / about 9.5.  The avoidance passes and the walls carry more arithmetic
+// per neighbour: k = 16, 10,000 7.5 / 16.7, 65,536 24 / about 24, k = 7 13.2 / 14.
+bool lanes_calls(unsigned n, unsigned k, bool avoid) {
+    return k <= 32 && n <= (avoid ? 65536u : 20000u);
+}
+
 template <int G, int R>
 static void launch_lanes_r(const FusedLaunch& L, const StepDev& p, unsigned nb, cudaStream_t st,
                            PhaseHook* hook) {

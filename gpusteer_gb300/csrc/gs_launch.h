@@ -110,6 +110,17 @@ gs_status launch_avoid_walls(GroupView g, const unsigned* knw, unsigned kw, cons
                              const float4* end, const float4* normal, unsigned n_lines,
                              float min_time, float w, unsigned mask, cudaStream_t st);
 gs_status launch_update(GroupView g, float dt, cudaStream_t st);
+// The same calls with a group of lanes per agent (gs_lanes.cu), for k <= 32
+// (kw <= 8); the launchers above take them where lanes_calls says so.
+bool lanes_calls(unsigned n, unsigned k, bool avoid);
+void launch_flock_lanes(int kind, GroupView g, const unsigned* knn, unsigned k, OtherView o,
+                        FlockParams fp, cudaStream_t st);
+void launch_avoid_lanes(GroupView g, const unsigned* knn, const float* knn_dist, unsigned k,
+                        OtherView o, float min_time, float min_sep, bool close, float w,
+                        unsigned mask, cudaStream_t st);
+void launch_avoid_walls_lanes(GroupView g, const unsigned* knw, unsigned kw, const float4* start,
+                              const float4* end, const float4* normal, unsigned n_lines,
+                              float min_time, float w, unsigned mask, cudaStream_t st);
 // MultiGroup (plugins/MultiGroup.cpp:558-601): one group's behaviour calls of
 // a frame in one pass, reading every group's current state and this group's
 // KNN lists against each of them.
