@@ -552,10 +552,8 @@ gs_status gs_group_destroy(gs_group g) {
     dfree(g->side);
     dfree(g->speed);
     db_release(g->db);
-    db_release(g->bf_a);
-    db_release(g->bf_b);
+    db_release(g->bf_db);
     dfree(g->bf_tmp);
-    dfree(g->bf_boxes);
     if (g->diag) cudaFree(g->diag);
     if (g->ap) cudaFree(g->ap);
     if (g->read_ev) cudaEventDestroy(g->read_ev);
@@ -1163,36 +1161,12 @@ gs_status gs_find_knn_walls(gs_group g, gs_knn out, gs_bins bins, gs_walls walls
     return GS_OK;
 }
 
-// A grid centred on the origin that covers every position of the other
-// group (largest |coordinate| per axis).  Its cell count per axis with extent
-// depends on n alone (about two agents per cell for an even spread), so a
-// moving crowd keeps the same database; only the cell size follows the
-// extent.  False when the extent is not finite.
-static bool brute_seed_grid(const float ext[3], unsigned n, Grid& grid, unsigned& C) {
-    double w[3], wmax = 0.0;
-    for (int a = 0; a < 3; ++a) {
-        if (!std::isfinite(ext[a])) return false;
-        w[a] = 2.0 * double(ext[a]) * 1.001 + 1e-6;
-        wmax = std::max(wmax, w[a]);
-    }
-    bool active[3];
-    int dims = 0;
-    for (int a = 0; a < 3; ++a) {
-        active[a] = w[a] > 1e-3 * wmax;
-        dims += active[a];
-    }
-    const double per_axis =
-        std::floor(std::pow(std::max(1.0, double(n) / 2.0), 1.0 / std::max(1, dims)));
-    unsigned long long cells = 1;
-    for (int a = 0; a < 3; ++a) {
-        grid.wc[a] = active[a] ? unsigned(std::min(std::max(per_axis, 1.0), 1024.0)) : 1u;
-        grid.ws[a] = float(w[a]);
-        cells *= grid.wc[a];
-    }
-    if (cells > (1ull << 22)) return false;
-    C = unsigned(cells);
-    return true;
-}
+// Queries from which brute force goes over cells; below, every pair is met.
+// Every pair / cells (us): k = 7, 500 queries 71 / 24, 4,096 92 / 31, 65,536
+// 180 / 80; k = 16, 500 94 / 23, 65,536 273 / 103; k = 40, 500 198 / 24, 65,536
+// 764 / 193 (from 4,096 on the former skipped chunks of bucketed candidates
+// beyond a seeded bound).
+constexpr unsigned kBruteCellsMin = 128;
 
 gs_status gs_knn_bruteforce(gs_group g, gs_knn out, gs_group other) {
     if (!g || !out || !other) return fail(GS_ERR_INVALID_ARG, "null argument");
@@ -1203,60 +1177,30 @@ gs_status gs_knn_bruteforce(gs_group g, gs_knn out, gs_group other) {
         GS_CUDA(cudaStreamSynchronize(other->stream));
     }
     cudaStream_t st = g->stream;
-    const float* seed = nullptr;
     g->bf_counted = false;
     g->bf_pairs = (unsigned long long)g->n * other->n;
-    // Seed every query's filter with the k-th distance among the candidates
-    // of its 3 x 3 x 3 cells on an automatic grid: the k-th distance among a
-    // subset of the candidates bounds the true one from above, so the full
-    // scan still sees every pair it needs and gives the same lists.  The
-    // scan then runs over the seed databases' bucketed arrays and skips
-    // chunks of candidates beyond every bound of a warp's queries.
-    if (g->n >= 4096 && other->n > out->k) {
-        if (!g->bf_tmp) GS_TRY(dalloc(&g->bf_tmp, 6));
-        float ext[3];
-        GS_TRY(abs_extent(other->position, other->n, g->bf_tmp, ext, st));
-        Grid grid;
-        unsigned C = 0;
-        if (brute_seed_grid(ext, other->n, grid, C)) {
-            Database& A = g->bf_a;
-            Database& B = other == g ? g->bf_a : g->bf_b;
-            GS_TRY(db_reserve(A, g->capacity, C));
-            GS_TRY(db_build(A, g->position, g->n, grid, st));
-            if (other != g) {
-                // sized for the other group's capacity (it may differ per call)
-                if (B.cell != nullptr && B.agent_cap < other->capacity) db_release(B);
-                GS_TRY(db_reserve(B, other->capacity, C));
-                B.agent_cap = other->capacity;
-                GS_TRY(db_build(B, other->position, other->n, grid, st));
-            }
-            // the seed goes to the k-th distance column, which the scan
-            // overwrites; a query whose box holds fewer than k candidates at
-            // every size tried starts unbounded (its block then takes the
-            // longest: it inserts most candidates of the first stages)
-            float* seed_col = out->dist + size_t(out->k - 1) * g->n;
-            GS_TRY(launch_brute_seed(A, g->n, B, other == g, out->k, seed_col, st));
-            seed = seed_col;
-            // chunk boxes of 64 candidates, then stage boxes of 32 chunks
-            const size_t chunks = (size_t(other->capacity) + 63) / 64;
-            const size_t boxes = chunks + (chunks + 31) / 32;
-            if (g->bf_boxes_cap < boxes) {
-                dfree(g->bf_boxes);
-                g->bf_boxes_cap = 0;
-                GS_TRY(dalloc(&g->bf_boxes, 2 * boxes));
-                g->bf_boxes_cap = boxes;
-            }
-            auto* evaluated = reinterpret_cast<unsigned long long*>(g->bf_tmp + 4);
-            GS_CUDA(cudaMemsetAsync(evaluated, 0, sizeof(unsigned long long), st));
-            GS_TRY(launch_knn_brute_bucketed(A.pos_id, g->n, B.pos_id, other->n, g->bf_boxes,
-                                             other == g, out->k, seed, evaluated, out->idx,
-                                             out->dist, st));
-            g->bf_counted = true;
-            return read_done(g, other);
+    if (g->n >= kBruteCellsMin && other->n > out->k) {
+        static_assert(sizeof(Grid) == 24, "bf_tmp layout");
+        if (!g->bf_tmp) GS_TRY(dalloc(&g->bf_tmp, 8));
+        // sized for the largest other group met so far
+        Database& B = g->bf_db;
+        const unsigned C = brute_cells(other->capacity, out->k);
+        if (B.cells < C || B.agent_cap < other->capacity) {
+            const unsigned cells = std::max(C, B.cells), cap = std::max(other->capacity, B.agent_cap);
+            GS_CUDA(cudaStreamSynchronize(st));
+            db_release(B);
+            GS_TRY(db_reserve(B, cap, cells));
+            B.agent_cap = cap;
         }
+        const BruteWork w{reinterpret_cast<Grid*>(g->bf_tmp),
+                          reinterpret_cast<unsigned long long*>(g->bf_tmp + 6)};
+        GS_TRY(launch_knn_brute_cells(g->position, g->n, other->position, other->n, other == g,
+                                      out->k, B, w, out->idx, out->dist, st));
+        g->bf_counted = true;
+        return read_done(g, other);
     }
     GS_TRY(launch_knn_brute(g->position, g->n, other->position, other->n, other == g, out->k,
-                            seed, out->idx, out->dist, st));
+                            out->idx, out->dist, st));
     return read_done(g, other);
 }
 
@@ -1264,7 +1208,7 @@ gs_status gs_knn_bruteforce_pairs(gs_group g, unsigned long long* pairs) {
     if (!g || !pairs) return fail(GS_ERR_INVALID_ARG, "null argument");
     *pairs = g->bf_pairs;
     if (!g->bf_counted) return GS_OK;
-    GS_CUDA(cudaMemcpyAsync(pairs, g->bf_tmp + 4, sizeof(unsigned long long),
+    GS_CUDA(cudaMemcpyAsync(pairs, g->bf_tmp + 6, sizeof(unsigned long long),
                             cudaMemcpyDeviceToHost, g->stream));
     GS_CUDA(cudaStreamSynchronize(g->stream));
     return GS_OK;

@@ -1,0 +1,220 @@
+// updateKNNDatabase for small groups: the whole counting sort in one launch.
+//
+// The rebuild's three passes (count, exclusive scan, scatter) each depend on
+// all of the one before, so over the whole chip they are five launches, about
+// 20 us whatever the size of a small group.  A cluster of 16 blocks on one GPC
+// runs them with hardware barriers between (no block waits on one that may not
+// be running: a cluster's blocks are resident together), and several groups'
+// databases are several clusters of one launch.
+#include <cooperative_groups.h>
+
+
+#include "gs_db.cuh"
+#include "gs_launch.h"
+
+namespace cg = cooperative_groups;
+
+namespace gs {
+
+constexpr unsigned kDbThreads = 1024;
+constexpr unsigned kDbCluster = 16;
+
+// Counts and starts are written by other SMs during the launch: read past L1.
+__device__ __forceinline__ uint4 load_counts(const unsigned* count, unsigned i, unsigned end) {
+    if (i + 4 <= end) return __ldcg(reinterpret_cast<const uint4*>(count + i));
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (i < end) v.x = __ldcg(count + i);
+    if (i + 1 < end) v.y = __ldcg(count + i + 1);
+    if (i + 2 < end) v.z = __ldcg(count + i + 2);
+    return v;
+}
+
+// Exclusive prefix of v over the block, and the block's total.
+__device__ __forceinline__ unsigned block_scan(unsigned v, unsigned* warp_sums, unsigned& total) {
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    unsigned x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= unsigned(o)) x += y;
+    }
+    if (lane == 31) warp_sums[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+        unsigned w = warp_sums[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= unsigned(o)) w += y;
+        }
+        warp_sums[lane] = w;
+    }
+    __syncthreads();
+    total = warp_sums[31];
+    const unsigned before = warp ? warp_sums[warp - 1] : 0u;
+    __syncthreads();
+    return before + x - v;
+}
+
+// A grid centred on the origin that covers every position (largest
+// |coordinate| per axis, as float bits): about two agents a cell over the
+// axes that have extent, one cell when a position is not finite.
+__device__ __forceinline__ Grid automatic_grid(const unsigned ext[3], const unsigned axis_cells[3]) {
+    Grid g;
+    float w[3], most = 0.f;
+    bool finite = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        finite = finite && ext[a] < 0x7e800000u;  // far enough below overflow to be doubled
+        w[a] = 2.002f * __uint_as_float(ext[a]) + 1e-6f;
+        most = fmaxf(most, w[a]);
+    }
+    int dims = 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) dims += w[a] > 1e-3f * most;
+    const unsigned cells = dims == 1 ? axis_cells[0] : dims == 2 ? axis_cells[1] : axis_cells[2];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        g.wc[a] = finite && w[a] > 1e-3f * most ? cells : 1u;
+        g.ws[a] = finite ? w[a] : 1.f;
+    }
+    return g;
+}
+
+__global__ void __launch_bounds__(kDbThreads) k_db_cluster(const __grid_constant__ DbJobs J) {
+    __shared__ unsigned ws[32];
+    __shared__ unsigned totals[kDbCluster], extents[kDbCluster][3];
+    cg::cluster_group cluster = cg::this_cluster();
+    const unsigned R = cluster.num_blocks(), rank = cluster.block_rank(), t = threadIdx.x;
+    const DbJob& j = J.job[blockIdx.x / R];
+    const unsigned first = rank * kDbThreads + t, step = R * kDbThreads, n = j.n;
+    Grid grid = j.grid;
+    if (first == 0 && j.zero) *j.zero = 0ull;
+    if (j.auto_axis[0]) {
+        unsigned m[3] = {0u, 0u, 0u};
+        for (unsigned i = first; i < n; i += step) {
+            const float4 p = j.pos[i];
+            m[0] = max(m[0], __float_as_uint(fabsf(p.x)));
+            m[1] = max(m[1], __float_as_uint(fabsf(p.y)));
+            m[2] = max(m[2], __float_as_uint(fabsf(p.z)));
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const unsigned w = __reduce_max_sync(0xffffffffu, m[a]);
+            if ((t & 31u) == 0) ws[t >> 5] = w;
+            __syncthreads();
+            const unsigned b = __reduce_max_sync(0xffffffffu, ws[t & 31u]);
+            if (t < R) cluster.map_shared_rank(&extents[0][0], t)[rank * 3 + a] = b;
+            __syncthreads();
+        }
+        cluster.sync();
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            m[a] = 0;
+            for (unsigned q = 0; q < R; ++q) m[a] = max(m[a], extents[q][a]);
+        }
+        grid = automatic_grid(m, j.auto_axis);
+        if (first == 0) *j.grid_out = grid;
+    }
+    const unsigned C = grid.wc[0] * grid.wc[1] * grid.wc[2];
+    for (unsigned i = first; i < n; i += step) {
+        V3 p = v3(j.pos[i]);
+        if (j.wrap_mode >= 0) {
+            p = wrap_world(p, j.wrap_ws, j.wrap_mode);
+            j.pos[i] = f4(p, 0.f);
+        }
+        const unsigned c = cell_of(grid, p);
+        j.cell[i] = c;
+        j.rank[i] = atomicAdd(j.count + c, 1u);
+        if (j.applied) j.applied[i] = 0u;
+    }
+    cluster.sync();
+    // this block's run of cells: its total, then its starts
+    const unsigned per = ((C + R - 1) / R + 3u) & ~3u;
+    const unsigned c0 = min(rank * per, C), c1 = min(c0 + per, C);
+    unsigned sum = 0;
+    for (unsigned i = c0 + 4 * t; i < c1; i += 4 * kDbThreads) {
+        const uint4 v = load_counts(j.count, i, c1);
+        sum += v.x + v.y + v.z + v.w;
+    }
+    unsigned total;
+    block_scan(sum, ws, total);
+    if (t < R) cluster.map_shared_rank(totals, t)[rank] = total;
+    cluster.sync();
+    unsigned base = 0;
+    for (unsigned q = 0; q < rank; ++q) base += totals[q];
+    for (unsigned b = c0; b < c1; b += 4 * kDbThreads) {
+        const unsigned i = b + 4 * t;
+        const uint4 v = load_counts(j.count, i, c1);
+        unsigned run = base + block_scan(v.x + v.y + v.z + v.w, ws, total);
+        const uint4 s = make_uint4(run, run + v.x, run + v.x + v.y, run + v.x + v.y + v.z);
+        if (i + 4 <= c1) {
+            *reinterpret_cast<uint4*>(j.start + i) = s;
+            *reinterpret_cast<uint4*>(j.count + i) = make_uint4(0u, 0u, 0u, 0u);
+        } else {
+            if (i < c1) {
+                j.start[i] = s.x;
+                j.count[i] = 0u;
+            }
+            if (i + 1 < c1) {
+                j.start[i + 1] = s.y;
+                j.count[i + 1] = 0u;
+            }
+            if (i + 2 < c1) {
+                j.start[i + 2] = s.z;
+                j.count[i + 2] = 0u;
+            }
+        }
+        base += total;
+    }
+    if (first == 0) j.start[C] = n;
+    cluster.sync();
+    for (unsigned i = first; i < n; i += step) {
+        const unsigned dst = __ldcg(j.start + j.cell[i]) + j.rank[i];
+        if (dst >= n) continue;
+        const float4 p = j.pos[i];
+        if (j.sorted) j.sorted[dst] = i;
+        j.pos_id[dst] = make_float4(p.x, p.y, p.z, __uint_as_float(i));
+    }
+}
+
+DbJob db_job(Database& db, const float4* pos, unsigned n, const Grid& grid) {
+    DbJob j;
+    std::memset(static_cast<void*>(&j), 0, sizeof(j));
+    j.pos = const_cast<float4*>(pos);  // written only when wrap_mode >= 0
+    j.n = n;
+    j.grid = grid;
+    j.wrap_mode = -1;
+    j.cell = db.cell;
+    j.rank = db.rank;
+    j.sorted = db.sorted;
+    j.start = db.start;
+    j.count = db.count;
+    j.pos_id = db.pos_id;
+    return j;
+}
+
+// Rebuild, cluster / five launches (us): 16,384 agents on 32,768 cells 10.6 /
+// 20.6, 32,768 on 64,000 14.4 / 20.6, 65,536 on 132,651 22.6 / 20.6.
+bool db_on_cluster(unsigned n, unsigned C) { return n <= 32768 && C <= 131072; }
+
+gs_status db_build_clusters(const DbJobs& J, unsigned count, cudaStream_t st) {
+    if (count == 0) return GS_OK;
+    if (count > kMaxDbJobs) return fail(GS_ERR_INVALID_ARG, "too many databases in one launch");
+    // 16 blocks a cluster is past the portable 8: allowed per kernel and device
+    GS_CUDA(cudaFuncSetAttribute(k_db_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kDbCluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kDbCluster * count);
+    cfg.blockDim = dim3(kDbThreads);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    GS_CUDA(cudaLaunchKernelEx(&cfg, k_db_cluster, J));
+    return GS_OK;
+}
+
+}  // namespace gs

@@ -155,14 +155,11 @@ struct gs_group_s {
     unsigned* knn_slot;    // [k * n] neighbour slots (wall phase)
     float* knn_dist;       // [k * n]
     gs::Database fdb;      // counts / starts of the fused step
-    // brute-force KNN's seed search: databases of the queries and of the
-    // other group on an automatic grid; scratch (words 0-2: the extent,
-    // words 4-5: the pairs the filter ran on); the candidates' chunk boxes
-    gs::Database bf_a, bf_b;
+    // brute-force KNN over cells: the other group's database on an automatic
+    // grid; scratch (words 0-5: that grid, words 6-7: the pairs met)
+    gs::Database bf_db;
     unsigned* bf_tmp;
-    float4* bf_boxes;
-    size_t bf_boxes_cap;         // boxes bf_boxes holds
-    bool bf_counted;             // the last call counted its pairs in bf_tmp
+    bool bf_counted;       // the last call counted its pairs in bf_tmp
     unsigned long long bf_pairs; // else the pairs it ran on (n * m)
     gs::Scene* d_scene;    // scene table (one entry for a plain group)
     unsigned scene_alloc;

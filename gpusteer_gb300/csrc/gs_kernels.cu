@@ -12,6 +12,7 @@
 #include <cstring>
 
 #include "gs_behaviours.cuh"
+#include "gs_db.cuh"
 #include "gs_knn.cuh"
 #include "gs_scan.cuh"
 
@@ -222,12 +223,19 @@ gs_status db_build(Database& db, const float4* pos, unsigned n, const Grid& grid
     const unsigned C = grid.wc[0] * grid.wc[1] * grid.wc[2];
     if (db.cells != C || (n > 0 && db.cell == nullptr))
         return fail(GS_ERR_STATE, "database not reserved for this grid");
-    if (n > 0) k_db_count<<<blocks_for(n), kBlock, 0, st>>>(pos, n, grid, db.cell, db.rank, db.count);
-    GS_TRY(scan_counts(db.count, db.start, C, db.tile, st));
-    if (n > 0)
-        k_db_scatter<<<blocks_for(n), kBlock, 0, st>>>(pos, n, db.cell, db.rank, db.start,
-                                                       db.sorted, db.pos_id);
-    GS_LAUNCHED("db_build");
+    if (n > 0 && db_on_cluster(n, C)) {
+        DbJobs J;
+        J.job[0] = db_job(db, pos, n, grid);
+        GS_TRY(db_build_clusters(J, 1, st));
+    } else {
+        if (n > 0)
+            k_db_count<<<blocks_for(n), kBlock, 0, st>>>(pos, n, grid, db.cell, db.rank, db.count);
+        GS_TRY(scan_counts(db.count, db.start, C, db.tile, st));
+        if (n > 0)
+            k_db_scatter<<<blocks_for(n), kBlock, 0, st>>>(pos, n, db.cell, db.rank, db.start,
+                                                           db.sorted, db.pos_id);
+        GS_LAUNCHED("db_build");
+    }
     db.grid = grid;
     db.valid = true;
     return GS_OK;
@@ -314,9 +322,8 @@ struct WarpList {
 // list); updates the filter bound.  Every lane runs it with the same
 // candidate.
 template <int L>
-__device__ __forceinline__ void warp_list_insert(WarpList<L>& w, float& bound, float seed_bound,
-                                                 V3 q, float x, float y, float z, unsigned id,
-                                                 unsigned k, unsigned lane) {
+__device__ __forceinline__ void warp_list_insert(WarpList<L>& w, float& bound, V3 q, float x, float y, float z, unsigned id, unsigned k,
+                                                 unsigned lane) {
     const unsigned long long key = knn_key(distance(q, v3(x, y, z)), id);
     if (!(key < w.kth(k))) return;  // warp-uniform
     const unsigned long long left0 = __shfl_up_sync(0xffffffffu, w.e[0], 1);
@@ -327,7 +334,7 @@ __device__ __forceinline__ void warp_list_insert(WarpList<L>& w, float& bound, f
         if (32 + lane < k && key < w.e[L - 1]) w.e[L - 1] = key > left1 ? key : left1;
     }
     if (lane < k && key < w.e[0]) w.e[0] = (lane == 0 || key > left0) ? key : left0;
-    bound = fminf(seed_bound, prefilter_bound(w.kth(k)));
+    bound = prefilter_bound(w.kth(k));
 }
 
 // Writes a warp list to idx / dist[a + rank * nA], ranks below k.
@@ -346,23 +353,16 @@ __device__ __forceinline__ void warp_list_store(const WarpList<L>& w, unsigned a
     }
 }
 
-// Rounded-up filter bound for a known upper bound d of the k-th distance.
-__device__ __forceinline__ float seed_prefilter(float d) {
-    return __fmul_ru(__fmul_ru(d, d), 1.000004f);
-}
-
 // The warp's step over the staged candidates t0 .. t0 + 63 (each lane the
 // pair t0 + 2 lane, t0 + 2 lane + 1): the packed filter against every query
-// of the warp, then the exact insertion of the candidates that passed.  sid:
-// the staged candidates' indices (null: base + their position in the stage).
+// of the warp, then the exact insertion of the candidates that passed.
 template <int L>
 __device__ __forceinline__ void brute_chunk(
-    const float* sx, const float* sy, const float* sz, const unsigned* sid, unsigned base,
-    unsigned t0, unsigned cnt, unsigned lane, bool self, unsigned k, const V3 (&q)[kBruteQW],
+    const float* sx, const float* sy, const float* sz, unsigned base, unsigned t0, unsigned cnt,
+    unsigned lane, bool self, unsigned k, const V3 (&q)[kBruteQW],
     const unsigned (&qid)[kBruteQW], const unsigned long long (&px)[kBruteQW],
     const unsigned long long (&py)[kBruteQW], const unsigned long long (&pz)[kBruteQW],
-    WarpList<L> (&entry)[kBruteQW], float (&bound)[kBruteQW],
-    const float (&seed_bound)[kBruteQW]) {
+    WarpList<L> (&entry)[kBruteQW], float (&bound)[kBruteQW]) {
     const unsigned t = t0 + 2 * lane;
     const unsigned long long x2 = *reinterpret_cast<const unsigned long long*>(sx + t);
     const unsigned long long y2 = *reinterpret_cast<const unsigned long long*>(sy + t);
@@ -391,24 +391,18 @@ __device__ __forceinline__ void brute_chunk(
                 m &= m - 1u;
                 const unsigned c = t0 + 2 * src + h;
                 if (c >= cnt) continue;
-                const unsigned id = sid ? sid[c] : base + c;
+                const unsigned id = base + c;
                 if (self && id == qid[j]) continue;
-                warp_list_insert(entry[j], bound[j], seed_bound[j], q[j], sx[c], sy[c], sz[c],
-                                 id, k, lane);
+                warp_list_insert(entry[j], bound[j], q[j], sx[c], sy[c], sz[c], id, k, lane);
             }
         }
     }
 }
 
-// seed (may be null): per query an upper bound of its k-th distance (the
-// k-th distance among any subset of the candidates is one); the filter then
-// starts at that bound instead of infinity, so a query's list takes little
-// more than its k final entries.
 template <int L>
 __global__ void __launch_bounds__(kBruteWarps * 32) k_knn_brute3(
     const float4* __restrict__ posA, unsigned nA, const float4* __restrict__ posB, unsigned nB,
-    bool self, unsigned k, const float* __restrict__ seed, unsigned* __restrict__ idx,
-    float* __restrict__ dist) {
+    bool self, unsigned k, unsigned* __restrict__ idx, float* __restrict__ dist) {
     __shared__ __align__(16) float sx[kBruteTile], sy[kBruteTile], sz[kBruteTile];
     const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned q0 = (blockIdx.x * kBruteWarps + warp) * kBruteQW;
@@ -416,7 +410,7 @@ __global__ void __launch_bounds__(kBruteWarps * 32) k_knn_brute3(
     unsigned qid[kBruteQW];
     unsigned long long px[kBruteQW], py[kBruteQW], pz[kBruteQW];
     WarpList<L> entry[kBruteQW];
-    float bound[kBruteQW], seed_bound[kBruteQW];
+    float bound[kBruteQW];
 #pragma unroll
     for (unsigned j = 0; j < kBruteQW; ++j) {
         const bool act = q0 + j < nA;
@@ -426,8 +420,7 @@ __global__ void __launch_bounds__(kBruteWarps * 32) k_knn_brute3(
         py[j] = pack2(q[j].y, q[j].y);
         pz[j] = pack2(q[j].z, q[j].z);
         entry[j].init();
-        seed_bound[j] = (act && seed) ? seed_prefilter(seed[q0 + j]) : prefilter_bound(KEY_EMPTY);
-        bound[j] = act ? seed_bound[j] : -1.f;
+        bound[j] = act ? prefilter_bound(KEY_EMPTY) : -1.f;
     }
     const float inf = __int_as_float(0x7f800000);
     for (unsigned base = 0; base < nB; base += kBruteTile) {
@@ -441,342 +434,24 @@ __global__ void __launch_bounds__(kBruteWarps * 32) k_knn_brute3(
         __syncthreads();
         const unsigned cnt = min(kBruteTile, nB - base);
         for (unsigned t0 = 0; t0 < cnt; t0 += 64)
-            brute_chunk(sx, sy, sz, nullptr, base, t0, cnt, lane, self, k, q, qid, px, py, pz,
-                        entry, bound, seed_bound);
+            brute_chunk(sx, sy, sz, base, t0, cnt, lane, self, k, q, qid, px, py, pz, entry, bound);
     }
 #pragma unroll
     for (unsigned j = 0; j < kBruteQW; ++j)
         if (q0 + j < nA) warp_list_store(entry[j], q0 + j, nA, k, lane, idx, dist);
 }
 
-// ---- brute force over bucketed candidates: chunks beyond every bound skipped ---------
-// With the seed's databases, queries and candidates are taken in bucket
-// order (the cell-sorted pos_id arrays: position and agent index), so a
-// warp's queries are neighbours and 64 consecutive candidates (a chunk) sit
-// in a few neighbouring cells.  Before each stage a lane tests one of the
-// stage's 32 chunks: the squared distance from each query of its warp to the
-// chunk's bounding box, in the reference's unfused operations.  Per axis the
-// gap to the box is fl(lo - q) or fl(q - hi), at most |fl(q - c)| for every
-// candidate c of the chunk (rounding is monotone), and squares and sums are
-// monotone too, so the box's squared distance is at most every candidate's
-// exact one: a chunk whose box lies beyond the filter bound of every query of
-// the warp holds no candidate the filter would pass, and the warp skips it
-// without changing a list.  The block stages only the chunks some warp needs.
-
-// Bounding box of each chunk of 64 consecutive slots: boxes[2c] = lower
-// corner, boxes[2c + 1] = upper corner (NaN coordinates ignored: such a
-// candidate's distance is NaN and never passes the filter).  With `merge`,
-// pos_id holds n such boxes and each output box covers 32 of them (a stage
-// of kBruteTile candidates).  One warp per output box.
-__global__ void k_chunk_boxes(const float4* __restrict__ pos_id, unsigned n, bool merge,
-                              float4* __restrict__ boxes) {
-    const unsigned c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    const unsigned per = merge ? 32u : 64u;
-    if (c >= (n + per - 1) / per) return;  // warp-uniform
-    const float inf = __int_as_float(0x7f800000);
-    float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
-    if (merge) {
-        const unsigned b = c * 32 + lane;
-        if (b < n) {
-            const float4 l = pos_id[2 * b], h = pos_id[2 * b + 1];
-            lo[0] = l.x;
-            lo[1] = l.y;
-            lo[2] = l.z;
-            hi[0] = h.x;
-            hi[1] = h.y;
-            hi[2] = h.z;
-        }
-    } else {
-#pragma unroll
-        for (unsigned h = 0; h < 2; ++h) {
-            const unsigned sl = c * 64 + 2 * lane + h;
-            if (sl < n) {
-                const float4 v = pos_id[sl];
-                lo[0] = fminf(lo[0], v.x);
-                lo[1] = fminf(lo[1], v.y);
-                lo[2] = fminf(lo[2], v.z);
-                hi[0] = fmaxf(hi[0], v.x);
-                hi[1] = fmaxf(hi[1], v.y);
-                hi[2] = fmaxf(hi[2], v.z);
-            }
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-        }
-    }
-    if (lane == 0) {
-        boxes[2 * c] = make_float4(lo[0], lo[1], lo[2], 0.f);
-        boxes[2 * c + 1] = make_float4(hi[0], hi[1], hi[2], 0.f);
-    }
-}
-
-// The scan's seed: per query (one thread each, in bucket order, so that
-// neighbouring threads read the same cells) the k-th smallest distance among
-// the other group's candidates in its 3 x 3 x 3 cells; in its 5 x 5 x 5, then
-// 9 x 9 x 9 cells when the smaller box holds fewer than k (grid corners and
-// edges); FLT_MAX when even that box does.  The k-th distance among a subset
-// of the candidates is at least the k-th among all of them, and an upper
-// bound is all the filter needs, so no list is kept: the k smallest squared
-// distances (the reference's unfused sum) stay in registers and one square
-// root is taken at the end (correctly rounded square roots keep their
-// order).  Candidates at an infinite or NaN distance never enter a list and
-// are not counted.  seed[a] by agent index.
-template <int KMAX>
-__global__ void __launch_bounds__(kBlock) k_brute_seed(const float4* __restrict__ a_pos_id,
-                                                       unsigned nA,
-                                                       const unsigned* __restrict__ b_start,
-                                                       const float4* __restrict__ b_pos_id,
-                                                       Grid g, unsigned k, bool self,
-                                                       float* __restrict__ seed) {
-    const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nA) return;
-    const float4 v = a_pos_id[s];
-    const unsigned a = __float_as_uint(v.w);
-    if (a >= nA) return;
-    const V3 p = v3(v);
-    unsigned ix, iy, iz;
-    cell_coords(g, p, ix, iy, iz);
-    const float inf = __int_as_float(0x7f800000);
-    float kth = FLT_MAX;
-    for (unsigned r = 1; r <= 4; r *= 2) {
-        // the k smallest in top[KMAX - k .. KMAX - 1], ascending; the slots
-        // below hold -1 (below every distance) and never change
-        float top[KMAX];
-#pragma unroll
-        for (int i = 0; i < KMAX; ++i) top[i] = i < KMAX - int(k) ? -1.f : inf;
-        unsigned found = 0;
-        const Box b = cell_box(g, ix, iy, iz, r);
-        for (unsigned cy = b.y0; cy <= b.y1; ++cy) {
-            for (unsigned cz = b.z0; cz <= b.z1; ++cz) {
-                const unsigned s0 = __ldg(b_start + cell_label(g, b.x0, cy, cz));
-                const unsigned s1 = __ldg(b_start + cell_label(g, b.x1, cy, cz) + 1);
-                for (unsigned t = s0; t < s1; ++t) {
-                    const float4 q = __ldg(b_pos_id + t);
-                    if (self && __float_as_uint(q.w) == a) continue;
-                    const V3 o = sub(p, v3(q));
-                    const float d2 = dot(o, o);
-                    if (!(d2 < inf)) continue;
-                    ++found;
-                    if (d2 < top[KMAX - 1]) {
-#pragma unroll
-                        for (int i = KMAX - 1; i > 0; --i)
-                            top[i] = fminf(top[i], fmaxf(top[i - 1], d2));
-                        top[0] = fminf(top[0], d2);
-                    }
-                }
-            }
-        }
-        if (found >= k) {
-            kth = sqrtf(top[KMAX - 1]);
-            break;
-        }
-    }
-    seed[a] = kth;
-}
-
-gs_status launch_brute_seed(const Database& A, unsigned nA, const Database& B, bool self,
-                            unsigned k, float* seed, cudaStream_t st) {
-    if (nA == 0) return GS_OK;
-    if (k == 0 || k > 64)
-        return fail(GS_ERR_UNSUPPORTED, "the brute-force seed needs 1 <= k <= 64");
-    if (k <= 8)
-        k_brute_seed<8><<<blocks_for(nA), kBlock, 0, st>>>(A.pos_id, nA, B.start, B.pos_id, B.grid,
-                                                           k, self, seed);
-    else if (k <= 16)
-        k_brute_seed<16><<<blocks_for(nA), kBlock, 0, st>>>(A.pos_id, nA, B.start, B.pos_id,
-                                                            B.grid, k, self, seed);
-    else if (k <= 32)
-        k_brute_seed<32><<<blocks_for(nA), kBlock, 0, st>>>(A.pos_id, nA, B.start, B.pos_id,
-                                                            B.grid, k, self, seed);
-    else
-        k_brute_seed<64><<<blocks_for(nA), kBlock, 0, st>>>(A.pos_id, nA, B.start, B.pos_id,
-                                                            B.grid, k, self, seed);
-    GS_LAUNCHED("brute_seed");
-    return GS_OK;
-}
-
-// Squared distance from q to the box [lo, hi], as a lower bound of every
-// inside candidate's exact squared distance (same operation order as dot).
-__device__ __forceinline__ float box_dist_sq(V3 q, float4 lo, float4 hi) {
-    const V3 gap = v3(fmaxf(fmaxf(lo.x - q.x, q.x - hi.x), 0.f),
-                      fmaxf(fmaxf(lo.y - q.y, q.y - hi.y), 0.f),
-                      fmaxf(fmaxf(lo.z - q.z, q.z - hi.z), 0.f));
-    return dot(gap, gap);
-}
-
-// qpos / cpos: the queries' and candidates' bucketed (position, agent index)
-// arrays; seed: per agent index an upper bound of its k-th distance; the
-// lists go to idx / dist by agent index.  evaluated (may be null): adds the
-// (query, candidate) pairs the packed filter ran on.
-// sboxes: the boxes of the stages (32 chunks each), tested first, 32 stages
-// at a time, so that a block visits only the stages some query may need.
-template <int L>
-__global__ void __launch_bounds__(kBruteWarps * 32) k_knn_brute3_bucketed(
-    const float4* __restrict__ qpos, unsigned nA, const float4* __restrict__ cpos, unsigned nB,
-    const float4* __restrict__ boxes, const float4* __restrict__ sboxes, bool self, unsigned k,
-    const float* __restrict__ seed, unsigned long long* __restrict__ evaluated,
-    unsigned* __restrict__ idx, float* __restrict__ dist) {
-    __shared__ __align__(16) float sx[kBruteTile], sy[kBruteTile], sz[kBruteTile];
-    __shared__ unsigned sid[kBruteTile];
-    __shared__ unsigned wmask[kBruteWarps], smask[kBruteWarps];
-    const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned s0 = (blockIdx.x * kBruteWarps + warp) * kBruteQW;
-    V3 q[kBruteQW];
-    unsigned qid[kBruteQW];
-    unsigned long long px[kBruteQW], py[kBruteQW], pz[kBruteQW];
-    WarpList<L> entry[kBruteQW];
-    float bound[kBruteQW], seed_bound[kBruteQW];
-    unsigned active = 0;
-#pragma unroll
-    for (unsigned j = 0; j < kBruteQW; ++j) {
-        const float4 v = s0 + j < nA ? qpos[s0 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
-        qid[j] = s0 + j < nA ? __float_as_uint(v.w) : UINT_MAX;
-        const bool act = qid[j] < nA;  // a slot holds an agent index below nA
-        active += act;
-        q[j] = v3(v);
-        px[j] = pack2(q[j].x, q[j].x);
-        py[j] = pack2(q[j].y, q[j].y);
-        pz[j] = pack2(q[j].z, q[j].z);
-        entry[j].init();
-        seed_bound[j] = act ? seed_prefilter(seed[qid[j]]) : prefilter_bound(KEY_EMPTY);
-        bound[j] = act ? seed_bound[j] : -1.f;
-    }
-    const float inf = __int_as_float(0x7f800000);
-    const unsigned chunks = (nB + 63) / 64, stages = (nB + kBruteTile - 1) / kBruteTile;
-    for (unsigned sg = 0; sg < stages; sg += 32) {
-        // lane l: may stage sg + l hold a candidate some query of the warp
-        // would pass?  (bounds only fall, so the answer stays safe)
-        bool swant = false;
-        if (sg + lane < stages) {
-            const float4 lo = sboxes[2 * (sg + lane)], hi = sboxes[2 * (sg + lane) + 1];
-#pragma unroll
-            for (unsigned j = 0; j < kBruteQW; ++j) swant |= box_dist_sq(q[j], lo, hi) <= bound[j];
-        }
-        const unsigned sm = __ballot_sync(0xffffffffu, swant);
-        __syncthreads();  // the previous group's reads of smask are done
-        if (lane == 0) smask[warp] = sm;
-        __syncthreads();
-        unsigned visit = 0;
-#pragma unroll
-        for (unsigned w = 0; w < kBruteWarps; ++w) visit |= smask[w];
-        for (; visit; visit &= visit - 1u) {
-            const unsigned base = (sg + unsigned(__ffs(visit)) - 1u) * kBruteTile;
-            // lane l: may chunk base / 64 + l hold a candidate some query of the
-            // warp would pass?  (bounds only fall within the stage)
-            const unsigned ch = base / 64 + lane;
-            bool want = false;
-            if (ch < chunks) {
-                const float4 lo = boxes[2 * ch], hi = boxes[2 * ch + 1];
-#pragma unroll
-                for (unsigned j = 0; j < kBruteQW; ++j)
-                    want |= box_dist_sq(q[j], lo, hi) <= bound[j];
-            }
-            const unsigned mask = __ballot_sync(0xffffffffu, want);
-            __syncthreads();  // the previous stage's reads of the staged chunks are done
-            if (lane == 0) wmask[warp] = mask;
-            __syncthreads();
-            unsigned need = 0;
-#pragma unroll
-            for (unsigned w = 0; w < kBruteWarps; ++w) need |= wmask[w];
-            if (need == 0) continue;  // block-uniform
-            for (unsigned c = threadIdx.x; c < kBruteTile; c += blockDim.x) {
-                if (!((need >> (c / 64)) & 1u)) continue;
-                const float4 v =
-                    base + c < nB ? cpos[base + c] : make_float4(inf, inf, inf, 0.f);
-                sx[c] = v.x;
-                sy[c] = v.y;
-                sz[c] = v.z;
-                sid[c] = __float_as_uint(v.w);
-            }
-            __syncthreads();
-            if (evaluated && lane == 0 && mask)
-                atomicAdd(evaluated, (unsigned long long)__popc(mask) * 64u * active);
-            const unsigned cnt = min(kBruteTile, nB - base);
-            for (unsigned m = mask; m; m &= m - 1u)
-                brute_chunk(sx, sy, sz, sid, base, 64u * (unsigned(__ffs(m)) - 1u), cnt, lane,
-                            self, k, q, qid, px, py, pz, entry, bound, seed_bound);
-        }
-    }
-#pragma unroll
-    for (unsigned j = 0; j < kBruteQW; ++j)
-        if (qid[j] < nA) warp_list_store(entry[j], qid[j], nA, k, lane, idx, dist);
-}
-
-gs_status launch_knn_brute_bucketed(const float4* qpos, unsigned nA, const float4* cpos,
-                                    unsigned nB, float4* boxes, bool self, unsigned k,
-                                    const float* seed, unsigned long long* evaluated,
-                                    unsigned* idx, float* dist, cudaStream_t st) {
-    if (nA == 0) return GS_OK;
-    if (k == 0 || k > 64 || seed == nullptr)
-        return fail(GS_ERR_UNSUPPORTED, "the bucketed brute force needs 1 <= k <= 64 and a seed");
-    const unsigned chunks = (nB + 63) / 64, stages = (chunks + 31) / 32;
-    float4* sboxes = boxes + 2 * size_t(chunks);
-    if (chunks) {
-        k_chunk_boxes<<<(chunks * 32 + kBlock - 1) / kBlock, kBlock, 0, st>>>(cpos, nB, false,
-                                                                               boxes);
-        k_chunk_boxes<<<(stages * 32 + kBlock - 1) / kBlock, kBlock, 0, st>>>(boxes, chunks, true,
-                                                                               sboxes);
-    }
-    const unsigned per_block = kBruteWarps * kBruteQW, blocks = (nA + per_block - 1) / per_block;
-    if (k <= 32)
-        k_knn_brute3_bucketed<1><<<blocks, kBruteWarps * 32, 0, st>>>(
-            qpos, nA, cpos, nB, boxes, sboxes, self, k, seed, evaluated, idx, dist);
-    else
-        k_knn_brute3_bucketed<2><<<blocks, kBruteWarps * 32, 0, st>>>(
-            qpos, nA, cpos, nB, boxes, sboxes, self, k, seed, evaluated, idx, dist);
-    GS_LAUNCHED("knn_brute_bucketed");
-    return GS_OK;
-}
-
-// Largest |coordinate| per axis of n positions, as float bits (non-negative
-// floats order like their bits), into out[0..2] (zeroed by the caller).
-__global__ void k_abs_extent(const float4* __restrict__ pos, unsigned n, unsigned* out) {
-    unsigned m[3] = {0u, 0u, 0u};
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 p = pos[i];
-        m[0] = max(m[0], __float_as_uint(fabsf(p.x)));
-        m[1] = max(m[1], __float_as_uint(fabsf(p.y)));
-        m[2] = max(m[2], __float_as_uint(fabsf(p.z)));
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m[a] = max(m[a], __shfl_down_sync(0xffffffffu, m[a], o));
-        if ((threadIdx.x & 31) == 0) atomicMax(out + a, m[a]);
-    }
-}
-
-gs_status abs_extent(const float4* pos, unsigned n, unsigned* d_tmp3, float out[3],
-                     cudaStream_t st) {
-    unsigned h[3] = {0u, 0u, 0u};
-    GS_CUDA(cudaMemsetAsync(d_tmp3, 0, 3 * sizeof(unsigned), st));
-    if (n > 0) {
-        k_abs_extent<<<std::min(blocks_for(n), 4u * 152u), kBlock, 0, st>>>(pos, n, d_tmp3);
-        GS_LAUNCHED("abs_extent");
-    }
-    GS_CUDA(cudaMemcpyAsync(h, d_tmp3, sizeof(h), cudaMemcpyDeviceToHost, st));
-    GS_CUDA(cudaStreamSynchronize(st));
-    for (int a = 0; a < 3; ++a) std::memcpy(&out[a], &h[a], 4);
-    return GS_OK;
-}
-
 gs_status launch_knn_brute(const float4* posA, unsigned nA, const float4* posB, unsigned nB,
-                           bool self, unsigned k, const float* seed, unsigned* idx, float* dist,
-                           cudaStream_t st) {
+                           bool self, unsigned k, unsigned* idx, float* dist, cudaStream_t st) {
     if (nA == 0) return GS_OK;
     if (k == 0 || k > 64) return fail(GS_ERR_UNSUPPORTED, "brute force needs 1 <= k <= 64");
     const unsigned per_block = kBruteWarps * kBruteQW, blocks = (nA + per_block - 1) / per_block;
     if (k <= 32)
-        k_knn_brute3<1><<<blocks, kBruteWarps * 32, 0, st>>>(posA, nA, posB, nB, self, k, seed,
-                                                             idx, dist);
+        k_knn_brute3<1><<<blocks, kBruteWarps * 32, 0, st>>>(posA, nA, posB, nB, self, k, idx,
+                                                             dist);
     else
-        k_knn_brute3<2><<<blocks, kBruteWarps * 32, 0, st>>>(posA, nA, posB, nB, self, k, seed,
-                                                             idx, dist);
+        k_knn_brute3<2><<<blocks, kBruteWarps * 32, 0, st>>>(posA, nA, posB, nB, self, k, idx,
+                                                             dist);
     GS_LAUNCHED("knn_brute");
     return GS_OK;
 }

@@ -52,26 +52,19 @@ struct KnnPairs {
     unsigned r, n_pairs;
 };
 gs_status launch_knn_binned_pairs(KnnPairs& P, cudaStream_t st);
-// seed (may be null): per query of A an upper bound of its k-th distance.
 gs_status launch_knn_brute(const float4* posA, unsigned nA, const float4* posB, unsigned nB,
-                           bool self, unsigned k, const float* seed, unsigned* idx, float* dist,
-                           cudaStream_t st);
-// Per query of A (by agent index) an upper bound of its k-th distance to B's
-// agents: the k-th among the candidates of a box of cells (1 <= k <= 64).
-gs_status launch_brute_seed(const Database& A, unsigned nA, const Database& B, bool self,
-                            unsigned k, float* seed, cudaStream_t st);
-// The same lists over bucketed queries and candidates (the seed databases'
-// pos_id arrays), skipping chunks of 64 candidates beyond every bound of a
-// warp's queries; k <= 64 and a seed.  boxes: 2 * (ceil(nB / 64) +
-// ceil(nB / 2048)) float4 of scratch (chunk, then stage boxes); evaluated
-// (may be null) adds the pairs the filter ran on.
-gs_status launch_knn_brute_bucketed(const float4* qpos, unsigned nA, const float4* cpos,
-                                    unsigned nB, float4* boxes, bool self, unsigned k,
-                                    const float* seed, unsigned long long* evaluated,
-                                    unsigned* idx, float* dist, cudaStream_t st);
-// Largest |coordinate| per axis of n positions (synchronises st); d_tmp3: 3 words.
-gs_status abs_extent(const float4* pos, unsigned n, unsigned* d_tmp3, float out[3],
-                     cudaStream_t st);
+                           bool self, unsigned k, unsigned* idx, float* dist, cudaStream_t st);
+// The same lists from the cells that can hold them (gs_brute.cu): B is a
+// database reserved for nB agents and brute_cells(nB, k) cells, `evaluated`
+// receives the (query, candidate) pairs met.
+struct BruteWork {
+    Grid* grid;
+    unsigned long long* evaluated;
+};
+unsigned brute_cells(unsigned n, unsigned k);
+gs_status launch_knn_brute_cells(const float4* posA, unsigned nA, const float4* posB, unsigned nB,
+                                 bool self, unsigned k, Database& B, const BruteWork& w,
+                                 unsigned* idx, float* dist, cudaStream_t st);
 gs_status launch_wrap(float4* pos, unsigned n, const float ws[3], int mode, cudaStream_t st);
 gs_status launch_cell_density(const Database& db, unsigned* out, cudaStream_t st);
 gs_status launch_cell_avg_velocity(const Database& db, const float4* dir, const float* speed,
