@@ -9,6 +9,7 @@
 #include <new>
 #include <string>
 
+#include "gs_db.cuh"
 #include "gs_launch.h"
 
 namespace gs {
@@ -1038,6 +1039,7 @@ gs_status gs_find_knn_groups(const gs_group* groups, unsigned n_groups, gs_bins 
 
 static gs_status antipen_enqueue(gs_group g, gs_knn knn, gs_group other, unsigned mask,
                                  cudaStream_t st);
+static gs_status group_scratch(gs_group g, size_t bytes, cudaStream_t st);
 
 gs_status gs_multigroup_step(const gs_group* groups, unsigned n_groups, gs_bins bins,
                              const gs_path* paths, gs_knn* knn, const gs_multigroup_params* p,
@@ -1071,13 +1073,27 @@ gs_status gs_multigroup_step(const gs_group* groups, unsigned n_groups, gs_bins 
         GS_TRY(db_reserve(groups[i]->db, groups[i]->capacity, bins->cells));
     }
     for (unsigned step = 0; step < steps; ++step) {
-        // Group::preUpdate for every group (MultiGroup.cpp:545-556)
+        // Group::preUpdate for every group (MultiGroup.cpp:545-556): small
+        // groups' wraps, databases and cleared bits in one launch
+        DbJobs J;
+        unsigned jobs = 0;
         for (unsigned i = 0; i < G; ++i) {
             gs_group g = groups[i];
+            if (db_on_cluster(g->n, bins->cells)) {
+                DbJob& job = J.job[jobs++];
+                job = db_job(g->db, g->position, g->n, bins->grid);
+                job.wrap_mode = p->wrap_mode;
+                std::memcpy(job.wrap_ws, p->world_size, sizeof(job.wrap_ws));
+                job.applied = g->applied;
+                g->db.grid = bins->grid;
+                g->db.valid = true;
+                continue;
+            }
             GS_TRY(launch_wrap(g->position, g->n, p->world_size, p->wrap_mode, st));
             GS_TRY(db_build(g->db, g->position, g->n, bins->grid, st));
             if (g->n) GS_CUDA(cudaMemsetAsync(g->applied, 0, size_t(g->n) * 4, st));
         }
+        GS_TRY(db_build_clusters(J, jobs, st));
         // every pair's KNN reads only those databases: one launch (:561-564)
         KnnPairs P;
         GS_TRY(knn_pairs(groups, G, bins, knn, P));
@@ -1116,6 +1132,17 @@ gs_status gs_multigroup_step(const gs_group* groups, unsigned n_groups, gs_bins 
                 M.w_seek = p->w_seek;
                 M.mask_seek = p->mask_seek;
                 for (int c = 0; c < 3; ++c) M.seek_target[c] = P_i->h_points[3 + c];
+            }
+            M.dt = p->dt;
+            M.mask_antipen = p->mask_antipen;
+            if (lanes_multigroup(M)) {
+                GS_TRY(group_scratch(g, size_t(g->n) * kGroupNextBytes, st));
+                M.next.position = static_cast<float4*>(g->ap);
+                M.next.direction = M.next.position + g->n;
+                M.next.speed = reinterpret_cast<float*>(M.next.direction + g->n);
+                M.next.applied = reinterpret_cast<unsigned*>(M.next.speed + g->n);
+                GS_TRY(launch_group_frame(M, st));
+                continue;
             }
             GS_TRY(launch_multigroup_steer(M, st));
             GS_TRY(launch_update(view(g), p->dt, st));
@@ -1492,18 +1519,23 @@ gs_status gs_anti_penetration_wall(gs_group g, gs_knn knw, gs_walls walls, float
 // AntiPenetrationAgentsCUDA does): the new positions, then a snapshot of the
 // other group's bits.  Queued on st; the groups' earlier work must be complete
 // or on st.
+// At least `bytes` of scratch in g->ap; grows after the work queued on st.
+static gs_status group_scratch(gs_group g, size_t bytes, cudaStream_t st) {
+    if (g->ap_bytes >= bytes) return GS_OK;
+    GS_CUDA(cudaStreamSynchronize(st));
+    if (g->ap) cudaFree(g->ap);
+    g->ap = nullptr;
+    g->ap_bytes = 0;
+    GS_CUDA(cudaMalloc(&g->ap, bytes));
+    g->ap_bytes = bytes;
+    return GS_OK;
+}
+
 static gs_status antipen_enqueue(gs_group g, gs_knn knn, gs_group other, unsigned mask,
                                  cudaStream_t st) {
     if (g->n == 0) return GS_OK;
     const size_t pos_bytes = size_t(g->n) * 16, snap_bytes = size_t(other->n ? other->n : 1) * 4;
-    if (g->ap_bytes < pos_bytes + snap_bytes) {
-        GS_CUDA(cudaStreamSynchronize(st));
-        if (g->ap) cudaFree(g->ap);
-        g->ap = nullptr;
-        g->ap_bytes = 0;
-        GS_CUDA(cudaMalloc(&g->ap, pos_bytes + snap_bytes));
-        g->ap_bytes = pos_bytes + snap_bytes;
-    }
+    GS_TRY(group_scratch(g, pos_bytes + snap_bytes, st));
     float4* pos_out = static_cast<float4*>(g->ap);
     unsigned* snap = reinterpret_cast<unsigned*>(static_cast<char*>(g->ap) + pos_bytes);
     if (other->n)

@@ -399,6 +399,147 @@ void launch_avoid_walls_lanes(GroupView g, const unsigned* knw, unsigned kw, con
         g, knw, kw, start, end, normal, n_lines, min_time, w, mask);
 }
 
+// ---- MultiGroup frames ------------------------------------------------------------------------
+// One group's part of a frame (Group::update, plugins/MultiGroup.cpp:558-610) in
+// two launches instead of one for steering, one for the update and three for
+// each group's anti-penetration: 72 launches and copies a frame of three groups
+// took 400 us, almost all of it between kernels.
+//
+// The first: steering as k_multigroup_steer (each list gathered once, lane r
+// its entry r), the update, and anti-penetration against the groups before
+// this one, whose agents have moved.  Other agents of this group read its
+// position, heading and speed of before the update meanwhile, so the new ones
+// go to M.next.
+__device__ __forceinline__ void push_apart(V3& pos, unsigned& applied, float radius, unsigned b,
+                                           float knn_dist, const OtherView& o,
+                                           const float4* o_pos, const unsigned* o_applied,
+                                           unsigned mask) {
+    // AntiPenetrationAgentsCUDAKernel.cu:72-108, as k_antipen
+    if ((applied & mask) || b >= o.n) return;
+    const float overlap = radius + o.radius[b] - knn_dist;
+    if (overlap < 0.f) return;
+    const V3 unit = normalize(sub(pos, v3(o_pos[b])));
+    pos = add(pos, mul(unit, (o_applied[b] & mask) ? overlap : 0.5f * overlap));
+    applied |= ANTI_PENETRATION_AGENT;
+}
+
+template <int G>
+__global__ void __launch_bounds__(kLaneBlock) k_group_move(const __grid_constant__ MultiSteer M) {
+    __shared__ __align__(16) float sh[kLaneBlock / G * LaneSums<G>::kWords];
+    const GroupView& g = M.g;
+    unsigned a, lane;
+    const bool act = lanes_agent<G>(g.n, a, lane);
+    const LaneSums<G> sums = LaneSums<G>::of(sh);
+    unsigned applied = g.applied[a];
+    V3 steer = v3(g.steering[a]);
+    Self me;
+    me.pos = v3(g.position[a]);
+    me.dir = v3(g.direction[a]);
+    me.speed = g.speed[a];
+    me.radius = g.radius[a];
+    const float3 sd = g.side[a];
+    me.side = v3(sd.x, sd.y, sd.z);
+    V3 mine = v3(0.f, 0.f, 0.f), r_ali = mine, r_coh = mine;  // lane j: separation from group j
+    for (unsigned j = 0; j < M.n_groups; ++j) {
+        const OtherView& o = M.o[j];
+        LaneNeighbour nb;
+        unsigned b;
+        nb.ok = lanes_entry<G>(M.idx[j], a, g.n, M.k[j], o.n, lane, b);
+        nb.pos = nb.dir = v3(0.f, 0.f, 0.f);
+        nb.speed = nb.radius = nb.dist = 0.f;
+        if (nb.ok) {
+            nb.pos = v3(o.position[b]);
+            nb.dir = v3(o.direction[b]);
+            nb.speed = o.speed[b];
+            nb.radius = o.radius[b];
+            nb.dist = M.dist[j][a + size_t(lane) * g.n];
+        }
+        V3 r_sep, none;
+        if (j != M.self) {
+            lanes_flock(NEED_SEP, M.sep, M.sep, M.sep, me, lane, nb, sums, r_sep, none, none);
+            if (M.avoid_close) {
+                const CloseAcc c = lanes_close<G>(me, M.min_sep, nb);
+                close_finish(c, M.w_avoid, M.mask_avoid, applied, steer);
+            }
+            const AvoidAcc v = lanes_avoid<G>(me, M.min_time, M.k[j], nb);
+            avoid_finish(v, M.w_avoid, M.mask_avoid, me, applied, steer);
+        } else {
+            lanes_flock(NEED_SEP | NEED_ALI | NEED_COH, M.sep, M.ali, M.coh, me, lane, nb, sums,
+                        r_sep, r_ali, r_coh);
+        }
+        if (lane == j) mine = r_sep;
+    }
+    for (unsigned j = 0; j < M.n_groups; ++j)
+        flock_apply(lanes_get<G>(mine, j), M.sep, SEPARATION_BIT, applied, steer);
+    if (!act || lane != 0) return;
+    flock_apply(r_ali, M.ali, ALIGNMENT_BIT, applied, steer);
+    flock_apply(r_coh, M.coh, COHESION_BIT, applied, steer);
+    if (M.has_path) {
+        follow_path_finish(M.path, M.path_time, M.w_path, M.mask_path, me, applied, steer);
+        seek_finish(v3(M.seek_target[0], M.seek_target[1], M.seek_target[2]), M.w_seek, M.mask_seek,
+                    me, applied, steer);
+    }
+    const float3 up = g.up[a];
+    me.up = v3(up.x, up.y, up.z);
+    me.max_speed = g.max_speed[a];
+    me.max_force = g.max_force[a];
+    me.mass = g.mass[a];
+    integrate(me, steer, M.dt);
+    applied = 0u;
+    for (unsigned j = 0; j < M.self; ++j)
+        push_apart(me.pos, applied, me.radius, M.idx[j][a], M.dist[j][a], M.o[j], M.o[j].position,
+                   M.o[j].applied, M.mask_antipen);
+    M.next.position[a] = f4(me.pos, 0.f);
+    M.next.direction[a] = f4(me.dir, 0.f);
+    M.next.speed[a] = me.speed;
+    M.next.applied[a] = applied;
+    g.side[a] = make_float3(me.side.x, me.side.y, me.side.z);
+    g.up[a] = make_float3(me.up.x, me.up.y, me.up.z);
+    g.steering[a] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// The second: anti-penetration within the group, whose agents have all moved
+// now, then against the groups after it, which have not; the result goes to
+// the group's arrays.
+__global__ void __launch_bounds__(kLaneBlock) k_group_settle(const __grid_constant__ MultiSteer M) {
+    const unsigned a = blockIdx.x * kLaneBlock + threadIdx.x;
+    const GroupView& g = M.g;
+    if (a >= g.n) return;
+    V3 pos = v3(M.next.position[a]);
+    unsigned applied = M.next.applied[a];
+    const float radius = g.radius[a];
+    for (unsigned j = M.self; j < M.n_groups; ++j) {
+        const bool own = j == M.self;
+        push_apart(pos, applied, radius, M.idx[j][a], M.dist[j][a], M.o[j],
+                   own ? M.next.position : M.o[j].position, own ? M.next.applied : M.o[j].applied,
+                   M.mask_antipen);
+    }
+    g.position[a] = f4(pos, 0.f);
+    g.direction[a] = M.next.direction[a];
+    g.speed[a] = M.next.speed[a];
+    g.applied[a] = applied;
+}
+
+// k <= 32 for every list; a group of a few agents a lane group each, larger
+// groups keep one thread per agent (k_multigroup_steer and the calls after it).
+bool lanes_multigroup(const MultiSteer& M) {
+    for (unsigned j = 0; j < M.n_groups; ++j)
+        if (M.k[j] > 32) return false;
+    return M.g.n <= 65536;
+}
+
+gs_status launch_group_frame(const MultiSteer& M, cudaStream_t st) {
+    if (M.g.n == 0) return GS_OK;
+    unsigned k = 0;
+    for (unsigned j = 0; j < M.n_groups; ++j) k = M.k[j] > k ? M.k[j] : k;
+    if (k <= 8) k_group_move<8><<<blocks_for(M.g.n, kLaneBlock / 8), kLaneBlock, 0, st>>>(M);
+    else if (k <= 16) k_group_move<16><<<blocks_for(M.g.n, kLaneBlock / 16), kLaneBlock, 0, st>>>(M);
+    else k_group_move<32><<<blocks_for(M.g.n, kLaneBlock / 32), kLaneBlock, 0, st>>>(M);
+    k_group_settle<<<blocks_for(M.g.n, kLaneBlock), kLaneBlock, 0, st>>>(M);
+    GS_LAUNCHED("group_frame");
+    return GS_OK;
+}
+
 // Under ncu, lanes / threads (us; a launch's floor is about 3): one flocking
 // behaviour, k = 7, 30,000 agents 7.5 / 6.5; k = 16, 10,000 6.5 / 11.3, 32,768
 // 10.2 / about 9.5.  The avoidance passes and the walls carry more arithmetic

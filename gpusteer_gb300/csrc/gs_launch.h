@@ -134,8 +134,22 @@ struct MultiSteer {
     float path_time, w_path, w_seek;
     unsigned mask_path, mask_seek;
     float seek_target[3];
+    // the frame's two-launch form: what the update needs besides, and where
+    // the first launch leaves the group's new state for the second
+    float dt;
+    unsigned mask_antipen;
+    struct {
+        float4 *position, *direction;
+        float* speed;
+        unsigned* applied;
+    } next;
 };
 gs_status launch_multigroup_steer(const MultiSteer& M, cudaStream_t st);
+// Steering, update and anti-penetration of one group of a frame in two
+// launches (gs_lanes.cu), where lanes_multigroup says so.
+constexpr size_t kGroupNextBytes = 40;  // of M.next, per agent
+bool lanes_multigroup(const MultiSteer& M);
+gs_status launch_group_frame(const MultiSteer& M, cudaStream_t st);
 gs_status launch_update_antipen_wall(GroupView g, const unsigned* knl, unsigned k,
                                      const float4* start, const float4* end,
                                      const float4* normal, unsigned n_lines, float dt,
