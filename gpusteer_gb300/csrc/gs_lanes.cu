@@ -410,17 +410,42 @@ void launch_avoid_walls_lanes(GroupView g, const unsigned* knw, unsigned kw, con
 // this one, whose agents have moved.  Other agents of this group read its
 // position, heading and speed of before the update meanwhile, so the new ones
 // go to M.next.
-__device__ __forceinline__ void push_apart(V3& pos, unsigned& applied, float radius, unsigned b,
-                                           float knn_dist, const OtherView& o,
-                                           const float4* o_pos, const unsigned* o_applied,
-                                           unsigned mask) {
-    // AntiPenetrationAgentsCUDAKernel.cu:72-108, as k_antipen
-    if ((applied & mask) || b >= o.n) return;
-    const float overlap = radius + o.radius[b] - knn_dist;
-    if (overlap < 0.f) return;
-    const V3 unit = normalize(sub(pos, v3(o_pos[b])));
-    pos = add(pos, mul(unit, (o_applied[b] & mask) ? overlap : 0.5f * overlap));
-    applied |= ANTI_PENETRATION_AGENT;
+//
+// Anti-penetration (AntiPenetrationAgentsCUDAKernel.cu:72-108, as k_antipen)
+// takes the groups one after another, but what it reads of each does not depend
+// on the ones before: lane t loads group first + t's nearest neighbour, then the
+// pushes are applied in order.
+template <int G>
+__device__ __forceinline__ void lanes_push_apart(const MultiSteer& M, unsigned a, unsigned lane,
+                                                 unsigned first, unsigned last, V3& pos,
+                                                 float radius, unsigned& applied) {
+    bool near = false;
+    V3 at = v3(0.f, 0.f, 0.f);
+    float overlap = 0.f;
+    unsigned bits = 0;
+    const unsigned j = first + lane;
+    if (j < last) {
+        const OtherView& o = M.o[j];
+        const bool own = j == M.self;  // this group's agents have moved to M.next
+        const unsigned b = M.idx[j][a];
+        const float d = M.dist[j][a];
+        if (b < o.n) {
+            at = v3(own ? M.next.position[b] : o.position[b]);
+            bits = own ? M.next.applied[b] : o.applied[b];
+            overlap = radius + o.radius[b] - d;
+            near = !(overlap < 0.f);
+        }
+    }
+    const unsigned m = lanes_ballot<G>(near);
+    for (unsigned t = 0; t < last - first; ++t) {
+        const V3 other = lanes_get<G>(at, t);
+        const float over = __shfl_sync(kAllLanes, overlap, int(t), G);
+        const unsigned ob = __shfl_sync(kAllLanes, bits, int(t), G);
+        if (!((m >> t) & 1u) || (applied & M.mask_antipen)) continue;
+        const V3 unit = normalize(sub(pos, other));
+        pos = add(pos, mul(unit, (ob & M.mask_antipen) ? over : 0.5f * over));
+        applied |= ANTI_PENETRATION_AGENT;
+    }
 }
 
 template <int G>
@@ -440,7 +465,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_group_move(const __grid_constant
     const float3 sd = g.side[a];
     me.side = v3(sd.x, sd.y, sd.z);
     V3 mine = v3(0.f, 0.f, 0.f), r_ali = mine, r_coh = mine;  // lane j: separation from group j
-    for (unsigned j = 0; j < M.n_groups; ++j) {
+    auto neighbour = [&](unsigned j) {
         const OtherView& o = M.o[j];
         LaneNeighbour nb;
         unsigned b;
@@ -454,6 +479,12 @@ __global__ void __launch_bounds__(kLaneBlock) k_group_move(const __grid_constant
             nb.radius = o.radius[b];
             nb.dist = M.dist[j][a + size_t(lane) * g.n];
         }
+        return nb;
+    };
+    // the next group's neighbours are on their way while one group is taken
+    LaneNeighbour nb = neighbour(0), next;
+    for (unsigned j = 0; j < M.n_groups; ++j, nb = next) {
+        next = neighbour(j + 1 < M.n_groups ? j + 1 : j);
         V3 r_sep, none;
         if (j != M.self) {
             lanes_flock(NEED_SEP, M.sep, M.sep, M.sep, me, lane, nb, sums, r_sep, none, none);
@@ -471,7 +502,6 @@ __global__ void __launch_bounds__(kLaneBlock) k_group_move(const __grid_constant
     }
     for (unsigned j = 0; j < M.n_groups; ++j)
         flock_apply(lanes_get<G>(mine, j), M.sep, SEPARATION_BIT, applied, steer);
-    if (!act || lane != 0) return;
     flock_apply(r_ali, M.ali, ALIGNMENT_BIT, applied, steer);
     flock_apply(r_coh, M.coh, COHESION_BIT, applied, steer);
     if (M.has_path) {
@@ -486,9 +516,8 @@ __global__ void __launch_bounds__(kLaneBlock) k_group_move(const __grid_constant
     me.mass = g.mass[a];
     integrate(me, steer, M.dt);
     applied = 0u;
-    for (unsigned j = 0; j < M.self; ++j)
-        push_apart(me.pos, applied, me.radius, M.idx[j][a], M.dist[j][a], M.o[j], M.o[j].position,
-                   M.o[j].applied, M.mask_antipen);
+    lanes_push_apart<G>(M, a, lane, 0, M.self, me.pos, me.radius, applied);
+    if (!act || lane != 0) return;
     M.next.position[a] = f4(me.pos, 0.f);
     M.next.direction[a] = f4(me.dir, 0.f);
     M.next.speed[a] = me.speed;
@@ -502,23 +531,21 @@ __global__ void __launch_bounds__(kLaneBlock) k_group_move(const __grid_constant
 // now, then against the groups after it, which have not; the result goes to
 // the group's arrays.
 __global__ void __launch_bounds__(kLaneBlock) k_group_settle(const __grid_constant__ MultiSteer M) {
-    const unsigned a = blockIdx.x * kLaneBlock + threadIdx.x;
     const GroupView& g = M.g;
-    if (a >= g.n) return;
+    unsigned a, lane;
+    const bool act = lanes_agent<8>(g.n, a, lane);
     V3 pos = v3(M.next.position[a]);
     unsigned applied = M.next.applied[a];
-    const float radius = g.radius[a];
-    for (unsigned j = M.self; j < M.n_groups; ++j) {
-        const bool own = j == M.self;
-        push_apart(pos, applied, radius, M.idx[j][a], M.dist[j][a], M.o[j],
-                   own ? M.next.position : M.o[j].position, own ? M.next.applied : M.o[j].applied,
-                   M.mask_antipen);
-    }
+    const float4 dir = M.next.direction[a];
+    const float speed = M.next.speed[a];
+    lanes_push_apart<8>(M, a, lane, M.self, M.n_groups, pos, g.radius[a], applied);
+    if (!act || lane != 0) return;
     g.position[a] = f4(pos, 0.f);
-    g.direction[a] = M.next.direction[a];
-    g.speed[a] = M.next.speed[a];
+    g.direction[a] = dir;
+    g.speed[a] = speed;
     g.applied[a] = applied;
 }
+static_assert(kMaxGroups <= 8, "a lane per group");
 
 // k <= 32 for every list; a group of a few agents a lane group each, larger
 // groups keep one thread per agent (k_multigroup_steer and the calls after it).
@@ -535,7 +562,7 @@ gs_status launch_group_frame(const MultiSteer& M, cudaStream_t st) {
     if (k <= 8) k_group_move<8><<<blocks_for(M.g.n, kLaneBlock / 8), kLaneBlock, 0, st>>>(M);
     else if (k <= 16) k_group_move<16><<<blocks_for(M.g.n, kLaneBlock / 16), kLaneBlock, 0, st>>>(M);
     else k_group_move<32><<<blocks_for(M.g.n, kLaneBlock / 32), kLaneBlock, 0, st>>>(M);
-    k_group_settle<<<blocks_for(M.g.n, kLaneBlock), kLaneBlock, 0, st>>>(M);
+    k_group_settle<<<blocks_for(M.g.n, kLaneBlock / 8), kLaneBlock, 0, st>>>(M);
     GS_LAUNCHED("group_frame");
     return GS_OK;
 }
