@@ -301,7 +301,8 @@ struct AdjointLaunch {
     // scratch (adjoint_scratch_bind): per-edge and own terms; per target agent
     // its fill count (fill[n]: overflow count) and kBucket edge slots; the
     // overflow list of (target, edge) pairs
-    float4 *edge_p, *edge_v, *own_p, *own_v;
+    float* edge;  // 8 floats an edge
+    float4 *own_p, *own_v;
     unsigned *fill, *bucket, *ovf;
 };
 constexpr unsigned kBucket = 48;
