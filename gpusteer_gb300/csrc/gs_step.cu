@@ -584,11 +584,13 @@ __global__ void __launch_bounds__(kBlock) k_knn_retry(FusedLaunch L, StepDev p) 
 }
 
 // ---- whole step without walls -------------------------------------------------------
-constexpr unsigned kNbrChunk = 1;  // measured best for the flock (2: +2.5 %, 4: +9 %)
 constexpr unsigned kRestChunk = 2;  // the rest phase's (1: +7 %, 3: +6 %, 4: +12 %; spills)
 
-template <int KMAX, unsigned ENUM, bool EXACT, unsigned NEEDC = kNeedRuntime, bool FLAT = false>
-__global__ void __launch_bounds__(kBlock, 3) k_fused(FusedLaunch L, StepDev p) {
+// kNbrChunk: neighbours whose gathers are in flight together (1 is best at
+// full occupancy: 2 there costs 2.5 %, 4 9 %).
+template <int KMAX, unsigned ENUM, bool EXACT, unsigned NEEDC = kNeedRuntime, bool FLAT = false,
+          unsigned kNbrChunk = 1>
+__global__ void __launch_bounds__(kBlock, kNbrChunk > 1 ? 2 : 3) k_fused(FusedLaunch L, StepDev p) {
     const unsigned need = NEEDC == kNeedRuntime ? p.need : NEEDC;
     extern __shared__ unsigned sh_col[];
     const unsigned bd = blockDim.x;
@@ -930,8 +932,15 @@ static gs_status launch_fused_k(const FusedLaunch& L, const StepDev& p, cudaStre
         bool done = false;
         if constexpr (ENUM == 32) {
             if ((p.need & kNeedList) == (NEED_SEP | NEED_ALI | NEED_COH)) {
-                GS_TRY(allow_smem(k_fused<KMAX, 32, false, NEED_SEP | NEED_ALI | NEED_COH>, smem));
-                k_fused<KMAX, 32, false, NEED_SEP | NEED_ALI | NEED_COH><<<nb, bs, smem, st>>>(L, p);
+                // a group whose blocks all fit at two to an SM has registers to
+                // spare: two neighbours' gathers in flight (k = 16: 32,768
+                // boids 31.0 -> 28.1 us a step, 65,536 37.4 -> 32.6; 100,003,
+                // in one wave only at three to an SM, 45.8 against 46.3)
+                auto kern = nb * bs <= 2 * 152 * kBlock
+                                ? k_fused<KMAX, 32, false, NEED_SEP | NEED_ALI | NEED_COH, false, 2>
+                                : k_fused<KMAX, 32, false, NEED_SEP | NEED_ALI | NEED_COH>;
+                GS_TRY(allow_smem(kern, smem));
+                kern<<<nb, bs, smem, st>>>(L, p);
                 done = true;
             }
         }
