@@ -24,67 +24,6 @@ namespace gs {
 constexpr unsigned kBruteBlock = 256;
 constexpr unsigned kBruteSegs = 64;
 
-// A query's exact (distance, index) list over its group's lanes: lane r holds
-// rank r in e[0] and, with L = 2 (32 < k <= 64, G = 32), rank 32 + r in e[1].
-template <int G, int L>
-struct LaneList {
-    unsigned long long e[L];
-
-    __device__ __forceinline__ unsigned long long kth(unsigned k) const {
-        if (L == 1 || k <= 32) return __shfl_sync(kAllLanes, e[0], int(k) - 1, G);
-        return __shfl_sync(kAllLanes, e[L - 1], int(k) - 33, G);
-    }
-    __device__ __forceinline__ static unsigned long long pick(unsigned long long a, int stride,
-                                                              bool keep_min) {
-        const unsigned long long b = __shfl_xor_sync(kAllLanes, a, stride);
-        return (b < a) == keep_min ? b : a;
-    }
-    // One candidate key per lane (KEY_EMPTY for none).  A few that enter are
-    // shifted in one after another; more are sorted and merged at once.
-    __device__ __forceinline__ void take(unsigned long long c, unsigned k, unsigned lane) {
-        const bool in = c < kth(k);
-        if (!__any_sync(kAllLanes, in)) return;
-        unsigned m = lanes_ballot<G>(in);
-        unsigned most = __reduce_max_sync(kAllLanes, unsigned(__popc(m)));
-        if (most <= 4) {
-            for (; most; --most) {
-                const int from = m ? __ffs(int(m)) - 1 : 0;
-                unsigned long long key = __shfl_sync(kAllLanes, c, from, G);
-                if (!m) key = KEY_EMPTY;
-                m &= m - 1u;
-                const unsigned long long up = __shfl_up_sync(kAllLanes, e[0], 1, G);
-                if (L == 2) {
-                    unsigned long long up1 = __shfl_up_sync(kAllLanes, e[L - 1], 1, G);
-                    const unsigned long long last = __shfl_sync(kAllLanes, e[0], G - 1, G);
-                    if (lane == 0) up1 = last;
-                    if (key < e[L - 1]) e[L - 1] = up1 > key ? up1 : key;
-                }
-                if (key < e[0]) e[0] = (lane && up > key) ? up : key;
-            }
-            return;
-        }
-#pragma unroll
-        for (int size = 2; size <= G; size <<= 1) {
-#pragma unroll
-            for (int stride = size >> 1; stride > 0; stride >>= 1)
-                c = pick(c, stride,
-                         ((lane & unsigned(stride)) == 0) == ((lane & unsigned(size)) == 0));
-        }
-        const unsigned long long r = __shfl_xor_sync(kAllLanes, c, G - 1);
-        if (r < e[L - 1]) e[L - 1] = r;
-        if (L == 2 && e[L - 1] < e[0]) {
-            const unsigned long long x = e[0];
-            e[0] = e[L - 1];
-            e[L - 1] = x;
-        }
-#pragma unroll
-        for (int h = 0; h < L; ++h)
-#pragma unroll
-            for (int stride = G >> 1; stride > 0; stride >>= 1)
-                e[h] = pick(e[h], stride, (lane & unsigned(stride)) == 0);
-    }
-};
-
 struct BruteQuery {
     V3 p;
     unsigned self_id;

@@ -11,6 +11,7 @@
 
 #include "gs_db.cuh"
 #include "gs_launch.h"
+#include "gs_table.cuh"
 
 namespace gs {
 
@@ -56,6 +57,8 @@ static void release_fused(gs_group g) {
     dfree(g->d_stat);
     dfree(g->d_bar);
     db_release(g->fdb);
+    if (g->table.block) cudaFree(g->table.block);
+    g->table.block = nullptr;
     g->fused_k_alloc = 0;
 }
 
@@ -67,7 +70,8 @@ static void drop_graph(gs_group g) {
 // Brings the reference-layout arrays up to date after fused steps.
 static gs_status ensure_reference(gs_group g) {
     if (!g->fused_current) return GS_OK;
-    GS_TRY(fused_to_reference(g->A, g->n, g->d_scene, g->slot_of, view(g), g->stream));
+    GS_TRY(fused_to_reference(g->A, g->n, g->d_scene, g->slot_of, g->table.valid, view(g),
+                              g->stream));
     g->fused_current = false;
     g->db.valid = false;
     return GS_OK;
@@ -580,6 +584,7 @@ gs_status gs_group_create(unsigned k, unsigned capacity, void* stream, gs_group*
     std::memset(static_cast<void*>(g), 0, sizeof(*g));
     new (&g->db) Database();
     new (&g->fdb) Database();
+    new (&g->table) CellTable();
     g->use_graph = true;
     g->block = kBlock;
     g->k = k;
@@ -1290,6 +1295,7 @@ static DiagSource diag_source(gs_group g, gs_bins bins) {
 }
 
 // Scratch of the diagnostics, kept with the group (no allocation per call).
+static TableStep table_buffers(gs_group g, unsigned step);
 static gs_status diag_scratch(gs_group g, size_t bytes, void** p) {
     if (g->diag_bytes < bytes) {
         if (g->diag) cudaFree(g->diag);
@@ -1321,6 +1327,9 @@ gs_status gs_cell_density(gs_group g, gs_bins bins, unsigned* counts) {
     const unsigned C = bins->cells;
     void* d = nullptr;
     GS_TRY(diag_scratch(g, size_t(C) * 4, &d));
+    if (src == DIAG_FRAME && g->table.frame)  // the frame's counts themselves
+        return diag_copy_out(g, counts, table_buffers(g, (g->table.step + 5) % 6).cnt,
+                             size_t(C) * 4, GS_OK);
     const gs_status s = src == DIAG_DB
                             ? launch_cell_density(g->db, static_cast<unsigned*>(d), g->stream)
                             : launch_frame_cell_density(g->fdb.start, g->fdb.live, C,
@@ -1341,6 +1350,8 @@ gs_status gs_cell_avg_velocity(gs_group g, gs_bins bins, float* avg3) {
     gs_status s;
     if (src == DIAG_DB) {
         s = launch_cell_avg_velocity(g->db, g->direction, g->speed, out, g->stream);
+    } else if (g->table.frame) {
+        s = table_avg_velocity(table_buffers(g, (g->table.step + 5) % 6), out, g->stream);
     } else {
         s = launch_frame_cell_avg_velocity(g->fdb.start, g->fdb.live, C, g->A.f[0], g->A.f[1],
                                            out, g->stream);
@@ -1673,6 +1684,24 @@ static bool gather_first_permute(gs_group g) {
     return most >= kGatherPermuteMinAgents;
 }
 
+// Measures the automatic KNN capacity from the cell counts where the last
+// measurement no longer holds: one synchronising read per upload that changes
+// the agent count, or grid change.
+static gs_status measure_capacity(gs_group g, const unsigned* count, unsigned C, const Grid& grid,
+                                  unsigned r) {
+    if (g->auto_cap_valid && g->auto_cap_r == r &&
+        std::memcmp(&g->auto_cap_grid, &grid, sizeof(Grid)) == 0)
+        return GS_OK;
+    unsigned occupied = 0;
+    unsigned long long sumsq = 0;
+    GS_TRY(count_occupied(count, C, g->d_stat, &occupied, &sumsq, g->stream));
+    g->auto_cap = knn_capacity(g->n, sumsq, grid, r);
+    g->auto_cap_grid = grid;
+    g->auto_cap_r = r;
+    g->auto_cap_valid = true;
+    return GS_OK;
+}
+
 // Brings the fused engine's bucketed state and pending cell counts up to
 // date for steps on `grid` and fills the launch block L; picks the KNN
 // capacity into d.  dirty: the first step must add the steering and applied
@@ -1695,7 +1724,7 @@ static gs_status fused_setup(gs_group g, StepDev& d, const Grid& grid, unsigned 
         GS_TRY(scan_tile_totals(g->fdb.count, C, g->fdb.tile, st));
         g->fused_current = true;
     } else if (std::memcmp(&g->fdb.grid, &grid, sizeof(Grid)) != 0 || !g->fdb.valid ||
-               g->pending_wrap != d.wrap_mode) {
+               g->pending_wrap != d.wrap_mode || g->table.valid) {
         GS_TRY(clear_counts(g, C, st));
         GS_TRY(fused_recount(g->A, g->n, g->d_scene, g->cellrank, g->fdb.count, d.wrap_mode,
                              st));
@@ -1704,20 +1733,12 @@ static gs_status fused_setup(gs_group g, StepDev& d, const Grid& grid, unsigned 
     g->fdb.grid = grid;
     g->fdb.valid = true;
     g->pending_wrap = d.wrap_mode;
+    g->table.valid = false;  // its rows are not kept up by the sorting step
+    g->table.frame = false;
     if (g->knn_cap) {
         d.enum_cap = g->knn_cap;
     } else {
-        if (!g->auto_cap_valid || g->auto_cap_r != d.r ||
-            std::memcmp(&g->auto_cap_grid, &grid, sizeof(Grid)) != 0) {
-            // one synchronising read per upload or grid change
-            unsigned occupied = 0;
-            unsigned long long sumsq = 0;
-            GS_TRY(count_occupied(g->fdb.count, C, g->d_stat, &occupied, &sumsq, st));
-            g->auto_cap = knn_capacity(g->n, sumsq, grid, d.r);
-            g->auto_cap_grid = grid;
-            g->auto_cap_r = d.r;
-            g->auto_cap_valid = true;
-        }
+        GS_TRY(measure_capacity(g, g->fdb.count, C, grid, d.r));
         d.enum_cap = g->auto_cap;
         // a capacity fixed by the caller asks for that scan; otherwise small
         // groups step with a group of lanes per agent
@@ -1760,6 +1781,124 @@ static void fill_launch(gs_group g, const StepDev& d, const WallsDev& w, FusedLa
     }
 }
 
+// ---- the small groups' step on cell tables (gs_table.cu) ---------------------------
+// Rows of 16 places a cell (32 in a flat world, whose cells are columns) and
+// at most 64 MiB a table; larger grids keep the sorting step.
+static unsigned table_row_log2(const StepDev& d) { return d.flat ? 5u : 4u; }
+static bool table_wanted(gs_group g, const StepDev& d, unsigned C, const unsigned* agent_scene) {
+    return agent_scene == nullptr && d.r == 1 && g->knn_cap == 0 && !g->profiling &&
+           !g->persistent && lanes_preferred(g->n, (d.need & NEED_WALLS) != 0) &&
+           (size_t(C) << table_row_log2(d)) <= (size_t(1) << 22);
+}
+
+static gs_status table_reserve(gs_group g, unsigned C, unsigned row_log2) {
+    CellTable& t = g->table;
+    if (t.block && t.cells == C && t.row_log2 == row_log2) return GS_OK;
+    if (t.block) {
+        GS_CUDA(cudaStreamSynchronize(g->stream));
+        cudaFree(t.block);
+        t = CellTable();
+    }
+    const size_t row = (size_t(C) << row_log2) * 16, over = size_t(g->capacity) * 16;
+    char* b = nullptr;
+    GS_TRY(dalloc(&b, 2 * (row + over) + (3 * size_t(C) + 4) * 4));
+    t.block = b;
+    for (int i = 0; i < 2; ++i) {
+        t.tab[i] = reinterpret_cast<float4*>(b + size_t(i) * row);
+        t.over[i] = reinterpret_cast<float4*>(b + 2 * row + size_t(i) * over);
+    }
+    t.cnt = reinterpret_cast<unsigned*>(b + 2 * (row + over));
+    t.cells = C;
+    t.row_log2 = row_log2;
+    return GS_OK;
+}
+
+// The buffers of step number `step` (0: the first after table_init).
+static TableStep table_buffers(gs_group g, unsigned step) {
+    const CellTable& t = g->table;
+    TableStep T;
+    std::memset(static_cast<void*>(&T), 0, sizeof(T));
+    const unsigned in = step % 2, out = 1 - in, ci = step % 3, co = (step + 1) % 3,
+                   cc = (step + 2) % 3;
+    unsigned* const over_n = t.cnt + 3 * size_t(t.cells);
+    T.tab = t.tab[in];
+    T.over = t.over[in];
+    T.cnt = t.cnt + size_t(ci) * t.cells;
+    T.over_n = over_n + ci;
+    T.tab_next = t.tab[out];
+    T.over_next = t.over[out];
+    T.cnt_next = t.cnt + size_t(co) * t.cells;
+    T.over_n_next = over_n + co;
+    T.cnt_clear = t.cnt + size_t(cc) * t.cells;
+    T.over_n_clear = over_n + cc;
+    T.f0 = T.f0_next = g->A.f[0];
+    T.f1 = T.f1_next = g->A.f[1];
+    T.f2 = g->A.f[2];
+    T.f3 = g->A.f[3];
+    T.f4 = g->A.f[4];
+    T.f5 = g->A.f[5];
+    T.w0 = g->w0;
+    T.w1 = g->w1;
+    T.w2 = g->w2;
+    T.near = g->knn_slot;
+    T.near_dist = g->knn_dist;
+    T.n = g->n;
+    T.cells = t.cells;
+    T.row_log2 = t.row_log2;
+    T.sc = (*g->h_scenes)[0];
+    return T;
+}
+
+static gs_status table_run(gs_group g, StepDev d, const Grid& grid, unsigned C,
+                           const WallsDev& w, unsigned steps) {
+    cudaStream_t st = g->stream;
+    CellTable& t = g->table;
+    bool dirty = false;
+    g->frame_cells = 0;
+    if (!g->fused_current || !t.valid || t.cells != C || t.row_log2 != table_row_log2(d) ||
+        std::memcmp(&t.grid, &grid, sizeof(Grid)) != 0 || t.wrap_mode != d.wrap_mode) {
+        GS_TRY(ensure_reference(g));
+        dirty = g->accum_dirty;
+        t.valid = t.frame = false;
+        GS_TRY(table_reserve(g, C, table_row_log2(d)));
+        GS_CUDA(cudaMemsetAsync(t.cnt, 0, (3 * size_t(C) + 4) * 4, st));
+        // step "-1" fills the table that step 0 reads
+        t.step = 0;
+        GS_TRY(table_init(view(g), table_buffers(g, 5), d.wrap_mode, dirty, g->A.f[5],
+                          g->retry_count, st));
+        t.grid = grid;
+        t.wrap_mode = d.wrap_mode;
+        t.valid = true;
+        g->fused_current = true;
+    }
+    GS_TRY(measure_capacity(g, t.cnt + size_t(t.step % 3) * C, C, grid, d.r));
+    g->fdb.grid = grid;
+    const bool walls = d.need & NEED_WALLS;
+    for (unsigned s = 0; s < steps; ++s) {
+        TableStep T = table_buffers(g, t.step % 6);
+        T.walls = WallRefs{w.start, w.end, w.normal, w.pos_id, w.cell_start};
+        // without walls the other agents read the old positions and headings
+        // while the new ones are written: the two sets take turns
+        if (!walls) {
+            T.f0_next = g->B.f[0];
+            T.f1_next = g->B.f[1];
+        }
+        d.dirty = dirty ? 1 : 0;
+        dirty = false;
+        GS_TRY(table_step(T, d, st));
+        if (!walls) {
+            std::swap(g->A.f[0], g->B.f[0]);
+            std::swap(g->A.f[1], g->B.f[1]);
+        }
+        t.step = (t.step + 1) % 6;
+    }
+    g->accum_dirty = false;
+    g->db.valid = false;
+    g->frame_cells = C;
+    t.frame = true;
+    return GS_OK;
+}
+
 // The fused engine for a group whose scene table is in g->h_scenes / d_scene
 // (one scene for a plain group, many for a batch).
 static gs_status fused_run(gs_group g, StepDev d, const Grid& grid, unsigned C,
@@ -1769,6 +1908,7 @@ static gs_status fused_run(gs_group g, StepDev d, const Grid& grid, unsigned C,
     bool dirty = false, fresh = false;
     g->frame_cells = 0;
     // part of the graph key: a changed form or limit captures again
+    if (table_wanted(g, d, C, agent_scene)) return table_run(g, d, grid, C, w, steps);
     d.persistent = g->persistent ? 1u : 0u;
     d.bar_limit = g->bar_limit ? g->bar_limit : kBarrierPollsDefault;
     GS_TRY(fused_setup(g, d, grid, C, agent_scene, w, L, dirty, fresh));
@@ -2135,7 +2275,7 @@ static gs_status io_compute_and_download(IoPart& q, unsigned steps, bool in_plac
         di.fresh = i == 0 && gather_first_permute(g) ? 1 : 0;
         GS_TRY(step_body(g, q.L, di, q.Ct, nullptr));
     }
-    GS_TRY(fused_to_reference(g->A, g->n, g->d_scene, g->slot_of, view(g), st));
+    GS_TRY(fused_to_reference(g->A, g->n, g->d_scene, g->slot_of, false, view(g), st));
     return download_copies(g, &q.ho, in_place);
 }
 

@@ -73,6 +73,19 @@ inline bool operator==(const Scene& a, const Scene& b) {
     return std::memcmp(&a, &b, sizeof(Scene)) == 0;
 }
 
+// Buffers of the fused step on cell tables (gs_table.cuh), in one block.
+struct CellTable {
+    void* block = nullptr;
+    float4 *tab[2] = {nullptr, nullptr}, *over[2] = {nullptr, nullptr};
+    unsigned* cnt = nullptr;  // three arrays of `cells`, then three overflow counts
+    unsigned cells = 0, row_log2 = 0;
+    unsigned step = 0;        // steps since the table was filled from the reference layout
+    bool valid = false;       // the group's state is in A, in agent order, and in the table
+    bool frame = false;       // `step - 1`'s table and counts describe frame_cells
+    Grid grid{};
+    int wrap_mode = 0;
+};
+
 // Bucketed ("fused") state: six float4 streams per agent.
 //   f0 = position.xyz, agent index (bits)    f1 = direction.xyz, speed
 //   f2 = side.xyz, radius                    f3 = up.xyz, mass
@@ -155,6 +168,7 @@ struct gs_group_s {
     unsigned* knn_slot;    // [k * n] neighbour slots (wall phase)
     float* knn_dist;       // [k * n]
     gs::Database fdb;      // counts / starts of the fused step
+    gs::CellTable table;   // the small groups' step without a sort
     // brute-force KNN over cells: the other group's database on an automatic
     // grid; scratch (words 0-5: that grid, words 6-7: the pairs met)
     gs::Database bf_db;

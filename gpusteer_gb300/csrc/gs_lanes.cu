@@ -12,51 +12,6 @@ namespace gs {
 
 constexpr unsigned kLaneBlock = 128;
 
-// The behaviours order[first..] of one agent over its lanes' neighbours.
-template <int G>
-__device__ __forceinline__ void lanes_behaviours(const StepDev& p, unsigned need, unsigned first,
-                                                 const Self& me, unsigned lane,
-                                                 const LaneNeighbour& nb, LaneSums<G> sums,
-                                                 unsigned& applied, V3& steer) {
-    const FlockParams fs = flock_params(p.sep, p.sep_dsq), fa = flock_params(p.ali, p.ali_dsq),
-                      fc = flock_params(p.coh, p.coh_dsq);
-    V3 r_sep, r_ali, r_coh;
-    lanes_flock(need, fs, fa, fc, me, lane, nb, sums, r_sep, r_ali, r_coh);
-    CloseAcc close;
-    AvoidAcc avoid;
-    if (need & NEED_CLOSE) close = lanes_close<G>(me, p.min_sep, nb);
-    if (need & NEED_AVOID) avoid = lanes_avoid<G>(me, p.min_time_col, p.k, nb);
-#pragma unroll 1
-    for (unsigned o = first; o < p.n_order; ++o) {
-        switch ((p.order_packed >> (3u * o)) & 7u) {
-            case GS_B_SEPARATION:
-                if (need & NEED_SEP) flock_apply(r_sep, fs, SEPARATION_BIT, applied, steer);
-                break;
-            case GS_B_ALIGNMENT:
-                if (need & NEED_ALI) flock_apply(r_ali, fa, ALIGNMENT_BIT, applied, steer);
-                break;
-            case GS_B_COHESION:
-                if (need & NEED_COH) flock_apply(r_coh, fc, COHESION_BIT, applied, steer);
-                break;
-            case GS_B_SEEK:
-                seek_finish(v3(p.seek_target[0], p.seek_target[1], p.seek_target[2]), p.w_seek,
-                            p.mask_seek, me, applied, steer);
-                break;
-            case GS_B_AVOID_NEIGHBORS:
-                if (need & NEED_AVOID) {
-                    if (need & NEED_CLOSE)
-                        close_finish(close, p.w_avoid, p.mask_avoid, applied, steer);
-                    avoid_finish(avoid, p.w_avoid, p.mask_avoid, me, applied, steer);
-                }
-                break;
-            case GS_B_FOLLOW_PATH:
-                follow_path_finish(p.path, p.path_time, p.w_path, p.mask_path, me, applied, steer);
-                break;
-            default: break;
-        }
-    }
-}
-
 // ---- whole step without walls -----------------------------------------------------------
 template <int G, int R, unsigned NEEDC>
 __global__ void __launch_bounds__(kLaneBlock) k_lanes_step(FusedLaunch L, StepDev p) {
@@ -100,39 +55,6 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_step(FusedLaunch L, StepDe
 }
 
 // ---- wall phase ---------------------------------------------------------------------------
-// The four tests of a wall line (touching, then the three feelers, walls_add)
-// on lanes 0 to 3 of the group; the line's result is then taken in their order.
-template <int G>
-__device__ __forceinline__ void lanes_wall_line(WallAcc& wa, const Self& me, unsigned lane,
-                                                unsigned line, bool on, V3 ls, V3 le, V3 ln) {
-    const unsigned t = lane & 3u;
-    const V3 end = t == 0 ? add(me.pos, mul(neg(ln), me.radius))
-                          : t == 1 ? wa.feelers[0] : t == 2 ? wa.feelers[1] : wa.feelers[2];
-    V3 ip = v3(0.f, 0.f, 0.f);
-    const bool hit = on && lines_intersect(me.pos, end, ls, le, ip);
-    const float d = distance(me.pos, ip);
-    const unsigned hits = lanes_ballot<G>(hit) & 15u;
-    unsigned from = 0;
-#pragma unroll
-    for (unsigned f = 0; f < 4; ++f) {
-        const float df = __shfl_sync(kAllLanes, d, int(f), G);
-        if (!((hits >> f) & 1u)) continue;
-        if (f == 0) {
-            wa.touching = true;
-            wa.nearest_normal = ln;
-            wa.nearest_d = df;
-        } else if (df < wa.nearest_d) {
-            wa.nearest_d = df;
-            wa.nearest_line = line;
-            wa.feeler_index = f - 1;
-            wa.nearest_normal = ln;
-            from = f;
-        }
-    }
-    const V3 at = lanes_get<G>(ip, from);
-    if (from) wa.nearest_ip = at;
-}
-
 template <int G, int R>
 __global__ void __launch_bounds__(kLaneBlock) k_lanes_walls(FusedLaunch L, StepDev p) {
     __shared__ unsigned row_sh[R ? 1 : kLaneBlock / G * kLaneRowWords];
@@ -159,34 +81,8 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_walls(FusedLaunch L, StepD
     }
     unsigned applied = p.clear_applied ? 0u : __float_as_uint(f4v.z);
     V3 steer = p.dirty ? v3(L.B.f[5][s]) : v3(0.f, 0.f, 0.f);
-    const bool walls = sc.n_walls > 0 && L.w_pos_id != nullptr;
-    if (__any_sync(kAllLanes, walls)) {
-        Box wb = box;
-        if (!walls) {  // a scene without walls searches an empty box
-            wb.y0 = 1;
-            wb.y1 = 0;
-        }
-        const LaneEntry<G> wl =
-            lanes_knn<G, R>(p.knw, lane, me.pos, UINT_MAX, sc.grid, wb, sc.wall_cell_offset,
-                            L.w_cell_start, L.w_pos_id, rows);
-        const unsigned found = lanes_ballot<G>(walls && lane < p.knw && wl.slot != UINT_MAX &&
-                                               key_id(wl.key) < sc.n_walls);
-        WallAcc wa;
-        walls_init(wa, me, p.min_time_wall);
-        const unsigned lines = __popc(found);  // the list is filled from rank 0
-        const unsigned most = __reduce_max_sync(kAllLanes, lines);
-        for (unsigned r = 0; r < most; ++r) {
-            const unsigned line = unsigned(__shfl_sync(kAllLanes, wl.key, int(r), G));
-            const bool on = r < lines;
-            const unsigned g = on ? sc.wall_offset + line : 0u;
-            lanes_wall_line<G>(wa, me, lane, line, on, v3(L.w_start[g]), v3(L.w_end[g]),
-                               v3(L.w_normal[g]));
-        }
-        if (walls) walls_finish(wa, p.w_walls, p.mask_walls, me, applied, steer);
-        else if (!(applied & p.mask_walls)) steer = add(mul(v3(0.f, 0.f, 0.f), p.w_walls), steer);
-    } else if (!(applied & p.mask_walls)) {
-        steer = add(mul(v3(0.f, 0.f, 0.f), p.w_walls), steer);
-    }
+    lanes_walls<G, R>(WallRefs{L.w_start, L.w_end, L.w_normal, L.w_pos_id, L.w_cell_start}, sc, p, me,
+                      lane, box, applied, steer, rows);
     if (act && lane == 0) {
         L.w0[s] = make_float4(me.pos.x, me.pos.y, me.pos.z, me.radius);
         L.w1[s] = make_float4(me.dir.x, me.dir.y, me.dir.z, me.speed);

@@ -227,6 +227,67 @@ __device__ __forceinline__ V3 lanes_get(V3 v, unsigned from) {
               __shfl_sync(kAllLanes, v.z, int(from), G));
 }
 
+// A query's exact (distance, index) list over its group's lanes: lane r holds
+// rank r in e[0] and, with L = 2 (32 < k <= 64, G = 32), rank 32 + r in e[1].
+template <int G, int L>
+struct LaneList {
+    unsigned long long e[L];
+
+    __device__ __forceinline__ unsigned long long kth(unsigned k) const {
+        if (L == 1 || k <= 32) return __shfl_sync(kAllLanes, e[0], int(k) - 1, G);
+        return __shfl_sync(kAllLanes, e[L - 1], int(k) - 33, G);
+    }
+    __device__ __forceinline__ static unsigned long long pick(unsigned long long a, int stride,
+                                                              bool keep_min) {
+        const unsigned long long b = __shfl_xor_sync(kAllLanes, a, stride);
+        return (b < a) == keep_min ? b : a;
+    }
+    // One candidate key per lane (KEY_EMPTY for none).  A few that enter are
+    // shifted in one after another; more are sorted and merged at once.
+    __device__ __forceinline__ void take(unsigned long long c, unsigned k, unsigned lane) {
+        const bool in = c < kth(k);
+        if (!__any_sync(kAllLanes, in)) return;
+        unsigned m = lanes_ballot<G>(in);
+        unsigned most = __reduce_max_sync(kAllLanes, unsigned(__popc(m)));
+        if (most <= 4) {
+            for (; most; --most) {
+                const int from = m ? __ffs(int(m)) - 1 : 0;
+                unsigned long long key = __shfl_sync(kAllLanes, c, from, G);
+                if (!m) key = KEY_EMPTY;
+                m &= m - 1u;
+                const unsigned long long up = __shfl_up_sync(kAllLanes, e[0], 1, G);
+                if (L == 2) {
+                    unsigned long long up1 = __shfl_up_sync(kAllLanes, e[L - 1], 1, G);
+                    const unsigned long long last = __shfl_sync(kAllLanes, e[0], G - 1, G);
+                    if (lane == 0) up1 = last;
+                    if (key < e[L - 1]) e[L - 1] = up1 > key ? up1 : key;
+                }
+                if (key < e[0]) e[0] = (lane && up > key) ? up : key;
+            }
+            return;
+        }
+#pragma unroll
+        for (int size = 2; size <= G; size <<= 1) {
+#pragma unroll
+            for (int stride = size >> 1; stride > 0; stride >>= 1)
+                c = pick(c, stride,
+                         ((lane & unsigned(stride)) == 0) == ((lane & unsigned(size)) == 0));
+        }
+        const unsigned long long r = __shfl_xor_sync(kAllLanes, c, G - 1);
+        if (r < e[L - 1]) e[L - 1] = r;
+        if (L == 2 && e[L - 1] < e[0]) {
+            const unsigned long long x = e[0];
+            e[0] = e[L - 1];
+            e[L - 1] = x;
+        }
+#pragma unroll
+        for (int h = 0; h < L; ++h)
+#pragma unroll
+            for (int stride = G >> 1; stride > 0; stride >>= 1)
+                e[h] = pick(e[h], stride, (lane & unsigned(stride)) == 0);
+    }
+};
+
 // One value per lane of a group summed in lane order, for up to 9 value
 // columns at once: each column is a row of shared memory and one lane adds
 // up one row from 0, as the reference's loop over the list does (a lane that
@@ -390,6 +451,121 @@ __device__ __forceinline__ AvoidAcc lanes_avoid(const Self& me, float min_time, 
         a.threat_speed = ts;
     }
     return a;
+}
+
+// The behaviours order[first..] of one agent over its lanes' neighbours.
+template <int G>
+__device__ __forceinline__ void lanes_behaviours(const StepDev& p, unsigned need, unsigned first,
+                                                 const Self& me, unsigned lane,
+                                                 const LaneNeighbour& nb, LaneSums<G> sums,
+                                                 unsigned& applied, V3& steer) {
+    const FlockParams fs = flock_params(p.sep, p.sep_dsq), fa = flock_params(p.ali, p.ali_dsq),
+                      fc = flock_params(p.coh, p.coh_dsq);
+    V3 r_sep, r_ali, r_coh;
+    lanes_flock(need, fs, fa, fc, me, lane, nb, sums, r_sep, r_ali, r_coh);
+    CloseAcc close;
+    AvoidAcc avoid;
+    if (need & NEED_CLOSE) close = lanes_close<G>(me, p.min_sep, nb);
+    if (need & NEED_AVOID) avoid = lanes_avoid<G>(me, p.min_time_col, p.k, nb);
+#pragma unroll 1
+    for (unsigned o = first; o < p.n_order; ++o) {
+        switch ((p.order_packed >> (3u * o)) & 7u) {
+            case GS_B_SEPARATION:
+                if (need & NEED_SEP) flock_apply(r_sep, fs, SEPARATION_BIT, applied, steer);
+                break;
+            case GS_B_ALIGNMENT:
+                if (need & NEED_ALI) flock_apply(r_ali, fa, ALIGNMENT_BIT, applied, steer);
+                break;
+            case GS_B_COHESION:
+                if (need & NEED_COH) flock_apply(r_coh, fc, COHESION_BIT, applied, steer);
+                break;
+            case GS_B_SEEK:
+                seek_finish(v3(p.seek_target[0], p.seek_target[1], p.seek_target[2]), p.w_seek,
+                            p.mask_seek, me, applied, steer);
+                break;
+            case GS_B_AVOID_NEIGHBORS:
+                if (need & NEED_AVOID) {
+                    if (need & NEED_CLOSE)
+                        close_finish(close, p.w_avoid, p.mask_avoid, applied, steer);
+                    avoid_finish(avoid, p.w_avoid, p.mask_avoid, me, applied, steer);
+                }
+                break;
+            case GS_B_FOLLOW_PATH:
+                follow_path_finish(p.path, p.path_time, p.w_path, p.mask_path, me, applied, steer);
+                break;
+            default: break;
+        }
+    }
+}
+
+// The four tests of a wall line (touching, then the three feelers, walls_add)
+// on lanes 0 to 3 of the group; the line's result is then taken in their order.
+template <int G>
+__device__ __forceinline__ void lanes_wall_line(WallAcc& wa, const Self& me, unsigned lane,
+                                                unsigned line, bool on, V3 ls, V3 le, V3 ln) {
+    const unsigned t = lane & 3u;
+    const V3 end = t == 0 ? add(me.pos, mul(neg(ln), me.radius))
+                          : t == 1 ? wa.feelers[0] : t == 2 ? wa.feelers[1] : wa.feelers[2];
+    V3 ip = v3(0.f, 0.f, 0.f);
+    const bool hit = on && lines_intersect(me.pos, end, ls, le, ip);
+    const float d = distance(me.pos, ip);
+    const unsigned hits = lanes_ballot<G>(hit) & 15u;
+    unsigned from = 0;
+#pragma unroll
+    for (unsigned f = 0; f < 4; ++f) {
+        const float df = __shfl_sync(kAllLanes, d, int(f), G);
+        if (!((hits >> f) & 1u)) continue;
+        if (f == 0) {
+            wa.touching = true;
+            wa.nearest_normal = ln;
+            wa.nearest_d = df;
+        } else if (df < wa.nearest_d) {
+            wa.nearest_d = df;
+            wa.nearest_line = line;
+            wa.feeler_index = f - 1;
+            wa.nearest_normal = ln;
+            from = f;
+        }
+    }
+    const V3 at = lanes_get<G>(ip, from);
+    if (from) wa.nearest_ip = at;
+}
+
+// Avoid-walls for one agent (its box: that of its KNN): the nearest walls'
+// list, then their lines in order; may move the agent.
+template <int G, int R>
+__device__ __forceinline__ void lanes_walls(const WallRefs& W, const Scene& sc, const StepDev& p,
+                                            Self& me, unsigned lane, const Box& box,
+                                            unsigned& applied, V3& steer,
+                                            unsigned* rows = nullptr) {
+    const bool walls = sc.n_walls > 0 && W.pos_id != nullptr;
+    if (__any_sync(kAllLanes, walls)) {
+        Box wb = box;
+        if (!walls) {  // a scene without walls searches an empty box
+            wb.y0 = 1;
+            wb.y1 = 0;
+        }
+        const LaneEntry<G> wl =
+            lanes_knn<G, R>(p.knw, lane, me.pos, UINT_MAX, sc.grid, wb, sc.wall_cell_offset,
+                            W.cell_start, W.pos_id, rows);
+        const unsigned found = lanes_ballot<G>(walls && lane < p.knw && wl.slot != UINT_MAX &&
+                                               key_id(wl.key) < sc.n_walls);
+        WallAcc wa;
+        walls_init(wa, me, p.min_time_wall);
+        const unsigned lines = __popc(found);  // the list is filled from rank 0
+        const unsigned most = __reduce_max_sync(kAllLanes, lines);
+        for (unsigned r = 0; r < most; ++r) {
+            const unsigned line = unsigned(__shfl_sync(kAllLanes, wl.key, int(r), G));
+            const bool on = r < lines;
+            const unsigned g = on ? sc.wall_offset + line : 0u;
+            lanes_wall_line<G>(wa, me, lane, line, on, v3(W.start[g]), v3(W.end[g]),
+                               v3(W.normal[g]));
+        }
+        if (walls) walls_finish(wa, p.w_walls, p.mask_walls, me, applied, steer);
+        else if (!(applied & p.mask_walls)) steer = add(mul(v3(0.f, 0.f, 0.f), p.w_walls), steer);
+    } else if (!(applied & p.mask_walls)) {
+        steer = add(mul(v3(0.f, 0.f, 0.f), p.w_walls), steer);
+    }
 }
 
 }  // namespace gs

@@ -220,6 +220,12 @@ constexpr unsigned kRetryListK = 32;
 constexpr unsigned kRetryListCap = 16384;
 constexpr unsigned kRetryNotListed = 0xfffffffeu;
 
+// A wall set on the device: segments, and their midpoints by cell.
+struct WallRefs {
+    const float4 *start, *end, *normal, *pos_id;
+    const unsigned* cell_start;
+};
+
 struct FusedLaunch {
     Fused A, B;
     uint2* cellrank;
@@ -283,8 +289,9 @@ gs_status fused_step_lanes(const FusedLaunch& L, const StepDev& p, cudaStream_t 
                            PhaseHook* hook);
 bool lanes_preferred(unsigned n, bool walls);
 // slot_of: capacity words of scratch (each agent's slot, then the gather).
+// in_order: A's slots are agent indices already.
 gs_status fused_to_reference(Fused A, unsigned n, const Scene* scenes, unsigned* slot_of,
-                             GroupView g, cudaStream_t st);
+                             bool in_order, GroupView g, cudaStream_t st);
 // ---- adjoint of the fused flocking step -------------------------------------------
 // Inputs recorded by a forward step (FusedLaunch::rec_*), the agents' constant
 // limits, and the adjoints of the step's outputs; accumulates the adjoints of

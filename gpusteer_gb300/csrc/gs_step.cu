@@ -1134,7 +1134,7 @@ __global__ void k_to_reference(Fused A, unsigned n, const unsigned* __restrict__
                                GroupView g) {
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const unsigned s = slot_of[i];
+    const unsigned s = slot_of ? slot_of[i] : i;
     const float4 f0 = A.f[0][s], f1 = A.f[1][s], f2 = A.f[2][s], f3 = A.f[3][s], f4v = A.f[4][s];
     g.position[i] = make_float4(f0.x, f0.y, f0.z, 0.f);
     g.direction[i] = make_float4(f1.x, f1.y, f1.z, 0.f);
@@ -1150,10 +1150,10 @@ __global__ void k_to_reference(Fused A, unsigned n, const unsigned* __restrict__
 }
 
 gs_status fused_to_reference(Fused A, unsigned n, const Scene* scenes, unsigned* slot_of,
-                             GroupView g, cudaStream_t st) {
+                             bool in_order, GroupView g, cudaStream_t st) {
     if (n == 0) return GS_OK;
-    k_slot_of<<<blocks_for(n), kBlock, 0, st>>>(A, n, scenes, slot_of);
-    k_to_reference<<<blocks_for(n), kBlock, 0, st>>>(A, n, slot_of, g);
+    if (!in_order) k_slot_of<<<blocks_for(n), kBlock, 0, st>>>(A, n, scenes, slot_of);
+    k_to_reference<<<blocks_for(n), kBlock, 0, st>>>(A, n, in_order ? nullptr : slot_of, g);
     GS_LAUNCHED("fused_to_reference");
     return GS_OK;
 }
