@@ -114,15 +114,16 @@ GS_HD void alignment_add(FlockAcc& a, const FlockParams& p, V3 dir, V3 offset, f
     }
 }
 // kind 0 separation, 1 alignment, 2 cohesion (…CUDAKernel.cu:119-134 of each).
+template <bool FLAT = false>
 GS_HD void flock_finish(int kind, const FlockAcc& a, const FlockParams& p, const Self& s,
                         unsigned& applied, V3& steer) {
     if (applied & p.mask) return;
     V3 r = a.sum;
     if (a.n > 0) {
-        const V3 mean = dvd(a.sum, float(a.n));
-        if (kind == 0) r = normalize(mean);
-        else if (kind == 1) r = normalize(sub(mean, s.dir));
-        else r = normalize(sub(mean, s.pos));
+        const V3 mean = dvd<FLAT>(a.sum, float(a.n));
+        if (kind == 0) r = normalize<FLAT>(mean);
+        else if (kind == 1) r = normalize<FLAT>(sub(mean, s.dir));
+        else r = normalize<FLAT>(sub(mean, s.pos));
     }
     r = mul(r, p.w);
     const unsigned bit = kind == 0 ? SEPARATION_BIT : kind == 1 ? ALIGNMENT_BIT : COHESION_BIT;
@@ -131,12 +132,13 @@ GS_HD void flock_finish(int kind, const FlockAcc& a, const FlockParams& p, const
 }
 
 // ---- SteerForSeekCUDAKernel.cu:41-71 ------------------------------------------------
+template <bool FLAT = false>
 GS_HD void seek_finish(V3 target, float w, unsigned mask, const Self& s, unsigned& applied,
                        V3& steer) {
     if (applied & mask) return;
     const V3 desired = sub(target, s.pos);
     V3 r = sub(desired, s.dir);
-    r = mul(normalize(r), w);
+    r = mul(normalize<FLAT>(r), w);
     if (!is_zero(r)) applied |= SEEK_BIT;
     steer = add(r, steer);
 }
@@ -273,9 +275,10 @@ GS_HD void close_add(CloseAcc& a, const Self& s, float min_sep, float knn_dist, 
         a.found = true;
     }
 }
+template <bool FLAT = false>
 GS_HD void close_finish(const CloseAcc& a, float w, unsigned mask, unsigned& applied, V3& steer) {
     if (applied & mask) return;
-    const V3 r = mul(normalize(a.steer), w);
+    const V3 r = mul(normalize<FLAT>(a.steer), w);
     if (!is_zero(r)) applied |= AVOID_CLOSE_NEIGHBORS_BIT;
     steer = add(r, steer);
 }
@@ -295,10 +298,11 @@ GS_HD void avoid_init(AvoidAcc& a, float min_time) {
 }
 // `threat_at` keeps the nearest-approach position of the last candidate that
 // passed the time test, as in the reference (:330-340).
+template <bool FLAT = false>
 GS_HD void avoid_add(AvoidAcc& a, const Self& s, unsigned bid, V3 bpos, V3 bdir, float bspeed,
                      float bradius) {
     const float danger = s.radius + bradius;
-    const float time = nearest_approach_time(s.pos, s.dir, s.speed, bpos, bdir, bspeed);
+    const float time = nearest_approach_time<FLAT>(s.pos, s.dir, s.speed, bpos, bdir, bspeed);
     if (time >= 0.f && time < a.min_t) {
         if (nearest_approach_positions(s.pos, s.dir, s.speed, bpos, bdir, bspeed, time,
                                        a.threat_at) < danger) {
@@ -310,6 +314,7 @@ GS_HD void avoid_add(AvoidAcc& a, const Self& s, unsigned bid, V3 bpos, V3 bdir,
         }
     }
 }
+template <bool FLAT = false>
 GS_HD void avoid_finish(const AvoidAcc& a, float w, unsigned mask, const Self& s,
                         unsigned& applied, V3& steer) {
     if (applied & (mask | AVOID_CLOSE_NEIGHBORS_BIT)) return;  // SteerToAvoidNeighborsCUDA.cu:159
@@ -328,7 +333,7 @@ GS_HD void avoid_finish(const AvoidAcc& a, float w, unsigned mask, const Self& s
         st = (side_dot > 0.f) ? -1.f : 1.f;
     }
     V3 r = mul(s.side, st);
-    r = mul(normalize(r), w);
+    r = mul(normalize<FLAT>(r), w);
     if (!is_zero(r)) applied |= AVOID_NEIGHBORS_BIT;
     steer = add(r, steer);
 }
@@ -349,10 +354,11 @@ GS_HD void avoid_lite_init(AvoidLite& a, float min_time) {
     a.last_t = 0.f;
     a.threat = a.last = UINT_MAX;
 }
+template <bool FLAT = false>
 GS_HD void avoid_lite_add(AvoidLite& a, const Self& s, unsigned rank, V3 bpos, V3 bdir,
                           float bspeed, float bradius) {
     const float danger = s.radius + bradius;
-    const float time = nearest_approach_time(s.pos, s.dir, s.speed, bpos, bdir, bspeed);
+    const float time = nearest_approach_time<FLAT>(s.pos, s.dir, s.speed, bpos, bdir, bspeed);
     if (time >= 0.f && time < a.min_t) {
         V3 at;
         a.last = rank;
@@ -454,6 +460,7 @@ GS_HD void walls_add(WallAcc& a, const Self& s, unsigned line, V3 ls, V3 le, V3 
 }
 // Applies the result: may move the agent (anti-penetration) and adds the
 // weighted wall steering.  Returns false when masked (nothing changes).
+template <bool FLAT = false>
 GS_HD bool walls_finish(const WallAcc& a, float w, unsigned mask, Self& s, unsigned& applied,
                         V3& steer) {
     if (applied & mask) return false;
@@ -461,7 +468,7 @@ GS_HD bool walls_finish(const WallAcc& a, float w, unsigned mask, Self& s, unsig
     if (a.touching) {
         const float pen = s.radius - a.nearest_d;
         s.pos = add(s.pos, mul(a.nearest_normal, pen));
-        s.dir = normalize(perpendicular_component(s.dir, a.nearest_normal));
+        s.dir = normalize<FLAT>(perpendicular_component(s.dir, a.nearest_normal));
         applied |= ANTI_PENETRATION_WALL;
     } else if (a.nearest_line != UINT_MAX) {
         const V3 f = a.feeler_index == 0 ? a.feelers[0]
@@ -478,15 +485,16 @@ GS_HD bool walls_finish(const WallAcc& a, float w, unsigned mask, Self& s, unsig
 // ---- UpdateCUDAKernel.cu:78-123 -----------------------------------------------------
 // A new speed of 0 keeps the previous side vector (the reference writes back
 // uninitialised shared memory there).
+template <bool FLAT = false>
 GS_HD void integrate(Self& s, V3 steer, float dt) {
     steer = truncate_length(steer, s.max_force);
-    const V3 acc = dvd(steer, s.mass);
+    const V3 acc = dvd<FLAT>(steer, s.mass);
     V3 vel = add(mul(s.dir, s.speed), mul(acc, dt));
     vel = truncate_length(vel, s.max_speed);
     s.speed = length(vel);
     if (s.speed > 0.f) {
-        s.dir = dvd(vel, s.speed);
-        s.side = normalize(cross(s.dir, s.up));
+        s.dir = dvd<FLAT>(vel, s.speed);
+        s.side = normalize<FLAT>(cross(s.dir, s.up));
         s.up = cross(s.side, s.dir);
     }
     s.pos = add(s.pos, mul(vel, dt));

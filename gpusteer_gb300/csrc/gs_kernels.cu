@@ -662,7 +662,7 @@ __global__ void k_flock(GroupView g, const unsigned* __restrict__ knn, unsigned 
                 in = ahead < 0 ? forward_component(dir, offset, dsq) > fp.cos_max : ahead > 0;
             }
             if (!in) continue;
-            acc.sum = add(acc.sum, KIND == 0 ? dvd(offset, -dsq) : KIND == 1 ? v3(bd[j]) : v3(bp[j]));
+            acc.sum = add(acc.sum, KIND == 0 ? dvd<true>(offset, -dsq) : KIND == 1 ? v3(bd[j]) : v3(bp[j]));
             acc.n++;
         }
         return true;
@@ -670,7 +670,7 @@ __global__ void k_flock(GroupView g, const unsigned* __restrict__ knn, unsigned 
     Self me;
     me.pos = pos;
     me.dir = dir;
-    flock_finish(KIND, acc, fp, me, applied, steer);
+    flock_finish<true>(KIND, acc, fp, me, applied, steer);
     g.steering[i] = f4(steer, 0.f);
     g.applied[i] = applied;
 }
@@ -702,7 +702,7 @@ __global__ void k_seek(GroupView g, float tx, float ty, float tz, float w, unsig
     me.pos = v3(g.position[i]);
     me.dir = v3(g.direction[i]);
     V3 steer = v3(g.steering[i]);
-    seek_finish(v3(tx, ty, tz), w, mask, me, applied, steer);
+    seek_finish<true>(v3(tx, ty, tz), w, mask, me, applied, steer);
     g.steering[i] = f4(steer, 0.f);
     g.applied[i] = applied;
 }
@@ -803,11 +803,11 @@ __global__ void __launch_bounds__(kBlock, 2) k_avoid(GroupView g, const unsigned
 #pragma unroll
         for (unsigned j = 0; j < kCallChunk; ++j)
             if (ok[j] && avoid_time_may_fall_in(me, min_time, v3(bp[j]), v3(bd[j]), bv[j]))
-                avoid_add(acc, me, b[j], v3(bp[j]), v3(bd[j]), bv[j], br[j]);
+                avoid_add<true>(acc, me, b[j], v3(bp[j]), v3(bd[j]), bv[j], br[j]);
         return true;
     });
     if (acc.threat == UINT_MAX) return;
-    avoid_finish(acc, w, mask, me, applied, steer);
+    avoid_finish<true>(acc, w, mask, me, applied, steer);
     g.steering[i] = f4(steer, 0.f);
     g.applied[i] = applied;
 }
@@ -873,7 +873,7 @@ __global__ void k_update(GroupView g, float dt) {
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     Self me = load_self(g, i);
-    integrate(me, v3(g.steering[i]), dt);
+    integrate<true>(me, v3(g.steering[i]), dt);
     g.side[i] = make_float3(me.side.x, me.side.y, me.side.z);
     g.up[i] = make_float3(me.up.x, me.up.y, me.up.z);
     g.direction[i] = f4(me.dir, 0.f);

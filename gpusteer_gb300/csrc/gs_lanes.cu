@@ -49,8 +49,8 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_step(FusedLaunch L, StepDe
     unsigned applied = p.clear_applied ? 0u : __float_as_uint(f4v.z);
     V3 steer = p.dirty ? v3(L.B.f[5][s]) : v3(0.f, 0.f, 0.f);
     const LaneNeighbour n{ok, v3(b0), v3(b1), b1.w, br, key_dist(nb.key)};
-    lanes_behaviours<G>(p, need, 0, me, lane, n, LaneSums<G>::of(sh), applied, steer);
-    integrate(me, steer, p.dt);
+    lanes_behaviours<G, R == 3>(p, need, 0, me, lane, n, LaneSums<G>::of(sh), applied, steer);
+    integrate<R == 3>(me, steer, p.dt);
     if (act && lane == 0) store_next(L, s, me, id, scene, sc, p.wrap_mode);
 }
 
@@ -115,14 +115,15 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_rest(FusedLaunch L, StepDe
     unsigned applied = __float_as_uint(w2.w);
     V3 steer = v3(w2);
     const LaneNeighbour n{ok, v3(b0), v3(b1), b1.w, b0.w, kd};
-    lanes_behaviours<G>(p, need, 1, me, lane, n, LaneSums<G>::of(sh), applied, steer);
-    integrate(me, steer, p.dt);
+    lanes_behaviours<G, true>(p, need, 1, me, lane, n, LaneSums<G>::of(sh), applied, steer);
+    integrate<true>(me, steer, p.dt);
     const Scene sc = L.scenes[scene];
     if (act && lane == 0) store_next(L, s, me, id, scene, sc, p.wrap_mode);
 }
 
 // ---- one behaviour per launch ------------------------------------------------------------------
-// The per-function behaviours of small groups: lane r of an agent's group takes
+// The per-function behaviours of small groups (whose worlds may be flat: they
+// divide vectors as flat ones): lane r of an agent's group takes
 // list entry r.  An index past the other group ends the list, as in the
 // reference's kernels.
 template <int G>
@@ -166,7 +167,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_flock_lanes(GroupView g,
     nb.pos = nb.ok ? v3(o.position[b]) : me.pos;
     nb.dir = nb.ok && KIND == 1 ? v3(o.direction[b]) : me.dir;
     V3 r_sep, r_ali, r_coh;
-    lanes_flock(need, fp, fp, fp, me, lane, nb, LaneSums<G>::of(sh), r_sep, r_ali, r_coh);
+    lanes_flock<true>(need, fp, fp, fp, me, lane, nb, LaneSums<G>::of(sh), r_sep, r_ali, r_coh);
     if (!act || lane != 0 || (applied & fp.mask)) return;
     flock_apply(KIND == 0 ? r_sep : KIND == 1 ? r_ali : r_coh, fp,
                 KIND == 0 ? SEPARATION_BIT : KIND == 1 ? ALIGNMENT_BIT : COHESION_BIT, applied,
@@ -210,11 +211,11 @@ __global__ void __launch_bounds__(kLaneBlock) k_avoid_lanes(GroupView g,
     if constexpr (CLOSE) {
         const CloseAcc c = lanes_close<G>(me, limit, nb);
         if (!act || lane != 0 || (applied & mask)) return;
-        close_finish(c, w, mask, applied, steer);
+        close_finish<true>(c, w, mask, applied, steer);
     } else {
-        const AvoidAcc a = lanes_avoid<G>(me, limit, k, nb);
+        const AvoidAcc a = lanes_avoid<G, true>(me, limit, k, nb);
         if (!act || lane != 0 || a.threat == UINT_MAX) return;
-        avoid_finish(a, w, mask, me, applied, steer);
+        avoid_finish<true>(a, w, mask, me, applied, steer);
     }
     g.steering[i] = f4(steer, 0.f);
     g.applied[i] = applied;

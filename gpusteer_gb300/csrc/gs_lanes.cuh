@@ -342,7 +342,7 @@ struct LaneNeighbour {
 
 // The weighted separation, alignment and cohesion vectors (flock_finish up to
 // its mask test) of the behaviours in `need`; the others' are left unset.
-template <int G>
+template <bool FLAT = false, int G = 32>
 __device__ __forceinline__ void lanes_flock(unsigned need, const FlockParams& fs,
                                             const FlockParams& fa, const FlockParams& fc,
                                             const Self& me, unsigned lane,
@@ -352,7 +352,7 @@ __device__ __forceinline__ void lanes_flock(unsigned need, const FlockParams& fs
     const V3 zero = v3(0.f, 0.f, 0.f);
     const V3 offset = sub(nb.pos, me.pos);
     const float dsq = dot(offset, offset), d = sqrtf(dsq);
-    const float ahead = dot(me.dir, dvd(offset, d));
+    const float ahead = dot(me.dir, dvd<FLAT>(offset, d));
     auto member = [&](const FlockParams& f) {  // inBoidNeighborhood, FlockingCommon.cuh:4-30
         return nb.ok && (d < f.min_d || (!(d > f.max_d) && ahead > f.cos_max));
     };
@@ -360,7 +360,7 @@ __device__ __forceinline__ void lanes_flock(unsigned need, const FlockParams& fs
     if (need & NEED_SEP) {
         const bool in = member(fs);
         n_sep = __popc(lanes_ballot<G>(in));
-        sums.put(0, lane, in ? dvd(offset, -dsq) : zero);
+        sums.put(0, lane, in ? dvd<FLAT>(offset, -dsq) : zero);
     }
     if (need & NEED_ALI) {
         const bool in = member(fa);
@@ -379,8 +379,8 @@ __device__ __forceinline__ void lanes_flock(unsigned need, const FlockParams& fs
     const float w = kind == 0 ? fs.w : kind == 1 ? fa.w : fc.w;
     V3 r = zero;
     if (n) {
-        const V3 mean = dvd(sums.sum(3 * kind), float(n));
-        r = normalize(kind == 0 ? mean : sub(mean, kind == 1 ? me.dir : me.pos));
+        const V3 mean = dvd<FLAT>(sums.sum(3 * kind), float(n));
+        r = normalize<FLAT>(kind == 0 ? mean : sub(mean, kind == 1 ? me.dir : me.pos));
     }
     r = mul(r, w);
     if (need & NEED_SEP) r_sep = lanes_get<G>(r, 0);
@@ -413,7 +413,7 @@ __device__ __forceinline__ CloseAcc lanes_close(const Self& me, float min_sep,
 // avoid_add over the list: every lane its neighbour's approach time and
 // distance, then the reference's pass over them, whose window [0, min_t) only
 // narrows (`at` keeps the last neighbour in it, threat or not).
-template <int G>
+template <int G, bool FLAT = false>
 __device__ __forceinline__ AvoidAcc lanes_avoid(const Self& me, float min_time, unsigned k,
                                                 const LaneNeighbour& nb) {
     AvoidAcc a;
@@ -423,7 +423,7 @@ __device__ __forceinline__ AvoidAcc lanes_avoid(const Self& me, float min_time, 
     bool danger = false;
     if (nb.ok) {
         const float time =
-            nearest_approach_time(me.pos, me.dir, me.speed, nb.pos, nb.dir, nb.speed);
+            nearest_approach_time<FLAT>(me.pos, me.dir, me.speed, nb.pos, nb.dir, nb.speed);
         if (time >= 0.f) t = time;
         danger = nearest_approach_positions(me.pos, me.dir, me.speed, nb.pos, nb.dir, nb.speed,
                                             time, at) < me.radius + nb.radius;
@@ -454,7 +454,7 @@ __device__ __forceinline__ AvoidAcc lanes_avoid(const Self& me, float min_time, 
 }
 
 // The behaviours order[first..] of one agent over its lanes' neighbours.
-template <int G>
+template <int G, bool FLAT>
 __device__ __forceinline__ void lanes_behaviours(const StepDev& p, unsigned need, unsigned first,
                                                  const Self& me, unsigned lane,
                                                  const LaneNeighbour& nb, LaneSums<G> sums,
@@ -462,11 +462,11 @@ __device__ __forceinline__ void lanes_behaviours(const StepDev& p, unsigned need
     const FlockParams fs = flock_params(p.sep, p.sep_dsq), fa = flock_params(p.ali, p.ali_dsq),
                       fc = flock_params(p.coh, p.coh_dsq);
     V3 r_sep, r_ali, r_coh;
-    lanes_flock(need, fs, fa, fc, me, lane, nb, sums, r_sep, r_ali, r_coh);
+    lanes_flock<FLAT>(need, fs, fa, fc, me, lane, nb, sums, r_sep, r_ali, r_coh);
     CloseAcc close;
     AvoidAcc avoid;
     if (need & NEED_CLOSE) close = lanes_close<G>(me, p.min_sep, nb);
-    if (need & NEED_AVOID) avoid = lanes_avoid<G>(me, p.min_time_col, p.k, nb);
+    if (need & NEED_AVOID) avoid = lanes_avoid<G, FLAT>(me, p.min_time_col, p.k, nb);
 #pragma unroll 1
     for (unsigned o = first; o < p.n_order; ++o) {
         switch ((p.order_packed >> (3u * o)) & 7u) {
@@ -480,14 +480,14 @@ __device__ __forceinline__ void lanes_behaviours(const StepDev& p, unsigned need
                 if (need & NEED_COH) flock_apply(r_coh, fc, COHESION_BIT, applied, steer);
                 break;
             case GS_B_SEEK:
-                seek_finish(v3(p.seek_target[0], p.seek_target[1], p.seek_target[2]), p.w_seek,
-                            p.mask_seek, me, applied, steer);
+                seek_finish<FLAT>(v3(p.seek_target[0], p.seek_target[1], p.seek_target[2]), p.w_seek,
+                                  p.mask_seek, me, applied, steer);
                 break;
             case GS_B_AVOID_NEIGHBORS:
                 if (need & NEED_AVOID) {
                     if (need & NEED_CLOSE)
-                        close_finish(close, p.w_avoid, p.mask_avoid, applied, steer);
-                    avoid_finish(avoid, p.w_avoid, p.mask_avoid, me, applied, steer);
+                        close_finish<FLAT>(close, p.w_avoid, p.mask_avoid, applied, steer);
+                    avoid_finish<FLAT>(avoid, p.w_avoid, p.mask_avoid, me, applied, steer);
                 }
                 break;
             case GS_B_FOLLOW_PATH:

@@ -29,12 +29,35 @@ GS_HD V3 add(V3 a, V3 b) { return V3{a.x + b.x, a.y + b.y, a.z + b.z}; }
 GS_HD V3 sub(V3 a, V3 b) { return V3{a.x - b.x, a.y - b.y, a.z - b.z}; }
 GS_HD V3 neg(V3 a) { return V3{-a.x, -a.y, -a.z}; }
 GS_HD V3 mul(V3 a, float s) { return V3{a.x * s, a.y * s, a.z * s}; }
-GS_HD V3 dvd(V3 a, float s) { return V3{a.x / s, a.y / s, a.z / s}; }
+// a / s where a is often zero: a flat world's components along y, in every
+// offset, heading and force.  A zero numerator takes the division's
+// out-of-line path (on GB300 three times the time of another), with the whole
+// warp of a flat world; here it divides 1 instead and the quotient, a zero
+// signed as the operands are, is put in its place.  Every other case (s zero
+// or NaN among them) is the division itself.
+GS_HD float div_often_zero(float a, float s) {
+#ifdef __CUDA_ARCH__
+    const bool zero = a == 0.f && fabsf(s) > 0.f;
+    const float q = (zero ? 1.f : a) / s;
+    return zero ? __uint_as_float(__float_as_uint(a) ^ (__float_as_uint(s) & 0x80000000u)) : q;
+#else
+    return a / s;
+#endif
+}
+// FLAT, here and in what divides vectors: the world is probably flat, so y
+// goes through div_often_zero.  The results do not depend on it; the choke
+// point's rest phase runs in 433 instead of 485 us (256 scenes), and the 3D
+// flock's kernel would take 1.2 % longer.
+template <bool FLAT = false>
+GS_HD V3 dvd(V3 a, float s) {
+    return V3{a.x / s, FLAT ? div_often_zero(a.y, s) : a.y / s, a.z / s};
+}
 GS_HD float dot(V3 a, V3 b) { return ((a.x * b.x) + (a.y * b.y)) + (a.z * b.z); }
 GS_HD float length(V3 a) { return sqrtf(dot(a, a)); }
+template <bool FLAT = false>
 GS_HD V3 normalize(V3 v) {
     const float len = length(v);
-    return (len > 0.f) ? dvd(v, len) : v;
+    return (len > 0.f) ? dvd<FLAT>(v, len) : v;
 }
 GS_HD V3 cross(V3 a, V3 b) {
     return V3{(a.y * b.z) - (a.z * b.y), (a.z * b.x) - (a.x * b.z), (a.x * b.y) - (a.y * b.x)};
@@ -132,13 +155,14 @@ GS_HD bool in_boid_neighborhood(V3 dir, V3 offset, float d, float min_d, float m
 }
 
 // ---- SteerToAvoidNeighborsCUDAKernel.cu:192-233 -----------------------------------
+template <bool FLAT = false>
 GS_HD float nearest_approach_time(V3 pos, V3 dir, float speed, V3 opos, V3 odir, float ospeed) {
     const V3 my_vel = mul(dir, speed);
     const V3 other_vel = mul(odir, ospeed);
     const V3 rel_vel = sub(other_vel, my_vel);
     const float rel_speed = length(rel_vel);
     if (rel_speed == 0.f) return 0.f;
-    const V3 rel_tangent = dvd(rel_vel, rel_speed);
+    const V3 rel_tangent = dvd<FLAT>(rel_vel, rel_speed);
     const V3 rel_pos = sub(pos, opos);
     const float projection = dot(rel_tangent, rel_pos);
     return projection / rel_speed;

@@ -207,6 +207,7 @@ struct Accs {
 // specialised for one configuration (the unused accumulators then vanish).
 // gs, ga, gc: the agent's angle gates of the three flocking behaviours.
 // offset = bpos - me.pos and dsq = dot(offset, offset), computed by the caller.
+template <bool FLAT = false>
 __device__ __forceinline__ void accumulate_at(Accs& a, const StepDev& p, unsigned need,
                                               const FlockParams& fs, const FlockParams& fa,
                                               const FlockParams& fc, AngleGate gs_, AngleGate ga,
@@ -246,7 +247,7 @@ __device__ __forceinline__ void accumulate_at(Accs& a, const StepDev& p, unsigne
         }
         if (need & NEED_SEP) {
             if (in_s) {
-                a.sep.sum = add(a.sep.sum, dvd(offset, -dsq));
+                a.sep.sum = add(a.sep.sum, dvd<FLAT>(offset, -dsq));
                 a.sep.n++;
             }
         }
@@ -331,7 +332,7 @@ __device__ __forceinline__ bool packed_avoid_time_may_fall_in(const PackedSelf& 
 // A runtime loop over the packed order (3 bits per entry), so each
 // behaviour's code appears once in the kernel rather than once per order
 // slot; `need` drops the code of behaviours a specialised kernel never runs.
-template <class Fetch>
+template <bool FLAT = false, class Fetch>
 __device__ __forceinline__ void finish_all(const Accs& a, const StepDev& p, unsigned need,
                                            unsigned first, const FlockParams& fs,
                                            const FlockParams& fa, const FlockParams& fc,
@@ -341,24 +342,24 @@ __device__ __forceinline__ void finish_all(const Accs& a, const StepDev& p, unsi
     for (unsigned o = first; o < p.n_order; ++o) {
         switch ((p.order_packed >> (3u * o)) & 7u) {
             case GS_B_SEPARATION:
-                if (need & NEED_SEP) flock_finish(0, a.sep, fs, me, applied, steer);
+                if (need & NEED_SEP) flock_finish<FLAT>(0, a.sep, fs, me, applied, steer);
                 break;
             case GS_B_ALIGNMENT:
-                if (need & NEED_ALI) flock_finish(1, a.ali, fa, me, applied, steer);
+                if (need & NEED_ALI) flock_finish<FLAT>(1, a.ali, fa, me, applied, steer);
                 break;
             case GS_B_COHESION:
-                if (need & NEED_COH) flock_finish(2, a.coh, fc, me, applied, steer);
+                if (need & NEED_COH) flock_finish<FLAT>(2, a.coh, fc, me, applied, steer);
                 break;
             case GS_B_SEEK:
-                seek_finish(v3(p.seek_target[0], p.seek_target[1], p.seek_target[2]), p.w_seek,
-                            p.mask_seek, me, applied, steer);
+                seek_finish<FLAT>(v3(p.seek_target[0], p.seek_target[1], p.seek_target[2]), p.w_seek,
+                                  p.mask_seek, me, applied, steer);
                 break;
             case GS_B_AVOID_NEIGHBORS:
                 if (need & NEED_AVOID) {
                     if (p.avoid_close)
-                        close_finish(a.close, p.w_avoid, p.mask_avoid, applied, steer);
-                    avoid_finish(avoid_lite_full(a.avoid, fetch), p.w_avoid, p.mask_avoid, me,
-                                 applied, steer);
+                        close_finish<FLAT>(a.close, p.w_avoid, p.mask_avoid, applied, steer);
+                    avoid_finish<FLAT>(avoid_lite_full(a.avoid, fetch), p.w_avoid, p.mask_avoid, me,
+                                       applied, steer);
                 }
                 break;
             case GS_B_FOLLOW_PATH:
@@ -740,7 +741,7 @@ __device__ __forceinline__ void walls_agent(const FusedLaunch& L, const StepDev&
                 const unsigned g = sc.wall_offset + line;
                 walls_add(wa, me, line, v3(L.w_start[g]), v3(L.w_end[g]), v3(L.w_normal[g]));
             }
-            walls_finish(wa, p.w_walls, p.mask_walls, me, applied, steer);
+            walls_finish<true>(wa, p.w_walls, p.mask_walls, me, applied, steer);
         } else if (!(applied & p.mask_walls)) {
             steer = add(mul(v3(0.f, 0.f, 0.f), p.w_walls), steer);
         }
@@ -817,7 +818,7 @@ __device__ __forceinline__ void rest_agent(const FusedLaunch& L, const StepDev& 
             V3 off;
             unsigned long long o_xy;
             const float dsq = packed_offset(pq, me, b0[j], off, o_xy);
-            accumulate_at(a, p, need & ~NEED_AVOID, fs, fa, fc, gs_, ga, gc, me, i, kd, off, dsq,
+            accumulate_at<true>(a, p, need & ~NEED_AVOID, fs, fa, fc, gs_, ga, gc, me, i, kd, off, dsq,
                           v3(b0[j]), v3(b1[j]), b1[j].w, b0[j].w);
             if ((need & NEED_AVOID) &&
                 packed_avoid_time_may_fall_in(pq, o_xy, off.z, p.min_time_col, b1[j]))
@@ -830,7 +831,7 @@ __device__ __forceinline__ void rest_agent(const FusedLaunch& L, const StepDev& 
         exact_avoid &= exact_avoid - 1;
         const unsigned bs = L.knn_slot[size_t(i) * L.n + s];
         const float4 b0 = L.w0[bs], b1 = L.w1[bs];
-        avoid_lite_add(a.avoid, me, i, v3(b0), v3(b1), b1.w, b0.w);
+        avoid_lite_add<true>(a.avoid, me, i, v3(b0), v3(b1), b1.w, b0.w);
     }
     const float4 w2 = L.w2[s];
     const float4 f2 = L.B.f[2][s], f3 = L.B.f[3][s], f4v = L.B.f[4][s];
@@ -842,7 +843,7 @@ __device__ __forceinline__ void rest_agent(const FusedLaunch& L, const StepDev& 
     const unsigned id = u(reinterpret_cast<const float*>(L.B.f[0] + s)[3]), scene = u(f4v.w);
     unsigned applied = u(w2.w);
     V3 steer = v3(w2);
-    finish_all(a, p, need, 1, fs, fa, fc, me, applied, steer,
+    finish_all<true>(a, p, need, 1, fs, fa, fc, me, applied, steer,
                [&](unsigned rank, V3& bp, V3& bh, float& bsp) {
                    const unsigned bs = L.knn_slot[size_t(rank) * L.n + s];
                    const float4 b0 = L.w0[bs], b1 = L.w1[bs];
@@ -850,7 +851,7 @@ __device__ __forceinline__ void rest_agent(const FusedLaunch& L, const StepDev& 
                    bh = v3(b1);
                    bsp = b1.w;
                });
-    integrate(me, steer, p.dt);
+    integrate<true>(me, steer, p.dt);
     const Scene sc = L.scenes[scene];
     store_next(L, s, me, id, scene, sc, p.wrap_mode);
 }
