@@ -93,6 +93,7 @@ __device__ __forceinline__ void get_edge(const AdjointLaunch& A, unsigned e, V3&
 }
 
 __global__ void __launch_bounds__(kAdjBlock) k_flock_adjoint(AdjointLaunch A, StepDev p) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     float gw[3] = {0.f, 0.f, 0.f};  // separation, alignment, cohesion
     if (i < A.n) {
@@ -264,6 +265,7 @@ __global__ void __launch_bounds__(kAdjBlock) k_flock_adjoint(AdjointLaunch A, St
 
 // Files edge e = i * k + r in the bucket of its target knn[e].
 __global__ void __launch_bounds__(kAdjBlock) k_bucket_edges(AdjointLaunch A) {
+    after_previous();
     const unsigned e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= A.n * A.k) return;
     const unsigned j = A.knn[e];
@@ -286,6 +288,7 @@ __global__ void __launch_bounds__(kAdjBlock) k_bucket_edges(AdjointLaunch A) {
 constexpr unsigned kGatherChunk = 4;
 constexpr unsigned kGatherBlock = 128;
 __global__ void __launch_bounds__(kGatherBlock) k_adjoint_gather(AdjointLaunch A) {
+    after_previous();
     const unsigned j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= A.n) return;
     const unsigned deg = A.fill[j];
@@ -375,10 +378,10 @@ gs_status launch_flock_adjoint(const AdjointLaunch& A, const StepDev& p, cudaStr
     if (size_t(A.n) * A.k > 0xffffffffull) return fail(GS_ERR_INVALID_ARG, "too many KNN edges");
     // bucket fill counts and the overflow count start at zero
     GS_CUDA(cudaMemsetAsync(A.fill, 0, (size_t(A.n) + 1) * 4, st));
-    k_bucket_edges<<<adjoint_blocks(A.n * A.k), kAdjBlock, 0, st>>>(A);
+    launch_after(k_bucket_edges, adjoint_blocks(A.n * A.k), kAdjBlock, 0, st, A);
     // each agent's terms and its edges' terms, then the gather
-    k_flock_adjoint<<<adjoint_blocks(A.n), kAdjBlock, 0, st>>>(A, p);
-    k_adjoint_gather<<<blocks_for(A.n, kGatherBlock), kGatherBlock, 0, st>>>(A);
+    launch_after(k_flock_adjoint, adjoint_blocks(A.n), kAdjBlock, 0, st, A, p);
+    launch_after(k_adjoint_gather, blocks_for(A.n, kGatherBlock), kGatherBlock, 0, st, A);
     GS_LAUNCHED("flock_adjoint");
     return GS_OK;
 }

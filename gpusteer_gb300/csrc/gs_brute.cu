@@ -110,10 +110,11 @@ __device__ __forceinline__ unsigned brute_region(LaneList<G, L>& list, const Bru
 // query's place otherwise.
 template <int G, int L>
 __global__ void __launch_bounds__(kBruteBlock) k_brute_cells(
-    const float4* __restrict__ q_pos, bool by_slot, unsigned nA, const float4* __restrict__ pos_id,
-    const unsigned* __restrict__ start, const Grid* __restrict__ grid, bool self, unsigned k,
-    unsigned long long* __restrict__ evaluated, unsigned* __restrict__ idx,
-    float* __restrict__ dist) {
+    const float4* q_pos, bool by_slot, unsigned nA, const float4* pos_id,
+    const unsigned* start, const Grid* grid, bool self, unsigned k,
+    unsigned long long* evaluated, unsigned* idx,
+    float* dist) {
+    after_previous();
     __shared__ unsigned sh[kBruteBlock / G * (2 * kBruteSegs + 1)];
     __shared__ unsigned met_sh[kBruteBlock / 32];
     unsigned* segs = sh + threadIdx.x / G * (2 * kBruteSegs + 1);
@@ -182,8 +183,7 @@ template <int G, int L>
 static void brute_go(const float4* q_pos, bool by_slot, unsigned nA, const Database& B,
                      const BruteWork& w, bool self, unsigned k, unsigned* idx, float* dist,
                      cudaStream_t st) {
-    k_brute_cells<G, L><<<blocks_for(nA, kBruteBlock / G), kBruteBlock, 0, st>>>(
-        q_pos, by_slot, nA, B.pos_id, B.start, w.grid, self, k, w.evaluated, idx, dist);
+    launch_after(k_brute_cells<G, L>, blocks_for(nA, kBruteBlock / G), kBruteBlock, 0, st, q_pos, by_slot, nA, B.pos_id, B.start, w.grid, self, k, w.evaluated, idx, dist);
 }
 
 // k / 8 candidates a cell: the 27 cells then hold about 3.4 k, 8 of them (a

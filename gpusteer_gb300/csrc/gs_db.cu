@@ -82,6 +82,7 @@ __device__ __forceinline__ Grid automatic_grid(const unsigned ext[3], const unsi
 }
 
 __global__ void __launch_bounds__(kDbThreads) k_db_cluster(const __grid_constant__ DbJobs J) {
+    after_previous();
     __shared__ unsigned ws[32];
     __shared__ unsigned totals[kDbCluster], extents[kDbCluster][3];
     cg::cluster_group cluster = cg::this_cluster();
@@ -203,16 +204,18 @@ gs_status db_build_clusters(const DbJobs& J, unsigned count, cudaStream_t st) {
     if (count > kMaxDbJobs) return fail(GS_ERR_INVALID_ARG, "too many databases in one launch");
     // 16 blocks a cluster is past the portable 8: allowed per kernel and device
     GS_CUDA(cudaFuncSetAttribute(k_db_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = kDbCluster;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kDbCluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_after
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kDbCluster * count);
     cfg.blockDim = dim3(kDbThreads);
     cfg.stream = st;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
     GS_CUDA(cudaLaunchKernelEx(&cfg, k_db_cluster, J));
     return GS_OK;
 }

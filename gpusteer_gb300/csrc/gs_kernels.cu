@@ -23,8 +23,9 @@ namespace gs {
 // ---- exclusive scan (device code in gs_scan.cuh) ----------------------------------
 unsigned scan_tile_count(unsigned C) { return (C + kScanTile - 1) / kScanTile; }
 
-__global__ void __launch_bounds__(kBlock) k_scan_reduce(const unsigned* __restrict__ count,
-                                                        unsigned C, unsigned* __restrict__ tile) {
+__global__ void __launch_bounds__(kBlock) k_scan_reduce(const unsigned* count,
+                                                        unsigned C, unsigned* tile) {
+    after_previous();
     __shared__ unsigned sh[kScanTile + kScanTile / 32];
     __shared__ unsigned ws[kBlock / 32];
     scan_reduce_tile(count, C, blockIdx.x, sh, ws, tile);
@@ -32,7 +33,8 @@ __global__ void __launch_bounds__(kBlock) k_scan_reduce(const unsigned* __restri
 
 // One block scans the tile totals in place (exclusive) and writes start[C].
 __global__ void __launch_bounds__(1024) k_scan_tiles(unsigned* tile, unsigned T,
-                                                     unsigned* __restrict__ start, unsigned C) {
+                                                     unsigned* start, unsigned C) {
+    after_previous();
     __shared__ unsigned ws[32];
     __shared__ unsigned carry;
     if (threadIdx.x == 0) carry = 0;
@@ -68,9 +70,10 @@ __global__ void __launch_bounds__(1024) k_scan_tiles(unsigned* tile, unsigned T,
     if (threadIdx.x == 0) start[C] = carry;
 }
 
-__global__ void __launch_bounds__(kBlock) k_scan_apply(unsigned* __restrict__ count, unsigned C,
-                                                       const unsigned* __restrict__ tile,
-                                                       unsigned* __restrict__ start) {
+__global__ void __launch_bounds__(kBlock) k_scan_apply(unsigned* count, unsigned C,
+                                                       const unsigned* tile,
+                                                       unsigned* start) {
+    after_previous();
     __shared__ unsigned sh[kScanTile + kScanTile / 32];
     __shared__ unsigned ws[kBlock / 32];
     unsigned items[kScanItems];
@@ -101,9 +104,9 @@ __global__ void __launch_bounds__(kBlock) k_scan_apply(unsigned* __restrict__ co
 gs_status scan_counts(unsigned* count, unsigned* start, unsigned C, unsigned* tile,
                       cudaStream_t st) {
     const unsigned T = scan_tile_count(C);
-    k_scan_reduce<<<T, kBlock, 0, st>>>(count, C, tile);
-    k_scan_tiles<<<1, 1024, 0, st>>>(tile, T, start, C);
-    k_scan_apply<<<T, kBlock, 0, st>>>(count, C, tile, start);
+    launch_after(k_scan_reduce, T, kBlock, 0, st, count, C, tile);
+    launch_after(k_scan_tiles, 1, 1024, 0, st, tile, T, start, C);
+    launch_after(k_scan_apply, T, kBlock, 0, st, count, C, tile, start);
     GS_LAUNCHED("scan");
     return GS_OK;
 }
@@ -114,12 +117,13 @@ gs_status scan_counts(unsigned* count, unsigned* start, unsigned C, unsigned* ti
 // on a new grid, takes one); every block sums the totals of the tiles before its own (a
 // few thousand words from L2) and writes its tile's starts, and no block
 // waits on another (scan_apply_sparse_tile).
-__global__ void __launch_bounds__(kBlock) k_scan_apply_sparse(unsigned* __restrict__ count,
+__global__ void __launch_bounds__(kBlock) k_scan_apply_sparse(unsigned* count,
                                                               unsigned C,
-                                                              const unsigned* __restrict__ tile,
-                                                              unsigned* __restrict__ start,
+                                                              const unsigned* tile,
+                                                              unsigned* start,
                                                               unsigned T, unsigned reach,
-                                                              unsigned* __restrict__ live) {
+                                                              unsigned* live) {
+    after_previous();
     __shared__ unsigned sh[kScanTile + kScanTile / 32];
     __shared__ unsigned ws[kBlock / 32];
     scan_apply_sparse_tile(count, C, tile, start, T, blockIdx.x, reach, live, sh, ws);
@@ -128,7 +132,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_apply_sparse(unsigned* __restri
 gs_status scan_tile_totals(const unsigned* count, unsigned C, unsigned* tile, cudaStream_t st) {
     const unsigned T = scan_tile_count(C);
     if (T == 0) return GS_OK;
-    k_scan_reduce<<<T, kBlock, 0, st>>>(count, C, tile);
+    launch_after(k_scan_reduce, T, kBlock, 0, st, count, C, tile);
     GS_LAUNCHED("scan_tile_totals");
     return GS_OK;
 }
@@ -137,7 +141,7 @@ gs_status scan_counts_sparse(unsigned* count, unsigned* start, unsigned C, const
                              unsigned* live, unsigned reach, cudaStream_t st) {
     const unsigned T = scan_tile_count(C);
     if (T == 0) return GS_OK;
-    k_scan_apply_sparse<<<T, kBlock, 0, st>>>(count, C, tile, start, T, reach, live);
+    launch_after(k_scan_apply_sparse, T, kBlock, 0, st, count, C, tile, start, T, reach, live);
     GS_LAUNCHED("scan_sparse");
     return GS_OK;
 }
@@ -195,9 +199,10 @@ void db_release(Database& db) {
     db.valid = false;
 }
 
-__global__ void k_db_count(const float4* __restrict__ pos, unsigned n, Grid g,
-                           unsigned* __restrict__ cell, unsigned* __restrict__ rank,
-                           unsigned* __restrict__ count) {
+__global__ void k_db_count(const float4* pos, unsigned n, Grid g,
+                           unsigned* cell, unsigned* rank,
+                           unsigned* count) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const unsigned c = cell_of(g, v3(pos[i]));
@@ -205,10 +210,11 @@ __global__ void k_db_count(const float4* __restrict__ pos, unsigned n, Grid g,
     rank[i] = atomicAdd(count + c, 1u);
 }
 
-__global__ void k_db_scatter(const float4* __restrict__ pos, unsigned n,
-                             const unsigned* __restrict__ cell, const unsigned* __restrict__ rank,
-                             const unsigned* __restrict__ start, unsigned* __restrict__ sorted,
-                             float4* __restrict__ pos_id) {
+__global__ void k_db_scatter(const float4* pos, unsigned n,
+                             const unsigned* cell, const unsigned* rank,
+                             const unsigned* start, unsigned* sorted,
+                             float4* pos_id) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const unsigned dst = start[cell[i]] + rank[i];
@@ -229,11 +235,10 @@ gs_status db_build(Database& db, const float4* pos, unsigned n, const Grid& grid
         GS_TRY(db_build_clusters(J, 1, st));
     } else {
         if (n > 0)
-            k_db_count<<<blocks_for(n), kBlock, 0, st>>>(pos, n, grid, db.cell, db.rank, db.count);
+            launch_after(k_db_count, blocks_for(n), kBlock, 0, st, pos, n, grid, db.cell, db.rank, db.count);
         GS_TRY(scan_counts(db.count, db.start, C, db.tile, st));
         if (n > 0)
-            k_db_scatter<<<blocks_for(n), kBlock, 0, st>>>(pos, n, db.cell, db.rank, db.start,
-                                                           db.sorted, db.pos_id);
+            launch_after(k_db_scatter, blocks_for(n), kBlock, 0, st, pos, n, db.cell, db.rank, db.start, db.sorted, db.pos_id);
         GS_LAUNCHED("db_build");
     }
     db.grid = grid;
@@ -566,6 +571,7 @@ static unsigned call_block(unsigned n) { return n <= 64u * 152u * 8u ? 64u : uns
 
 // ---- WrapWorldCUDAKernel.cu:11-48 ---------------------------------------------------
 __global__ void k_wrap(float4* pos, unsigned n, float wx, float wy, float wz, int mode) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float ws[3] = {wx, wy, wz};
@@ -575,7 +581,7 @@ __global__ void k_wrap(float4* pos, unsigned n, float wx, float wy, float wz, in
 gs_status launch_wrap(float4* pos, unsigned n, const float ws[3], int mode, cudaStream_t st) {
     if (n == 0) return GS_OK;
     const unsigned bs = call_block(n);
-    k_wrap<<<blocks_for(n, bs), bs, 0, st>>>(pos, n, ws[0], ws[1], ws[2], mode);
+    launch_after(k_wrap, blocks_for(n, bs), bs, 0, st, pos, n, ws[0], ws[1], ws[2], mode);
     GS_LAUNCHED("wrap_world");
     return GS_OK;
 }
@@ -607,7 +613,7 @@ constexpr unsigned kCallChunk = 8;
 // Calls body(s0, b, ok) for each chunk: ok[j]: entry s0 + j holds neighbour b[j]
 // (b[j] is 0 where there is none, a safe index to load).
 template <class Body>
-__device__ __forceinline__ void for_each_chunk(const unsigned* __restrict__ knn, unsigned i,
+__device__ __forceinline__ void for_each_chunk(const unsigned* knn, unsigned i,
                                                unsigned n, unsigned k, unsigned n_other,
                                                Body&& body) {
     bool more = true;
@@ -631,8 +637,9 @@ __device__ __forceinline__ void for_each_chunk(const unsigned* __restrict__ knn,
 // KIND: 0 separation, 1 alignment, 2 cohesion
 // (SteerFor{Separation,Alignment,Cohesion}CUDAKernel.cu:85-134)
 template <int KIND>
-__global__ void k_flock(GroupView g, const unsigned* __restrict__ knn, unsigned k, OtherView o,
+__global__ void k_flock(GroupView g, const unsigned* knn, unsigned k, OtherView o,
                         FlockParams fp) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     unsigned applied = g.applied[i];
@@ -686,14 +693,15 @@ gs_status launch_flock(int kind, GroupView g, const unsigned* knn, unsigned k, O
         return GS_OK;
     }
     const unsigned bs = call_block(g.n), nb = blocks_for(g.n, bs);
-    if (kind == 0) k_flock<0><<<nb, bs, 0, st>>>(g, knn, k, o, fp);
-    else if (kind == 1) k_flock<1><<<nb, bs, 0, st>>>(g, knn, k, o, fp);
-    else k_flock<2><<<nb, bs, 0, st>>>(g, knn, k, o, fp);
+    if (kind == 0) launch_after(k_flock<0>, nb, bs, 0, st, g, knn, k, o, fp);
+    else if (kind == 1) launch_after(k_flock<1>, nb, bs, 0, st, g, knn, k, o, fp);
+    else launch_after(k_flock<2>, nb, bs, 0, st, g, knn, k, o, fp);
     GS_LAUNCHED("steer_flock");
     return GS_OK;
 }
 
 __global__ void k_seek(GroupView g, float tx, float ty, float tz, float w, unsigned mask) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     unsigned applied = g.applied[i];
@@ -711,13 +719,14 @@ gs_status launch_seek(GroupView g, const float target[3], float w, unsigned mask
                       cudaStream_t st) {
     if (g.n == 0) return GS_OK;
     const unsigned bs = call_block(g.n);
-    k_seek<<<blocks_for(g.n, bs), bs, 0, st>>>(g, target[0], target[1], target[2], w, mask);
+    launch_after(k_seek, blocks_for(g.n, bs), bs, 0, st, g, target[0], target[1], target[2], w, mask);
     GS_LAUNCHED("steer_seek");
     return GS_OK;
 }
 
 __global__ void k_follow_path(GroupView g, PathDev path, float prediction_time, float w,
                               unsigned mask) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     unsigned applied = g.applied[i];
@@ -735,14 +744,15 @@ __global__ void k_follow_path(GroupView g, PathDev path, float prediction_time, 
 gs_status launch_follow_path(GroupView g, const PathDev& path, float prediction_time, float w,
                              unsigned mask, cudaStream_t st) {
     if (g.n == 0) return GS_OK;
-    k_follow_path<<<blocks_for(g.n), kBlock, 0, st>>>(g, path, prediction_time, w, mask);
+    launch_after(k_follow_path, blocks_for(g.n), kBlock, 0, st, g, path, prediction_time, w, mask);
     GS_LAUNCHED("steer_follow_path");
     return GS_OK;
 }
 
-__global__ void k_avoid_close(GroupView g, const unsigned* __restrict__ knn,
-                              const float* __restrict__ knn_dist, unsigned k, OtherView o,
+__global__ void k_avoid_close(GroupView g, const unsigned* knn,
+                              const float* knn_dist, unsigned k, OtherView o,
                               float min_sep, float w, unsigned mask) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     unsigned applied = g.applied[i];
@@ -780,8 +790,9 @@ __device__ __forceinline__ bool avoid_time_may_fall_in(const Self& me, float min
                                   (fabsf(h.x) + fabsf(h.y)) + fabsf(h.z), min_t);
 }
 
-__global__ void __launch_bounds__(kBlock, 2) k_avoid(GroupView g, const unsigned* __restrict__ knn, unsigned k, OtherView o,
+__global__ void __launch_bounds__(kBlock, 2) k_avoid(GroupView g, const unsigned* knn, unsigned k, OtherView o,
                         float min_time, float w, unsigned mask) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     unsigned applied = g.applied[i];
@@ -823,16 +834,17 @@ gs_status launch_avoid_neighbors(GroupView g, const unsigned* knn, const float* 
     }
     const unsigned bs = call_block(g.n), nb = blocks_for(g.n, bs);
     if (avoid_close)
-        k_avoid_close<<<nb, bs, 0, st>>>(g, knn, knn_dist, k, o, min_sep, w, mask);
-    k_avoid<<<nb, bs, 0, st>>>(g, knn, k, o, min_time, w, mask);
+        launch_after(k_avoid_close, nb, bs, 0, st, g, knn, knn_dist, k, o, min_sep, w, mask);
+    launch_after(k_avoid, nb, bs, 0, st, g, knn, k, o, min_time, w, mask);
     GS_LAUNCHED("steer_avoid_neighbors");
     return GS_OK;
 }
 
-__global__ void k_avoid_walls(GroupView g, const unsigned* __restrict__ knw, unsigned kw,
-                              const float4* __restrict__ ls, const float4* __restrict__ le,
-                              const float4* __restrict__ ln, unsigned n_lines, float min_time,
+__global__ void k_avoid_walls(GroupView g, const unsigned* knw, unsigned kw,
+                              const float4* ls, const float4* le,
+                              const float4* ln, unsigned n_lines, float min_time,
                               float w, unsigned mask) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     unsigned applied = g.applied[i];
@@ -863,13 +875,13 @@ gs_status launch_avoid_walls(GroupView g, const unsigned* knw, unsigned kw, cons
         return GS_OK;
     }
     const unsigned bs = call_block(g.n);
-    k_avoid_walls<<<blocks_for(g.n, bs), bs, 0, st>>>(g, knw, kw, start, end, normal, n_lines,
-                                                      min_time, w, mask);
+    launch_after(k_avoid_walls, blocks_for(g.n, bs), bs, 0, st, g, knw, kw, start, end, normal, n_lines, min_time, w, mask);
     GS_LAUNCHED("steer_avoid_walls");
     return GS_OK;
 }
 
 __global__ void k_update(GroupView g, float dt) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     Self me = load_self(g, i);
@@ -886,7 +898,7 @@ __global__ void k_update(GroupView g, float dt) {
 gs_status launch_update(GroupView g, float dt, cudaStream_t st) {
     if (g.n == 0) return GS_OK;
     const unsigned bs = call_block(g.n);
-    k_update<<<blocks_for(g.n, bs), bs, 0, st>>>(g, dt);
+    launch_after(k_update, blocks_for(g.n, bs), bs, 0, st, g, dt);
     GS_LAUNCHED("update_group");
     return GS_OK;
 }

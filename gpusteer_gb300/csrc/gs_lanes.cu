@@ -15,6 +15,7 @@ constexpr unsigned kLaneBlock = 128;
 // ---- whole step without walls -----------------------------------------------------------
 template <int G, int R, unsigned NEEDC>
 __global__ void __launch_bounds__(kLaneBlock) k_lanes_step(FusedLaunch L, StepDev p) {
+    after_previous();
     __shared__ unsigned row_sh[R ? 1 : kLaneBlock / G * kLaneRowWords];
     unsigned* rows = row_sh + (R ? 0u : threadIdx.x / G * kLaneRowWords);
     __shared__ __align__(16) float sh[kLaneBlock / G * LaneSums<G>::kWords];
@@ -57,6 +58,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_step(FusedLaunch L, StepDe
 // ---- wall phase ---------------------------------------------------------------------------
 template <int G, int R>
 __global__ void __launch_bounds__(kLaneBlock) k_lanes_walls(FusedLaunch L, StepDev p) {
+    after_previous();
     __shared__ unsigned row_sh[R ? 1 : kLaneBlock / G * kLaneRowWords];
     unsigned* rows = row_sh + (R ? 0u : threadIdx.x / G * kLaneRowWords);
     const unsigned lane = threadIdx.x & unsigned(G - 1);
@@ -93,6 +95,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_walls(FusedLaunch L, StepD
 // ---- rest of the step after the wall phase -------------------------------------------------
 template <int G, unsigned NEEDC>
 __global__ void __launch_bounds__(kLaneBlock) k_lanes_rest(FusedLaunch L, StepDev p) {
+    after_previous();
     __shared__ __align__(16) float sh[kLaneBlock / G * LaneSums<G>::kWords];
     const unsigned need = NEEDC == kNeedRuntime ? p.need : NEEDC;
     const unsigned lane = threadIdx.x & unsigned(G - 1);
@@ -127,7 +130,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_lanes_rest(FusedLaunch L, StepDe
 // list entry r.  An index past the other group ends the list, as in the
 // reference's kernels.
 template <int G>
-__device__ __forceinline__ bool lanes_entry(const unsigned* __restrict__ knn, unsigned i,
+__device__ __forceinline__ bool lanes_entry(const unsigned* knn, unsigned i,
                                             unsigned n, unsigned k, unsigned n_other,
                                             unsigned lane, unsigned& b) {
     b = lane < k ? knn[i + size_t(lane) * n] : UINT_MAX;
@@ -150,9 +153,10 @@ __device__ __forceinline__ bool lanes_agent(unsigned n, unsigned& i, unsigned& l
 // KIND: 0 separation, 1 alignment, 2 cohesion
 template <int G, int KIND>
 __global__ void __launch_bounds__(kLaneBlock) k_flock_lanes(GroupView g,
-                                                            const unsigned* __restrict__ knn,
+                                                            const unsigned* knn,
                                                             unsigned k, OtherView o,
                                                             FlockParams fp) {
+    after_previous();
     __shared__ __align__(16) float sh[kLaneBlock / G * LaneSums<G>::kWords];
     constexpr unsigned need = KIND == 0 ? NEED_SEP : KIND == 1 ? NEED_ALI : NEED_COH;
     unsigned i, lane, b;
@@ -179,10 +183,11 @@ __global__ void __launch_bounds__(kLaneBlock) k_flock_lanes(GroupView g,
 // steerToAvoidNeighbors: the close pass (CLOSE) or the main pass.
 template <int G, bool CLOSE>
 __global__ void __launch_bounds__(kLaneBlock) k_avoid_lanes(GroupView g,
-                                                            const unsigned* __restrict__ knn,
-                                                            const float* __restrict__ knn_dist,
+                                                            const unsigned* knn,
+                                                            const float* knn_dist,
                                                             unsigned k, OtherView o, float limit,
                                                             float w, unsigned mask) {
+    after_previous();
     unsigned i, lane, b;
     const bool act = lanes_agent<G>(g.n, i, lane);
     LaneNeighbour nb;
@@ -223,9 +228,10 @@ __global__ void __launch_bounds__(kLaneBlock) k_avoid_lanes(GroupView g,
 
 template <int G>
 __global__ void __launch_bounds__(kLaneBlock) k_avoid_walls_lanes(
-    GroupView g, const unsigned* __restrict__ knw, unsigned kw, const float4* __restrict__ ls,
-    const float4* __restrict__ le, const float4* __restrict__ ln, unsigned n_lines, float min_time,
+    GroupView g, const unsigned* knw, unsigned kw, const float4* ls,
+    const float4* le, const float4* ln, unsigned n_lines, float min_time,
     float w, unsigned mask) {
+    after_previous();
     unsigned i, lane, line;
     const bool act = lanes_agent<G>(g.n, i, lane);
     const bool ok = lanes_entry<G>(knw, i, g.n, kw, n_lines, lane, line);
@@ -260,9 +266,9 @@ template <int G>
 static void flock_lanes_go(int kind, GroupView g, const unsigned* knn, unsigned k, OtherView o,
                            FlockParams fp, cudaStream_t st) {
     const unsigned nb = blocks_for(g.n, kLaneBlock / G);
-    if (kind == 0) k_flock_lanes<G, 0><<<nb, kLaneBlock, 0, st>>>(g, knn, k, o, fp);
-    else if (kind == 1) k_flock_lanes<G, 1><<<nb, kLaneBlock, 0, st>>>(g, knn, k, o, fp);
-    else k_flock_lanes<G, 2><<<nb, kLaneBlock, 0, st>>>(g, knn, k, o, fp);
+    if (kind == 0) launch_after(k_flock_lanes<G, 0>, nb, kLaneBlock, 0, st, g, knn, k, o, fp);
+    else if (kind == 1) launch_after(k_flock_lanes<G, 1>, nb, kLaneBlock, 0, st, g, knn, k, o, fp);
+    else launch_after(k_flock_lanes<G, 2>, nb, kLaneBlock, 0, st, g, knn, k, o, fp);
 }
 void launch_flock_lanes(int kind, GroupView g, const unsigned* knn, unsigned k, OtherView o,
                         FlockParams fp, cudaStream_t st) {
@@ -277,8 +283,8 @@ static void avoid_lanes_go(GroupView g, const unsigned* knn, const float* knn_di
                            unsigned mask, cudaStream_t st) {
     const unsigned nb = blocks_for(g.n, kLaneBlock / G);
     if (close)
-        k_avoid_lanes<G, true><<<nb, kLaneBlock, 0, st>>>(g, knn, knn_dist, k, o, min_sep, w, mask);
-    k_avoid_lanes<G, false><<<nb, kLaneBlock, 0, st>>>(g, knn, nullptr, k, o, min_time, w, mask);
+        launch_after(k_avoid_lanes<G, true>, nb, kLaneBlock, 0, st, g, knn, knn_dist, k, o, min_sep, w, mask);
+    launch_after(k_avoid_lanes<G, false>, nb, kLaneBlock, 0, st, g, knn, nullptr, k, o, min_time, w, mask);
 }
 void launch_avoid_lanes(GroupView g, const unsigned* knn, const float* knn_dist, unsigned k,
                         OtherView o, float min_time, float min_sep, bool close, float w,
@@ -292,8 +298,7 @@ void launch_avoid_lanes(GroupView g, const unsigned* knn, const float* knn_dist,
 void launch_avoid_walls_lanes(GroupView g, const unsigned* knw, unsigned kw, const float4* start,
                               const float4* end, const float4* normal, unsigned n_lines,
                               float min_time, float w, unsigned mask, cudaStream_t st) {
-    k_avoid_walls_lanes<8><<<blocks_for(g.n, kLaneBlock / 8), kLaneBlock, 0, st>>>(
-        g, knw, kw, start, end, normal, n_lines, min_time, w, mask);
+    launch_after(k_avoid_walls_lanes<8>, blocks_for(g.n, kLaneBlock / 8), kLaneBlock, 0, st, g, knw, kw, start, end, normal, n_lines, min_time, w, mask);
 }
 
 // ---- MultiGroup frames ------------------------------------------------------------------------
@@ -347,6 +352,7 @@ __device__ __forceinline__ void lanes_push_apart(const MultiSteer& M, unsigned a
 
 template <int G>
 __global__ void __launch_bounds__(kLaneBlock) k_group_move(const __grid_constant__ MultiSteer M) {
+    after_previous();
     __shared__ __align__(16) float sh[kLaneBlock / G * LaneSums<G>::kWords];
     const GroupView& g = M.g;
     unsigned a, lane;
@@ -428,6 +434,7 @@ __global__ void __launch_bounds__(kLaneBlock) k_group_move(const __grid_constant
 // now, then against the groups after it, which have not; the result goes to
 // the group's arrays.
 __global__ void __launch_bounds__(kLaneBlock) k_group_settle(const __grid_constant__ MultiSteer M) {
+    after_previous();
     const GroupView& g = M.g;
     unsigned a, lane;
     const bool act = lanes_agent<8>(g.n, a, lane);
@@ -456,10 +463,10 @@ gs_status launch_group_frame(const MultiSteer& M, cudaStream_t st) {
     if (M.g.n == 0) return GS_OK;
     unsigned k = 0;
     for (unsigned j = 0; j < M.n_groups; ++j) k = M.k[j] > k ? M.k[j] : k;
-    if (k <= 8) k_group_move<8><<<blocks_for(M.g.n, kLaneBlock / 8), kLaneBlock, 0, st>>>(M);
-    else if (k <= 16) k_group_move<16><<<blocks_for(M.g.n, kLaneBlock / 16), kLaneBlock, 0, st>>>(M);
-    else k_group_move<32><<<blocks_for(M.g.n, kLaneBlock / 32), kLaneBlock, 0, st>>>(M);
-    k_group_settle<<<blocks_for(M.g.n, kLaneBlock / 8), kLaneBlock, 0, st>>>(M);
+    if (k <= 8) launch_after(k_group_move<8>, blocks_for(M.g.n, kLaneBlock / 8), kLaneBlock, 0, st, M);
+    else if (k <= 16) launch_after(k_group_move<16>, blocks_for(M.g.n, kLaneBlock / 16), kLaneBlock, 0, st, M);
+    else launch_after(k_group_move<32>, blocks_for(M.g.n, kLaneBlock / 32), kLaneBlock, 0, st, M);
+    launch_after(k_group_settle, blocks_for(M.g.n, kLaneBlock / 8), kLaneBlock, 0, st, M);
     GS_LAUNCHED("group_frame");
     return GS_OK;
 }
@@ -478,20 +485,20 @@ static void launch_lanes_r(const FusedLaunch& L, const StepDev& p, unsigned nb, 
     if (!(p.need & NEED_WALLS)) {
         if (hook) hook->mark(2, true);
         if ((p.need & kNeedList) == (NEED_SEP | NEED_ALI | NEED_COH))
-            k_lanes_step<G, R, NEED_SEP | NEED_ALI | NEED_COH><<<nb, kLaneBlock, 0, st>>>(L, p);
+            launch_after(k_lanes_step<G, R, NEED_SEP | NEED_ALI | NEED_COH>, nb, kLaneBlock, 0, st, L, p);
         else
-            k_lanes_step<G, R, kNeedRuntime><<<nb, kLaneBlock, 0, st>>>(L, p);
+            launch_after(k_lanes_step<G, R, kNeedRuntime>, nb, kLaneBlock, 0, st, L, p);
         if (hook) hook->mark(2, false);
         return;
     }
     if (hook) hook->mark(2, true);
-    k_lanes_walls<G, R><<<nb, kLaneBlock, 0, st>>>(L, p);
+    launch_after(k_lanes_walls<G, R>, nb, kLaneBlock, 0, st, L, p);
     if (hook) hook->mark(2, false);
     if (hook) hook->mark(3, true);
     if ((p.need & kNeedList) == (NEED_SEP | NEED_AVOID))
-        k_lanes_rest<G, NEED_SEP | NEED_AVOID><<<nb, kLaneBlock, 0, st>>>(L, p);
+        launch_after(k_lanes_rest<G, NEED_SEP | NEED_AVOID>, nb, kLaneBlock, 0, st, L, p);
     else
-        k_lanes_rest<G, kNeedRuntime><<<nb, kLaneBlock, 0, st>>>(L, p);
+        launch_after(k_lanes_rest<G, kNeedRuntime>, nb, kLaneBlock, 0, st, L, p);
     if (hook) hook->mark(3, false);
 }
 

@@ -43,6 +43,7 @@ __device__ __forceinline__ void lists_lanes(const KnnPair& pr, const Grid& grid,
 
 template <int G, int R>
 __global__ void __launch_bounds__(kListBlock) k_lists_lanes(KnnPair pr, Grid grid, unsigned r) {
+    after_previous();
     __shared__ unsigned row_sh[R ? 1 : kListBlock / G * kLaneRowWords];
     lists_lanes<G, R>(pr, grid, r, blockIdx.x * kListBlock + threadIdx.x,
                       row_sh + (R ? 0u : threadIdx.x / G * kLaneRowWords));
@@ -58,6 +59,7 @@ __device__ __forceinline__ unsigned pair_of_block(const KnnPairs& P) {
 
 template <int G, int R>
 __global__ void __launch_bounds__(kListBlock) k_lists_lanes_pairs(const __grid_constant__ KnnPairs P) {
+    after_previous();
     __shared__ unsigned row_sh[R ? 1 : kListBlock / G * kLaneRowWords];
     const KnnPair& pr = P.pair[pair_of_block(P)];
     lists_lanes<G, R>(pr, P.grid, P.r, (blockIdx.x - pr.block_begin) * kListBlock + threadIdx.x,
@@ -120,12 +122,14 @@ __device__ __forceinline__ void lists_thread(const KnnPair& pr, const Grid& grid
 
 template <int KMAX, bool FLAT>
 __global__ void __launch_bounds__(kListBlock) k_lists_thread(KnnPair pr, Grid grid) {
+    after_previous();
     __shared__ unsigned sh[KMAX * kListBlock];
     lists_thread<KMAX, FLAT>(pr, grid, blockIdx.x * kListBlock + threadIdx.x, sh);
 }
 
 template <int KMAX, bool FLAT>
 __global__ void __launch_bounds__(kListBlock) k_lists_thread_pairs(const __grid_constant__ KnnPairs P) {
+    after_previous();
     __shared__ unsigned sh[KMAX * kListBlock];
     const KnnPair& pr = P.pair[pair_of_block(P)];
     lists_thread<KMAX, FLAT>(pr, P.grid, (blockIdx.x - pr.block_begin) * kListBlock + threadIdx.x,
@@ -151,9 +155,11 @@ __device__ __forceinline__ void lists_wide(const KnnPair& pr, const Grid& grid, 
 }
 
 __global__ void __launch_bounds__(kListBlock) k_lists_wide(KnnPair pr, Grid grid, unsigned r) {
+    after_previous();
     lists_wide(pr, grid, r, blockIdx.x * kListBlock + threadIdx.x);
 }
 __global__ void __launch_bounds__(kListBlock) k_lists_wide_pairs(const __grid_constant__ KnnPairs P) {
+    after_previous();
     const KnnPair& pr = P.pair[pair_of_block(P)];
     lists_wide(pr, P.grid, P.r, (blockIdx.x - pr.block_begin) * kListBlock + threadIdx.x);
 }
@@ -173,22 +179,22 @@ static bool lists_on_lanes(size_t queries, unsigned k, unsigned r) {
 template <int G>
 static void lists_lanes_go(const KnnPair& pr, const Grid& grid, unsigned r, cudaStream_t st) {
     const unsigned nb = blocks_for(pr.nA, kListBlock / G);
-    if (r != 1) k_lists_lanes<G, 0><<<nb, kListBlock, 0, st>>>(pr, grid, r);
-    else if (grid.wc[1] == 1) k_lists_lanes<G, 3><<<nb, kListBlock, 0, st>>>(pr, grid, r);
-    else k_lists_lanes<G, 9><<<nb, kListBlock, 0, st>>>(pr, grid, r);
+    if (r != 1) launch_after(k_lists_lanes<G, 0>, nb, kListBlock, 0, st, pr, grid, r);
+    else if (grid.wc[1] == 1) launch_after(k_lists_lanes<G, 3>, nb, kListBlock, 0, st, pr, grid, r);
+    else launch_after(k_lists_lanes<G, 9>, nb, kListBlock, 0, st, pr, grid, r);
 }
 template <int KMAX>
 static void lists_thread_go(const KnnPair& pr, const Grid& grid, cudaStream_t st) {
     const unsigned nb = blocks_for(pr.nA, kListBlock);
-    if (grid.wc[1] == 1) k_lists_thread<KMAX, true><<<nb, kListBlock, 0, st>>>(pr, grid);
-    else k_lists_thread<KMAX, false><<<nb, kListBlock, 0, st>>>(pr, grid);
+    if (grid.wc[1] == 1) launch_after(k_lists_thread<KMAX, true>, nb, kListBlock, 0, st, pr, grid);
+    else launch_after(k_lists_thread<KMAX, false>, nb, kListBlock, 0, st, pr, grid);
 }
 
 gs_status launch_knn_binned(const Database& A, unsigned nA, const Database& B, bool self,
                             unsigned r, unsigned k, unsigned* idx, float* dist, cudaStream_t st) {
     if (nA == 0) return GS_OK;
     const KnnPair pr{A.pos_id, B.start, B.pos_id, idx, dist, nA, k, 0u, self};
-    if (k > 32) k_lists_wide<<<blocks_for(nA, kListBlock), kListBlock, 0, st>>>(pr, B.grid, r);
+    if (k > 32) launch_after(k_lists_wide, blocks_for(nA, kListBlock), kListBlock, 0, st, pr, B.grid, r);
     else if (lists_on_lanes(nA, k, r)) {
         if (k <= 8) lists_lanes_go<8>(pr, B.grid, r, st);
         else if (k <= 16) lists_lanes_go<16>(pr, B.grid, r, st);
@@ -205,14 +211,14 @@ static_assert(sizeof(KnnPairs) <= 4096, "batched KNN parameters exceed 4 KiB");
 
 template <int G>
 static void pairs_lanes_go(const KnnPairs& P, unsigned nb, cudaStream_t st) {
-    if (P.r != 1) k_lists_lanes_pairs<G, 0><<<nb, kListBlock, 0, st>>>(P);
-    else if (P.grid.wc[1] == 1) k_lists_lanes_pairs<G, 3><<<nb, kListBlock, 0, st>>>(P);
-    else k_lists_lanes_pairs<G, 9><<<nb, kListBlock, 0, st>>>(P);
+    if (P.r != 1) launch_after(k_lists_lanes_pairs<G, 0>, nb, kListBlock, 0, st, P);
+    else if (P.grid.wc[1] == 1) launch_after(k_lists_lanes_pairs<G, 3>, nb, kListBlock, 0, st, P);
+    else launch_after(k_lists_lanes_pairs<G, 9>, nb, kListBlock, 0, st, P);
 }
 template <int KMAX>
 static void pairs_thread_go(const KnnPairs& P, unsigned nb, cudaStream_t st) {
-    if (P.grid.wc[1] == 1) k_lists_thread_pairs<KMAX, true><<<nb, kListBlock, 0, st>>>(P);
-    else k_lists_thread_pairs<KMAX, false><<<nb, kListBlock, 0, st>>>(P);
+    if (P.grid.wc[1] == 1) launch_after(k_lists_thread_pairs<KMAX, true>, nb, kListBlock, 0, st, P);
+    else launch_after(k_lists_thread_pairs<KMAX, false>, nb, kListBlock, 0, st, P);
 }
 
 gs_status launch_knn_binned_pairs(KnnPairs& P, cudaStream_t st) {
@@ -232,7 +238,7 @@ gs_status launch_knn_binned_pairs(KnnPairs& P, cudaStream_t st) {
         blocks += blocks_for(P.pair[q].nA, lanes ? kListBlock / G : kListBlock);
     }
     if (blocks == 0) return GS_OK;
-    if (kmax > 32) k_lists_wide_pairs<<<blocks, kListBlock, 0, st>>>(P);
+    if (kmax > 32) launch_after(k_lists_wide_pairs, blocks, kListBlock, 0, st, P);
     else if (lanes) {
         if (G == 8) pairs_lanes_go<8>(P, blocks, st);
         else if (G == 16) pairs_lanes_go<16>(P, blocks, st);

@@ -36,10 +36,11 @@
 namespace gs {
 
 // Reference layout -> A (identity order), counting the first step's cells.
-__global__ void k_from_reference(GroupView g, const unsigned* __restrict__ agent_scene,
-                                 const Scene* __restrict__ scenes, Fused A,
-                                 uint2* __restrict__ cellrank, unsigned* __restrict__ count,
+__global__ void k_from_reference(GroupView g, const unsigned* agent_scene,
+                                 const Scene* scenes, Fused A,
+                                 uint2* cellrank, unsigned* count,
                                  int wrap_mode, int dirty) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.n) return;
     const unsigned si = agent_scene ? agent_scene[i] : 0u;
@@ -62,8 +63,7 @@ gs_status fused_from_reference(GroupView g, const unsigned* agent_scene, const S
                                Fused A, uint2* cellrank, unsigned* count, int wrap_mode,
                                bool dirty, cudaStream_t st) {
     if (g.n == 0) return GS_OK;
-    k_from_reference<<<blocks_for(g.n), kBlock, 0, st>>>(g, agent_scene, scenes, A, cellrank,
-                                                         count, wrap_mode, dirty ? 1 : 0);
+    launch_after(k_from_reference, blocks_for(g.n), kBlock, 0, st, g, agent_scene, scenes, A, cellrank, count, wrap_mode, dirty ? 1 : 0);
     GS_LAUNCHED("fused_from_reference");
     return GS_OK;
 }
@@ -105,10 +105,10 @@ __device__ __forceinline__ void move_agent(const Fused& A, const Fused& B,
 
 // A (slot i) -> B (slot start[cell] + rank), wrapping the position.
 __device__ __forceinline__ void permute_agent(const Fused& A, const Fused& B, unsigned n,
-                                              const uint2* __restrict__ cellrank,
-                                              const unsigned* __restrict__ start,
+                                              const uint2* cellrank,
+                                              const unsigned* start,
                                               const Scene* __restrict__ scenes, int wrap_mode,
-                                              int dirty, unsigned* __restrict__ err, unsigned i) {
+                                              int dirty, unsigned* err, unsigned i) {
     const uint2 cr = cellrank[i];
     const unsigned dst = start[cr.x] + cr.y;
     if (dst >= n) {  // inconsistent counts: record and write nothing
@@ -119,13 +119,14 @@ __device__ __forceinline__ void permute_agent(const Fused& A, const Fused& B, un
 }
 
 __global__ void __launch_bounds__(kBlock) k_permute(Fused A, Fused B, unsigned n,
-                                                    const uint2* __restrict__ cellrank,
-                                                    const unsigned* __restrict__ start,
-                                                    const Scene* __restrict__ scenes,
+                                                    const uint2* cellrank,
+                                                    const unsigned* start,
+                                                    const Scene* scenes,
                                                     int wrap_mode, int dirty,
-                                                    unsigned* __restrict__ err,
-                                                    unsigned* __restrict__ retry_count,
-                                                    unsigned* __restrict__ tile, unsigned tiles) {
+                                                    unsigned* err,
+                                                    unsigned* retry_count,
+                                                    unsigned* tile, unsigned tiles) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) *retry_count = 0u;  // the fused launch that follows refills it
     // the scan has read the tile totals; the step's counting adds them anew
@@ -140,9 +141,10 @@ __global__ void __launch_bounds__(kBlock) k_permute(Fused A, Fused B, unsigned n
 // times the steady step's permute).  Instead, one scattered 4-byte store per
 // agent records which agent each slot takes, and the permute gathers:
 // scattered 16-byte reads, coalesced writes.
-__global__ void k_agent_at(unsigned n, const uint2* __restrict__ cellrank,
-                           const unsigned* __restrict__ start, unsigned* __restrict__ err,
-                           unsigned* __restrict__ agent_at) {
+__global__ void k_agent_at(unsigned n, const uint2* cellrank,
+                           const unsigned* start, unsigned* err,
+                           unsigned* agent_at) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint2 cr = cellrank[i];
@@ -155,13 +157,14 @@ __global__ void k_agent_at(unsigned n, const uint2* __restrict__ cellrank,
 }
 
 __global__ void __launch_bounds__(kBlock) k_permute_gather(Fused A, Fused B, unsigned n,
-                                                           const unsigned* __restrict__ agent_at,
-                                                           const Scene* __restrict__ scenes,
+                                                           const unsigned* agent_at,
+                                                           const Scene* scenes,
                                                            int wrap_mode, int dirty,
-                                                           unsigned* __restrict__ err,
-                                                           unsigned* __restrict__ retry_count,
-                                                           unsigned* __restrict__ tile,
+                                                           unsigned* err,
+                                                           unsigned* retry_count,
+                                                           unsigned* tile,
                                                            unsigned tiles) {
+    after_previous();
     const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s == 0) *retry_count = 0u;
     for (unsigned t = s; t < tiles; t += gridDim.x * blockDim.x) tile[t] = 0u;
@@ -181,17 +184,12 @@ gs_status fused_permute(const FusedLaunch& L, int wrap_mode, bool dirty, bool fr
                         cudaStream_t st) {
     if (L.n == 0) return GS_OK;
     if (fresh) {
-        k_agent_at<<<blocks_for(L.n), kBlock, 0, st>>>(L.n, L.cellrank, L.start, L.err,
-                                                        L.agent_at);
-        k_permute_gather<<<blocks_for(L.n), kBlock, 0, st>>>(L.A, L.B, L.n, L.agent_at, L.scenes,
-                                                             wrap_mode, dirty ? 1 : 0, L.err,
-                                                             L.retry_count, L.tile, L.tiles);
+        launch_after(k_agent_at, blocks_for(L.n), kBlock, 0, st, L.n, L.cellrank, L.start, L.err, L.agent_at);
+        launch_after(k_permute_gather, blocks_for(L.n), kBlock, 0, st, L.A, L.B, L.n, L.agent_at, L.scenes, wrap_mode, dirty ? 1 : 0, L.err, L.retry_count, L.tile, L.tiles);
         GS_LAUNCHED("fused_permute");
         return GS_OK;
     }
-    k_permute<<<blocks_for(L.n), kBlock, 0, st>>>(L.A, L.B, L.n, L.cellrank, L.start, L.scenes,
-                                                  wrap_mode, dirty ? 1 : 0, L.err, L.retry_count,
-                                                  L.tile, L.tiles);
+    launch_after(k_permute, blocks_for(L.n), kBlock, 0, st, L.A, L.B, L.n, L.cellrank, L.start, L.scenes, wrap_mode, dirty ? 1 : 0, L.err, L.retry_count, L.tile, L.tiles);
     GS_LAUNCHED("fused_permute");
     return GS_OK;
 }
@@ -575,6 +573,7 @@ __device__ __forceinline__ void retry_lists(const FusedLaunch& L, const StepDev&
 
 template <int KMAX, bool TO_SLOTS>
 __global__ void __launch_bounds__(kBlock) k_knn_retry(FusedLaunch L, StepDev p) {
+    after_previous();
     __shared__ unsigned long long sk[kBlock / 32][kRetryWarpKeys];
     __shared__ unsigned ss[kBlock / 32][kRetryWarpKeys];
     const unsigned w = threadIdx.x >> 5;
@@ -592,6 +591,7 @@ constexpr unsigned kRestChunk = 2;  // the rest phase's (1: +7 %, 3: +6 %, 4: +1
 template <int KMAX, unsigned ENUM, bool EXACT, unsigned NEEDC = kNeedRuntime, bool FLAT = false,
           unsigned kNbrChunk = 1>
 __global__ void __launch_bounds__(kBlock, kNbrChunk > 1 ? 2 : 3) k_fused(FusedLaunch L, StepDev p) {
+    after_previous();
     const unsigned need = NEEDC == kNeedRuntime ? p.need : NEEDC;
     extern __shared__ unsigned sh_col[];
     const unsigned bd = blockDim.x;
@@ -755,6 +755,7 @@ __device__ __forceinline__ void walls_agent(const FusedLaunch& L, const StepDev&
 
 template <int KMAX, int KW, unsigned ENUM, bool EXACT, bool FLAT = false>
 __global__ void __launch_bounds__(kBlock, 4) k_fused_walls(FusedLaunch L, StepDev p) {
+    after_previous();
     extern __shared__ unsigned sh_col[];
     const unsigned bd = blockDim.x;
     unsigned* col = sh_col + threadIdx.x;
@@ -858,6 +859,7 @@ __device__ __forceinline__ void rest_agent(const FusedLaunch& L, const StepDev& 
 
 template <int KMAX, unsigned NEEDC>
 __global__ void __launch_bounds__(kBlock, 5) k_fused_rest(FusedLaunch L, StepDev p) {
+    after_previous();
     const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < L.n) rest_agent<KMAX, NEEDC>(L, p, s);
 }
@@ -907,23 +909,23 @@ static gs_status launch_fused_k(const FusedLaunch& L, const StepDev& p, cudaStre
         if constexpr (ENUM > 64) {
             if (p.flat) {
                 GS_TRY(allow_smem(k_fused_walls<KMAX, 8, ENUM, false, true>, smem));
-                k_fused_walls<KMAX, 8, ENUM, false, true><<<nb, bs, smem, st>>>(L, p);
+                launch_after(k_fused_walls<KMAX, 8, ENUM, false, true>, nb, bs, smem, st, L, p);
                 launched = true;
             }
         }
         if (!launched) {
             GS_TRY(allow_smem(k_fused_walls<KMAX, 8, ENUM, false>, smem));
-            k_fused_walls<KMAX, 8, ENUM, false><<<nb, bs, smem, st>>>(L, p);
+            launch_after(k_fused_walls<KMAX, 8, ENUM, false>, nb, bs, smem, st, L, p);
         }
         // the redo agents' exact lists, straight into the neighbour lists
-        if (ENUM > 64) k_knn_retry<KMAX, true><<<nb_retry, kBlock, 0, st>>>(L, p);
+        if (ENUM > 64) launch_after(k_knn_retry<KMAX, true>, nb_retry, kBlock, 0, st, L, p);
         if (hook) hook->mark(2, false);
         if (hook) hook->mark(3, true);
         // the choke-point step (separation and neighbour avoidance) has its own build
         if ((p.need & kNeedList) == (NEED_SEP | NEED_AVOID))
-            k_fused_rest<KMAX, NEED_SEP | NEED_AVOID><<<nb, bs, 0, st>>>(L, p);
+            launch_after(k_fused_rest<KMAX, NEED_SEP | NEED_AVOID>, nb, bs, 0, st, L, p);
         else
-            k_fused_rest<KMAX, kNeedRuntime><<<nb, bs, 0, st>>>(L, p);
+            launch_after(k_fused_rest<KMAX, kNeedRuntime>, nb, bs, 0, st, L, p);
         if (hook) hook->mark(3, false);
     } else {
         GS_TRY(allow_smem(k_fused<KMAX, ENUM, false>, smem));
@@ -941,21 +943,21 @@ static gs_status launch_fused_k(const FusedLaunch& L, const StepDev& p, cudaStre
                                 ? k_fused<KMAX, 32, false, NEED_SEP | NEED_ALI | NEED_COH, false, 2>
                                 : k_fused<KMAX, 32, false, NEED_SEP | NEED_ALI | NEED_COH>;
                 GS_TRY(allow_smem(kern, smem));
-                kern<<<nb, bs, smem, st>>>(L, p);
+                launch_after(kern, nb, bs, smem, st, L, p);
                 done = true;
             }
         }
         if constexpr (ENUM > 64) {
             if (p.flat) {
                 GS_TRY(allow_smem(k_fused<KMAX, ENUM, false, kNeedRuntime, true>, smem));
-                k_fused<KMAX, ENUM, false, kNeedRuntime, true><<<nb, bs, smem, st>>>(L, p);
+                launch_after(k_fused<KMAX, ENUM, false, kNeedRuntime, true>, nb, bs, smem, st, L, p);
                 done = true;
             }
         }
-        if (!done) k_fused<KMAX, ENUM, false><<<nb, bs, smem, st>>>(L, p);
+        if (!done) launch_after(k_fused<KMAX, ENUM, false>, nb, bs, smem, st, L, p);
         if (ENUM > 64) {
-            k_knn_retry<KMAX, false><<<nb_retry, kBlock, 0, st>>>(L, p);
-            k_fused<KMAX, 32, true><<<nb_retry, kBlock, smem_x, st>>>(L, p);
+            launch_after(k_knn_retry<KMAX, false>, nb_retry, kBlock, 0, st, L, p);
+            launch_after(k_fused<KMAX, 32, true>, nb_retry, kBlock, smem_x, st, L, p);
         }
         if (hook) hook->mark(2, false);
     }
@@ -1123,16 +1125,18 @@ gs_status fused_step(const FusedLaunch& L, const StepDev& p, cudaStream_t st, Ph
 // order, so the conversion first records each agent's slot (one scattered
 // 4-byte store per agent), then writes the reference arrays in agent order,
 // coalesced, reading each agent's five float4 from its slot.
-__global__ void k_slot_of(Fused A, unsigned n, const Scene* __restrict__ scenes,
-                          unsigned* __restrict__ slot_of) {
+__global__ void k_slot_of(Fused A, unsigned n, const Scene* scenes,
+                          unsigned* slot_of) {
+    after_previous();
     const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const unsigned id = u(A.f[0][s].w), scene = u(A.f[4][s].w);
     slot_of[scenes[scene].agent_offset + id] = s;
 }
 
-__global__ void k_to_reference(Fused A, unsigned n, const unsigned* __restrict__ slot_of,
+__global__ void k_to_reference(Fused A, unsigned n, const unsigned* slot_of,
                                GroupView g) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const unsigned s = slot_of ? slot_of[i] : i;
@@ -1153,8 +1157,8 @@ __global__ void k_to_reference(Fused A, unsigned n, const unsigned* __restrict__
 gs_status fused_to_reference(Fused A, unsigned n, const Scene* scenes, unsigned* slot_of,
                              bool in_order, GroupView g, cudaStream_t st) {
     if (n == 0) return GS_OK;
-    if (!in_order) k_slot_of<<<blocks_for(n), kBlock, 0, st>>>(A, n, scenes, slot_of);
-    k_to_reference<<<blocks_for(n), kBlock, 0, st>>>(A, n, in_order ? nullptr : slot_of, g);
+    if (!in_order) launch_after(k_slot_of, blocks_for(n), kBlock, 0, st, A, n, scenes, slot_of);
+    launch_after(k_to_reference, blocks_for(n), kBlock, 0, st, A, n, in_order ? nullptr : slot_of, g);
     GS_LAUNCHED("fused_to_reference");
     return GS_OK;
 }

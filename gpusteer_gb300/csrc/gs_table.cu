@@ -164,6 +164,7 @@ __device__ __forceinline__ void table_store(const TableStep& T, unsigned a, cons
 template <int G, bool FLAT, unsigned NEEDC>
 __global__ void __launch_bounds__(kTableBlock) k_table_step(const __grid_constant__ TableStep T,
                                                             const __grid_constant__ StepDev p) {
+    after_previous();
     __shared__ __align__(16) float sh[kTableBlock / G * LaneSums<G>::kWords];
     __shared__ unsigned place_sh[kTableBlock / G * kTablePlaces];
     const unsigned need = NEEDC == kNeedRuntime ? p.need : NEEDC;
@@ -196,6 +197,7 @@ __global__ void __launch_bounds__(kTableBlock) k_table_step(const __grid_constan
 template <int G, bool FLAT>
 __global__ void __launch_bounds__(kTableBlock) k_table_walls(const __grid_constant__ TableStep T,
                                                              const __grid_constant__ StepDev p) {
+    after_previous();
     __shared__ unsigned place_sh[kTableBlock / G * kTablePlaces];
     unsigned a, lane;
     const bool act = table_agent<G>(T.n, a, lane);
@@ -225,6 +227,7 @@ __global__ void __launch_bounds__(kTableBlock) k_table_walls(const __grid_consta
 template <int G, unsigned NEEDC>
 __global__ void __launch_bounds__(kTableBlock) k_table_rest(const __grid_constant__ TableStep T,
                                                             const __grid_constant__ StepDev p) {
+    after_previous();
     __shared__ __align__(16) float sh[kTableBlock / G * LaneSums<G>::kWords];
     const unsigned need = NEEDC == kNeedRuntime ? p.need : NEEDC;
     unsigned a, lane;
@@ -252,6 +255,7 @@ __global__ void __launch_bounds__(kTableBlock) k_table_rest(const __grid_constan
 // A in agent order and the first table (T's `next` one; its counts are zero).
 __global__ void k_table_init(GroupView g, const __grid_constant__ TableStep T, int wrap_mode,
                              int dirty, float4* f5, unsigned* redo_count) {
+    after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) *redo_count = 0u;
     if (i >= g.n) return;
@@ -268,7 +272,7 @@ __global__ void k_table_init(GroupView g, const __grid_constant__ TableStep T, i
 
 gs_status table_init(GroupView g, const TableStep& T, int wrap_mode, bool dirty, float4* f5,
                      unsigned* redo_count, cudaStream_t st) {
-    k_table_init<<<blocks_for(g.n, 64), 64, 0, st>>>(g, T, wrap_mode, dirty ? 1 : 0, f5, redo_count);
+    launch_after(k_table_init, blocks_for(g.n, 64), 64, 0, st, g, T, wrap_mode, dirty ? 1 : 0, f5, redo_count);
     GS_LAUNCHED("table_init");
     return GS_OK;
 }
@@ -278,16 +282,16 @@ static void table_go(const TableStep& T, const StepDev& p, cudaStream_t st) {
     const unsigned nb = blocks_for(T.n, kTableBlock / G);
     if (!(p.need & NEED_WALLS)) {
         if ((p.need & kNeedList) == (NEED_SEP | NEED_ALI | NEED_COH))
-            k_table_step<G, FLAT, NEED_SEP | NEED_ALI | NEED_COH><<<nb, kTableBlock, 0, st>>>(T, p);
+            launch_after(k_table_step<G, FLAT, NEED_SEP | NEED_ALI | NEED_COH>, nb, kTableBlock, 0, st, T, p);
         else
-            k_table_step<G, FLAT, kNeedRuntime><<<nb, kTableBlock, 0, st>>>(T, p);
+            launch_after(k_table_step<G, FLAT, kNeedRuntime>, nb, kTableBlock, 0, st, T, p);
         return;
     }
-    k_table_walls<G, FLAT><<<nb, kTableBlock, 0, st>>>(T, p);
+    launch_after(k_table_walls<G, FLAT>, nb, kTableBlock, 0, st, T, p);
     if ((p.need & kNeedList) == (NEED_SEP | NEED_AVOID))
-        k_table_rest<G, NEED_SEP | NEED_AVOID><<<nb, kTableBlock, 0, st>>>(T, p);
+        launch_after(k_table_rest<G, NEED_SEP | NEED_AVOID>, nb, kTableBlock, 0, st, T, p);
     else
-        k_table_rest<G, kNeedRuntime><<<nb, kTableBlock, 0, st>>>(T, p);
+        launch_after(k_table_rest<G, kNeedRuntime>, nb, kTableBlock, 0, st, T, p);
 }
 
 gs_status table_step(const TableStep& T, const StepDev& p, cudaStream_t st) {
