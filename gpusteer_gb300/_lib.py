@@ -175,4 +175,6 @@ def check(status: int) -> None:
 
 
 def call(name: str, *args) -> None:
-    check(getattr(load(), name)(*args))
+    status = getattr(_lib or load(), name)(*args)
+    if status != GS_OK:
+        check(status)

@@ -50,6 +50,8 @@ static void release_fused(gs_group g) {
     dfree(g->knn_dist);
     dfree(g->d_scene);
     dfree(g->d_err);
+    if (g->h_err) cudaFreeHost(g->h_err);
+    g->h_err = nullptr;
     dfree(g->retry);
     dfree(g->slot_of);
     dfree(g->retry_count);
@@ -699,7 +701,7 @@ static gs_status upload_enqueue(gs_group g, const gs_agent_arrays* h, unsigned n
     return GS_OK;
 }
 
-static gs_status check_device_flags(gs_group g);
+static gs_status sync_and_check(gs_group g);
 
 // Queues the copies of gs_group_download on the group's stream.  With
 // skip_constants the per-agent constants (maxSpeed, maxForce, radius, mass),
@@ -761,8 +763,7 @@ static gs_status download_copies(gs_group g, const gs_agent_arrays* h, bool skip
 gs_status gs_group_download(gs_group g, const gs_agent_arrays* h) {
     if (!g || !h) return fail(GS_ERR_INVALID_ARG, "null argument");
     GS_TRY(download_enqueue(g, h));
-    GS_CUDA(cudaStreamSynchronize(g->stream));
-    return check_device_flags(g);
+    return sync_and_check(g);
 }
 
 gs_status gs_group_size(gs_group g, unsigned* n) {
@@ -799,14 +800,20 @@ gs_status gs_group_stream(gs_group g, void** stream) {
     return GS_OK;
 }
 
-// Reads and clears the device error flags of the fused step.
-static gs_status check_device_flags(gs_group g) {
-    if (!g->d_err) return GS_OK;
-    unsigned flags = 0;
-    GS_CUDA(cudaMemcpyAsync(&flags, g->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost,
-                            g->stream));
+// Waits for the group's stream, then reads and clears the device error flags
+// of the fused step: they come with the work they describe, in page-locked
+// memory, so one wait serves both.
+static gs_status sync_and_check(gs_group g) {
+    if (g->d_err && !g->h_err) {
+        GS_CUDA(cudaMallocHost(reinterpret_cast<void**>(&g->h_err), sizeof(unsigned)));
+        *g->h_err = 0;
+    }
+    if (g->d_err)
+        GS_CUDA(cudaMemcpyAsync(g->h_err, g->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                                g->stream));
     GS_CUDA(cudaStreamSynchronize(g->stream));
-    if (flags) {
+    if (!g->d_err) return GS_OK;
+    if (const unsigned flags = *g->h_err) {
         GS_CUDA(cudaMemsetAsync(g->d_err, 0, sizeof(unsigned), g->stream));
         if (flags & kErrBarrierTimeout)
             return fail(GS_ERR_TIMEOUT,
@@ -818,8 +825,7 @@ static gs_status check_device_flags(gs_group g) {
 
 gs_status gs_group_synchronize(gs_group g) {
     if (!g) return fail(GS_ERR_INVALID_ARG, "null group");
-    GS_CUDA(cudaStreamSynchronize(g->stream));
-    return check_device_flags(g);
+    return sync_and_check(g);
 }
 
 // ---- KNN data -----------------------------------------------------------------------
@@ -2009,8 +2015,7 @@ gs_status gs_step_host(gs_group g, gs_bins bins, gs_walls walls, const gs_step_p
     const bool in_place = out->max_speed == in->max_speed && out->max_force == in->max_force &&
                           out->radius == in->radius && out->mass == in->mass;
     GS_TRY(download_enqueue(g, out, in_place));
-    GS_CUDA(cudaStreamSynchronize(g->stream));
-    return check_device_flags(g);
+    return sync_and_check(g);
 }
 
 gs_status gs_group_set_persistent(gs_group g, int enable) {
@@ -2412,10 +2417,9 @@ gs_status gs_batches_step_host(const gs_batch* parts, unsigned n_parts, const gs
     }
     gs_status s = GS_OK;
     for (unsigned i = 0; i < n_parts; ++i) {
-        const cudaError_t e = cudaStreamSynchronize(parts[i]->g->stream);
-        if (e != cudaSuccess && s == GS_OK) s = cuda_fail(e, "batches step");
+        const gs_status e = sync_and_check(parts[i]->g);  // waits for every part
+        if (s == GS_OK) s = e;
     }
-    for (unsigned i = 0; i < n_parts && s == GS_OK; ++i) s = check_device_flags(parts[i]->g);
     return s;
 }
 
@@ -2507,6 +2511,9 @@ struct gs_rollout_s {
     unsigned steps = 0, every = 0, n_seg = 0, cap = 0, k = 0;
     unsigned n = 0;           // agents at the last forward pass
     bool have_forward = false;
+    // the segment whose step records rec_* hold (n_seg: none).  The forward
+    // pass records its last one, so the backward pass need not run that again.
+    unsigned recorded = 0;
     gs_step_params params{};  // of the last forward pass
     // checkpoints [n_seg + 1][cap]: the state at the start of each segment, then the final state
     float4 *ck_pos = nullptr, *ck_dir = nullptr;
@@ -2637,6 +2644,9 @@ static gs_status rollout_restore(gs_rollout r, unsigned c) {
     return GS_OK;
 }
 
+static gs_status rollout_record(gs_rollout r, StepDev d, const Grid& grid, unsigned C,
+                                unsigned len);
+
 gs_status gs_rollout_forward(gs_rollout r, const gs_step_params* p) {
     if (!r) return fail(GS_ERR_INVALID_ARG, "null rollout");
     gs_group g = r->g;
@@ -2659,20 +2669,26 @@ gs_status gs_rollout_forward(gs_rollout r, const gs_step_params* p) {
     g->frame_cells = 0;
     g->accum_dirty = false;
     GS_TRY(rollout_save(r, 0));
+    r->recorded = r->n_seg;
     for (unsigned c = 0; c < r->n_seg; ++c) {
         const unsigned len = std::min(r->every, r->steps - c * r->every);
-        GS_TRY(gs_step(g, r->bins, nullptr, p, len));
+        if (c + 1 == r->n_seg && !g->profiling) {
+            GS_TRY(rollout_record(r, d, grid, C, len));
+            r->recorded = c;
+            g->frame_cells = C;
+        } else {
+            GS_TRY(gs_step(g, r->bins, nullptr, p, len));
+        }
         GS_TRY(rollout_save(r, c + 1));
     }
     r->have_forward = true;
     return GS_OK;
 }
 
-// Re-runs segment c from its checkpoint, recording every step's inputs.
-static gs_status rollout_record(gs_rollout r, unsigned c, StepDev d, const Grid& grid,
-                                unsigned C, unsigned len) {
+// Runs `len` steps from the group's state, recording every step's inputs.
+static gs_status rollout_record(gs_rollout r, StepDev d, const Grid& grid, unsigned C,
+                                unsigned len) {
     gs_group g = r->g;
-    GS_TRY(rollout_restore(r, c));
     GS_TRY(reserve_fused(g, C, false, d.k, 1));
     Scene sc{};
     sc.grid = grid;
@@ -2727,7 +2743,12 @@ gs_status gs_rollout_backward(gs_rollout r, const float* adj_position, const flo
     int cur = 0;
     for (unsigned c = r->n_seg; c-- > 0;) {
         const unsigned len = std::min(r->every, r->steps - c * r->every);
-        GS_TRY(rollout_record(r, c, d, grid, C, len));
+        if (c != r->recorded) {
+            r->recorded = r->n_seg;
+            GS_TRY(rollout_restore(r, c));
+            GS_TRY(rollout_record(r, d, grid, C, len));
+            r->recorded = c;
+        }
         for (unsigned j = len; j-- > 0;) {
             AdjointLaunch A;
             A.pos = r->rec_pos + size_t(j) * r->cap;
@@ -2756,8 +2777,7 @@ gs_status gs_rollout_backward(gs_rollout r, const float* adj_position, const flo
     GS_CUDA(cudaMemcpyAsync(part.data(), r->wpart, part.size() * 4, cudaMemcpyDeviceToHost, st));
     // leave the group at the rollout's final state
     GS_TRY(rollout_restore(r, r->n_seg));
-    GS_CUDA(cudaStreamSynchronize(st));
-    GS_TRY(check_device_flags(g));
+    GS_TRY(sync_and_check(g));
     if (grad_weights) {
         for (int b = 0; b < 3; ++b) {
             double sum = 0.0;  // host-side sum of the per-block partials

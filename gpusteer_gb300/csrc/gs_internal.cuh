@@ -179,6 +179,7 @@ struct gs_group_s {
     unsigned scene_alloc;
     std::vector<gs::Scene>* h_scenes;  // host copy of the table on the device
     unsigned* d_err;       // device error flags (see FusedLaunch::err)
+    unsigned* h_err;       // their page-locked copy
     unsigned* retry;       // [capacity] exact-redo list and its counter
     unsigned* slot_of;     // [capacity] each agent's slot (conversion to the reference layout)
     unsigned* retry_count;

@@ -435,7 +435,7 @@ gs_status gs_batch_cell_avg_velocity(gs_batch b, float* avg3);
  * every `checkpoint_every` steps, and then runs the hand-written adjoint of
  * the fused steering-plus-integrate step backwards through it: each segment
  * between checkpoints is re-run once with its steps' inputs and KNN lists
- * recorded, so memory grows with steps / checkpoint_every + checkpoint_every
+ * recorded (the last one is recorded by the forward pass), so memory grows with steps / checkpoint_every + checkpoint_every
  * states.  KNN lists and neighbourhood memberships are frozen at the
  * forward pass's values (piecewise constant); the derivative of the world
  * wrap is the identity.  Velocities are heading * speed. */
