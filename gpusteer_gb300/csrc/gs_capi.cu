@@ -385,6 +385,8 @@ static gs_status validate_step(const gs_step_params* p, gs_walls walls, StepDev&
             default: return fail(GS_ERR_INVALID_ARG, "unknown behaviour code");
         }
     }
+    d.same_flock = std::memcmp(&d.sep[2], &d.ali[2], 4) == 0 &&
+                   std::memcmp(d.ali, d.coh, 3 * sizeof(float)) == 0;
     if ((d.need & NEED_WALLS) && (p->knw == 0 || p->knw > 8))
         return fail(GS_ERR_INVALID_ARG, "knw must be in 1..8");
     (void)walls;

@@ -221,6 +221,7 @@ struct StepDev {
     unsigned n_order;
     float dt;
     unsigned need;      // NEED_* bits
+    unsigned same_flock;  // one cosine, and alignment's distances are cohesion's
     unsigned enum_cap;  // candidate capacity of the fast KNN scan (32, 64: collecting; 128, 256: streaming)
     unsigned block;     // threads per block of the fused launches (0: 256)
     unsigned flat;      // the grid is one cell high (y): boxes hold 3 rows of cells

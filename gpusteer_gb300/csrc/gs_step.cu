@@ -325,6 +325,36 @@ __device__ __forceinline__ bool packed_avoid_time_may_fall_in(const PackedSelf& 
     return avoid_time_window_test(ss, h, S, min_t);
 }
 
+// The flock's three behaviours where they share an angle and alignment and
+// cohesion their distances too (StepDev::same_flock: the usual flock): one
+// angle decision and one membership serve both, and separation, whose
+// distance few neighbours are within, only leaves a bit per member, so that
+// its divisions run as often as a warp's busiest lane has members instead of
+// once per neighbour that any lane separates from.  Same tests, same sums.
+// k = 16, a step: 1M boids 265.5 -> 253.5 us, 65,536 32.6 -> 31.1 (8 steps of
+// 1,048,576: 2358 -> 2242 with their conversions).
+__device__ __forceinline__ void accumulate_same(Accs& a, unsigned& sep_members,
+                                                const FlockParams& fs, const FlockParams& fa,
+                                                AngleGate gate, const Self& me, unsigned rank,
+                                                V3 bpos, V3 bdir) {
+    const V3 offset = sub(bpos, me.pos);
+    const float dsq = dot(offset, offset);
+    bool in_s = dsq < fs.lt, in_a = dsq < fa.lt;
+    const bool ang_s = !in_s && !(dsq > fs.gt), ang_a = !in_a && !(dsq > fa.gt);
+    if (ang_s || ang_a) {
+        const int t = angle_decide(dot(me.dir, offset), d_estimate(dsq), fs.cos_max, gate);
+        const bool ahead = t < 0 ? forward_component(me.dir, offset, dsq) > fs.cos_max : t > 0;
+        in_s = in_s || (ang_s && ahead);
+        in_a = in_a || (ang_a && ahead);
+    }
+    if (in_s) sep_members |= 1u << rank;
+    if (in_a) {
+        a.ali.sum = add(a.ali.sum, bdir);
+        a.coh.sum = add(a.coh.sum, bpos);
+        a.ali.n++;
+    }
+}
+
 // Behaviours order[first..] in order, then nothing else.  fetch(rank, pos,
 // dir, speed) reads neighbour list entry `rank` again (neighbour avoidance).
 // A runtime loop over the packed order (3 bits per entry), so each
@@ -589,7 +619,7 @@ constexpr unsigned kRestChunk = 2;  // the rest phase's (1: +7 %, 3: +6 %, 4: +1
 // kNbrChunk: neighbours whose gathers are in flight together (1 is best at
 // full occupancy: 2 there costs 2.5 %, 4 9 %).
 template <int KMAX, unsigned ENUM, bool EXACT, unsigned NEEDC = kNeedRuntime, bool FLAT = false,
-          unsigned kNbrChunk = 1>
+          unsigned kNbrChunk = 1, bool SAME = false>
 __global__ void __launch_bounds__(kBlock, kNbrChunk > 1 ? 2 : 3) k_fused(FusedLaunch L, StepDev p) {
     after_previous();
     const unsigned need = NEEDC == kNeedRuntime ? p.need : NEEDC;
@@ -627,6 +657,7 @@ __global__ void __launch_bounds__(kBlock, kNbrChunk > 1 ? 2 : 3) k_fused(FusedLa
                         gc = angle_gate(me.dir, fc.cos_max);
         Accs a;
         init_accs(a, p);
+        unsigned sep_members = 0;  // SAME: bit r for list entry r
         unsigned* rec_knn = L.rec_knn ? L.rec_knn + size_t(id) * p.k : nullptr;
         unsigned r = 0;
         // Neighbours kNbrChunk at a time: their loads are issued together, so
@@ -654,9 +685,21 @@ __global__ void __launch_bounds__(kBlock, kNbrChunk > 1 ? 2 : 3) k_fused(FusedLa
                     break;
                 }
                 if (rec_knn) rec_knn[r] = u(b0[j].w);
-                accumulate(a, p, need, fs, fa, fc, gs_, ga, gc, me, r, -1.f, v3(b0[j]), v3(b1[j]),
-                           b1[j].w, br[j]);
+                if constexpr (SAME)
+                    accumulate_same(a, sep_members, fs, fa, gs_, me, r, v3(b0[j]), v3(b1[j]));
+                else
+                    accumulate(a, p, need, fs, fa, fc, gs_, ga, gc, me, r, -1.f, v3(b0[j]),
+                               v3(b1[j]), b1[j].w, br[j]);
                 ++r;
+            }
+        }
+        if constexpr (SAME) {
+            a.coh.n = a.ali.n;
+            a.sep.n = unsigned(__popc(sep_members));
+            for (; sep_members; sep_members &= sep_members - 1u) {
+                const unsigned bs = col[(base + unsigned(__ffs(int(sep_members)) - 1)) * bd];
+                const V3 offset = sub(v3(L.B.f[0][bs]), me.pos);
+                a.sep.sum = add(a.sep.sum, dvd(offset, -dot(offset, offset)));
             }
         }
         if (rec_knn) {
@@ -939,9 +982,12 @@ static gs_status launch_fused_k(const FusedLaunch& L, const StepDev& p, cudaStre
                 // spare: two neighbours' gathers in flight (k = 16: 32,768
                 // boids 31.0 -> 28.1 us a step, 65,536 37.4 -> 32.6; 100,003,
                 // in one wave only at three to an SM, 45.8 against 46.3)
-                auto kern = nb * bs <= 2 * 152 * kBlock
-                                ? k_fused<KMAX, 32, false, NEED_SEP | NEED_ALI | NEED_COH, false, 2>
-                                : k_fused<KMAX, 32, false, NEED_SEP | NEED_ALI | NEED_COH>;
+                constexpr unsigned flock = NEED_SEP | NEED_ALI | NEED_COH;
+                const bool two = nb * bs <= 2 * 152 * kBlock;
+                auto kern = p.same_flock ? (two ? k_fused<KMAX, 32, false, flock, false, 2, true>
+                                                : k_fused<KMAX, 32, false, flock, false, 1, true>)
+                                         : (two ? k_fused<KMAX, 32, false, flock, false, 2>
+                                                : k_fused<KMAX, 32, false, flock>);
                 GS_TRY(allow_smem(kern, smem));
                 launch_after(kern, nb, bs, smem, st, L, p);
                 done = true;
