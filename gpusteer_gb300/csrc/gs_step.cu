@@ -331,8 +331,8 @@ __device__ __forceinline__ bool packed_avoid_time_may_fall_in(const PackedSelf& 
 // distance few neighbours are within, only leaves a bit per member, so that
 // its divisions run as often as a warp's busiest lane has members instead of
 // once per neighbour that any lane separates from.  Same tests, same sums.
-// k = 16, a step: 1M boids 265.5 -> 253.5 us, 65,536 32.6 -> 31.1 (8 steps of
-// 1,048,576: 2358 -> 2242 with their conversions).
+// k = 16, a step: 1,048,576 boids 265.5 -> 253.5 us, 65,536 32.6 -> 31.1; with
+// more gathers in flight (k_fused) 242.9 and 30.9.
 __device__ __forceinline__ void accumulate_same(Accs& a, unsigned& sep_members,
                                                 const FlockParams& fs, const FlockParams& fa,
                                                 AngleGate gate, const Self& me, unsigned rank,
@@ -616,11 +616,14 @@ __global__ void __launch_bounds__(kBlock) k_knn_retry(FusedLaunch L, StepDev p) 
 // ---- whole step without walls -------------------------------------------------------
 constexpr unsigned kRestChunk = 2;  // the rest phase's (1: +7 %, 3: +6 %, 4: +12 %; spills)
 
-// kNbrChunk: neighbours whose gathers are in flight together (1 is best at
-// full occupancy: 2 there costs 2.5 %, 4 9 %).
+// kNbrChunk: neighbours whose gathers are in flight together.  At three blocks
+// to an SM the general pass has registers for one (2 cost 2.5 %, 4 9 %); the
+// shared-angle pass is smaller and takes four (1,048,576 boids, k = 16: 253.2
+// -> 242.9 us a step; two 243.3), two where lists are short (k = 7: 203.1 ->
+// 199.9, four 203.2).
 template <int KMAX, unsigned ENUM, bool EXACT, unsigned NEEDC = kNeedRuntime, bool FLAT = false,
-          unsigned kNbrChunk = 1, bool SAME = false>
-__global__ void __launch_bounds__(kBlock, kNbrChunk > 1 ? 2 : 3) k_fused(FusedLaunch L, StepDev p) {
+          unsigned kNbrChunk = 1, int kBlocks = 3, bool SAME = false>
+__global__ void __launch_bounds__(kBlock, kBlocks) k_fused(FusedLaunch L, StepDev p) {
     after_previous();
     const unsigned need = NEEDC == kNeedRuntime ? p.need : NEEDC;
     extern __shared__ unsigned sh_col[];
@@ -976,17 +979,28 @@ static gs_status launch_fused_k(const FusedLaunch& L, const StepDev& p, cudaStre
         // the flock (separation, alignment, cohesion) on the collecting scan has
         // its own build
         bool done = false;
+        constexpr unsigned flock = NEED_SEP | NEED_ALI | NEED_COH;
+        constexpr unsigned kAhead = KMAX > 8 ? 4 : 2;
+        // larger candidate capacities: the shared-angle pass in place of the
+        // build that asks at run time (1,048,576 boids, k = 16: capacity 64
+        // 631 -> 466 us a step, 128 395 -> 336; k = 7: 482 -> 407, 283 -> 245)
+        if (ENUM > 32 && p.same_flock && (p.need & kNeedList) == flock && !(ENUM > 64 && p.flat)) {
+            auto kern = k_fused<KMAX, ENUM, false, flock, false, kAhead, 3, true>;
+            GS_TRY(allow_smem(kern, smem));
+            launch_after(kern, nb, bs, smem, st, L, p);
+            done = true;
+        }
         if constexpr (ENUM == 32) {
             if ((p.need & kNeedList) == (NEED_SEP | NEED_ALI | NEED_COH)) {
                 // a group whose blocks all fit at two to an SM has registers to
-                // spare: two neighbours' gathers in flight (k = 16: 32,768
+                // spare: more neighbours' gathers in flight (k = 16, two: 32,768
                 // boids 31.0 -> 28.1 us a step, 65,536 37.4 -> 32.6; 100,003,
-                // in one wave only at three to an SM, 45.8 against 46.3)
-                constexpr unsigned flock = NEED_SEP | NEED_ALI | NEED_COH;
+                // in one wave only at three to an SM, 45.8 against 46.3; the
+                // shared-angle pass, four against two: 30.8 against 31.4)
                 const bool two = nb * bs <= 2 * 152 * kBlock;
-                auto kern = p.same_flock ? (two ? k_fused<KMAX, 32, false, flock, false, 2, true>
-                                                : k_fused<KMAX, 32, false, flock, false, 1, true>)
-                                         : (two ? k_fused<KMAX, 32, false, flock, false, 2>
+                auto kern = p.same_flock ? (two ? k_fused<KMAX, 32, false, flock, false, 4, 2, true>
+                                                : k_fused<KMAX, 32, false, flock, false, kAhead, 3, true>)
+                                         : (two ? k_fused<KMAX, 32, false, flock, false, 2, 2>
                                                 : k_fused<KMAX, 32, false, flock>);
                 GS_TRY(allow_smem(kern, smem));
                 launch_after(kern, nb, bs, smem, st, L, p);
@@ -994,7 +1008,7 @@ static gs_status launch_fused_k(const FusedLaunch& L, const StepDev& p, cudaStre
             }
         }
         if constexpr (ENUM > 64) {
-            if (p.flat) {
+            if (p.flat && !done) {
                 GS_TRY(allow_smem(k_fused<KMAX, ENUM, false, kNeedRuntime, true>, smem));
                 launch_after(k_fused<KMAX, ENUM, false, kNeedRuntime, true>, nb, bs, smem, st, L, p);
                 done = true;

@@ -47,6 +47,20 @@ def test_flock_kernel_with_and_without_a_shared_angle(n, k, change):
     same(g.download(), want, f"n={n} k={k}")
 
 
+@pytest.mark.parametrize("change", [{}, dict(coh_cos=0.1)])
+@pytest.mark.parametrize("capacity", [64, 128, 256])
+@pytest.mark.parametrize("n,k", [(65, 3), (2049, 7), (1501, 16), (3001, 32)])
+def test_flock_kernel_at_larger_capacities(n, k, capacity, change):
+    """Dense enough that some agents' boxes hold more than the capacity."""
+    p = sc.boids_params(k=k, world=128.0).replace(**change)
+    s = sc.boids_sphere(n, radius=1.0 + 0.5 * n ** (1 / 3), seed=n + capacity)
+    g = group_of(s, p, capacity)
+    gs.step(g, gs.KNNBinData(p.world_cells, p.world_size, p.search_radius), None, p, 2)
+    want = s.copy()
+    ol.run(want, p, 2)
+    same(g.download(), want, f"n={n} k={k} capacity={capacity}")
+
+
 def clump(n, inside, seed):
     """`inside` of n boids within one cell, so that its row overflows."""
     s = sc.boids_sphere(n, radius=12.0, seed=seed)
