@@ -211,11 +211,27 @@ struct KList32 {
         cmpx(c[0], c[2]);
         cmpx(c[1], c[3]);
         cmpx(c[1], c[2]);
+        return take_sorted(c);
+    }
+    // The same for 8 keys (19 compare-exchanges): the list's own sort, the
+    // dearer part, runs half as often.
+    __device__ __forceinline__ unsigned merge8(unsigned (&c)[8]) {
+        static_assert(KMAX >= 8, "chunk merge needs KMAX >= 8");
+        cmpx(c[0], c[1]), cmpx(c[2], c[3]), cmpx(c[4], c[5]), cmpx(c[6], c[7]);
+        cmpx(c[0], c[2]), cmpx(c[1], c[3]), cmpx(c[4], c[6]), cmpx(c[5], c[7]);
+        cmpx(c[1], c[2]), cmpx(c[5], c[6]);
+        cmpx(c[0], c[4]), cmpx(c[1], c[5]), cmpx(c[2], c[6]), cmpx(c[3], c[7]);
+        cmpx(c[2], c[4]), cmpx(c[3], c[5]);
+        cmpx(c[1], c[2]), cmpx(c[3], c[4]), cmpx(c[5], c[6]);
+        return take_sorted(c);
+    }
+    template <int N>
+    __device__ __forceinline__ unsigned take_sorted(const unsigned (&c)[N]) {
         unsigned out = KEY32_EMPTY;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const unsigned a = key[KMAX - 4 + j], b = c[3 - j];
-            key[KMAX - 4 + j] = min(a, b);
+        for (int j = 0; j < N; ++j) {
+            const unsigned a = key[KMAX - N + j], b = c[N - 1 - j];
+            key[KMAX - N + j] = min(a, b);
             out = min(out, max(a, b));
         }
 #pragma unroll
@@ -419,15 +435,12 @@ __device__ __forceinline__ bool knn_neighbours_fast(int k, V3 p, unsigned self_i
     return near_pairs_ordered<KMAX, EBITS>(L.key, k, p, pos_id, key_tab, stride);
 }
 
-// The order the streaming scan visits the nine rows of a 3 x 3 x 3 (or
-// 3 x 3) box in (kRowOrderFlat: the three rows of a flat box): the middle
-// row first, then the rows beside it, then the corners, so the list fills with near candidates early and later candidates
-// insert less (1.5 % of a 256-scene choke-point step).  The result does not
-// depend on it: the list ends as the k smallest keys, whose enumeration
-// indices do not change, and ties of truncated distance send the agent to the
-// exact path.
+// The order the streaming scan visits the nine rows of a 3 x 3 x 3 box in: the
+// middle row first, then the rows beside it, then the corners, so the list
+// fills with near candidates early.  The result does not depend on it: the
+// list ends as the k smallest keys, whose enumeration indices do not change,
+// and ties of truncated distance send the agent to the exact path.
 __device__ constexpr int kRowOrder[9] = {4, 1, 3, 5, 7, 0, 2, 6, 8};
-__device__ constexpr int kRowOrderFlat[3] = {1, 0, 2};
 
 // Streaming fast path for crowded boxes: the same 32-bit keys, but the
 // candidates go straight into the register list, four at a time (no
@@ -438,12 +451,8 @@ __device__ constexpr int kRowOrderFlat[3] = {1, 0, 2};
 // row starts and the running row offsets alone.  Boxes of more than 3 x 3
 // rows (search radius above 1) are left to the exact path.  Writes the k
 // slots to out[r * stride]; returns false when the exact path must redo the
-// agent, on the same conditions as the collecting scan.  FLAT: the grid is
-// one cell high in y (the 2D worlds on the x-z plane), so a box has at most 3
-// rows; that build keeps 3 row starts instead of 9 (no register spills at
-// 64 registers) and drops the 6 empty row loops.  The rows and their
-// enumeration are those of the 9-row build (rows 3-8 are empty there).
-template <int KMAX, unsigned EBITS, bool FLAT = false>
+// agent, on the same conditions as the collecting scan.
+template <int KMAX, unsigned EBITS>
 __device__ __forceinline__ bool knn_neighbours_stream(int k, V3 p, unsigned self_id,
                                                       const Grid& g, const Box& b,
                                                       unsigned cell_offset,
@@ -451,14 +460,14 @@ __device__ __forceinline__ bool knn_neighbours_stream(int k, V3 p, unsigned self
                                                       const float4* __restrict__ pos_id,
                                                       unsigned* out, unsigned stride) {
     constexpr unsigned ENUM = 1u << EBITS, mask = ENUM - 1;
-    constexpr int R = FLAT ? 3 : 9;
-    if ((FLAT ? b.y1 != b.y0 : b.y1 - b.y0 > 2) || b.z1 - b.z0 > 2) return false;
+    constexpr int R = 9;
+    if (b.y1 - b.y0 > 2 || b.z1 - b.z0 > 2) return false;
     const unsigned span = b.x1 - b.x0 + 1;
     unsigned rs[R], pre[R + 1];
     pre[0] = 0;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-        const unsigned cy = b.y0 + unsigned(FLAT ? 0 : i / 3), cz = b.z0 + unsigned(i % 3);
+        const unsigned cy = b.y0 + unsigned(i / 3), cz = b.z0 + unsigned(i % 3);
         const bool ok = cy <= b.y1 && cz <= b.z1;
         const unsigned c0 = cell_offset + cell_label(g, b.x0, ok ? cy : b.y0, ok ? cz : b.z0);
         const unsigned s0 = ok ? __ldg(cell_start + c0) : 0u;
@@ -474,7 +483,7 @@ __device__ __forceinline__ bool knn_neighbours_stream(int k, V3 p, unsigned self
     const unsigned long long pxy = pack_xy(p.x, p.y);
 #pragma unroll
     for (int ii = 0; ii < R; ++ii) {
-        const int i = FLAT ? kRowOrderFlat[ii] : kRowOrder[ii];
+        const int i = kRowOrder[ii];
         const unsigned n_row = pre[i + 1] - pre[i];
         // four candidates at a time: their loads and distances overlap, and
         // one chunk merge costs less than four insertions
@@ -508,6 +517,80 @@ __device__ __forceinline__ bool knn_neighbours_stream(int k, V3 p, unsigned self
                 if (e >= pre[j]) slot = rs[j] + (e - pre[j]);
         }
         out[(i - (KMAX - k)) * stride] = slot;
+    }
+    return near_pairs_ordered<KMAX, EBITS>(L.key, k, p, pos_id, out, stride);
+}
+
+// The same in a flat world (one cell high in y: the 2D worlds on the x-z
+// plane), whose boxes have at most three rows.  They are walked end to end,
+// eight candidates to a merge: a warp runs as many merges as its busiest
+// lane's box needs, not each row's busiest in turn (256 crowded scenes, a
+// step's wall phase 381 -> 350 us).  SKIP_SELF: e leaves the agent itself out,
+// as the collecting scan's numbering does, so that a box of 2^EBITS others
+// still fits.
+template <int KMAX, unsigned EBITS, bool SKIP_SELF = false>
+__device__ __forceinline__ bool knn_neighbours_flat(int k, V3 p, unsigned self_id, const Grid& g,
+                                                    const Box& b, unsigned cell_offset,
+                                                    const unsigned* __restrict__ cell_start,
+                                                    const float4* __restrict__ pos_id,
+                                                    unsigned* out, unsigned stride) {
+    constexpr unsigned ENUM = 1u << EBITS, mask = ENUM - 1;
+    if (b.y1 != b.y0 || b.z1 - b.z0 > 2) return false;
+    const unsigned span = b.x1 - b.x0 + 1;
+    unsigned off[3], pre[4];  // the slot of the box's e-th agent is off[its row] + e
+    pre[0] = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const unsigned cz = b.z0 + unsigned(i);
+        const bool ok = cz <= b.z1;
+        const unsigned c0 = cell_offset + cell_label(g, b.x0, b.y0, ok ? cz : b.z0);
+        const unsigned s0 = ok ? __ldg(cell_start + c0) : 0u;
+        const unsigned s1 = ok ? __ldg(cell_start + c0 + span) : 0u;
+        off[i] = s0 - pre[i];
+        pre[i + 1] = pre[i] + (s1 - s0);
+    }
+    if (pre[3] > ENUM + (SKIP_SELF ? 1u : 0u)) return false;
+    const auto slot_of = [&](unsigned e) {
+        return e + (e < pre[1] ? off[0] : e < pre[2] ? off[1] : off[2]);
+    };
+    KList32<KMAX> L;
+#pragma unroll
+    for (int i = 0; i < KMAX; ++i) L.key[i] = i < KMAX - k ? 0u : KEY32_EMPTY;
+    unsigned out_min = KEY32_EMPTY;  // smallest key not (or no longer) in the list
+    const unsigned long long pxy = pack_xy(p.x, p.y);
+    unsigned self_e = UINT_MAX;
+    for (unsigned e0 = 0; e0 < pre[3]; e0 += 8) {
+        unsigned c[8];
+#pragma unroll
+        for (int h = 0; h < 8; h += 4) {
+            float4 q[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const unsigned e = e0 + unsigned(h + j);
+                q[j] = e < pre[3] ? __ldg(pos_id + slot_of(e))
+                                  : make_float4(0.f, 0.f, 0.f, __uint_as_float(self_id));
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const unsigned e = e0 + unsigned(h + j);
+                const unsigned bits = __float_as_uint(dist_sq_xy2(pxy, p.z, q[j]));
+                const bool self = __float_as_uint(q[j].w) == self_id;
+                if (SKIP_SELF && self && e < pre[3]) self_e = e;
+                c[h + j] = !self && bits <= 0x7f7fffffu
+                               ? (bits & ~mask) | (SKIP_SELF ? e - (e > self_e ? 1u : 0u) : e)
+                               : KEY32_EMPTY;
+            }
+        }
+        out_min = min(out_min, L.merge8(c));
+    }
+    if (SKIP_SELF && pre[3] > ENUM && self_e == UINT_MAX) return false;
+    if (boundary_unsure<EBITS>(L.key[KMAX - 1], out_min)) return false;
+#pragma unroll
+    for (int i = 0; i < KMAX; ++i) {
+        if (i < KMAX - k) continue;
+        const unsigned key = L.key[i], e = key & mask;
+        out[(i - (KMAX - k)) * stride] =
+            key != KEY32_EMPTY ? slot_of(e + (SKIP_SELF && e >= self_e ? 1u : 0u)) : UINT_MAX;
     }
     return near_pairs_ordered<KMAX, EBITS>(L.key, k, p, pos_id, out, stride);
 }

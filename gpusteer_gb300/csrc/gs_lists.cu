@@ -90,9 +90,15 @@ __device__ __forceinline__ void lists_thread(const KnnPair& pr, const Grid& grid
     cell_coords(grid, p, ix, iy, iz);
     const Box box = cell_box(grid, ix, iy, iz, 1);
     unsigned* col = sh + threadIdx.x;
-    const bool ok =
-        !act || knn_neighbours_stream<KMAX, 8, FLAT>(int(pr.k), p, self_id, grid, box, 0u,
-                                                     pr.b_start, pr.b_pos_id, col, kListBlock);
+    bool ok = true;
+    if (act) {
+        if constexpr (FLAT)
+            ok = knn_neighbours_flat<KMAX, 8>(int(pr.k), p, self_id, grid, box, 0u, pr.b_start,
+                                              pr.b_pos_id, col, kListBlock);
+        else
+            ok = knn_neighbours_stream<KMAX, 8>(int(pr.k), p, self_id, grid, box, 0u, pr.b_start,
+                                                pr.b_pos_id, col, kListBlock);
+    }
     __syncwarp();
     unsigned redo = __ballot_sync(kAllLanes, !ok);
     if (__popc(redo) >= int(kListsRedoThreads)) {

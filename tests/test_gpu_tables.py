@@ -172,3 +172,37 @@ def test_diagnostics_of_a_table_frame(inside, steps):
         cell_avg_velocity(g, bins),
         ol.cell_avg_velocity(frame.position, want.direction, want.speed, p.world_size,
                              p.world_cells))
+
+
+@pytest.mark.parametrize("capacity", [32, 64, 128])
+@pytest.mark.parametrize("n,k,width", [(33, 16, 5.0), (34, 16, 5.0), (900, 7, 60.0), (3001, 16, 70.0),
+                                       (2500, 32, 40.0)])
+@pytest.mark.parametrize("radius", [1, 2])
+def test_flat_rows_end_to_end(n, k, width, capacity, radius):
+    """The flat worlds' three-row scan at a fixed capacity: boxes below, at
+    and above it, and radius 2, which sparse boxes leave to the other scan."""
+    p = sc.chokepoint_params(k=k).replace(search_radius=radius)
+    s = sc.chokepoint_agents(n, x_range=(-width / 2, width / 2), z_range=(14.0, 14.0 + width),
+                             seed=n + k)
+    bins = gs.KNNBinData(p.world_cells, p.world_size, p.search_radius)
+    walls = gs.WallGroup(sc.chokepoint_walls(10.0), bins=bins, knw=p.knw)
+    g = group_of(s, p, capacity)
+    gs.step(g, bins, walls, p, 3)
+    want = s.copy()
+    ol.run(want, p, 3, walls=walls.download())
+    same(g.download(), want, f"n={n} k={k} capacity={capacity} radius={radius}")
+
+
+@pytest.mark.parametrize("inside", [32, 33, 34])
+def test_a_flat_box_at_its_capacity(inside):
+    """Capacity 32 holds an agent's box of 32 others, itself left out:
+    clumps of one agent fewer, as many and one more than fit."""
+    p = sc.chokepoint_params(k=16)
+    s = sc.chokepoint_agents(inside, x_range=(0.1, 1.9), z_range=(20.1, 21.9), seed=4)
+    bins = gs.KNNBinData(p.world_cells, p.world_size, p.search_radius)
+    walls = gs.WallGroup(sc.chokepoint_walls(10.0), bins=bins, knw=p.knw)
+    g = group_of(s, p, 32)
+    gs.step(g, bins, walls, p, 1)
+    want = s.copy()
+    ol.run(want, p, 1, walls=walls.download())
+    same(g.download(), want, f"inside={inside}")
