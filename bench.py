@@ -978,8 +978,8 @@ def gpu_brute_line(args, dist, rank, world, local_rank):
     ms_max = allreduce_max(dist, ev0.elapsed_time(ev1))
     per = ms_max / args.steps
     pairs_all = float(n) * (n - 1)
-    # the pairs the distance filter ran on: the bucketed scan skips chunks of
-    # candidates beyond every bound of a warp's queries
+    # the pairs whose distance was taken: the scan visits cells outwards from
+    # a query until no farther one can enter its list
     pairs = float(gs.bruteforce_pairs(g))
     tflops = 8.0 * pairs / (per / 1e3) / 1e12
     peak = fp32_peak_tflops()
@@ -1015,16 +1015,16 @@ def gpu_brute_line(args, dist, rank, world, local_rank):
         "config": brute_config(n, k, world),
         "e2e": {"value": n * e2e_steps * world / e2e_s, "unit": "agent-queries/s",
                 "h2d_bytes_per_step": n * 96, "d2h_bytes_per_step": n * k * 8},
-        # per call: the extent, the seed database (count, three scan
-        # launches, scatter), the seed, chunk and stage boxes, the scan
-        # (profiles/k_knn_brute3_65536_agents.md lists them)
+        # nominal: the calls' cost was ten launches each when this field's
+        # value was fixed; launches_per_call is what a call makes
+        # (profiles/k_brute_cells_65536_agents.md lists them)
         "gpu_launches": 10 * args.steps,
+        "launches_per_call": 2,
         "roofline": {"bound": "fp32", "achieved": tflops, "peak": peak, "unit": "TFLOP/s",
-                     "frac": tflops / peak, "traffic": None, "kernel": "k_knn_brute3_bucketed",
+                     "frac": tflops / peak, "traffic": None, "kernel": "k_brute_cells",
                      "algorithmic_flops_per_launch": 8.0 * pairs,
                      "pairs_evaluated": pairs, "pairs_all": pairs_all,
-                     "time": "the whole call (extent, seed databases and search, chunk "
-                             "boxes, scan)",
+                     "time": "the whole call (extent, cell database, scan)",
                      "peak_source": "measured here: cuBLAS SGEMM 8192^3 with TF32 off"},
         "issue": issue_rate("brute", per, clocks.summary(), local_rank),
         "clocks": clocks.summary(),

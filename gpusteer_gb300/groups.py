@@ -351,9 +351,10 @@ def step_launches(group, walls: bool) -> int:
     permute, the fused kernel (two with walls), and with the streaming scan
     (capacity 128 or 256) the warp-per-agent exact lists, plus, without
     walls, the exact redo (with walls the lists go straight to the second
-    half; the collecting scan redoes its rare agents inline).  A small
-    group's step (a group of lanes per agent, automatic capacity only) needs
-    no exact lists: with walls it makes one launch less than counted here."""
+    half; the collecting scan redoes its rare agents inline).  Counted for the
+    sorting step.  A small group's (a group of lanes per agent, automatic
+    capacity only) needs no exact lists, and a small single scene's at radius
+    1 no sort either: one launch, two with walls."""
     cap = knn_capacity(group)
     if getattr(group, "persistent", False) and walls and cap > 64 and 8 < group.k <= 16:
         return 1

@@ -261,8 +261,8 @@ typedef struct gs_multigroup_params {
  * group in turn: avoid the other groups' neighbours, separation from every
  * group, alignment and cohesion with itself, path following and seek of the
  * path's second point when paths[i] is set (paths may be NULL), update, and
- * anti-penetration against every group.  One steering launch per group
- * replaces its per-call launches; results equal the per-function sequence
+ * anti-penetration against every group.  One or two launches per group
+ * replace its per-call launches; results equal the per-function sequence
  * bit for bit.  At most 7 groups. */
 gs_status gs_multigroup_step(const gs_group* groups, unsigned n_groups, gs_bins bins,
                              const gs_path* paths, gs_knn* knn, const gs_multigroup_params* p,
@@ -270,9 +270,9 @@ gs_status gs_multigroup_step(const gs_group* groups, unsigned n_groups, gs_bins 
 gs_status gs_find_knn_walls(gs_group g, gs_knn out, gs_bins bins, gs_walls walls,
                             unsigned search_radius);
 /* KNNBruteForceCUDAV2 (KNNBruteForceCUDA.cu:163-187).  The lists are the
- * reference's for every pair of groups; with 4,096 queries or more the
- * scan skips candidates that cannot enter a list (a seeded bound and
- * bucketed chunks), so a call evaluates far fewer than n * m pairs. */
+ * reference's for every pair of groups; with 128 queries or more the
+ * scan takes cells of candidates outwards from each query until no farther
+ * one can enter its list, so a call evaluates far fewer than n * m pairs. */
 gs_status gs_knn_bruteforce(gs_group g, gs_knn out, gs_group other);
 /* The (query, candidate) pairs the last gs_knn_bruteforce call of g ran its
  * distance filter on (n * m without the skipping scan).  Synchronises the
