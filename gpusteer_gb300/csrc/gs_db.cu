@@ -8,7 +8,6 @@
 // databases are several clusters of one launch.
 #include <cooperative_groups.h>
 
-
 #include "gs_db.cuh"
 #include "gs_launch.h"
 
@@ -92,6 +91,10 @@ __global__ void __launch_bounds__(kDbThreads) k_db_cluster(const __grid_constant
     Grid grid = j.grid;
     if (first == 0 && j.zero) *j.zero = 0ull;
     if (j.auto_axis[0]) {
+        // the peers' shared memory is written below: every block of the
+        // cluster has to run by then, which this barrier waits for, under the
+        // pass over the positions
+        cluster.barrier_arrive();
         unsigned m[3] = {0u, 0u, 0u};
         for (unsigned i = first; i < n; i += step) {
             const float4 p = j.pos[i];
@@ -99,6 +102,7 @@ __global__ void __launch_bounds__(kDbThreads) k_db_cluster(const __grid_constant
             m[1] = max(m[1], __float_as_uint(fabsf(p.y)));
             m[2] = max(m[2], __float_as_uint(fabsf(p.z)));
         }
+        cluster.barrier_wait();
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
             const unsigned w = __reduce_max_sync(0xffffffffu, m[a]);
