@@ -37,8 +37,8 @@ template <int G, int L>
 __device__ __forceinline__ unsigned brute_region(LaneList<G, L>& list, const BruteQuery& q,
                                                  unsigned k, unsigned lane, bool on, const Box& out,
                                                  bool any, const Box& in, const Grid& g,
-                                                 const unsigned* __restrict__ start,
-                                                 const float4* __restrict__ pos_id,
+                                                 const unsigned* start,
+                                                 const float4* pos_id,
                                                  unsigned* segs) {
     unsigned* s0s = segs;
     unsigned* pre = segs + kBruteSegs;
@@ -62,8 +62,8 @@ __device__ __forceinline__ unsigned brute_region(LaneList<G, L>& list, const Bru
                 else if (cross) x1 = in.x0;
                 if (x0 < x1) {
                     const unsigned c = cell_label(g, x0, y, z);
-                    s0 = __ldg(start + c);
-                    len = __ldg(start + c + (x1 - x0)) - s0;
+                    s0 = start[c];
+                    len = start[c + (x1 - x0)] - s0;
                 }
             }
             unsigned sum = len;
@@ -86,7 +86,7 @@ __device__ __forceinline__ unsigned brute_region(LaneList<G, L>& list, const Bru
         auto load = [&](unsigned j) {
             if (j >= total) return make_float4(0.f, 0.f, 0.f, 0.f);
             while (j >= pre[at + 1]) ++at;
-            return __ldg(pos_id + s0s[at] + (j - pre[at]));
+            return pos_id[s0s[at] + (j - pre[at])];
         };
         float4 v = load(lane);
         for (unsigned j = lane; j < rounds + lane; j += G) {

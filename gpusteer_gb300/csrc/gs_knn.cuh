@@ -93,15 +93,15 @@ GS_HD Box cell_box(const Grid& g, unsigned ix, unsigned iy, unsigned iz, unsigne
 template <int KMAX>
 __device__ __forceinline__ void knn_scan_box(KList<KMAX>& L, V3 p, unsigned self_id,
                                              const Grid& g, const Box& b, unsigned cell_offset,
-                                             const unsigned* __restrict__ cell_start,
-                                             const float4* __restrict__ pos_id) {
+                                             const unsigned* cell_start,
+                                             const float4* pos_id) {
     for (unsigned cy = b.y0; cy <= b.y1; ++cy) {
         for (unsigned cz = b.z0; cz <= b.z1; ++cz) {
             const unsigned c0 = cell_offset + cell_label(g, b.x0, cy, cz);
             const unsigned c1 = cell_offset + cell_label(g, b.x1, cy, cz) + 1;
-            const unsigned s0 = __ldg(cell_start + c0), s1 = __ldg(cell_start + c1);
+            const unsigned s0 = cell_start[c0], s1 = cell_start[c1];
             for (unsigned s = s0; s < s1; ++s) {
-                const float4 q = __ldg(pos_id + s);
+                const float4 q = pos_id[s];
                 const unsigned id = __float_as_uint(q.w);
                 if (id == self_id) continue;
                 const float d = distance(p, v3(q));
@@ -153,14 +153,14 @@ __device__ __forceinline__ bool boundary_unsure(unsigned last, unsigned out_min)
 // register list, first listed entry at register `first`), out of line: few
 // agents have any.
 static __device__ __noinline__ bool near_pairs_check(unsigned near, int first, V3 p,
-                                                     const float4* __restrict__ pos_id,
+                                                     const float4* pos_id,
                                                      const unsigned* out, unsigned stride) {
     while (near) {
         const int i = __ffs(int(near)) - 1;
         near &= near - 1;
         const unsigned r = unsigned(i - first);
-        const float4 qa = __ldg(pos_id + out[(r - 1) * stride]);
-        const float4 qb = __ldg(pos_id + out[r * stride]);
+        const float4 qa = pos_id[out[(r - 1) * stride]];
+        const float4 qb = pos_id[out[r * stride]];
         if (!knn_less(distance(p, v3(qa)), __float_as_uint(qa.w), distance(p, v3(qb)),
                       __float_as_uint(qb.w)))
             return false;
@@ -170,7 +170,7 @@ static __device__ __noinline__ bool near_pairs_check(unsigned near, int first, V
 
 template <int KMAX, unsigned EBITS>
 __device__ __forceinline__ bool near_pairs_ordered(const unsigned (&key)[KMAX], int k, V3 p,
-                                                   const float4* __restrict__ pos_id,
+                                                   const float4* pos_id,
                                                    const unsigned* out, unsigned stride) {
     unsigned near = 0;
 #pragma unroll
@@ -296,10 +296,10 @@ __device__ __forceinline__ float dist_sq_xy2(unsigned long long pxy, float pz, f
 // No early exits: the warp's lanes reconverge after every candidate.
 template <unsigned ENUM>
 __device__ __forceinline__ void collect_one(unsigned s, V3 p, unsigned self_id,
-                                            const float4* __restrict__ pos_id, unsigned& e,
+                                            const float4* pos_id, unsigned& e,
                                             unsigned* slot_tab, unsigned* key_tab,
                                             unsigned stride) {
-    const float4 q = __ldg(pos_id + s);
+    const float4 q = pos_id[s];
     const unsigned bits = __float_as_uint(dist_sq(p, v3(q)));
     // inf or NaN (the distance is then inf or NaN: never below FLT_MAX, never
     // listed); a finite square gives a finite root, which is
@@ -319,8 +319,8 @@ constexpr unsigned kCollectChunk = 4;
 template <unsigned ENUM>
 __device__ __forceinline__ unsigned collect_box(V3 p, unsigned self_id, const Grid& g,
                                                 const Box& b, unsigned cell_offset,
-                                                const unsigned* __restrict__ cell_start,
-                                                const float4* __restrict__ pos_id,
+                                                const unsigned* cell_start,
+                                                const float4* pos_id,
                                                 unsigned* slot_tab, unsigned* key_tab,
                                                 unsigned stride) {
     unsigned e = 0;
@@ -336,8 +336,8 @@ __device__ __forceinline__ unsigned collect_box(V3 p, unsigned self_id, const Gr
             const unsigned cy = b.y0 + unsigned(i / 3), cz = b.z0 + unsigned(i % 3);
             const bool ok = cy <= b.y1 && cz <= b.z1;
             const unsigned c0 = cell_offset + cell_label(g, b.x0, ok ? cy : b.y0, ok ? cz : b.z0);
-            const unsigned s0 = ok ? __ldg(cell_start + c0) : 0u;
-            const unsigned s1 = ok ? __ldg(cell_start + c0 + span) : 0u;
+            const unsigned s0 = ok ? cell_start[c0] : 0u;
+            const unsigned s1 = ok ? cell_start[c0 + span] : 0u;
             rs[i] = s0;
             rn[i] = s1 - s0;
         }
@@ -361,7 +361,7 @@ __device__ __forceinline__ unsigned collect_box(V3 p, unsigned self_id, const Gr
                 sl[u] = j0 + u < total ? slot_tab[(j0 + u) * stride] : 0u;
 #pragma unroll
             for (unsigned u = 0; u < kCollectChunk; ++u)
-                q[u] = j0 + u < total ? __ldg(pos_id + sl[u]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                q[u] = j0 + u < total ? pos_id[sl[u]] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (unsigned u = 0; u < kCollectChunk; ++u) {
                 if (j0 + u >= total) break;
@@ -378,7 +378,7 @@ __device__ __forceinline__ unsigned collect_box(V3 p, unsigned self_id, const Gr
     for (unsigned cy = b.y0; cy <= b.y1; ++cy)
         for (unsigned cz = b.z0; cz <= b.z1; ++cz) {
             const unsigned c0 = cell_offset + cell_label(g, b.x0, cy, cz);
-            const unsigned s0 = __ldg(cell_start + c0), s1 = __ldg(cell_start + c0 + span);
+            const unsigned s0 = cell_start[c0], s1 = cell_start[c0 + span];
             for (unsigned s = s0; s < s1; ++s)
                 collect_one<ENUM>(s, p, self_id, pos_id, e, slot_tab, key_tab, stride);
         }
@@ -391,8 +391,8 @@ __device__ __forceinline__ unsigned collect_box(V3 p, unsigned self_id, const Gr
 template <int KMAX, unsigned ENUM>
 __device__ __forceinline__ bool knn_neighbours_fast(int k, V3 p, unsigned self_id, const Grid& g,
                                                     const Box& b, unsigned cell_offset,
-                                                    const unsigned* __restrict__ cell_start,
-                                                    const float4* __restrict__ pos_id,
+                                                    const unsigned* cell_start,
+                                                    const float4* pos_id,
                                                     unsigned* slot_tab, unsigned* key_tab,
                                                     unsigned stride) {
     constexpr unsigned mask = ENUM - 1, EBITS = Log2<ENUM>::value;
@@ -447,8 +447,8 @@ template <int KMAX, unsigned EBITS>
 __device__ __forceinline__ bool knn_neighbours_stream(int k, V3 p, unsigned self_id,
                                                       const Grid& g, const Box& b,
                                                       unsigned cell_offset,
-                                                      const unsigned* __restrict__ cell_start,
-                                                      const float4* __restrict__ pos_id,
+                                                      const unsigned* cell_start,
+                                                      const float4* pos_id,
                                                       unsigned* out, unsigned stride) {
     constexpr unsigned ENUM = 1u << EBITS, mask = ENUM - 1;
     constexpr int R = 9;
@@ -461,8 +461,8 @@ __device__ __forceinline__ bool knn_neighbours_stream(int k, V3 p, unsigned self
         const unsigned cy = b.y0 + unsigned(i / 3), cz = b.z0 + unsigned(i % 3);
         const bool ok = cy <= b.y1 && cz <= b.z1;
         const unsigned c0 = cell_offset + cell_label(g, b.x0, ok ? cy : b.y0, ok ? cz : b.z0);
-        const unsigned s0 = ok ? __ldg(cell_start + c0) : 0u;
-        const unsigned s1 = ok ? __ldg(cell_start + c0 + span) : 0u;
+        const unsigned s0 = ok ? cell_start[c0] : 0u;
+        const unsigned s1 = ok ? cell_start[c0 + span] : 0u;
         rs[i] = s0;
         pre[i + 1] = pre[i] + (s1 - s0);
     }
@@ -485,7 +485,7 @@ __device__ __forceinline__ bool knn_neighbours_stream(int k, V3 p, unsigned self
                 const unsigned t = t0 + unsigned(j);
                 c[j] = KEY32_EMPTY;
                 if (t < n_row) {
-                    const float4 q = __ldg(pos_id + rs[i] + t);
+                    const float4 q = pos_id[rs[i] + t];
                     const unsigned bits = __float_as_uint(dist_sq_xy2(pxy, p.z, q));
                     if (__float_as_uint(q.w) != self_id && bits <= 0x7f7fffffu)
                         c[j] = (bits & ~mask) | (pre[i] + t);
@@ -522,8 +522,8 @@ __device__ __forceinline__ bool knn_neighbours_stream(int k, V3 p, unsigned self
 template <int KMAX, unsigned EBITS, bool SKIP_SELF = false>
 __device__ __forceinline__ bool knn_neighbours_flat(int k, V3 p, unsigned self_id, const Grid& g,
                                                     const Box& b, unsigned cell_offset,
-                                                    const unsigned* __restrict__ cell_start,
-                                                    const float4* __restrict__ pos_id,
+                                                    const unsigned* cell_start,
+                                                    const float4* pos_id,
                                                     unsigned* out, unsigned stride) {
     constexpr unsigned ENUM = 1u << EBITS, mask = ENUM - 1;
     if (b.y1 != b.y0 || b.z1 - b.z0 > 2) return false;
@@ -535,8 +535,8 @@ __device__ __forceinline__ bool knn_neighbours_flat(int k, V3 p, unsigned self_i
         const unsigned cz = b.z0 + unsigned(i);
         const bool ok = cz <= b.z1;
         const unsigned c0 = cell_offset + cell_label(g, b.x0, b.y0, ok ? cz : b.z0);
-        const unsigned s0 = ok ? __ldg(cell_start + c0) : 0u;
-        const unsigned s1 = ok ? __ldg(cell_start + c0 + span) : 0u;
+        const unsigned s0 = ok ? cell_start[c0] : 0u;
+        const unsigned s1 = ok ? cell_start[c0 + span] : 0u;
         off[i] = s0 - pre[i];
         pre[i + 1] = pre[i] + (s1 - s0);
     }
@@ -558,7 +558,7 @@ __device__ __forceinline__ bool knn_neighbours_flat(int k, V3 p, unsigned self_i
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const unsigned e = e0 + unsigned(h + j);
-                q[j] = e < pre[3] ? __ldg(pos_id + slot_of(e))
+                q[j] = e < pre[3] ? pos_id[slot_of(e)]
                                   : make_float4(0.f, 0.f, 0.f, __uint_as_float(self_id));
             }
 #pragma unroll
@@ -590,8 +590,8 @@ __device__ __forceinline__ bool knn_neighbours_flat(int k, V3 p, unsigned self_i
 template <int KMAX>
 __device__ __forceinline__ void knn_neighbours_exact(int k, V3 p, unsigned self_id, const Grid& g,
                                                      const Box& b, unsigned cell_offset,
-                                                     const unsigned* __restrict__ cell_start,
-                                                     const float4* __restrict__ pos_id,
+                                                     const unsigned* cell_start,
+                                                     const float4* pos_id,
                                                      unsigned* col, unsigned stride) {
     KList<KMAX> L;
     L.init(k);

@@ -107,8 +107,8 @@ template <int G, int R>
 __device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 p,
                                                   unsigned self_id, const Grid& g, const Box& b,
                                                   unsigned cell_offset,
-                                                  const unsigned* __restrict__ start,
-                                                  const float4* __restrict__ pos_id,
+                                                  const unsigned* start,
+                                                  const float4* pos_id,
                                                   unsigned* rows = nullptr) {
     LaneEntry<G> list{KEY_EMPTY, UINT_MAX};
     const unsigned span = b.x1 - b.x0 + 1;
@@ -122,8 +122,8 @@ __device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 
             s0[q] = len[q] = 0;
             if (i < unsigned(R) && cy <= b.y1 && cz <= b.z1) {
                 const unsigned c0 = cell_offset + cell_label(g, b.x0, cy, cz);
-                s0[q] = __ldg(start + c0);
-                len[q] = __ldg(start + c0 + span) - s0[q];
+                s0[q] = start[c0];
+                len[q] = start[c0 + span] - s0[q];
             }
         }
         unsigned rs[R], pre[R + 1];
@@ -143,11 +143,11 @@ __device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 
         };
         // the next chunk's position is on its way while this one is sorted in
         unsigned sl = at(lane);
-        float4 q = lane < total ? __ldg(pos_id + sl) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 q = lane < total ? pos_id[sl] : make_float4(0.f, 0.f, 0.f, 0.f);
         for (unsigned j0 = 0; j0 < rounds; j0 += G) {
             const unsigned j = j0 + lane, jn = j + G;
             const unsigned sn = at(jn);
-            const float4 qn = jn < total ? __ldg(pos_id + sn) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 qn = jn < total ? pos_id[sn] : make_float4(0.f, 0.f, 0.f, 0.f);
             lanes_take(list, lanes_candidate<G>(p, self_id, q, sl, j < total), j0 == 0, k, lane);
             sl = sn;
             q = qn;
@@ -159,8 +159,8 @@ __device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 
         const unsigned most = __reduce_max_sync(kAllLanes, nr);
         auto row = [&](unsigned i, unsigned& s0) {
             const unsigned c0 = cell_offset + cell_label(g, b.x0, b.y0 + i / nz, b.z0 + i % nz);
-            s0 = __ldg(start + c0);
-            return __ldg(start + c0 + span) - s0;
+            s0 = start[c0];
+            return start[c0 + span] - s0;
         };
         if (most <= kLaneRows) {
             unsigned* rs = rows;
@@ -191,7 +191,7 @@ __device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 
                     while (j >= pre[at + 1]) ++at;
                     sl = rs[at] + (j - pre[at]);
                 }
-                const float4 q = ok ? __ldg(pos_id + sl) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 q = ok ? pos_id[sl] : make_float4(0.f, 0.f, 0.f, 0.f);
                 lanes_take(list, lanes_candidate<G>(p, self_id, q, sl, ok), j < G, k, lane);
             }
             __syncwarp();  // the rows may be written again
@@ -203,7 +203,7 @@ __device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 
                 const unsigned rounds = __reduce_max_sync(kAllLanes, len);
                 for (unsigned j = lane; j < rounds + lane; j += G) {
                     const float4 q =
-                        j < len ? __ldg(pos_id + s0 + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        j < len ? pos_id[s0 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
                     lanes_take(list, lanes_candidate<G>(p, self_id, q, s0 + j, j < len), first, k,
                                lane);
                     first = false;

@@ -7,15 +7,23 @@
 namespace gs {
 
 // ---- launches that follow one another --------------------------------------------
-// Every kernel of a step or of a call sequence starts with after_previous() and
-// is launched with launch_after(): its blocks may become resident once the
-// kernel before it in the stream has all of its own running, and wait there for
-// that kernel's end and its writes.  The launch latency and the blocks' start
-// then pass under the previous kernel.  Nothing is read or written before the
-// wait; a kernel completes only after its predecessor has, so the order of a
-// whole chain holds.  The pointer parameters of these kernels are not
-// __restrict__: loads through a const __restrict__ parameter count as invariant
-// and the compiler may move the first of them above the wait.
+// A kernel launched with launch_after() starts with after_previous(): its blocks
+// may become resident once the kernel before it in the stream has all of its
+// own running, and wait there for that kernel's end and its writes.  The launch
+// latency and the blocks' start then pass under the previous kernel.  Nothing is
+// read or written before the wait; a kernel completes only after its predecessor
+// has, so the order of a whole chain holds.
+//
+// Since such a kernel is resident while its predecessor writes, what it reads is
+// not constant for its lifetime: neither its pointer parameters nor those of the
+// helpers are const __restrict__ (loads through them count as invariant and may
+// be moved above the wait), and every load is an ordinary one, not the read-only
+// path's.
+//
+// Kernels launched with <<<>>> (a new grid's recount, the diagnostics, brute
+// force over every pair, the thread-per-agent group frames and
+// anti-penetration) keep plain stream order: they start after their predecessor
+// has ended, and what follows them waits for their end as for any other's.
 __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");

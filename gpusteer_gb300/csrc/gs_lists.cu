@@ -69,8 +69,8 @@ __global__ void __launch_bounds__(kListBlock) k_lists_lanes_pairs(const __grid_c
 // ---- one thread per query --------------------------------------------------------------------
 template <int KMAX>
 static __device__ __noinline__ void lists_exact(int k, V3 p, unsigned self_id, const Grid& g, Box b,
-                                                const unsigned* __restrict__ start,
-                                                const float4* __restrict__ pos_id, unsigned* col) {
+                                                const unsigned* start,
+                                                const float4* pos_id, unsigned* col) {
     knn_neighbours_exact<KMAX>(k, p, self_id, g, b, 0u, start, pos_id, col, kListBlock);
 }
 

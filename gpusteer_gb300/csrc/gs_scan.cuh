@@ -58,9 +58,9 @@ __device__ __forceinline__ void load_tile(const unsigned* count, unsigned C, uns
 
 // Tile t's total into tile[t] (sh: kScanTile + kScanTile / 32 words, ws:
 // kBlock / 32 words of shared memory).
-__device__ __forceinline__ void scan_reduce_tile(const unsigned* __restrict__ count, unsigned C,
+__device__ __forceinline__ void scan_reduce_tile(const unsigned* count, unsigned C,
                                                  unsigned t, unsigned* sh, unsigned* ws,
-                                                 unsigned* __restrict__ tile) {
+                                                 unsigned* tile) {
     unsigned items[kScanItems];
     load_tile(count, C, t, sh, items);
     unsigned s = 0;
@@ -74,9 +74,9 @@ __device__ __forceinline__ void scan_reduce_tile(const unsigned* __restrict__ co
 
 // Tile t's starts (its prefix summed from the totals of the tiles before it),
 // zeroing its counts; the last tile also writes start[C].
-__device__ __forceinline__ void scan_apply_tile(unsigned* __restrict__ count, unsigned C,
-                                                const unsigned* __restrict__ tile,
-                                                unsigned* __restrict__ start, unsigned T,
+__device__ __forceinline__ void scan_apply_tile(unsigned* count, unsigned C,
+                                                const unsigned* tile,
+                                                unsigned* start, unsigned T,
                                                 unsigned t, unsigned* sh, unsigned* ws) {
     unsigned before = 0;
     for (unsigned u = threadIdx.x; u < t; u += blockDim.x) before += tile[u];
@@ -118,11 +118,11 @@ __device__ __forceinline__ void scan_apply_tile(unsigned* __restrict__ count, un
 // holds agents; live[t] records which.  The other tiles' counts are already
 // zero and their starts, stale, are not read.  reach >= kBlock / 2: every
 // tile is written.
-__device__ __forceinline__ void scan_apply_sparse_tile(unsigned* __restrict__ count, unsigned C,
-                                                       const unsigned* __restrict__ tile,
-                                                       unsigned* __restrict__ start, unsigned T,
+__device__ __forceinline__ void scan_apply_sparse_tile(unsigned* count, unsigned C,
+                                                       const unsigned* tile,
+                                                       unsigned* start, unsigned T,
                                                        unsigned t, unsigned reach,
-                                                       unsigned* __restrict__ live, unsigned* sh,
+                                                       unsigned* live, unsigned* sh,
                                                        unsigned* ws) {
     unsigned v = reach >= kBlock / 2 ? 1u : 0u;
     if (!v && threadIdx.x <= 2 * reach) {

@@ -89,7 +89,7 @@ gs_status fused_recount(Fused A, unsigned n, const Scene* scenes, uint2* cellran
 
 // A (slot i) -> B (slot dst), wrapping the position.
 __device__ __forceinline__ void move_agent(const Fused& A, const Fused& B,
-                                           const Scene* __restrict__ scenes, int wrap_mode,
+                                           const Scene* scenes, int wrap_mode,
                                            int dirty, unsigned i, unsigned dst) {
     const float4 f0 = A.f[0][i];
     const float4 f4v = A.f[4][i];
@@ -107,7 +107,7 @@ __device__ __forceinline__ void move_agent(const Fused& A, const Fused& B,
 __device__ __forceinline__ void permute_agent(const Fused& A, const Fused& B, unsigned n,
                                               const uint2* cellrank,
                                               const unsigned* start,
-                                              const Scene* __restrict__ scenes, int wrap_mode,
+                                              const Scene* scenes, int wrap_mode,
                                               int dirty, unsigned* err, unsigned i) {
     const uint2 cr = cellrank[i];
     const unsigned dst = start[cr.x] + cr.y;
@@ -415,8 +415,8 @@ template <int KMAX>
 static __device__ __noinline__ void knn_exact_out_of_line(int k, V3 p, unsigned self_id,
                                                           const Grid& g, Box b,
                                                           unsigned cell_offset,
-                                                          const unsigned* __restrict__ start,
-                                                          const float4* __restrict__ pos_id,
+                                                          const unsigned* start,
+                                                          const float4* pos_id,
                                                           unsigned* col, unsigned stride) {
     knn_neighbours_exact<KMAX>(k, p, self_id, g, b, cell_offset, start, pos_id, col, stride);
 }

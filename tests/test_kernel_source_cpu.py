@@ -63,3 +63,41 @@ def test_clusters_have_started_before_remote_shared_memory_is_touched():
                 assert re.search(r"\bcluster\.(sync|barrier_wait)\s*\(", passed), \
                     f"{path.name} {name}: {body[m.start() - 20:m.end() + 40]!r}"
     assert met >= 2
+
+
+LAUNCHED_EARLY = sorted({m for p in SOURCES
+                         for m in re.findall(r"\blaunch_after\(\s*(k_\w+)", code(p))} | {"k_db_cluster"})
+
+
+def test_kernels_found():
+    assert len(LAUNCHED_EARLY) >= 20
+    assert any("*kern" in code(p) or "auto kern" in code(p) for p in SOURCES)  # named through a variable
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_no_read_only_path_loads(path):
+    """A kernel whose blocks may be resident before its predecessor has ended
+    reads what that predecessor writes: the read-only path is for data that
+    nobody writes while the reading kernel runs."""
+    text = code(path)
+    for form in (r"__ldg\s*\(", r"ld\.global\.nc", r"__ldlu\s*\("):
+        assert not re.search(form, text), f"{path.name}: {form}"
+
+
+def test_early_launched_kernels_wait_first_and_take_no_invariant_pointers():
+    """They begin with the wait, and no const __restrict__ pointer (whose
+    loads count as invariant) is among their parameters or in the helpers that
+    read the databases."""
+    found = set()
+    for path in SOURCES:
+        text = code(path)
+        for name, params, body in kernels(text):
+            if name in LAUNCHED_EARLY or name == "k_fused":
+                found.add(name)
+                assert "__restrict__" not in params, f"{path.name} {name}"
+                assert re.match(r"\{\s*after_previous\(\);", body), f"{path.name} {name}"
+        if path.suffix == ".cuh" or path.name in ("gs_lists.cu", "gs_brute.cu", "gs_step.cu"):
+            for m in re.finditer(r"__device__[^;{]*?\(([^;{]*?)\)\s*(?:const\s*)?\{", text):
+                assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", m.group(1)), \
+                    f"{path.name}: {m.group(0)[:120]}"
+    assert found == set(LAUNCHED_EARLY) | {"k_fused"}
