@@ -1692,18 +1692,25 @@ static bool gather_first_permute(gs_group g) {
     return most >= kGatherPermuteMinAgents;
 }
 
+// Whether the group's measurement holds for this grid and radius.
+static bool measured(gs_group g, const Grid& grid, unsigned r) {
+    return g->auto_cap_valid && g->auto_cap_r == r &&
+           std::memcmp(&g->auto_cap_grid, &grid, sizeof(Grid)) == 0;
+}
+
 // Measures the automatic KNN capacity from the cell counts where the last
 // measurement no longer holds: one synchronising read per upload that changes
 // the agent count, or grid change.
 static gs_status measure_capacity(gs_group g, const unsigned* count, unsigned C, const Grid& grid,
                                   unsigned r) {
-    if (g->auto_cap_valid && g->auto_cap_r == r &&
-        std::memcmp(&g->auto_cap_grid, &grid, sizeof(Grid)) == 0)
-        return GS_OK;
-    unsigned occupied = 0;
+    if (measured(g, grid, r)) return GS_OK;
+    unsigned occupied = 0, met = 0;
     unsigned long long sumsq = 0;
-    GS_TRY(count_occupied(count, C, g->d_stat, &occupied, &sumsq, g->stream));
+    const bool boxes = r == 1 && g->n <= kLanesMost && C == grid.wc[0] * grid.wc[1] * grid.wc[2];
+    GS_TRY(count_occupied(count, C, g->d_stat, &occupied, &sumsq, boxes ? &grid : nullptr, &met,
+                          g->stream));
     g->auto_cap = knn_capacity(g->n, sumsq, grid, r);
+    g->auto_met = met;
     g->auto_cap_grid = grid;
     g->auto_cap_r = r;
     g->auto_cap_valid = true;
@@ -1790,13 +1797,35 @@ static void fill_launch(gs_group g, const StepDev& d, const WallsDev& w, FusedLa
 }
 
 // ---- the small groups' step on cell tables (gs_table.cu) ---------------------------
-// Rows of 16 places a cell (32 in a flat world, whose cells are columns) and
-// at most 64 MiB a table; larger grids keep the sorting step.
-static unsigned table_row_log2(const StepDev& d) { return d.flat ? 5u : 4u; }
-static bool table_wanted(gs_group g, const StepDev& d, unsigned C, const unsigned* agent_scene) {
+// Places in a cell's row: at least 16 (32 in a flat world, whose cells are
+// columns), longer ones (up to 256) where the grid is coarse and a table stays
+// within 16 MiB, as crowded cells then need no further rows (8 steps of 10,000
+// boids, 40 in a cell of 4,096: 1065 us with rows of 16, 865 of 64, 830 of 256).
+// Grids whose tables would pass 64 MiB keep the sorting step.
+static unsigned table_row_log2(const StepDev& d, unsigned C) {
+    unsigned log2 = d.flat ? 5u : 4u;
+    while (log2 < 8u && (size_t(C) << (log2 + 1)) <= (size_t(1) << 20)) ++log2;
+    return log2;
+}
+// Candidates that all agents' boxes hold together, up to which the table is the
+// faster form: a lane group reads a box's 27 rows dearer than 9 sorted runs, but
+// saves two launches.  Table / sorting lanes (us, 8 steps): 2,000 boids, k = 16,
+// 843 to a box 258 / 280; 8,192, 221 to a box 255 / 256, 432 348 / 329; 16,384,
+// 131 310 / 321, 201 363 / 370, 606 617 / 602 and at k = 7 131 283 / 287, 201
+// 344 / 331, 606 627 / 524; a crowd of 10,000 (4 steps), 200 167 / 174, 500
+// 257 / 235.
+constexpr unsigned kTableMostCandidates = 2500000;
+static bool table_wanted(gs_group g, const StepDev& d, const Grid& grid, unsigned C,
+                         const unsigned* agent_scene) {
     return agent_scene == nullptr && d.r == 1 && g->knn_cap == 0 && !g->profiling &&
            !g->persistent && lanes_preferred(g->n, (d.need & NEED_WALLS) != 0) &&
-           (size_t(C) << table_row_log2(d)) <= (size_t(1) << 22);
+           (size_t(C) << table_row_log2(d, C)) <= (size_t(1) << 22) &&
+           !(measured(g, grid, 1) && g->auto_met > kTableMostCandidates);
+}
+
+// Words of the counts and tags, three arrays of each.
+static size_t table_words(unsigned C, unsigned ext_log2) {
+    return 3 * (size_t(C) + (size_t(1) << ext_log2));
 }
 
 static gs_status table_reserve(gs_group g, unsigned C, unsigned row_log2) {
@@ -1807,17 +1836,19 @@ static gs_status table_reserve(gs_group g, unsigned C, unsigned row_log2) {
         cudaFree(t.block);
         t = CellTable();
     }
-    const size_t row = (size_t(C) << row_log2) * 16, over = size_t(g->capacity) * 16;
+    // m agents fill at most m >> row_log2 further rows; twice as many slots
+    const unsigned rows = std::min(g->capacity, kLanesMost) >> row_log2;
+    unsigned ext_log2 = 4;
+    while (1u << ext_log2 < 2 * rows) ++ext_log2;
+    const size_t tab = ((size_t(C) + (size_t(1) << ext_log2)) << row_log2) * sizeof(float4);
     char* b = nullptr;
-    GS_TRY(dalloc(&b, 2 * (row + over) + (3 * size_t(C) + 4) * 4));
+    GS_TRY(dalloc(&b, 2 * tab + 4 * table_words(C, ext_log2)));
     t.block = b;
-    for (int i = 0; i < 2; ++i) {
-        t.tab[i] = reinterpret_cast<float4*>(b + size_t(i) * row);
-        t.over[i] = reinterpret_cast<float4*>(b + 2 * row + size_t(i) * over);
-    }
-    t.cnt = reinterpret_cast<unsigned*>(b + 2 * (row + over));
+    for (int i = 0; i < 2; ++i) t.tab[i] = reinterpret_cast<float4*>(b + size_t(i) * tab);
+    t.cnt = reinterpret_cast<unsigned*>(b + 2 * tab);
     t.cells = C;
     t.row_log2 = row_log2;
+    t.ext_log2 = ext_log2;
     return GS_OK;
 }
 
@@ -1828,17 +1859,16 @@ static TableStep table_buffers(gs_group g, unsigned step) {
     std::memset(static_cast<void*>(&T), 0, sizeof(T));
     const unsigned in = step % 2, out = 1 - in, ci = step % 3, co = (step + 1) % 3,
                    cc = (step + 2) % 3;
-    unsigned* const over_n = t.cnt + 3 * size_t(t.cells);
+    unsigned* const tags = t.cnt + 3 * size_t(t.cells);
+    const size_t slots = size_t(1) << t.ext_log2;
     T.tab = t.tab[in];
-    T.over = t.over[in];
     T.cnt = t.cnt + size_t(ci) * t.cells;
-    T.over_n = over_n + ci;
+    T.tag = tags + ci * slots;
     T.tab_next = t.tab[out];
-    T.over_next = t.over[out];
     T.cnt_next = t.cnt + size_t(co) * t.cells;
-    T.over_n_next = over_n + co;
+    T.tag_next = tags + co * slots;
     T.cnt_clear = t.cnt + size_t(cc) * t.cells;
-    T.over_n_clear = over_n + cc;
+    T.tag_clear = tags + cc * slots;
     T.f0 = T.f0_next = g->A.f[0];
     T.f1 = T.f1_next = g->A.f[1];
     T.f2 = g->A.f[2];
@@ -1853,23 +1883,26 @@ static TableStep table_buffers(gs_group g, unsigned step) {
     T.n = g->n;
     T.cells = t.cells;
     T.row_log2 = t.row_log2;
+    T.ext_log2 = t.ext_log2;
     T.sc = (*g->h_scenes)[0];
     return T;
 }
 
+// taken: false where the cells just counted are too full for the table; nothing
+// has then been done to the group's state.
 static gs_status table_run(gs_group g, StepDev d, const Grid& grid, unsigned C,
-                           const WallsDev& w, unsigned steps) {
+                           const WallsDev& w, unsigned steps, bool& taken) {
     cudaStream_t st = g->stream;
     CellTable& t = g->table;
     bool dirty = false;
-    g->frame_cells = 0;
-    if (!g->fused_current || !t.valid || t.cells != C || t.row_log2 != table_row_log2(d) ||
+    taken = true;
+    if (!g->fused_current || !t.valid || t.cells != C || t.row_log2 != table_row_log2(d, C) ||
         std::memcmp(&t.grid, &grid, sizeof(Grid)) != 0 || t.wrap_mode != d.wrap_mode) {
         GS_TRY(ensure_reference(g));
         dirty = g->accum_dirty;
         t.valid = t.frame = false;
-        GS_TRY(table_reserve(g, C, table_row_log2(d)));
-        GS_CUDA(cudaMemsetAsync(t.cnt, 0, (3 * size_t(C) + 4) * 4, st));
+        GS_TRY(table_reserve(g, C, table_row_log2(d, C)));
+        GS_CUDA(cudaMemsetAsync(t.cnt, 0, 4 * table_words(C, t.ext_log2), st));
         // step "-1" fills the table that step 0 reads
         t.step = 0;
         GS_TRY(table_init(view(g), table_buffers(g, 5), d.wrap_mode, dirty, g->A.f[5],
@@ -1879,7 +1912,17 @@ static gs_status table_run(gs_group g, StepDev d, const Grid& grid, unsigned C,
         t.valid = true;
         g->fused_current = true;
     }
-    GS_TRY(measure_capacity(g, t.cnt + size_t(t.step % 3) * C, C, grid, d.r));
+    if (!measured(g, grid, d.r)) {
+        GS_TRY(measure_capacity(g, t.cnt + size_t(t.step % 3) * C, C, grid, d.r));
+        if (g->auto_met > kTableMostCandidates) {
+            // the reference layout still holds the state: an unmeasured grid is
+            // a table just filled from it
+            t.valid = false;
+            g->fused_current = false;
+            taken = false;
+            return GS_OK;
+        }
+    }
     g->fdb.grid = grid;
     const bool walls = d.need & NEED_WALLS;
     for (unsigned s = 0; s < steps; ++s) {
@@ -1915,8 +1958,12 @@ static gs_status fused_run(gs_group g, StepDev d, const Grid& grid, unsigned C,
     FusedLaunch L;
     bool dirty = false, fresh = false;
     g->frame_cells = 0;
+    if (table_wanted(g, d, grid, C, agent_scene)) {
+        bool taken = false;
+        GS_TRY(table_run(g, d, grid, C, w, steps, taken));
+        if (taken) return GS_OK;
+    }
     // part of the graph key: a changed form or limit captures again
-    if (table_wanted(g, d, C, agent_scene)) return table_run(g, d, grid, C, w, steps);
     d.persistent = g->persistent ? 1u : 0u;
     d.bar_limit = g->bar_limit ? g->bar_limit : kBarrierPollsDefault;
     GS_TRY(fused_setup(g, d, grid, C, agent_scene, w, L, dirty, fresh));

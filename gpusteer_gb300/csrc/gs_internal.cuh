@@ -76,9 +76,9 @@ inline bool operator==(const Scene& a, const Scene& b) {
 // Buffers of the fused step on cell tables (gs_table.cuh), in one block.
 struct CellTable {
     void* block = nullptr;
-    float4 *tab[2] = {nullptr, nullptr}, *over[2] = {nullptr, nullptr};
-    unsigned* cnt = nullptr;  // three arrays of `cells`, then three overflow counts
-    unsigned cells = 0, row_log2 = 0;
+    float4* tab[2] = {nullptr, nullptr};
+    unsigned* cnt = nullptr;  // three arrays of `cells`, then three of the further rows' tags
+    unsigned cells = 0, row_log2 = 0, ext_log2 = 0;
     unsigned step = 0;        // steps since the table was filled from the reference layout
     bool valid = false;       // the group's state is in A, in agent order, and in the table
     bool frame = false;       // `step - 1`'s table and counts describe frame_cells
@@ -191,6 +191,7 @@ struct gs_group_s {
     unsigned knn_cap, auto_cap, auto_cap_r;
     bool auto_cap_valid;
     gs::Grid auto_cap_grid;
+    unsigned auto_met;     // candidates that all boxes of a small group held then
     bool fused_current;    // true: A holds the state, reference arrays stale
     // cells of the last completed fused step's database while the state is still
     // that step's result (0 once anything changes it): fdb.start then holds the

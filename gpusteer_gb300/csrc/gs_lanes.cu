@@ -520,7 +520,7 @@ static gs_status launch_lanes(const FusedLaunch& L, const StepDev& p, cudaStream
 // k = 24, 4,096 29.3 / 20.6, 16,384 38.3 / 39.0; a crowd with walls (which
 // also drops the exact lists' launch), 10,000 53.5 / 31.0, 20,000 59.9 / 47.9;
 // eight of them, 20,219 agents together, 40.8 / 43.1.
-bool lanes_preferred(unsigned n, bool walls) { return n <= (walls ? 20000u : 16384u); }
+bool lanes_preferred(unsigned n, bool walls) { return n <= (walls ? kLanesMost : 16384u); }
 
 gs_status fused_step_lanes(const FusedLaunch& L, const StepDev& p, cudaStream_t st,
                            PhaseHook* hook) {

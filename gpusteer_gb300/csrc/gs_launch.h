@@ -333,6 +333,7 @@ gs_status fused_step(const FusedLaunch& L, const StepDev& p, cudaStream_t st,
 // it when p.lanes is set.  lanes_preferred: the sizes where it is the faster.
 gs_status fused_step_lanes(const FusedLaunch& L, const StepDev& p, cudaStream_t st,
                            PhaseHook* hook);
+constexpr unsigned kLanesMost = 20000;  // agents, at most
 bool lanes_preferred(unsigned n, bool walls);
 // slot_of: capacity words of scratch (each agent's slot, then the gather).
 // in_order: A's slots are agent indices already.
@@ -364,9 +365,12 @@ size_t adjoint_scratch_bytes(unsigned n, unsigned k);
 void adjoint_scratch_bind(AdjointLaunch& A, void* base, unsigned n, unsigned k);
 gs_status launch_flock_adjoint(const AdjointLaunch& A, const StepDev& p, cudaStream_t st);
 
-// Number of non-zero entries of count[0..C) and the sum of their squares,
-// read back to the host (syncs st); d_tmp: 4 words of device scratch.
+// Number of non-zero entries of count[0..C) and the sum of their squares and,
+// with the cells' grid in `boxes`, the candidates in all agents' boxes of radius
+// 1 (at most 65,535 agents), read back to the host (syncs st); d_tmp: 4 words of
+// device scratch.
 gs_status count_occupied(const unsigned* count, unsigned C, unsigned* d_tmp, unsigned* h_out,
-                         unsigned long long* h_sumsq, cudaStream_t st);
+                         unsigned long long* h_sumsq, const Grid* boxes, unsigned* h_met,
+                         cudaStream_t st);
 
 }  // namespace gs

@@ -1246,40 +1246,53 @@ gs_status fused_to_reference(Fused A, unsigned n, const Scene* scenes, unsigned*
 namespace gs {
 
 // Occupied cells and the sum of squared cell counts (out[0], and the 64-bit
-// word at out + 2).
+// word at out + 2); with `boxes`, the candidates that all agents' boxes of
+// radius 1 hold together (out[1]; g the cells' grid, at most 65,535 agents).
 __global__ void k_count_occupied(const unsigned* __restrict__ count, unsigned C,
-                                 unsigned* __restrict__ out) {
-    unsigned local = 0;
+                                 unsigned* __restrict__ out, Grid g, bool boxes) {
+    unsigned local = 0, met = 0;
     unsigned long long sq = 0;
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < C; i += gridDim.x * blockDim.x) {
         const unsigned c = count[i];
         local += c != 0u;
         sq += (unsigned long long)c * c;
+        if (!boxes || c == 0u) continue;
+        const Box b = cell_box(g, i % g.wc[0], i / (g.wc[0] * g.wc[2]), i / g.wc[0] % g.wc[2], 1);
+        unsigned held = 0;
+        for (unsigned y = b.y0; y <= b.y1; ++y)
+            for (unsigned z = b.z0; z <= b.z1; ++z)
+                for (unsigned x = b.x0; x <= b.x1; ++x) held += count[cell_label(g, x, y, z)];
+        met += c * held;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         local += __shfl_down_sync(0xffffffffu, local, o);
         sq += __shfl_down_sync(0xffffffffu, sq, o);
+        met += __shfl_down_sync(0xffffffffu, met, o);
     }
     if ((threadIdx.x & 31) == 0 && local) {
         atomicAdd(out, local);
+        if (boxes) atomicAdd(out + 1, met);
         atomicAdd(reinterpret_cast<unsigned long long*>(out + 2), sq);
     }
 }
 
 gs_status count_occupied(const unsigned* count, unsigned C, unsigned* d_tmp, unsigned* h_out,
-                         unsigned long long* h_sumsq, cudaStream_t st) {
-    *h_out = 0;
+                         unsigned long long* h_sumsq, const Grid* boxes, unsigned* h_met,
+                         cudaStream_t st) {
+    *h_out = *h_met = 0;
     *h_sumsq = 0;
     if (C == 0) return GS_OK;
     GS_CUDA(cudaMemsetAsync(d_tmp, 0, 4 * sizeof(unsigned), st));
     const unsigned nb = std::min(blocks_for(C, kBlock), 8u * 152u);
-    k_count_occupied<<<nb, kBlock, 0, st>>>(count, C, d_tmp);
+    k_count_occupied<<<nb, kBlock, 0, st>>>(count, C, d_tmp, boxes ? *boxes : Grid{},
+                                            boxes != nullptr);
     GS_LAUNCHED("count_occupied");
     unsigned h[4];
     GS_CUDA(cudaMemcpyAsync(h, d_tmp, sizeof(h), cudaMemcpyDeviceToHost, st));
     GS_CUDA(cudaStreamSynchronize(st));
     *h_out = h[0];
+    *h_met = h[1];
     std::memcpy(h_sumsq, h + 2, sizeof(*h_sumsq));
     return GS_OK;
 }

@@ -7,9 +7,16 @@
 // (position, index) into the next table at its cell's count, and the next
 // step's search reads the counts and rows of its box.  Two tables and three
 // count arrays take turns: a step reads one, fills the next, and clears the
-// third, which the step after fills.  What does not fit a row goes to an
-// overflow list that every search also reads, so nothing depends on the row
-// length but speed.
+// third, which the step after fills.
+//
+// A cell that holds more than a row goes on in further rows, found by hashing
+// (cell, row number): whoever puts an agent there claims the hashed slot's tag,
+// or finds it claimed for the same row, and takes the next slot otherwise.
+// Nothing is allocated and nobody waits, and a search reads what its box holds
+// and no more, however crowded the rest of the world is.  (One overflow list
+// for the whole world, which every agent scanned, took 8 steps of 16,384 boids
+// in clumps of 60 to 3844 us instead of 279, and of a choke point's 10,000
+// agents 1,200 steps on to 407 instead of 272; sorted, 276 and 290.)
 //
 // A group of lanes serves each agent (gs_lanes.cuh): lane by lane it loads the
 // box's counts, lays the candidates' places end to end in shared memory, and
@@ -23,25 +30,57 @@ namespace gs {
 constexpr unsigned kTableBlock = 128;
 constexpr unsigned kTablePlaces = 128;  // candidates laid end to end per lane group
 
+// Row `number` (from 1) of cell c, as its tag.  The tables' sizes keep both in
+// their bits: at most 2^22 places in rows of 16 or more, and the lanes' groups
+// have at most kLanesMost agents.
+constexpr unsigned kTagCellBits = 18;
+static_assert((kLanesMost >> 4) < 1u << (32 - kTagCellBits), "row numbers overflow a tag");
+__device__ __forceinline__ unsigned row_tag(unsigned c, unsigned number) {
+    return number << kTagCellBits | c;
+}
+__device__ __forceinline__ unsigned tag_slot(unsigned tag, unsigned ext_log2) {
+    return (tag * 0x9e3779b1u) >> (32u - ext_log2);
+}
+// There are twice as many slots as further rows of n agents (table_reserve),
+// so both loops end at their row.
+__device__ __forceinline__ unsigned claim_row(const TableStep& T, unsigned c, unsigned number) {
+    const unsigned tag = row_tag(c, number), last = (1u << T.ext_log2) - 1u;
+    unsigned s = tag_slot(tag, T.ext_log2);
+    for (unsigned i = 0; i < last; ++i, s = (s + 1u) & last) {
+        const unsigned old = atomicCAS(T.tag_next + s, 0u, tag);
+        if (old == 0u || old == tag) break;
+    }
+    return s;
+}
+__device__ __forceinline__ unsigned find_row(const TableStep& T, unsigned c, unsigned number) {
+    const unsigned tag = row_tag(c, number), last = (1u << T.ext_log2) - 1u;
+    unsigned s = tag_slot(tag, T.ext_log2);
+    for (unsigned i = 0; i < last && T.tag[s] != tag; ++i) s = (s + 1u) & last;
+    return s;
+}
+// Entry t of cell c.
+__device__ __forceinline__ float4 table_entry(const TableStep& T, unsigned c, unsigned t) {
+    const unsigned number = t >> T.row_log2;
+    const unsigned row = number == 0 ? c : T.cells + find_row(T, c, number);
+    return T.tab[(row << T.row_log2) + (t & ((1u << T.row_log2) - 1u))];
+}
+
 // Puts the agent in the next step's table.
 __device__ __forceinline__ void table_put(const TableStep& T, V3 pos, int wrap_mode, unsigned id) {
     const V3 p = wrap_world(pos, T.sc.grid.ws, wrap_mode);
     const unsigned c = cell_of(T.sc.grid, p);
     const unsigned at = atomicAdd(T.cnt_next + c, 1u);
     const float4 e = make_float4(p.x, p.y, p.z, __uint_as_float(id));
-    if (at < (1u << T.row_log2)) {
-        T.tab_next[(size_t(c) << T.row_log2) + at] = e;
-    } else {
-        const unsigned o = atomicAdd(T.over_n_next, 1u);
-        if (o < T.n) T.over_next[o] = e;
-    }
+    const unsigned number = at >> T.row_log2;
+    const unsigned row = number == 0 ? c : T.cells + claim_row(T, c, number);
+    T.tab_next[(row << T.row_log2) + (at & ((1u << T.row_log2) - 1u))] = e;
 }
 
-// Clears the counts that the step after this one fills.
+// Clears the counts and tags that the step after this one fills.
 __device__ __forceinline__ void table_clear(const TableStep& T) {
     const unsigned t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
     for (unsigned i = t; i < T.cells; i += nt) T.cnt_clear[i] = 0u;
-    if (t == 0) *T.over_n_clear = 0u;
+    for (unsigned i = t; i < 1u << T.ext_log2; i += nt) T.tag_clear[i] = 0u;
 }
 
 // The k nearest of the 27 (FLAT: 9) cells of box b, over the group's lanes.
@@ -58,20 +97,19 @@ __device__ __forceinline__ LaneList<G, 1> table_knn(const TableStep& T, unsigned
         const unsigned long long key = knn_key(distance(p, v3(v)), id);
         list.take(ok && id != self_id && key < KEY_EMPTY ? key : KEY_EMPTY, k, lane);
     };
-    unsigned row[Q], len[Q];
+    unsigned cell[Q], len[Q];
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const unsigned i = lane + unsigned(q * G);
         const unsigned x = b.x0 + i % 3u, z = b.z0 + (i / 3u) % 3u, y = b.y0 + i / 9u;
-        row[q] = len[q] = 0;
+        cell[q] = len[q] = 0;
         if (i < unsigned(CELLS) && x <= b.x1 && y <= b.y1 && z <= b.z1) {
-            const unsigned c = cell_label(g, x, y, z);
-            row[q] = c << T.row_log2;
-            len[q] = min(T.cnt[c], 1u << T.row_log2);
+            cell[q] = cell_label(g, x, y, z);
+            len[q] = T.cnt[cell[q]];
         }
     }
-    const unsigned over = *T.over_n;
     unsigned total = 0, first[Q];
+    bool rows = true;  // this lane's cells are within their rows
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         unsigned sum = len[q];
@@ -82,12 +120,14 @@ __device__ __forceinline__ LaneList<G, 1> table_knn(const TableStep& T, unsigned
         }
         first[q] = total + sum - len[q];
         total += __shfl_sync(kAllLanes, sum, G - 1, G);
+        rows = rows && len[q] <= 1u << T.row_log2;
     }
     const unsigned most = __reduce_max_sync(kAllLanes, total);
-    if (most <= kTablePlaces) {
+    if (most <= kTablePlaces && __all_sync(kAllLanes, rows)) {
 #pragma unroll
         for (int q = 0; q < Q; ++q)
-            for (unsigned t = 0; t < len[q]; ++t) places[first[q] + t] = row[q] + t;
+            for (unsigned t = 0; t < len[q]; ++t)
+                places[first[q] + t] = (cell[q] << T.row_log2) + t;
         __syncwarp();
         // the next candidate is on its way while this one is taken
         auto load = [&](unsigned j) {
@@ -99,24 +139,36 @@ __device__ __forceinline__ LaneList<G, 1> table_knn(const TableStep& T, unsigned
             take(v, j < total);
             v = next;
         }
-    } else {  // crowded boxes: cell by cell
+    } else {  // crowded boxes: the cells end to end, a lane's cell found as it goes
+        unsigned* cells = places;
+        unsigned* pre = places + CELLS;
 #pragma unroll
-        for (int q = 0; q < Q; ++q)
-            for (int l = 0; l < G; ++l) {
-                const unsigned r = __shfl_sync(kAllLanes, row[q], l, G);
-                const unsigned n = __shfl_sync(kAllLanes, len[q], l, G);
-                const unsigned rounds = __reduce_max_sync(kAllLanes, n);
-                for (unsigned j = lane; j < rounds + lane; j += G)
-                    take(j < n ? T.tab[r + j] : make_float4(0.f, 0.f, 0.f, 0.f), j < n);
+        for (int q = 0; q < Q; ++q) {
+            const unsigned i = lane + unsigned(q * G);
+            if (i < unsigned(CELLS)) {
+                cells[i] = cell[q];
+                pre[i] = first[q];
             }
-    }
-    const unsigned n_over = min(over, T.n);
-    for (unsigned j = lane; j < n_over + lane; j += G) {
-        const float4 v = j < n_over ? T.over[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-        unsigned x, y, z;
-        cell_coords(g, v3(v), x, y, z);
-        take(v, j < n_over && x >= b.x0 && x <= b.x1 && y >= b.y0 && y <= b.y1 && z >= b.z0 &&
-                    z <= b.z1);
+        }
+        if (lane == 0) pre[CELLS] = total;
+        __syncwarp();
+        unsigned at = UINT_MAX, begin = 0, end = 0, c = 0;
+        auto load = [&](unsigned j) {
+            if (j >= total) return make_float4(0.f, 0.f, 0.f, 0.f);
+            if (j >= end) {
+                do end = pre[++at + 1];
+                while (j >= end);
+                begin = pre[at];
+                c = cells[at];
+            }
+            return table_entry(T, c, j - begin);
+        };
+        float4 v = load(lane);
+        for (unsigned j = lane; j < most + lane; j += G) {
+            const float4 next = load(j + G);
+            take(v, j < total);
+            v = next;
+        }
     }
     return list;
 }
@@ -308,24 +360,20 @@ gs_status table_step(const TableStep& T, const StepDev& p, cudaStream_t st) {
 }
 
 // ---- frame diagnostics (ProcessData.cu:132-237) ----------------------------------------------------
-// The counts are the density.  A cell's agents, its row and the overflow's of
-// that cell, are added in ascending index, picked by increasing index.
+// The counts are the density.  A cell's agents are added in ascending index,
+// picked by increasing index.
 __global__ void k_table_avg_velocity(const __grid_constant__ TableStep T, float3* __restrict__ out) {
     const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= T.cells) return;
-    const unsigned n = T.cnt[c], in_row = min(n, 1u << T.row_log2);
-    const unsigned over = n > in_row ? min(*T.over_n, T.n) : 0u;
+    const unsigned n = T.cnt[c];
     V3 sum = v3(0.f, 0.f, 0.f);
     unsigned last = 0;
     for (unsigned t = 0; t < n; ++t) {
         unsigned next = UINT_MAX;
-        auto see = [&](float4 v) {
-            const unsigned id = __float_as_uint(v.w);
+        for (unsigned s = 0; s < n; ++s) {
+            const unsigned id = __float_as_uint(table_entry(T, c, s).w);
             if ((t == 0 || id > last) && id < next) next = id;
-        };
-        for (unsigned s = 0; s < in_row; ++s) see(T.tab[(size_t(c) << T.row_log2) + s]);
-        for (unsigned s = 0; s < over; ++s)
-            if (cell_of(T.sc.grid, v3(T.over[s])) == c) see(T.over[s]);
+        }
         if (next == UINT_MAX) break;
         last = next;
         const float4 h = T.f1_next[next];

@@ -5,26 +5,25 @@
 
 namespace gs {
 
-// One step's buffers.  tab / cnt / over: this step's table, counts and
-// overflow list; *_next the ones it fills, *_clear the counts it clears.
+// One step's buffers.  tab / cnt: this step's rows, one a cell and then the
+// further ones, and the cells' counts; tag: what each further row is; *_next
+// the ones it fills, *_clear the counts and tags it clears.
 struct TableStep {
     const float4 *f0, *f1;
     float4 *f0_next, *f1_next, *f2, *f3, *f4;
     const float4* f5;
     const float4* tab;
     const unsigned* cnt;
-    const float4* over;
-    const unsigned* over_n;
+    const unsigned* tag;
     float4* tab_next;
     unsigned* cnt_next;
-    float4* over_next;
-    unsigned* over_n_next;
-    unsigned *cnt_clear, *over_n_clear;
+    unsigned* tag_next;
+    unsigned *cnt_clear, *tag_clear;
     WallRefs walls;
     float4 *w0, *w1, *w2;
     unsigned* near;    // [n * k] neighbour lists, agent by agent (walls)
     float* near_dist;
-    unsigned n, cells, row_log2;
+    unsigned n, cells, row_log2, ext_log2;
     Scene sc;
 };
 
