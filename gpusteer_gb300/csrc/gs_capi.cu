@@ -1818,7 +1818,7 @@ constexpr unsigned kTableMostCandidates = 2500000;
 static bool table_wanted(gs_group g, const StepDev& d, const Grid& grid, unsigned C,
                          const unsigned* agent_scene) {
     return agent_scene == nullptr && d.r == 1 && g->knn_cap == 0 && !g->profiling &&
-           !g->persistent && lanes_preferred(g->n, (d.need & NEED_WALLS) != 0) &&
+           !g->persistent && g->table.refused != C && lanes_preferred(g->n, (d.need & NEED_WALLS) != 0) &&
            (size_t(C) << table_row_log2(d, C)) <= (size_t(1) << 22) &&
            !(measured(g, grid, 1) && g->auto_met > kTableMostCandidates);
 }
@@ -1849,6 +1849,7 @@ static gs_status table_reserve(gs_group g, unsigned C, unsigned row_log2) {
     t.cells = C;
     t.row_log2 = row_log2;
     t.ext_log2 = ext_log2;
+    t.refused = 0;
     return GS_OK;
 }
 
@@ -1888,8 +1889,8 @@ static TableStep table_buffers(gs_group g, unsigned step) {
     return T;
 }
 
-// taken: false where the cells just counted are too full for the table; nothing
-// has then been done to the group's state.
+// taken: false where the device has no memory for the table or the cells just
+// counted are too full for it; nothing has then been done to the group's state.
 static gs_status table_run(gs_group g, StepDev d, const Grid& grid, unsigned C,
                            const WallsDev& w, unsigned steps, bool& taken) {
     cudaStream_t st = g->stream;
@@ -1901,7 +1902,13 @@ static gs_status table_run(gs_group g, StepDev d, const Grid& grid, unsigned C,
         GS_TRY(ensure_reference(g));
         dirty = g->accum_dirty;
         t.valid = t.frame = false;
-        GS_TRY(table_reserve(g, C, table_row_log2(d, C)));
+        const gs_status s = table_reserve(g, C, table_row_log2(d, C));
+        if (s == GS_ERR_OOM) {  // not asked for again before another grid's was had
+            t.refused = C;
+            taken = false;
+            return GS_OK;
+        }
+        GS_TRY(s);
         GS_CUDA(cudaMemsetAsync(t.cnt, 0, 4 * table_words(C, t.ext_log2), st));
         // step "-1" fills the table that step 0 reads
         t.step = 0;

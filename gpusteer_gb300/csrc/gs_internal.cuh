@@ -79,6 +79,7 @@ struct CellTable {
     float4* tab[2] = {nullptr, nullptr};
     unsigned* cnt = nullptr;  // three arrays of `cells`, then three of the further rows' tags
     unsigned cells = 0, row_log2 = 0, ext_log2 = 0;
+    unsigned refused = 0;     // cells of the last grid whose table could not be allocated
     unsigned step = 0;        // steps since the table was filled from the reference layout
     bool valid = false;       // the group's state is in A, in agent order, and in the table
     bool frame = false;       // `step - 1`'s table and counts describe frame_cells
