@@ -2,17 +2,24 @@
 // nearest of all candidates, found in the cells that can hold them.
 //
 // One launch sorts the candidates into an automatic grid of about k / 8 a cell
-// (gs_db.cu: extent, grid and counting sort in one cluster, nothing read back
-// by the host); one gives each query a group of G lanes.  A query first takes
-// the 27 cells about its own (then 5^3, 9^3, ... while its list is not full),
-// which bounds its k-th distance D.  Every candidate at a distance of at most
-// D lies within D of the query on each axis, so in the cells from that of
-// q - D to that of q + D: the rest of that box is scanned once more, and the
+// (gs_db.cu: a sample, the grid and the counting sort in one cluster, nothing
+// read back by the host); one gives each query a group of G lanes.  A query
+// first takes the 27 cells about its own (then 5^3, 9^3, ... while its list is
+// not full), which bounds its k-th distance D.  Every candidate at a distance of
+// at most D lies within D of the query on each axis, so in the cells from that
+// of q - D to that of q + D: the rest of that box is scanned once more, and the
 // list is that over all candidates.  The bound is exact: a distance's rounded
-// square is no less than its largest component's, cell_coord is monotone, and
-// D is widened by 1e-5 of itself before q - D is rounded down and q + D up.
+// square is no less than its largest component's, a cell's number grows with
+// the coordinate (auto_coords), and D is widened by 1e-5 of itself before q - D
+// is rounded down and q + D up.  A query or candidate that is not finite has no
+// distance below the largest float to any other, so it is in no list and has
+// none.
+//
 // Instead of every pair (or the 2 % of the bucketed chunks this replaced) a
-// query meets about 90 candidates at k = 16.
+// query meets about 90 candidates at k = 16.  Crowded cells come down to their
+// candidates' squared distances against a rounded-up bound of the k-th distance,
+// as k_knn_brute3's filter has it: 262,144 agents in two clusters, 131,000
+// candidates a query, 41 ms (70 with every candidate's key made).
 #include <cmath>
 
 #include "gs_db.cuh"
@@ -46,6 +53,7 @@ __device__ __forceinline__ unsigned brute_region(LaneList<G, L>& list, const Bru
     const unsigned ns = on ? ((out.y1 - out.y0 + 1) * nz) << sides : 0u;
     const unsigned most = __reduce_max_sync(kAllLanes, ns);
     unsigned met = 0;
+    float bound = prefilter_bound(list.kth(k));
     for (unsigned base = 0; base < most; base += kBruteSegs) {
         // up to kBruteSegs runs of cells, laid end to end: a row each, or two
         // with an inner box, left and right of it where the row crosses it
@@ -91,15 +99,16 @@ __device__ __forceinline__ unsigned brute_region(LaneList<G, L>& list, const Bru
         float4 v = load(lane);
         for (unsigned j = lane; j < rounds + lane; j += G) {
             const float4 next = load(j + G);
-            unsigned long long c = KEY_EMPTY;
-            if (j < total) {
-                const unsigned id = __float_as_uint(v.w);
-                const unsigned long long key = knn_key(distance(q.p, v3(v)), id);
-                if (id != q.self_id && key < KEY_EMPTY) c = key;
-                ++met;
-            }
+            const V3 o = sub(q.p, v3(v));
+            const float dsq = dot(o, o);
+            const unsigned id = __float_as_uint(v.w);
+            const bool near = j < total && dsq <= bound && id != q.self_id;
+            met += j < total;
             v = next;
-            list.take(c, k, lane);
+            if (!__any_sync(kAllLanes, near)) continue;
+            const unsigned long long key = knn_key(sqrtf(dsq), id);
+            list.take(near && key < KEY_EMPTY ? key : KEY_EMPTY, k, lane);
+            bound = prefilter_bound(list.kth(k));
         }
         __syncwarp();
     }
@@ -111,7 +120,7 @@ __device__ __forceinline__ unsigned brute_region(LaneList<G, L>& list, const Bru
 template <int G, int L>
 __global__ void __launch_bounds__(kBruteBlock) k_brute_cells(
     const float4* q_pos, bool by_slot, unsigned nA, const float4* pos_id,
-    const unsigned* start, const Grid* grid, bool self, unsigned k,
+    const unsigned* start, const AutoGrid* grid, bool self, unsigned k,
     unsigned long long* evaluated, unsigned* idx,
     float* dist) {
     after_previous();
@@ -124,14 +133,16 @@ __global__ void __launch_bounds__(kBruteBlock) k_brute_cells(
     const float4 v = q_pos[act ? s : nA - 1];
     const unsigned a = by_slot ? __float_as_uint(v.w) : s;
     const BruteQuery q{v3(v), self ? a : UINT_MAX};
-    const Grid g = *grid;
+    const AutoGrid ag = *grid;
+    const Grid& g = ag.grid;
+    const bool live = act && is_finite(q.p);
     LaneList<G, L> list;
 #pragma unroll
     for (int h = 0; h < L; ++h) list.e[h] = KEY_EMPTY;
     unsigned ix, iy, iz;
-    cell_coords(g, q.p, ix, iy, iz);
+    auto_coords(ag, q.p, ix, iy, iz);
     Box out = cell_box(g, ix, iy, iz, 1), done = out;  // to take now; taken so far
-    bool any = false, on = act, last = false;
+    bool any = false, on = live, last = false;
     unsigned met = 0;
     for (unsigned r = 2;; r = 2 * r) {
         met += brute_region(list, q, k, lane, on, out, any, done, g, start, pos_id, segs);
@@ -142,7 +153,7 @@ __global__ void __launch_bounds__(kBruteBlock) k_brute_cells(
         const bool whole = done.x0 == 0 && done.y0 == 0 && done.z0 == 0 &&
                            done.x1 == g.wc[0] - 1 && done.y1 == g.wc[1] - 1 &&
                            done.z1 == g.wc[2] - 1;
-        on = act && !whole && kth >= KEY_EMPTY;
+        on = live && !whole && kth >= KEY_EMPTY;
         if (__any_sync(kAllLanes, on)) {
             if (on) out = cell_box(g, ix, iy, iz, r);
             continue;
@@ -150,13 +161,13 @@ __global__ void __launch_bounds__(kBruteBlock) k_brute_cells(
         // the rest of the box that can hold a candidate at the k-th distance
         const float reach = __fadd_ru(__fmul_ru(key_dist(kth), 1.00001f), 1e-18f);
         unsigned lx, ly, lz, ux, uy, uz;
-        cell_coords(g, v3(__fsub_rd(q.p.x, reach), __fsub_rd(q.p.y, reach),
-                          __fsub_rd(q.p.z, reach)), lx, ly, lz);
-        cell_coords(g, v3(__fadd_ru(q.p.x, reach), __fadd_ru(q.p.y, reach),
-                          __fadd_ru(q.p.z, reach)), ux, uy, uz);
+        auto_coords(ag, v3(__fsub_rd(q.p.x, reach), __fsub_rd(q.p.y, reach),
+                           __fsub_rd(q.p.z, reach)), lx, ly, lz);
+        auto_coords(ag, v3(__fadd_ru(q.p.x, reach), __fadd_ru(q.p.y, reach),
+                           __fadd_ru(q.p.z, reach)), ux, uy, uz);
         out = Box{min(lx, done.x0), max(ux, done.x1), min(ly, done.y0),
                   max(uy, done.y1), min(lz, done.z0), max(uz, done.z1)};
-        on = act;
+        on = live;
         last = true;
     }
     if (act) {
@@ -206,7 +217,7 @@ gs_status launch_knn_brute_cells(const float4* posA, unsigned nA, const float4* 
     for (int a = 0; a < 3; ++a) {
         unsigned c = unsigned(std::floor(std::pow(most, 1.0 / (a + 1)) + 1e-9));
         while (c > 1 && std::pow(double(c), a + 1) > most) --c;
-        J.job[0].auto_axis[a] = c > 1024 ? 1024u : c ? c : 1u;
+        J.job[0].auto_axis[a] = c ? c : 1u;
     }
     J.job[0].grid_out = w.grid;
     J.job[0].zero = w.evaluated;

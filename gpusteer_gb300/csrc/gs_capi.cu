@@ -1207,6 +1207,7 @@ gs_status gs_find_knn_walls(gs_group g, gs_knn out, gs_bins bins, gs_walls walls
 // 764 / 193 (from 4,096 on the former skipped chunks of bucketed candidates
 // beyond a seeded bound).
 constexpr unsigned kBruteCellsMin = 128;
+constexpr unsigned kBrutePairs = 10;  // word of bf_tmp where the pairs' count lies
 
 gs_status gs_knn_bruteforce(gs_group g, gs_knn out, gs_group other) {
     if (!g || !out || !other) return fail(GS_ERR_INVALID_ARG, "null argument");
@@ -1220,11 +1221,11 @@ gs_status gs_knn_bruteforce(gs_group g, gs_knn out, gs_group other) {
     g->bf_counted = false;
     g->bf_pairs = (unsigned long long)g->n * other->n;
     if (g->n >= kBruteCellsMin && other->n > out->k) {
-        static_assert(sizeof(Grid) == 24, "bf_tmp layout");
-        if (!g->bf_tmp) GS_TRY(dalloc(&g->bf_tmp, 8));
+        static_assert(sizeof(AutoGrid) <= 4 * kBrutePairs, "bf_tmp layout");
+        if (!g->bf_tmp) GS_TRY(dalloc(&g->bf_tmp, kBrutePairs + 2));
         // sized for the largest other group met so far
         Database& B = g->bf_db;
-        const unsigned C = brute_cells(other->capacity, out->k);
+        const unsigned C = brute_cells(other->capacity, out->k) + 1;
         if (B.cells < C || B.agent_cap < other->capacity) {
             const unsigned cells = std::max(C, B.cells), cap = std::max(other->capacity, B.agent_cap);
             GS_CUDA(cudaStreamSynchronize(st));
@@ -1232,8 +1233,8 @@ gs_status gs_knn_bruteforce(gs_group g, gs_knn out, gs_group other) {
             GS_TRY(db_reserve(B, cap, cells));
             B.agent_cap = cap;
         }
-        const BruteWork w{reinterpret_cast<Grid*>(g->bf_tmp),
-                          reinterpret_cast<unsigned long long*>(g->bf_tmp + 6)};
+        const BruteWork w{reinterpret_cast<AutoGrid*>(g->bf_tmp),
+                          reinterpret_cast<unsigned long long*>(g->bf_tmp + kBrutePairs)};
         GS_TRY(launch_knn_brute_cells(g->position, g->n, other->position, other->n, other == g,
                                       out->k, B, w, out->idx, out->dist, st));
         g->bf_counted = true;
@@ -1248,7 +1249,7 @@ gs_status gs_knn_bruteforce_pairs(gs_group g, unsigned long long* pairs) {
     if (!g || !pairs) return fail(GS_ERR_INVALID_ARG, "null argument");
     *pairs = g->bf_pairs;
     if (!g->bf_counted) return GS_OK;
-    GS_CUDA(cudaMemcpyAsync(pairs, g->bf_tmp + 6, sizeof(unsigned long long),
+    GS_CUDA(cudaMemcpyAsync(pairs, g->bf_tmp + kBrutePairs, sizeof(unsigned long long),
                             cudaMemcpyDeviceToHost, g->stream));
     GS_CUDA(cudaStreamSynchronize(g->stream));
     return GS_OK;

@@ -55,27 +55,101 @@ __device__ __forceinline__ unsigned block_scan(unsigned v, unsigned* warp_sums, 
     return before + x - v;
 }
 
-// A grid centred on the origin that covers every position (largest
-// |coordinate| per axis, as float bits): about two agents a cell over the
-// axes that have extent, one cell when a position is not finite.
-__device__ __forceinline__ Grid automatic_grid(const unsigned ext[3], const unsigned axis_cells[3]) {
-    Grid g;
-    float w[3], most = 0.f;
-    bool finite = true;
+// The grid of a sample of kSample positions spread evenly over the agents, by
+// one block; every block of a cluster computes the same.  Per axis, a centre and
+// a reach start from all of the sample; each round takes the mean and four times
+// the mean distance from the centre of what lies within the reach, so that a few
+// positions far off, at whatever distance, drop out and a box or a cloud keeps
+// everything.  The sample's extent within the last reach, a little widened, is
+// the axis' (a grid over the extent of all positions, about the origin, lost
+// most of its cells to one far position, to one that is not finite, or to a
+// crowd far from the origin: 65,536 agents, k = 16, 9.2 ms for each of these
+// and 0.1 ms for a cube about the origin).
+constexpr unsigned kSample = 256;
+constexpr int kSampleRounds = 4;
+struct Sample {
+    float x[3][kSample];                   // NaN: not a finite position
+    float low[3], high[3], count[3];
+};
+template <class Op>
+__device__ __forceinline__ float warp_all(float v, Op op) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ AutoGrid automatic_grid(const float4* pos, unsigned n,
+                                                   const unsigned axis_cells[3], Sample& sh) {
+    const unsigned t = threadIdx.x, lane = t & 31u, warp = t >> 5, take = min(n, kSample);
+    constexpr float kScale = 0x1p-12f;  // sums of the largest floats stay finite
+    if (t < kSample) {
+        const V3 p = v3(pos[t < take ? size_t(t) * n / take : 0]);
+        const bool ok = t < take && is_finite(p);
+        const float none = __int_as_float(0x7fffffff);
+        sh.x[0][t] = ok ? p.x * kScale : none;
+        sh.x[1][t] = ok ? p.y * kScale : none;
+        sh.x[2][t] = ok ? p.z * kScale : none;
+    }
+    __syncthreads();
+    if (warp < 3) {  // a warp an axis
+        const auto sum = [](float u, float v) { return u + v; };
+        const auto least = [](float u, float v) { return fminf(u, v); };
+        const auto most = [](float u, float v) { return fmaxf(u, v); };
+        float x[kSample / 32];
+#pragma unroll
+        for (unsigned i = 0; i < kSample / 32; ++i) x[i] = sh.x[warp][32 * i + lane];
+        float centre = 0.f, reach = FLT_MAX;
+        for (int round = 0; round < kSampleRounds; ++round) {
+            float m = 0.f, u = 0.f, v = 0.f;
+#pragma unroll
+            for (unsigned i = 0; i < kSample / 32; ++i) {
+                const float d = x[i] - centre;
+                const bool in = fabsf(d) <= reach;
+                m += in ? 1.f : 0.f;
+                u += in ? d : 0.f;
+                v += in ? fabsf(d) : 0.f;
+            }
+            m = warp_all(m, sum);
+            u = warp_all(u, sum);
+            v = warp_all(v, sum);
+            if (m > 0.f) {
+                centre += u / m;
+                reach = 4.f * (v / m);
+            }
+        }
+        float m = 0.f, low = FLT_MAX, high = -FLT_MAX;
+#pragma unroll
+        for (unsigned i = 0; i < kSample / 32; ++i) {
+            const bool in = fabsf(x[i] - centre) <= reach;
+            m += in ? 1.f : 0.f;
+            low = in ? fminf(low, x[i]) : low;
+            high = in ? fmaxf(high, x[i]) : high;
+        }
+        m = warp_all(m, sum);
+        low = warp_all(low, least);
+        high = warp_all(high, most);
+        if (lane == 0) {
+            sh.low[warp] = m > 0.f ? low : 0.f;
+            sh.high[warp] = m > 0.f ? high : 0.f;
+            sh.count[warp] = m;
+        }
+    }
+    __syncthreads();
+    AutoGrid g;
+    float width[3], most = 0.f;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        finite = finite && ext[a] < 0x7e800000u;  // far enough below overflow to be doubled
-        w[a] = 2.002f * __uint_as_float(ext[a]) + 1e-6f;
-        most = fmaxf(most, w[a]);
+        width[a] = (sh.high[a] - sh.low[a]) * (1.f + 2.f / fmaxf(sh.count[a], 2.f));
+        most = fmaxf(most, width[a]);
     }
     int dims = 0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) dims += w[a] > 1e-3f * most;
+    for (int a = 0; a < 3; ++a) dims += width[a] > 1e-3f * most;
     const unsigned cells = dims == 1 ? axis_cells[0] : dims == 2 ? axis_cells[1] : axis_cells[2];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        g.wc[a] = finite && w[a] > 1e-3f * most ? cells : 1u;
-        g.ws[a] = finite ? w[a] : 1.f;
+        g.grid.wc[a] = width[a] > 1e-3f * most ? cells : 1u;
+        g.grid.ws[a] = fminf(fmaxf(width[a], 1e-30f), FLT_MAX * kScale * 0.25f) * (1.f / kScale);
+        g.mid[a] = (0.5f * sh.low[a] + 0.5f * sh.high[a]) * (1.f / kScale);
     }
     return g;
 }
@@ -83,52 +157,35 @@ __device__ __forceinline__ Grid automatic_grid(const unsigned ext[3], const unsi
 __global__ void __launch_bounds__(kDbThreads) k_db_cluster(const __grid_constant__ DbJobs J) {
     after_previous();
     __shared__ unsigned ws[32];
-    __shared__ unsigned totals[kDbCluster], extents[kDbCluster][3];
+    __shared__ unsigned totals[kDbCluster];
+    __shared__ Sample sample;
     cg::cluster_group cluster = cg::this_cluster();
     const unsigned R = cluster.num_blocks(), rank = cluster.block_rank(), t = threadIdx.x;
     const DbJob& j = J.job[blockIdx.x / R];
     const unsigned first = rank * kDbThreads + t, step = R * kDbThreads, n = j.n;
-    Grid grid = j.grid;
+    const bool automatic = j.auto_axis[0] != 0;
+    AutoGrid a{j.grid, {0.f, 0.f, 0.f}};
     if (first == 0 && j.zero) *j.zero = 0ull;
-    if (j.auto_axis[0]) {
-        // the peers' shared memory is written below: every block of the
-        // cluster has to run by then, which this barrier waits for, under the
-        // pass over the positions
-        cluster.barrier_arrive();
-        unsigned m[3] = {0u, 0u, 0u};
-        for (unsigned i = first; i < n; i += step) {
-            const float4 p = j.pos[i];
-            m[0] = max(m[0], __float_as_uint(fabsf(p.x)));
-            m[1] = max(m[1], __float_as_uint(fabsf(p.y)));
-            m[2] = max(m[2], __float_as_uint(fabsf(p.z)));
-        }
-        cluster.barrier_wait();
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            const unsigned w = __reduce_max_sync(0xffffffffu, m[a]);
-            if ((t & 31u) == 0) ws[t >> 5] = w;
-            __syncthreads();
-            const unsigned b = __reduce_max_sync(0xffffffffu, ws[t & 31u]);
-            if (t < R) cluster.map_shared_rank(&extents[0][0], t)[rank * 3 + a] = b;
-            __syncthreads();
-        }
-        cluster.sync();
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            m[a] = 0;
-            for (unsigned q = 0; q < R; ++q) m[a] = max(m[a], extents[q][a]);
-        }
-        grid = automatic_grid(m, j.auto_axis);
-        if (first == 0) *j.grid_out = grid;
+    if (automatic) {
+        a = automatic_grid(j.pos, n, j.auto_axis, sample);
+        if (first == 0) *j.grid_out = a;
     }
-    const unsigned C = grid.wc[0] * grid.wc[1] * grid.wc[2];
+    const unsigned cells = a.grid.wc[0] * a.grid.wc[1] * a.grid.wc[2];
+    const unsigned C = cells + (automatic ? 1u : 0u);
     for (unsigned i = first; i < n; i += step) {
         V3 p = v3(j.pos[i]);
         if (j.wrap_mode >= 0) {
             p = wrap_world(p, j.wrap_ws, j.wrap_mode);
             j.pos[i] = f4(p, 0.f);
         }
-        const unsigned c = cell_of(grid, p);
+        unsigned c;
+        if (automatic) {
+            unsigned x, y, z;
+            auto_coords(a, p, x, y, z);
+            c = is_finite(p) ? cell_label(a.grid, x, y, z) : cells;
+        } else {
+            c = cell_of(a.grid, p);
+        }
         j.cell[i] = c;
         j.rank[i] = atomicAdd(j.count + c, 1u);
         if (j.applied) j.applied[i] = 0u;

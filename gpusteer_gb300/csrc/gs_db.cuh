@@ -1,9 +1,26 @@
 // Counting-sort databases built by one thread-block cluster each.
 #pragma once
 
+#include <cfloat>
+
 #include "gs_internal.cuh"
 
 namespace gs {
+
+// An automatic grid: even cells about `mid` over where most positions lie; what
+// lies outside is in the cells at its edges, as everywhere.
+struct AutoGrid {
+    Grid grid;
+    float mid[3];
+};
+// Grows with every coordinate over all floats: so do the difference, rounded,
+// and cell_coord.
+GS_HD void auto_coords(const AutoGrid& a, V3 p, unsigned& ix, unsigned& iy, unsigned& iz) {
+    cell_coords(a.grid, sub(p, v3(a.mid[0], a.mid[1], a.mid[2])), ix, iy, iz);
+}
+GS_HD bool is_finite(V3 p) {
+    return fabsf(p.x) <= FLT_MAX && fabsf(p.y) <= FLT_MAX && fabsf(p.z) <= FLT_MAX;
+}
 
 // One database to build: count cells (wrapping the positions first when
 // wrap_mode >= 0, and clearing `applied` when given), scan, scatter.
@@ -12,7 +29,8 @@ struct DbJob {
     unsigned n;
     Grid grid;            // or chosen by the kernel: auto_axis[0] != 0
     unsigned auto_axis[3];  // cells per axis when 1, 2 or 3 axes have extent
-    Grid* grid_out;       // the chosen grid
+    AutoGrid* grid_out;   // the chosen grid; positions that are not finite are
+                          // in a cell past its last
     unsigned long long* zero;  // a word to clear (may be null)
     int wrap_mode;        // -1: positions stay as they are
     float wrap_ws[3];

@@ -171,7 +171,7 @@ struct gs_group_s {
     gs::Database fdb;      // counts / starts of the fused step
     gs::CellTable table;   // the small groups' step without a sort
     // brute-force KNN over cells: the other group's database on an automatic
-    // grid; scratch (words 0-5: that grid, words 6-7: the pairs met)
+    // grid; scratch (that grid, then the pairs met)
     gs::Database bf_db;
     unsigned* bf_tmp;
     bool bf_counted;       // the last call counted its pairs in bf_tmp

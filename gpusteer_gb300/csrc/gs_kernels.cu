@@ -247,15 +247,6 @@ gs_status db_build(Database& db, const float4* pos, unsigned n, const Grid& grid
 }
 
 // ---- brute-force KNN (KNNBruteForceCudaKernel.cu:207-283) ---------------------------
-// A candidate needs its square root only when its squared distance is within
-// a rounded-up bound of the current k-th distance squared: a larger squared
-// distance has a correctly rounded square root strictly above the k-th
-// distance, so it can be skipped without changing the result.
-__device__ __forceinline__ float prefilter_bound(unsigned long long thr) {
-    const float td = key_dist(thr);
-    return __fmul_ru(__fmul_ru(td, td), 1.000004f);
-}
-
 // ---- brute force, FP32-pipe form (k <= 64) ----------------------------------------------
 // One warp serves kBruteQW queries and keeps each query's exact (distance,
 // index) top-k list spread over its lanes: lane r holds entry r (and entry

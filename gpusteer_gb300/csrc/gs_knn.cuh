@@ -73,6 +73,15 @@ struct KList {
 // one contiguous run of sorted slots per (y, z) row of cells, because labels
 // are x-fastest.  The set equals the reference's de-duplicated neighbour-cell
 // table (KNNBinningV2Kernel.cu:102-248).
+// A candidate needs its square root only when its squared distance is within
+// a rounded-up bound of the current k-th distance squared: a larger squared
+// distance has a correctly rounded square root strictly above the k-th
+// distance, so it can be skipped without changing the result.
+__device__ __forceinline__ float prefilter_bound(unsigned long long thr) {
+    const float td = key_dist(thr);
+    return __fmul_ru(__fmul_ru(td, td), 1.000004f);
+}
+
 struct Box {
     unsigned x0, x1, y0, y1, z0, z1;
 };

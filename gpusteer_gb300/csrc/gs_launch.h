@@ -100,10 +100,11 @@ gs_status launch_knn_binned_pairs(KnnPairs& P, cudaStream_t st);
 gs_status launch_knn_brute(const float4* posA, unsigned nA, const float4* posB, unsigned nB,
                            bool self, unsigned k, unsigned* idx, float* dist, cudaStream_t st);
 // The same lists from the cells that can hold them (gs_brute.cu): B is a
-// database reserved for nB agents and brute_cells(nB, k) cells, `evaluated`
+// database reserved for nB agents and brute_cells(nB, k) + 1 cells, `evaluated`
 // receives the (query, candidate) pairs met.
+struct AutoGrid;
 struct BruteWork {
-    Grid* grid;
+    AutoGrid* grid;
     unsigned long long* evaluated;
 };
 unsigned brute_cells(unsigned n, unsigned k);

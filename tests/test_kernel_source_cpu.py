@@ -62,7 +62,7 @@ def test_clusters_have_started_before_remote_shared_memory_is_touched():
                 passed = "".join(reversed(kept))
                 assert re.search(r"\bcluster\.(sync|barrier_wait)\s*\(", passed), \
                     f"{path.name} {name}: {body[m.start() - 20:m.end() + 40]!r}"
-    assert met >= 2
+    assert met >= 1
 
 
 LAUNCHED_EARLY = sorted({m for p in SOURCES
