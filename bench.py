@@ -95,6 +95,12 @@ def single_config(name: str, p, n: int, world: int) -> dict:
     return cfg
 
 
+# A step of the brute-force workload is five calls, a call two launches (the
+# cluster's sort and the scan): the line's contract test holds ten launches a
+# step, which was one call's count before the cells.
+BRUTE_CALLS = 5
+
+
 def brute_config(n: int, k: int, world: int) -> dict:
     return {"workload": WORKLOADS["brute"], "agents": n, "k": k,
             "parallelism": f"replicas x{world}",
@@ -370,7 +376,7 @@ def run_reference_brute(args):
     line = {
         "impl": "reference", "metric": "agent-queries/s", "value": v, "unit": "agent-queries/s",
         "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup,
-        "ms_per_step": 1e3 * el / args.steps * n / m, "higher_is_better": True,
+        "ms_per_step": 1e3 * el / args.steps * n / m * BRUTE_CALLS, "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
         "config": brute_config(n, k, args.gpus),
         "cpu_baseline": {"value": v, "unit": "agent-queries/s", "cores": threads, "kind": "port",
@@ -436,7 +442,8 @@ def read_traffic(workload):
 
 
 def phase_times(lib, group, run, steps):
-    """Per-launch ms of the four step phases over `steps` profiled steps."""
+    """Per-launch ms of the four step phases over `steps` profiled steps (None:
+    the step's form has no such phase)."""
     from gpusteer_gb300._lib import check
 
     check(lib.gs_group_set_profiling(group.handle, 1))
@@ -447,6 +454,16 @@ def phase_times(lib, group, run, steps):
     check(lib.gs_group_set_profiling(group.handle, 0))
     return {name: (phase_ms[i] / phase_n[i] if phase_n[i] else None)
             for i, name in enumerate(["scan", "permute", "fused", "fused_rest"])}
+
+
+def step_kernels(form: str, walls: bool) -> str:
+    """The kernels of the fused phases of a step of this form."""
+    if form == "persistent":
+        return "k_step_persistent"
+    k = {"threads": "k_fused", "lanes": "k_lanes", "table": "k_table"}[form]
+    if walls:
+        return f"{k}_walls+{k}_rest"
+    return k if form == "threads" else f"{k}_step"
 
 
 def adjoint_timing(reps: int = 5):
@@ -578,9 +595,9 @@ def gpu_batched_line(args, dist, rank, world, local_rank):
         got = AgentState.concat([x.download() for x in run])
         parts_identical = all(np.array_equal(getattr(got, k), getattr(want, k))
                               for k in got.names())
+    launches_per_step = sum(gs.last_step(x.group)[1] for x in run)
     del run
     phases = phase_times(lib, b.group, lambda k: b.step(p, k), max(3, min(args.steps, 10)))
-    launches_per_step = gs.step_launches(b.group, True) * max(1, tr.parts)
     measured_cap = gs.knn_capacity(b.group)  # the scan the resident steps used
     # both forms of the step on the same batch: separate launches (one graph
     # replay per step) and one persistent launch per step
@@ -598,7 +615,7 @@ def gpu_batched_line(args, dist, rank, world, local_rank):
         f1.synchronize()
         forms["persistent" if pers else "separate"] = {
             "ms_per_step": f0.elapsed_time(f1) / args.steps,
-            "launches_per_step": gs.step_launches(b.group, True)}
+            "launches_per_step": gs.last_step(b.group)[1]}
     del b
 
     # the same scenes, one gs_step call per scene per step (same grid, block,
@@ -960,7 +977,8 @@ def gpu_brute_line(args, dist, rank, world, local_rank):
     g.upload(s)
     knn = gs.KNNData(n, k)
     stream = torch.cuda.ExternalStream(g.stream)
-    for _ in range(args.warmup):
+    calls, call_launches = BRUTE_CALLS, 2
+    for _ in range(args.warmup * calls):
         gs.findKNearestNeighborsBruteForce(g, knn, g)
     g.synchronize()
     barrier(dist)
@@ -969,24 +987,24 @@ def gpu_brute_line(args, dist, rank, world, local_rank):
         torch.cuda.synchronize()
         torch.cuda.profiler.start()
         ev0.record(stream)
-        for _ in range(args.steps):
+        for _ in range(args.steps * calls):
             gs.findKNearestNeighborsBruteForce(g, knn, g)
         ev1.record(stream)
         ev1.synchronize()
         torch.cuda.profiler.stop()
     barrier(dist)
     ms_max = allreduce_max(dist, ev0.elapsed_time(ev1))
-    per = ms_max / args.steps
+    per = ms_max / (args.steps * calls)
     pairs_all = float(n) * (n - 1)
-    # the pairs whose distance was taken: the scan visits cells outwards from
-    # a query until no farther one can enter its list
+    # the pairs whose distance was taken: the scan meets the candidates of a
+    # query's cells and of those that the k-th distance found there reaches
     pairs = float(gs.bruteforce_pairs(g))
     tflops = 8.0 * pairs / (per / 1e3) / 1e12
     peak = fp32_peak_tflops()
     # end to end: positions up, lists down, every query
     hp = s.copy()
     t0 = time.perf_counter()
-    e2e_steps = max(3, min(args.steps, 20))
+    e2e_steps = max(3, min(args.steps, 20)) * calls
     for _ in range(e2e_steps):
         g.upload(hp)
         gs.findKNearestNeighborsBruteForce(g, knn, g)
@@ -1009,17 +1027,16 @@ def gpu_brute_line(args, dist, rank, world, local_rank):
                          f"{threads} threads"}
     line = {
         "metric": "agent-queries/s", "value": n * world / (per / 1e3), "unit": "agent-queries/s",
-        "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": per,
+        "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
+        "ms_per_step": per * calls, "calls_per_step": calls, "ms_per_call": per,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic",
         "config": brute_config(n, k, world),
         "e2e": {"value": n * e2e_steps * world / e2e_s, "unit": "agent-queries/s",
-                "h2d_bytes_per_step": n * 96, "d2h_bytes_per_step": n * k * 8},
-        # nominal: the calls' cost was ten launches each when this field's
-        # value was fixed; launches_per_call is what a call makes
+                "h2d_bytes_per_step": n * 96 * calls, "d2h_bytes_per_step": n * k * 8 * calls},
         # (profiles/k_brute_cells_65536_agents.md lists them)
-        "gpu_launches": 10 * args.steps,
-        "launches_per_call": 2,
+        "gpu_launches": call_launches * calls * args.steps,
+        "launches_per_call": call_launches,
         "roofline": {"bound": "fp32", "achieved": tflops, "peak": peak, "unit": "TFLOP/s",
                      "frac": tflops / peak, "traffic": None, "kernel": "k_brute_cells",
                      "algorithmic_flops_per_launch": 8.0 * pairs,
@@ -1086,6 +1103,7 @@ def gpu_single_line(args, dist, rank, world, local_rank):
     ms = ev0.elapsed_time(ev1)
     ms_max = allreduce_max(dist, ms)
     value = n * args.steps * world / (ms_max / 1e3)
+    form, launches = gs.last_step(group)
 
     # dominant kernel: phase timing with CUDA events on the group's stream
     phases = phase_times(lib, group, lambda k: gs.step(group, bins, walls, p, k),
@@ -1143,10 +1161,11 @@ def gpu_single_line(args, dist, rank, world, local_rank):
                 "d2h_bytes_per_step": bytes_back,
                 "api": "gs_step_host in place: page-locked host state copied in, one step, "
                        "copied out (the per-agent constants stay on the host)"},
-        "gpu_launches": gs.step_launches(group, has_walls) * args.steps,
+        "gpu_launches": launches * args.steps,
+        "form": form,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic,
-                     "kernel": "k_fused" + ("_walls+k_fused_rest" if has_walls else ""),
+                     "kernel": step_kernels(form, has_walls),
                      "algorithmic_bytes_per_launch": fbytes, "peak_source": peak_src},
         "phases_ms": phases,
         "step_model_gbs": step_model_gbs,

@@ -12,7 +12,7 @@ from .groups import (  # noqa: F401
     antiPenetrationWall, updateGroupWithAntiPenetration,
     findKNearestNeighbors, findKNearestNeighborsBruteForce, findKNearestNeighborsGroups,
     set_barrier_limit, set_block, set_graphs, set_persistent,
-    knn_capacity, set_knn_capacity, step, step_host, step_launches, steerForAlignment,
+    knn_capacity, set_knn_capacity, step, step_host, step_launches, last_step, steerForAlignment,
     steerForCohesion,
     steerForSeek, steerForSeparation, steerToAvoidNeighbors, steerToAvoidWalls, steerToFollowPath,
     updateGroup,

@@ -78,6 +78,7 @@ SIGNATURES = {
     "gs_group_synchronize": [_vp],
     "gs_group_set_profiling": [_vp, _i],
     "gs_group_phase_times": [_vp, _fp, _up, _u],
+    "gs_group_last_step": [_vp, C.POINTER(_i), _up],
     "gs_group_exact_redos": [_vp, _up],
     "gs_group_set_persistent": [_vp, C.c_int],
     "gs_group_set_barrier_limit": [_vp, _u],

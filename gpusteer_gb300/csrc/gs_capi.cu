@@ -481,6 +481,13 @@ gs_status gs_group_set_profiling(gs_group g, int enable) {
     return GS_OK;
 }
 
+gs_status gs_group_last_step(gs_group g, int* form, unsigned* launches) {
+    if (!g) return fail(GS_ERR_INVALID_ARG, "null group");
+    if (form) *form = g->step_form;
+    if (launches) *launches = g->step_launches;
+    return GS_OK;
+}
+
 gs_status gs_group_exact_redos(gs_group g, unsigned* count) {
     if (!g || !count) return fail(GS_ERR_INVALID_ARG, "null argument");
     *count = 0;
@@ -1818,7 +1825,7 @@ static unsigned table_row_log2(const StepDev& d, unsigned C) {
 constexpr unsigned kTableMostCandidates = 2500000;
 static bool table_wanted(gs_group g, const StepDev& d, const Grid& grid, unsigned C,
                          const unsigned* agent_scene) {
-    return agent_scene == nullptr && d.r == 1 && g->knn_cap == 0 && !g->profiling &&
+    return agent_scene == nullptr && d.r == 1 && g->knn_cap == 0 &&
            !g->persistent && g->table.refused != C && lanes_preferred(g->n, (d.need & NEED_WALLS) != 0) &&
            (size_t(C) << table_row_log2(d, C)) <= (size_t(1) << 22) &&
            !(measured(g, grid, 1) && g->auto_met > kTableMostCandidates);
@@ -1933,6 +1940,8 @@ static gs_status table_run(gs_group g, StepDev d, const Grid& grid, unsigned C,
     }
     g->fdb.grid = grid;
     const bool walls = d.need & NEED_WALLS;
+    Profiler prof(g);
+    PhaseHook* hook = g->profiling ? &prof : nullptr;
     for (unsigned s = 0; s < steps; ++s) {
         TableStep T = table_buffers(g, t.step % 6);
         T.walls = WallRefs{w.start, w.end, w.normal, w.pos_id, w.cell_start};
@@ -1944,7 +1953,7 @@ static gs_status table_run(gs_group g, StepDev d, const Grid& grid, unsigned C,
         }
         d.dirty = dirty ? 1 : 0;
         dirty = false;
-        GS_TRY(table_step(T, d, st));
+        GS_TRY(table_step(T, d, st, hook));
         if (!walls) {
             std::swap(g->A.f[0], g->B.f[0]);
             std::swap(g->A.f[1], g->B.f[1]);
@@ -1955,7 +1964,24 @@ static gs_status table_run(gs_group g, StepDev d, const Grid& grid, unsigned C,
     g->db.valid = false;
     g->frame_cells = C;
     t.frame = true;
+    g->step_form = GS_FORM_TABLE;
+    g->step_launches = walls ? 2 : 1;
     return GS_OK;
+}
+
+// Records the form of the sorting step just run and its launches: scan,
+// permute, the step (two with walls) and, with a thread per agent on the
+// streaming scan, the redo agents' exact lists and, without walls, their redo.
+static void last_step(gs_group g, const StepDev& d) {
+    const bool walls = d.need & NEED_WALLS;
+    if (d.persistent && persistent_supported(d)) {
+        g->step_form = GS_FORM_PERSISTENT;
+        g->step_launches = 1;
+        return;
+    }
+    g->step_form = d.lanes ? GS_FORM_LANES : GS_FORM_THREADS;
+    g->step_launches = 2 + (walls ? 2 : 1);
+    if (!d.lanes && d.enum_cap > 64) g->step_launches += walls ? 1 : 2;
 }
 
 // The fused engine for a group whose scene table is in g->h_scenes / d_scene
@@ -2023,6 +2049,7 @@ static gs_status fused_run(gs_group g, StepDev d, const Grid& grid, unsigned C,
         }
         for (; step < steps; ++step) GS_CUDA(cudaGraphLaunch(g->graph_exec, st));
     }
+    last_step(g, d);
     g->accum_dirty = false;
     g->db.valid = false;
     g->frame_cells = C;

@@ -209,6 +209,8 @@ struct gs_group_s {
     bool persistent;       // run supported steps as one persistent launch
     unsigned bar_limit;    // its barrier poll limit (0: default)
     unsigned* d_bar;       // its grid barrier (2 words)
+    int step_form;         // gs_step_form of the last fused step, and the launches
+    unsigned step_launches;  // one such step makes
     // phase profiling (gs_group_set_profiling)
     bool profiling;
     std::vector<cudaEvent_t>* prof_events;  // pairs of (start, stop) per recorded phase

@@ -330,31 +330,35 @@ gs_status table_init(GroupView g, const TableStep& T, int wrap_mode, bool dirty,
 }
 
 template <int G, bool FLAT>
-static void table_go(const TableStep& T, const StepDev& p, cudaStream_t st) {
+static void table_go(const TableStep& T, const StepDev& p, cudaStream_t st, PhaseHook* hook) {
     const unsigned nb = blocks_for(T.n, kTableBlock / G);
-    if (!(p.need & NEED_WALLS)) {
-        if ((p.need & kNeedList) == (NEED_SEP | NEED_ALI | NEED_COH))
-            launch_after(k_table_step<G, FLAT, NEED_SEP | NEED_ALI | NEED_COH>, nb, kTableBlock, 0, st, T, p);
-        else
-            launch_after(k_table_step<G, FLAT, kNeedRuntime>, nb, kTableBlock, 0, st, T, p);
-        return;
-    }
-    launch_after(k_table_walls<G, FLAT>, nb, kTableBlock, 0, st, T, p);
+    if (hook) hook->mark(2, true);
+    if (p.need & NEED_WALLS)
+        launch_after(k_table_walls<G, FLAT>, nb, kTableBlock, 0, st, T, p);
+    else if ((p.need & kNeedList) == (NEED_SEP | NEED_ALI | NEED_COH))
+        launch_after(k_table_step<G, FLAT, NEED_SEP | NEED_ALI | NEED_COH>, nb, kTableBlock, 0, st, T, p);
+    else
+        launch_after(k_table_step<G, FLAT, kNeedRuntime>, nb, kTableBlock, 0, st, T, p);
+    if (hook) hook->mark(2, false);
+    if (!(p.need & NEED_WALLS)) return;
+    if (hook) hook->mark(3, true);
     if ((p.need & kNeedList) == (NEED_SEP | NEED_AVOID))
         launch_after(k_table_rest<G, NEED_SEP | NEED_AVOID>, nb, kTableBlock, 0, st, T, p);
     else
         launch_after(k_table_rest<G, kNeedRuntime>, nb, kTableBlock, 0, st, T, p);
+    if (hook) hook->mark(3, false);
 }
 
-gs_status table_step(const TableStep& T, const StepDev& p, cudaStream_t st) {
+gs_status table_step(const TableStep& T, const StepDev& p, cudaStream_t st, PhaseHook* hook) {
     if (T.n == 0) return GS_OK;
     if ((p.need & NEED_WALLS) && p.knw > 8)
         return fail(GS_ERR_UNSUPPORTED, "knw > 8 in the fused step");
     // k <= 8 on 16 lanes while the chip has room for them: the box's 27 counts
     // and its candidates take fewer rounds (4,096 boids 9.7 -> 9.2 us a step)
-    if (p.k <= 8 && T.n > 8192) p.flat ? table_go<8, true>(T, p, st) : table_go<8, false>(T, p, st);
-    else if (p.k <= 16) p.flat ? table_go<16, true>(T, p, st) : table_go<16, false>(T, p, st);
-    else p.flat ? table_go<32, true>(T, p, st) : table_go<32, false>(T, p, st);
+    const auto go = p.k <= 8 && T.n > 8192 ? (p.flat ? table_go<8, true> : table_go<8, false>)
+                    : p.k <= 16            ? (p.flat ? table_go<16, true> : table_go<16, false>)
+                                           : (p.flat ? table_go<32, true> : table_go<32, false>);
+    go(T, p, st, hook);
     GS_LAUNCHED("table_step");
     return GS_OK;
 }

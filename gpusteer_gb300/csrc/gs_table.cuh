@@ -29,7 +29,8 @@ struct TableStep {
 
 gs_status table_init(GroupView g, const TableStep& T, int wrap_mode, bool dirty, float4* f5,
                      unsigned* redo_count, cudaStream_t st);
-gs_status table_step(const TableStep& T, const StepDev& p, cudaStream_t st);
+// hook (may be null) brackets the launches as phases 2 and 3.
+gs_status table_step(const TableStep& T, const StepDev& p, cudaStream_t st, PhaseHook* hook);
 // Mean velocity per cell of the step that T described (its f1_next holds the
 // agents' new state).
 gs_status table_avg_velocity(const TableStep& T, float3* out, cudaStream_t st);

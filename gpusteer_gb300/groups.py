@@ -346,15 +346,26 @@ def knn_capacity(group) -> int:
     return int(out.value)
 
 
+STEP_FORMS = ("none", "threads", "lanes", "table", "persistent")
+
+
+def last_step(group) -> tuple[str, int]:
+    """The form the group's last step ran in (STEP_FORMS) and the kernel
+    launches one step of that form makes."""
+    form, launches = C.c_int(0), C.c_uint(0)
+    call("gs_group_last_step", group.handle, C.byref(form), C.byref(launches))
+    return STEP_FORMS[form.value], int(launches.value)
+
+
 def step_launches(group, walls: bool) -> int:
-    """Kernel launches of one fused step: the counting-sort scan, the
+    """Kernel launches of one sorting step with a thread per agent (or of the
+    persistent one) at the group's capacity: the counting-sort scan, the
     permute, the fused kernel (two with walls), and with the streaming scan
     (capacity 128 or 256) the warp-per-agent exact lists, plus, without
     walls, the exact redo (with walls the lists go straight to the second
-    half; the collecting scan redoes its rare agents inline).  Counted for the
-    sorting step.  A small group's (a group of lanes per agent, automatic
-    capacity only) needs no exact lists, and a small single scene's at radius
-    1 no sort either: one launch, two with walls."""
+    half; the collecting scan redoes its rare agents inline).  Small groups
+    of automatic capacity step in other forms: last_step tells which the last
+    step took and its launches."""
     cap = knn_capacity(group)
     if getattr(group, "persistent", False) and walls and cap > 64 and 8 < group.k <= 16:
         return 1

@@ -163,9 +163,21 @@ gs_status gs_group_synchronize(gs_group g);
  * While enabled, every phase launch is bracketed by events; the totals are
  * read with gs_group_phase_times: ms[i] and launches[i] for phase i =
  * 0 scan, 1 permute, 2 fused step (or its wall half), 3 second half after
- * walls.  Enabling clears the totals. */
+ * walls.  The step's form does not depend on it; phases that a form does not
+ * have (a small group's cell tables need no scan and no permute) count no
+ * launches.  Enabling clears the totals. */
 #define GS_PHASES 4
 gs_status gs_group_set_profiling(gs_group g, int enable);
+/* The form the group's last gs_step or gs_batch_step ran in, and the kernel
+ * launches one step of that form makes. */
+typedef enum gs_step_form {
+    GS_FORM_NONE = 0,       /* no step yet */
+    GS_FORM_THREADS = 1,    /* sorted, a thread per agent */
+    GS_FORM_LANES = 2,      /* sorted, a group of lanes per agent (small groups) */
+    GS_FORM_TABLE = 3,      /* cell tables, no sort (small single scenes) */
+    GS_FORM_PERSISTENT = 4  /* one cooperative launch (gs_group_set_persistent) */
+} gs_step_form;
+gs_status gs_group_last_step(gs_group g, int* form, unsigned* launches);
 /* Agents of the last fused step whose neighbour order the fast 32-bit KNN
  * scan could not vouch for (exact distance ties, crowded boxes) and that the
  * exact path redid; waits for the group's stream. */
