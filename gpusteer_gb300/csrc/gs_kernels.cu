@@ -9,6 +9,7 @@
 // deterministic; nothing downstream depends on it because every KNN uses the
 // total order (distance, agent index).
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 
 #include "gs_behaviours.cuh"
@@ -19,6 +20,16 @@
 #include "gs_launch.h"
 
 namespace gs {
+
+unsigned sm_count() {
+    static std::atomic<int> known[64];
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+    if ((sms = known[dev].load(std::memory_order_relaxed)) > 0) return unsigned(sms);
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 1;
+    known[dev].store(sms, std::memory_order_relaxed);
+    return unsigned(sms);
+}
 
 // ---- exclusive scan (device code in gs_scan.cuh) ----------------------------------
 unsigned scan_tile_count(unsigned C) { return (C + kScanTile - 1) / kScanTile; }
@@ -558,7 +569,7 @@ gs_status launch_cell_avg_velocity(const Database& db, const float4* dir, const 
 
 // Threads per block of the per-function launches: small groups in small
 // blocks, so that their few warps spread over all SMs.
-static unsigned call_block(unsigned n) { return n <= 64u * 152u * 8u ? 64u : unsigned(kBlock); }
+static unsigned call_block(unsigned n) { return n <= 64u * 8u * sm_count() ? 64u : unsigned(kBlock); }
 
 // ---- WrapWorldCUDAKernel.cu:11-48 ---------------------------------------------------
 __global__ void k_wrap(float4* pos, unsigned n, float wx, float wy, float wz, int mode) {

@@ -51,6 +51,9 @@ void launch_after(void (*kernel)(P...), unsigned grid, unsigned block, size_t sm
     (void)cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
+// SMs of the current device (asked of it once).
+unsigned sm_count();
+
 // ---- counting-sort binning ---------------------------------------------------
 // Exclusive scan of count[0..C) into start[0..C]; zeroes count.
 gs_status scan_counts(unsigned* count, unsigned* start, unsigned C, unsigned* tile,

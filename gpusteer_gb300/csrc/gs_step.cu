@@ -950,14 +950,14 @@ static gs_status allow_smem(K kernel, size_t bytes) {
 // Redo launches over the retry list: a grid of up to four blocks per SM that
 // strides over however many agents the fast launch appended (read on the
 // device); agents that all overflowed still spread over the whole GPU.
-constexpr unsigned kRetryBlocksMax = 4 * 152;
+constexpr unsigned kRetryBlocksPerSM = 4;
 
 template <int KMAX, unsigned ENUM>
 static gs_status launch_fused_k(const FusedLaunch& L, const StepDev& p, cudaStream_t st,
                                 PhaseHook* hook) {
     const unsigned bs = p.block ? p.block : kBlock;
     const unsigned nb = blocks_for(L.n, bs);
-    const unsigned nb_retry = std::min(blocks_for(L.n, kBlock), kRetryBlocksMax);
+    const unsigned nb_retry = std::min(blocks_for(L.n, kBlock), kRetryBlocksPerSM * sm_count());
     // collecting scan: slot and key tables of ENUM words per thread;
     // streaming scan: the k result slots only
     const size_t smem = ENUM > 64 ? size_t(KMAX > 8 ? KMAX : 8) * bs * sizeof(unsigned)
@@ -1015,7 +1015,7 @@ static gs_status launch_fused_k(const FusedLaunch& L, const StepDev& p, cudaStre
                 // boids 31.0 -> 28.1 us a step, 65,536 37.4 -> 32.6; 100,003,
                 // in one wave only at three to an SM, 45.8 against 46.3; the
                 // shared-angle pass, four against two: 30.8 against 31.4)
-                const bool two = nb * bs <= 2 * 152 * kBlock;
+                const bool two = nb * bs <= 2 * sm_count() * kBlock;
                 auto kern = p.same_flock ? (two ? k_fused<KMAX, 32, false, flock, false, 4, 2, true>
                                                 : k_fused<KMAX, 32, false, flock, false, kAhead, 3, true>)
                                          : (two ? k_fused<KMAX, 32, false, flock, false, 2, 2>
@@ -1160,12 +1160,10 @@ static gs_status launch_persistent_k(const FusedLaunch& L, const StepDev& p,
     auto kern = k_step_persistent<16, ENUM, NEEDC>;
     constexpr size_t smem = persistent_smem<16>();
     GS_TRY(allow_smem(kern, smem));
-    int dev = 0, sms = 0, per_sm = 0;
-    GS_CUDA(cudaGetDevice(&dev));
-    GS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int per_sm = 0;
     GS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, smem));
     if (per_sm < 1) return fail(GS_ERR_UNSUPPORTED, "the persistent step does not fit on an SM");
-    const unsigned grid = unsigned(per_sm) * unsigned(sms);
+    const unsigned grid = unsigned(per_sm) * sm_count();
     // the barrier starts from zero on every launch, also after a step that gave up
     GS_CUDA(cudaMemsetAsync(P.bar, 0, sizeof(GridBarrier), st));
     FusedLaunch l = L;
@@ -1284,7 +1282,7 @@ gs_status count_occupied(const unsigned* count, unsigned C, unsigned* d_tmp, uns
     *h_sumsq = 0;
     if (C == 0) return GS_OK;
     GS_CUDA(cudaMemsetAsync(d_tmp, 0, 4 * sizeof(unsigned), st));
-    const unsigned nb = std::min(blocks_for(C, kBlock), 8u * 152u);
+    const unsigned nb = std::min(blocks_for(C, kBlock), 8u * sm_count());
     k_count_occupied<<<nb, kBlock, 0, st>>>(count, C, d_tmp, boxes ? *boxes : Grid{},
                                             boxes != nullptr);
     GS_LAUNCHED("count_occupied");

@@ -101,3 +101,9 @@ def test_early_launched_kernels_wait_first_and_take_no_invariant_pointers():
                 assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", m.group(1)), \
                     f"{path.name}: {m.group(0)[:120]}"
     assert found == set(LAUNCHED_EARLY) | {"k_fused"}
+
+
+@pytest.mark.parametrize("path", SOURCES + sorted(CSRC.glob("*.h")), ids=lambda p: p.name)
+def test_no_rule_holds_the_chips_sm_count(path):
+    """Launch rules ask the device (sm_count)."""
+    assert not re.search(r"\b152u?\b", code(path))
