@@ -282,9 +282,10 @@ gs_status gs_multigroup_step(const gs_group* groups, unsigned n_groups, gs_bins 
 gs_status gs_find_knn_walls(gs_group g, gs_knn out, gs_bins bins, gs_walls walls,
                             unsigned search_radius);
 /* KNNBruteForceCUDAV2 (KNNBruteForceCUDA.cu:163-187).  The lists are the
- * reference's for every pair of groups; with 128 queries or more the
- * scan takes cells of candidates outwards from each query until no farther
- * one can enter its list, so a call evaluates far fewer than n * m pairs. */
+ * reference's for every pair of groups; with 128 queries or more a query
+ * meets the candidates of the cells about its own, whose k-th distance bounds
+ * what else can enter its list, and of the cells within that bound, so a call
+ * evaluates far fewer than n * m pairs. */
 gs_status gs_knn_bruteforce(gs_group g, gs_knn out, gs_group other);
 /* The (query, candidate) pairs the last gs_knn_bruteforce call of g ran its
  * distance filter on (n * m without the skipping scan).  Synchronises the
@@ -365,7 +366,10 @@ gs_status gs_anti_penetration_wall(gs_group g, gs_knn knw, gs_walls walls, float
 /* Runs `steps` whole steps; the result equals the per-function sequence
  * wrap -> rebuild -> KNN (+ wall KNN) -> behaviours in p->order -> update.
  * Requires knn_mode GS_KNN_BINNED, and avoid-walls (if present) first in order.
- * `walls` may be NULL when the order has no GS_B_AVOID_WALLS. */
+ * `walls` may be NULL when the order has no GS_B_AVOID_WALLS.
+ * A small group (16,384 agents, 20,000 with avoid-walls) at radius 1 and
+ * automatic KNN capacity steps on cell tables, up to 128 MiB of the device's
+ * memory, kept with the group; where they cannot be had it sorts instead. */
 gs_status gs_step(gs_group g, gs_bins bins, gs_walls walls, const gs_step_params* p,
                   unsigned steps);
 /* As gs_step but the state comes from and goes back to host arrays, each copy
