@@ -8,11 +8,13 @@ namespace gs {
 
 // ---- launches that follow one another --------------------------------------------
 // A kernel launched with launch_after() starts with after_previous(): its blocks
-// may become resident once the kernel before it in the stream has all of its
-// own running, and wait there for that kernel's end and its writes.  The launch
+// may become resident once the kernel before it in the stream runs (has passed
+// its own wait), and wait there for that kernel's end and its writes.  The launch
 // latency and the blocks' start then pass under the previous kernel.  Nothing is
 // read or written before the wait; a kernel completes only after its predecessor
-// has, so the order of a whole chain holds.
+// has, so the order of a whole chain holds.  The wait stands before the trigger,
+// so no more than one kernel waits on the SMs: the other way round a whole chain's
+// blocks took their places at once (four frames of three groups 343 us, 302 so).
 //
 // Since such a kernel is resident while its predecessor writes, what it reads is
 // not constant for its lifetime: neither its pointer parameters nor those of the
@@ -20,13 +22,13 @@ namespace gs {
 // be moved above the wait), and every load is an ordinary one, not the read-only
 // path's.
 //
-// Kernels launched with <<<>>> (a new grid's recount, the diagnostics, brute
-// force over every pair, the thread-per-agent group frames and
+// Kernels launched with launch_in_order() or <<<>>> (a new grid's recount, the
+// diagnostics, brute force over every pair, the thread-per-agent group frames and
 // anti-penetration) keep plain stream order: they start after their predecessor
 // has ended, and what follows them waits for their end as for any other's.
 __device__ __forceinline__ void after_previous() {
-    asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
 }
 // Starts of launches up to this many threads pass under the kernel before
 // (us a pass, without / with: 16 steps of 4,096 boids 183 / 156, a boids
@@ -35,11 +37,11 @@ __device__ __forceinline__ void after_previous() {
 // waves anyway, is slower with it (4217 / 4297).
 constexpr size_t kAfterMaxThreads = size_t(1) << 21;
 template <class... P, class... A>
-void launch_after(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
-                  cudaStream_t st, const A&... args) {
+void launch_kernel(bool early, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                   cudaStream_t st, const A&... args) {
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = size_t(grid) * block <= kAfterMaxThreads;
+    at.val.programmaticStreamSerializationAllowed = early;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -49,6 +51,25 @@ void launch_after(void (*kernel)(P...), unsigned grid, unsigned block, size_t sm
     cfg.numAttrs = 1;
     // an error stays with the runtime for the GS_LAUNCHED that follows
     (void)cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+template <class... P, class... A>
+void launch_after(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                  cudaStream_t st, const A&... args) {
+    launch_kernel(size_t(grid) * block <= kAfterMaxThreads, kernel, grid, block, smem, st, args...);
+}
+// In plain stream order, for the sorting step's long kernels with a thread per
+// agent: blocks that take their places while the short kernel before still holds
+// some SMs crowd onto the others and stay there, a few hundred blocks of a group
+// that would otherwise lie one or two to an SM (8 steps, this / launch_after / the
+// sorting step before either: 30,000 boids in boxes of 400 1277 / 1483 / 1272 us,
+// 65,536 at 13 to a box and capacity 128 554 / 614 / 622, a crowd of 40,000 335 /
+// 385 / 386).  The collecting scan's kernel, which no redo launch follows, gains
+// by the early start (a 12-step fit of 65,536 1904 / 1886, one step of 100,003
+// boids through host memory 227 / 221).
+template <class... P, class... A>
+void launch_in_order(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem,
+                     cudaStream_t st, const A&... args) {
+    launch_kernel(false, kernel, grid, block, smem, st, args...);
 }
 
 // SMs of the current device (asked of it once).

@@ -976,24 +976,28 @@ static gs_status launch_fused_k(const FusedLaunch& L, const StepDev& p, cudaStre
         // 74.0 us with it, at a quarter of the shared memory.
         if (p.flat && (ENUM > 64 || p.r == 1)) {
             const size_t cols = size_t(KMAX > 8 ? KMAX : 8) * bs * sizeof(unsigned);
-            launch_after(k_fused_walls<KMAX, 8, ENUM, false, true>, nb, bs, cols, st, L, p);
+            launch_in_order(k_fused_walls<KMAX, 8, ENUM, false, true>, nb, bs, cols, st, L, p);
         } else {
             GS_TRY(allow_smem(k_fused_walls<KMAX, 8, ENUM, false>, smem));
-            launch_after(k_fused_walls<KMAX, 8, ENUM, false>, nb, bs, smem, st, L, p);
+            launch_in_order(k_fused_walls<KMAX, 8, ENUM, false>, nb, bs, smem, st, L, p);
         }
         // the redo agents' exact lists, straight into the neighbour lists
-        if (ENUM > 64) launch_after(k_knn_retry<KMAX, true>, nb_retry, kBlock, 0, st, L, p);
+        if (ENUM > 64) launch_in_order(k_knn_retry<KMAX, true>, nb_retry, kBlock, 0, st, L, p);
         if (hook) hook->mark(2, false);
         if (hook) hook->mark(3, true);
         // the choke-point step (separation and neighbour avoidance) has its own build
         if ((p.need & kNeedList) == (NEED_SEP | NEED_AVOID))
-            launch_after(k_fused_rest<KMAX, NEED_SEP | NEED_AVOID>, nb, bs, 0, st, L, p);
+            launch_in_order(k_fused_rest<KMAX, NEED_SEP | NEED_AVOID>, nb, bs, 0, st, L, p);
         else
-            launch_after(k_fused_rest<KMAX, kNeedRuntime>, nb, bs, 0, st, L, p);
+            launch_in_order(k_fused_rest<KMAX, kNeedRuntime>, nb, bs, 0, st, L, p);
         if (hook) hook->mark(3, false);
     } else {
         GS_TRY(allow_smem(k_fused<KMAX, ENUM, false>, smem));
         if (hook) hook->mark(2, true);
+        const auto start = [&](auto kern) {
+            if (ENUM > 64) launch_in_order(kern, nb, bs, smem, st, L, p);
+            else launch_after(kern, nb, bs, smem, st, L, p);
+        };
         // the flock (separation, alignment, cohesion) on the collecting scan has
         // its own build
         bool done = false;
@@ -1005,7 +1009,7 @@ static gs_status launch_fused_k(const FusedLaunch& L, const StepDev& p, cudaStre
         if (ENUM > 32 && p.same_flock && (p.need & kNeedList) == flock && !(ENUM > 64 && p.flat)) {
             auto kern = k_fused<KMAX, ENUM, false, flock, false, kAhead, 3, true>;
             GS_TRY(allow_smem(kern, smem));
-            launch_after(kern, nb, bs, smem, st, L, p);
+            start(kern);
             done = true;
         }
         if constexpr (ENUM == 32) {
@@ -1021,21 +1025,21 @@ static gs_status launch_fused_k(const FusedLaunch& L, const StepDev& p, cudaStre
                                          : (two ? k_fused<KMAX, 32, false, flock, false, 2, 2>
                                                 : k_fused<KMAX, 32, false, flock>);
                 GS_TRY(allow_smem(kern, smem));
-                launch_after(kern, nb, bs, smem, st, L, p);
+                start(kern);
                 done = true;
             }
         }
         if constexpr (ENUM > 64) {
             if (p.flat && !done) {
                 GS_TRY(allow_smem(k_fused<KMAX, ENUM, false, kNeedRuntime, true>, smem));
-                launch_after(k_fused<KMAX, ENUM, false, kNeedRuntime, true>, nb, bs, smem, st, L, p);
+                start(k_fused<KMAX, ENUM, false, kNeedRuntime, true>);
                 done = true;
             }
         }
-        if (!done) launch_after(k_fused<KMAX, ENUM, false>, nb, bs, smem, st, L, p);
+        if (!done) start(k_fused<KMAX, ENUM, false>);
         if (ENUM > 64) {
-            launch_after(k_knn_retry<KMAX, false>, nb_retry, kBlock, 0, st, L, p);
-            launch_after(k_fused<KMAX, 32, true>, nb_retry, kBlock, smem_x, st, L, p);
+            launch_in_order(k_knn_retry<KMAX, false>, nb_retry, kBlock, 0, st, L, p);
+            launch_in_order(k_fused<KMAX, 32, true>, nb_retry, kBlock, smem_x, st, L, p);
         }
         if (hook) hook->mark(2, false);
     }
