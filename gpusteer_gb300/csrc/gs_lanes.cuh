@@ -94,23 +94,19 @@ __device__ __forceinline__ LaneEntry<G> lanes_candidate(V3 p, unsigned self_id, 
     return c;
 }
 
-// The k nearest of the box around cell (ix, iy, iz), in (distance, index)
-// order over the group's lanes: lane r holds rank r (ranks past the last
-// neighbour hold the empty entry; lanes r >= k hold leftovers).
+// Calls take(q, slot, ok, first) for the candidates of box b, one per lane of the
+// group at a time, in warp-converged rounds (ok: this lane has one; first: the
+// first round).
 // R: rows of cells in the box at search radius 1 (9, or 3 on a grid one cell
 // high in y); 0 for any radius.  The rows are laid end to end, so a group
 // takes ceil(candidates / G) chunks whatever the rows' lengths; with R = 0
 // their table is the group's kLaneRowWords words `rows` of shared memory, and
 // a box of more than kLaneRows rows is taken row by row.
 constexpr unsigned kLaneRows = 64, kLaneRowWords = 2 * kLaneRows + 1;
-template <int G, int R>
-__device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 p,
-                                                  unsigned self_id, const Grid& g, const Box& b,
-                                                  unsigned cell_offset,
-                                                  const unsigned* start,
-                                                  const float4* pos_id,
-                                                  unsigned* rows = nullptr) {
-    LaneEntry<G> list{KEY_EMPTY, UINT_MAX};
+template <int G, int R, class Take>
+__device__ __forceinline__ void lanes_box(unsigned lane, const Grid& g, const Box& b,
+                                          unsigned cell_offset, const unsigned* start,
+                                          const float4* pos_id, unsigned* rows, Take&& take) {
     const unsigned span = b.x1 - b.x0 + 1;
     if constexpr (R > 0) {
         constexpr int Q = (R + G - 1) / G;
@@ -148,7 +144,7 @@ __device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 
             const unsigned j = j0 + lane, jn = j + G;
             const unsigned sn = at(jn);
             const float4 qn = jn < total ? pos_id[sn] : make_float4(0.f, 0.f, 0.f, 0.f);
-            lanes_take(list, lanes_candidate<G>(p, self_id, q, sl, j < total), j0 == 0, k, lane);
+            take(q, sl, j < total, j0 == 0);
             sl = sn;
             q = qn;
         }
@@ -192,7 +188,7 @@ __device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 
                     sl = rs[at] + (j - pre[at]);
                 }
                 const float4 q = ok ? pos_id[sl] : make_float4(0.f, 0.f, 0.f, 0.f);
-                lanes_take(list, lanes_candidate<G>(p, self_id, q, sl, ok), j < G, k, lane);
+                take(q, sl, ok, j < G);
             }
             __syncwarp();  // the rows may be written again
         } else {
@@ -204,13 +200,29 @@ __device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 
                 for (unsigned j = lane; j < rounds + lane; j += G) {
                     const float4 q =
                         j < len ? pos_id[s0 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    lanes_take(list, lanes_candidate<G>(p, self_id, q, s0 + j, j < len), first, k,
-                               lane);
+                    take(q, s0 + j, j < len, first);
                     first = false;
                 }
             }
         }
     }
+}
+
+// The k nearest of the box around cell (ix, iy, iz), in (distance, index)
+// order over the group's lanes: lane r holds rank r (ranks past the last
+// neighbour hold the empty entry; lanes r >= k hold leftovers).
+template <int G, int R>
+__device__ __forceinline__ LaneEntry<G> lanes_knn(unsigned k, unsigned lane, V3 p,
+                                                  unsigned self_id, const Grid& g, const Box& b,
+                                                  unsigned cell_offset,
+                                                  const unsigned* start,
+                                                  const float4* pos_id,
+                                                  unsigned* rows = nullptr) {
+    LaneEntry<G> list{KEY_EMPTY, UINT_MAX};
+    lanes_box<G, R>(lane, g, b, cell_offset, start, pos_id, rows,
+                    [&](float4 q, unsigned slot, bool ok, bool first) {
+                        lanes_take(list, lanes_candidate<G>(p, self_id, q, slot, ok), first, k, lane);
+                    });
     return list;
 }
 

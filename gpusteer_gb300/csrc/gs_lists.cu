@@ -142,32 +142,50 @@ __global__ void __launch_bounds__(kListBlock) k_lists_thread_pairs(const __grid_
                              sh);
 }
 
-// 32 < k <= 64: one thread per query on the exact register list.
+// 32 < k <= 64: a warp per query, two ranks a lane.  One thread per query on a
+// register list of 64 keys was one long chain whatever its box held (k = 40, 13
+// candidates to a box: 3,000 queries 76.5 us, 131,072 231).
+template <int R>
 __device__ __forceinline__ void lists_wide(const KnnPair& pr, const Grid& grid, unsigned r,
-                                           unsigned s) {
-    if (s >= pr.nA) return;
-    const float4 v = pr.a_pos_id[s];
+                                           unsigned thread, unsigned* rows) {
+    const unsigned lane = threadIdx.x & 31u, q = thread / 32u;
+    const bool act = q < pr.nA;  // (whole warps)
+    const float4 v = pr.a_pos_id[act ? q : pr.nA - 1];
     const V3 p = v3(v);
-    const unsigned a = __float_as_uint(v.w);
+    const unsigned a = __float_as_uint(v.w), self_id = pr.self ? a : UINT_MAX;
     unsigned ix, iy, iz;
     cell_coords(grid, p, ix, iy, iz);
-    KList<64> list;
-    list.init(int(pr.k));
-    knn_scan_box<64>(list, p, pr.self ? a : UINT_MAX, grid, cell_box(grid, ix, iy, iz, r), 0u,
-                     pr.b_start, pr.b_pos_id);
-    list.for_each(int(pr.k), [&](int rank, unsigned long long key, unsigned) {
-        put_entry(pr, a, unsigned(rank), key_id(key), key_dist(key));
-    });
+    LaneList<32, 2> list;
+    list.e[0] = list.e[1] = KEY_EMPTY;
+    lanes_box<32, R>(lane, grid, cell_box(grid, ix, iy, iz, r), 0u, pr.b_start, pr.b_pos_id, rows,
+                     [&](float4 c, unsigned, bool ok, bool) {
+                         const unsigned id = __float_as_uint(c.w);
+                         const unsigned long long key = knn_key(distance(p, v3(c)), id);
+                         list.take(ok && id != self_id && key < KEY_EMPTY ? key : KEY_EMPTY, pr.k,
+                                   lane);
+                     });
+    if (!act) return;
+#pragma unroll
+    for (unsigned h = 0; h < 2; ++h) {
+        const unsigned rank = 32u * h + lane;
+        if (rank < pr.k) put_entry(pr, a, rank, key_id(list.e[h]), key_dist(list.e[h]));
+    }
 }
 
+template <int R>
 __global__ void __launch_bounds__(kListBlock) k_lists_wide(KnnPair pr, Grid grid, unsigned r) {
     after_previous();
-    lists_wide(pr, grid, r, blockIdx.x * kListBlock + threadIdx.x);
+    __shared__ unsigned row_sh[R ? 1 : kListBlock / 32 * kLaneRowWords];
+    lists_wide<R>(pr, grid, r, blockIdx.x * kListBlock + threadIdx.x,
+                  row_sh + (R ? 0u : threadIdx.x / 32u * kLaneRowWords));
 }
+template <int R>
 __global__ void __launch_bounds__(kListBlock) k_lists_wide_pairs(const __grid_constant__ KnnPairs P) {
     after_previous();
+    __shared__ unsigned row_sh[R ? 1 : kListBlock / 32 * kLaneRowWords];
     const KnnPair& pr = P.pair[pair_of_block(P)];
-    lists_wide(pr, P.grid, P.r, (blockIdx.x - pr.block_begin) * kListBlock + threadIdx.x);
+    lists_wide<R>(pr, P.grid, P.r, (blockIdx.x - pr.block_begin) * kListBlock + threadIdx.x,
+                  row_sh + (R ? 0u : threadIdx.x / 32u * kLaneRowWords));
 }
 
 // ---- dispatch ----------------------------------------------------------------------------------
@@ -200,8 +218,12 @@ gs_status launch_knn_binned(const Database& A, unsigned nA, const Database& B, b
                             unsigned r, unsigned k, unsigned* idx, float* dist, cudaStream_t st) {
     if (nA == 0) return GS_OK;
     const KnnPair pr{A.pos_id, B.start, B.pos_id, idx, dist, nA, k, 0u, self};
-    if (k > 32) launch_after(k_lists_wide, blocks_for(nA, kListBlock), kListBlock, 0, st, pr, B.grid, r);
-    else if (lists_on_lanes(nA, k, r)) {
+    if (k > 32) {
+        const unsigned nb = blocks_for(nA, kListBlock / 32);
+        if (r != 1) launch_after(k_lists_wide<0>, nb, kListBlock, 0, st, pr, B.grid, r);
+        else if (B.grid.wc[1] == 1) launch_after(k_lists_wide<3>, nb, kListBlock, 0, st, pr, B.grid, r);
+        else launch_after(k_lists_wide<9>, nb, kListBlock, 0, st, pr, B.grid, r);
+    } else if (lists_on_lanes(nA, k, r)) {
         if (k <= 8) lists_lanes_go<8>(pr, B.grid, r, st);
         else if (k <= 16) lists_lanes_go<16>(pr, B.grid, r, st);
         else lists_lanes_go<32>(pr, B.grid, r, st);
@@ -237,15 +259,19 @@ gs_status launch_knn_binned_pairs(KnnPairs& P, cudaStream_t st) {
         queries += P.pair[q].nA;
     }
     const unsigned G = kmax <= 8 ? 8 : kmax <= 16 ? 16 : 32;
-    const bool lanes = kmax <= 32 && lists_on_lanes(queries, kmax, P.r);
+    // (beyond k = 32 a warp per query)
+    const bool lanes = kmax > 32 || lists_on_lanes(queries, kmax, P.r);
     unsigned blocks = 0;
     for (unsigned q = 0; q < P.n_pairs; ++q) {
         P.pair[q].block_begin = blocks;
         blocks += blocks_for(P.pair[q].nA, lanes ? kListBlock / G : kListBlock);
     }
     if (blocks == 0) return GS_OK;
-    if (kmax > 32) launch_after(k_lists_wide_pairs, blocks, kListBlock, 0, st, P);
-    else if (lanes) {
+    if (kmax > 32) {
+        if (P.r != 1) launch_after(k_lists_wide_pairs<0>, blocks, kListBlock, 0, st, P);
+        else if (P.grid.wc[1] == 1) launch_after(k_lists_wide_pairs<3>, blocks, kListBlock, 0, st, P);
+        else launch_after(k_lists_wide_pairs<9>, blocks, kListBlock, 0, st, P);
+    } else if (lanes) {
         if (G == 8) pairs_lanes_go<8>(P, blocks, st);
         else if (G == 16) pairs_lanes_go<16>(P, blocks, st);
         else pairs_lanes_go<32>(P, blocks, st);
