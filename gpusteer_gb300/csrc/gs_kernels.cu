@@ -614,19 +614,19 @@ constexpr unsigned kCallChunk = 8;
 
 // Calls body(s0, b, ok) for each chunk: ok[j]: entry s0 + j holds neighbour b[j]
 // (b[j] is 0 where there is none, a safe index to load).
-template <class Body>
+template <unsigned CHUNK = kCallChunk, class Body>
 __device__ __forceinline__ void for_each_chunk(const unsigned* knn, unsigned i,
                                                unsigned n, unsigned k, unsigned n_other,
                                                Body&& body) {
     bool more = true;
-    for (unsigned s0 = 0; s0 < k && more; s0 += kCallChunk) {
-        unsigned b[kCallChunk];
-        bool ok[kCallChunk];
+    for (unsigned s0 = 0; s0 < k && more; s0 += CHUNK) {
+        unsigned b[CHUNK];
+        bool ok[CHUNK];
 #pragma unroll
-        for (unsigned j = 0; j < kCallChunk; ++j)
+        for (unsigned j = 0; j < CHUNK; ++j)
             b[j] = s0 + j < k ? knn[i + size_t(s0 + j) * n] : UINT_MAX;
 #pragma unroll
-        for (unsigned j = 0; j < kCallChunk; ++j) {
+        for (unsigned j = 0; j < CHUNK; ++j) {
             more = more && b[j] < n_other;
             ok[j] = more;
             b[j] = ok[j] ? b[j] : 0u;
@@ -751,6 +751,7 @@ gs_status launch_follow_path(GroupView g, const PathDev& path, float prediction_
     return GS_OK;
 }
 
+template <unsigned CHUNK>
 __global__ void k_avoid_close(GroupView g, const unsigned* knn,
                               const float* knn_dist, unsigned k, OtherView o,
                               float min_sep, float w, unsigned mask) {
@@ -763,17 +764,17 @@ __global__ void k_avoid_close(GroupView g, const unsigned* knn,
     if (applied & mask) return;
     CloseAcc acc;
     close_init(acc);
-    for_each_chunk(knn, i, g.n, k, o.n, [&](unsigned s0, const unsigned* b, const bool* ok) {
-        float4 bp[kCallChunk];
-        float br[kCallChunk], kd[kCallChunk];
+    for_each_chunk<CHUNK>(knn, i, g.n, k, o.n, [&](unsigned s0, const unsigned* b, const bool* ok) {
+        float4 bp[CHUNK];
+        float br[CHUNK], kd[CHUNK];
 #pragma unroll
-        for (unsigned j = 0; j < kCallChunk; ++j) {
+        for (unsigned j = 0; j < CHUNK; ++j) {
             bp[j] = o.position[b[j]];
             br[j] = o.radius[b[j]];
             kd[j] = ok[j] ? knn_dist[i + size_t(s0 + j) * g.n] : 0.f;
         }
 #pragma unroll
-        for (unsigned j = 0; j < kCallChunk; ++j)
+        for (unsigned j = 0; j < CHUNK; ++j)
             if (ok[j]) close_add(acc, me, min_sep, kd[j], v3(bp[j]), br[j]);
         return !acc.found;
     });
@@ -792,7 +793,8 @@ __device__ __forceinline__ bool avoid_time_may_fall_in(const Self& me, float min
                                   (fabsf(h.x) + fabsf(h.y)) + fabsf(h.z), min_t);
 }
 
-__global__ void __launch_bounds__(kBlock, 2) k_avoid(GroupView g, const unsigned* knn, unsigned k, OtherView o,
+template <unsigned CHUNK, int BLOCKS>
+__global__ void __launch_bounds__(kBlock, BLOCKS) k_avoid(GroupView g, const unsigned* knn, unsigned k, OtherView o,
                         float min_time, float w, unsigned mask) {
     after_previous();
     const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -803,18 +805,18 @@ __global__ void __launch_bounds__(kBlock, 2) k_avoid(GroupView g, const unsigned
     if (applied & (mask | AVOID_CLOSE_NEIGHBORS_BIT)) return;
     AvoidAcc acc;
     avoid_init(acc, min_time);
-    for_each_chunk(knn, i, g.n, k, o.n, [&](unsigned, const unsigned* b, const bool* ok) {
-        float4 bp[kCallChunk], bd[kCallChunk];
-        float bv[kCallChunk], br[kCallChunk];
+    for_each_chunk<CHUNK>(knn, i, g.n, k, o.n, [&](unsigned, const unsigned* b, const bool* ok) {
+        float4 bp[CHUNK], bd[CHUNK];
+        float bv[CHUNK], br[CHUNK];
 #pragma unroll
-        for (unsigned j = 0; j < kCallChunk; ++j) {
+        for (unsigned j = 0; j < CHUNK; ++j) {
             bp[j] = o.position[b[j]];
             bd[j] = o.direction[b[j]];
             bv[j] = o.speed[b[j]];
             br[j] = o.radius[b[j]];
         }
 #pragma unroll
-        for (unsigned j = 0; j < kCallChunk; ++j)
+        for (unsigned j = 0; j < CHUNK; ++j)
             if (ok[j] && avoid_time_may_fall_in(me, min_time, v3(bp[j]), v3(bd[j]), bv[j]))
                 avoid_add<true>(acc, me, b[j], v3(bp[j]), v3(bd[j]), bv[j], br[j]);
         return true;
@@ -835,9 +837,17 @@ gs_status launch_avoid_neighbors(GroupView g, const unsigned* knn, const float* 
         return GS_OK;
     }
     const unsigned bs = call_block(g.n), nb = blocks_for(g.n, bs);
-    if (avoid_close)
-        launch_after(k_avoid_close, nb, bs, 0, st, g, knn, knn_dist, k, o, min_sep, w, mask);
-    launch_after(k_avoid, nb, bs, 0, st, g, knn, k, o, min_time, w, mask);
+    // Groups that pass the blocks that fit at two to an SM have warps enough to
+    // hide the loads' latency, and gain by more blocks instead (us a call, a chunk
+    // of 8 / 1: 200,000 agents, k = 7 32.2 / 24.7, k = 16 44.6 / 41.1, 400,000,
+    // k = 16 79 / 64; with the close pass, 8 / 2: 36.1 / 27.7 and 42.2 / 33.6).
+    const bool many = g.n > 2 * kBlock * sm_count();
+    if (avoid_close) {
+        const auto close = many ? k_avoid_close<2> : k_avoid_close<kCallChunk>;
+        launch_after(close, nb, bs, 0, st, g, knn, knn_dist, k, o, min_sep, w, mask);
+    }
+    const auto avoid = many ? k_avoid<1, 4> : k_avoid<kCallChunk, 2>;
+    launch_after(avoid, nb, bs, 0, st, g, knn, k, o, min_time, w, mask);
     GS_LAUNCHED("steer_avoid_neighbors");
     return GS_OK;
 }

@@ -474,9 +474,14 @@ gs_status launch_group_frame(const MultiSteer& M, cudaStream_t st) {
 // Under ncu, lanes / threads (us; a launch's floor is about 3): one flocking
 // behaviour, k = 7, 30,000 agents 7.5 / 6.5; k = 16, 10,000 6.5 / 11.3, 32,768
 // 10.2 / about 9.5.  The avoidance passes and the walls carry more arithmetic
-// per neighbour: k = 16, 10,000 7.5 / 16.7, 65,536 24 / about 24, k = 7 13.2 / 14.
+// per neighbour, and their line lies by the lanes in all (us a call of the main
+// pass: k = 7, 50,000 agents 9.7 / 11.4, 65,536 11.5 / 11.7; k = 16, 20,000 7.9 /
+// 12.0, 30,000 10.5 / 11.6, 65,536 19.1 / 16.0; k = 32, 10,000 9.2 / 11.5, 14,000
+// 11.6 / 12.2, 20,000 15.5 / 13.0, 65,536 43 / 18; the close pass turns at two
+// thirds of that).
 bool lanes_calls(unsigned n, unsigned k, bool avoid) {
-    return k <= 32 && n <= (avoid ? 65536u : 20000u);
+    const unsigned G = k <= 8 ? 8u : k <= 16 ? 16u : 32u;
+    return k <= 32 && (avoid ? size_t(n) * G <= 450000 : n <= 20000u);
 }
 
 template <int G, int R>
