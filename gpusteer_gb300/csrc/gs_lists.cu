@@ -3,7 +3,7 @@
 // frame in one launch.  Queries are taken in bucketed order (neighbouring
 // threads scan the same cells); results go to idx / dist[a + rank * nA].
 //
-// Two forms.  Few queries: a group of lanes per query (gs_lanes.cuh), whose
+// Two forms up to k = 32, and a warp per query beyond.  Few queries: a group of lanes per query (gs_lanes.cuh), whose
 // serial chain is a few chunks of candidates.  Many: one thread per query on
 // the streaming scan, whose list is in registers and whose candidates take no
 // shared memory, so many warps stay resident; a query that scan cannot vouch
