@@ -3,12 +3,13 @@
 // frame in one launch.  Queries are taken in bucketed order (neighbouring
 // threads scan the same cells); results go to idx / dist[a + rank * nA].
 //
-// Two forms up to k = 32, and a warp per query beyond.  Few queries: a group of lanes per query (gs_lanes.cuh), whose
-// serial chain is a few chunks of candidates.  Many: one thread per query on
-// the streaming scan, whose list is in registers and whose candidates take no
-// shared memory, so many warps stay resident; a query that scan cannot vouch
-// for (ties, more than 256 candidates) is searched again by its whole warp, or,
-// where a warp has many of them, by its own thread.
+// Two forms up to k = 32, and a warp per query beyond.  Few queries: a group of
+// lanes per query (gs_lanes.cuh), whose serial chain is a few chunks of
+// candidates.  Many: one thread per query on the streaming scan, whose list is in
+// registers and whose candidates take no shared memory, so many warps stay
+// resident; a query that scan cannot vouch for (ties, more than 256 candidates)
+// is searched again by its whole warp, or, where a warp has many of them, by its
+// own thread.
 #include <algorithm>
 
 #include "gs_lanes.cuh"
